@@ -127,7 +127,7 @@ struct ddc_ctx {
   DBuf gord;
   // geometry
   DBuf sph, grid, basis, bw, fi, ui, zi, inl, nl, rev, pn_ptr, pn, pn_pair, ls_ptr, ls, ntri_pt;
-  DBuf lsstart, fxa, fda, fvec, xk;
+  DBuf lsstart, fxa, fda, fvec;
   DBuf pn_bits;  // per pair, which grid points lie inside the neighbour (ddinit scratch)
   // batched molecules: partition, per-target N-body ranges, per-molecule DIIS state
   int nmol = 1;
@@ -150,22 +150,22 @@ struct ddc_ctx {
   DBuf rcount;  // arrival counter of the solver kernels' last-block sums (kept zero)
   DBuf phi, psi, sigma, s, q, fx, zeta, ef1, ef2, ef_scratch, uchi;
   DBuf in1, in2, in3, in4, out1;  // staging for host-pointer calls
-  // mixed precision: FP32 grid/basis copies, FP32 grid fields, refinement vectors
-  DBuf gridf, basis_f, bw_f, pot_f, xi_f, rres, dres, eres;
-  // FP32 static geometry of the gather-list triples (mixed path)
-  DBuf tgeo4, tgeo2;
+  // mixed precision: FP32 basis copy, FP32 grid fields, refinement vectors
+  DBuf bw_f, pot_f, xi_f, rres, dres, eres;
+  // static geometry of the gather-list triples: FP32 (mixed path)
+  DBuf tgeo4;
   bool tgeo_on = false;
-  // FP64 static geometry of the gather-list triples (FP64 path)
-  DBuf tgeo4d, tgeo2d;
+  // and FP64 (FP64 path)
+  DBuf tgeo4d;
   bool tgeo64_on = false;
   // second solve set (direct and adjoint solved together) and the fused
   // operator's per-triple lx values
   DBuf y2, xn2, hist_x2, hist_e2, rres2, dres2, eres2, tval;
   // the two dense contractions of every operator application (projection
   // onto the harmonics, expansion to the grid): basisT[Y][G] is the basis
-  // transposed for the FP64 expansion; tc plans the tensor-core kernels of
+  // transposed for the FP64 expansion, bwT[Y][G] with the weights; tc plans the tensor-core kernels of
   // the mixed path, whose FP32 grid field pot_f has rows ldp_f floats apart
-  DBuf basisT;
+  DBuf basisT, bwT;
   TcPlan tc;
   int ldp_f = 0;
   // learned initial guess: the attached model, its feature rows, and flags
@@ -203,7 +203,6 @@ struct ddc_ctx {
     g.ntri = ntri;
     g.sph = sph.as<double4>();
     g.grid = grid.as<double4>();
-    g.gridf = gridf.as<float4>();
     g.basis = basis.as<double>();
     g.bw = bw.as<double>();
     g.fi = fi.as<double>();
@@ -217,11 +216,9 @@ struct ddc_ctx {
     g.pn_pair = pn_pair.as<uint8_t>();
     g.maxnb = maxnb;
     g.tgeo4 = tgeo_on ? tgeo4.as<float4>() : nullptr;
-    g.tgeo2 = tgeo_on ? tgeo2.as<float2>() : nullptr;
     g.tgeo4d = tgeo64_on ? tgeo4d.as<double4>() : nullptr;
-    g.tgeo2d = tgeo64_on ? tgeo2d.as<double2>() : nullptr;
     g.ls_ptr = ls_ptr.as<int>();
-    g.ls = ls.as<int2>();
+    g.ls = ls.as<int>();
     g.lsstart = lsstart.as<int>();
     g.ntri_pt = ntri_pt.as<uint8_t>();
     g.cavoff = cavoff.as<int>();
@@ -394,11 +391,10 @@ void build_tables_for(YlmTables& tb, int lmax, double eta, int ngrid) {
       gm1 = gam;
     }
   }
-  for (int e = 0; e < DDC_NLM_CAP; e++) {
-    tb.Kf[e] = (float)tb.K[e];
-    tb.Af[e] = (float)tb.A[e];
-    tb.Bf[e] = (float)tb.B[e];
-    tb.Bnf[e] = (float)tb.Bn[e];
+  double pre = 1.0;  // (-1)^m (2m-1)!!
+  for (int m = 0; m <= lmax; m++) {
+    if (m > 0) pre *= -(2.0 * m - 1.0);
+    for (int l = m; l <= lmax; l++) tb.Kp[l * (l + 1) / 2 + m] = pre * tb.Kg[l * (l + 1) / 2 + m];
   }
   tb.eta = eta;
   tb.lmax = lmax;
@@ -627,11 +623,11 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
                      ctx->cnt.as<int>()));
   CK(scan_exclusive(L, ctx->cnt.as<int>(), ctx->ls_ptr.as<int>(), N, ctx->scan_tmp.p,
                     ctx->scan_tmp.bytes));
-  CK(ctx->ls.ensure(sizeof(int2) * std::max(ntri, 1)));
+  CK(ctx->ls.ensure(sizeof(int) * std::max(ntri, 1)));
   CK(ctx->lsstart.ensure(sizeof(int) * std::max(npair, 1)));
   CK(launch_ls_fill(L, N, ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->rev.as<int>(),
-                    ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>(), ctx->ls_ptr.as<int>(),
-                    ctx->ls.as<int2>(), ctx->lsstart.as<int>()));
+                    ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>(), ctx->ls_ptr.as<int>(), G,
+                    ctx->ls.as<int>(), ctx->lsstart.as<int>()));
   // centres for the electrostatics
   CK(ctx->csph.ensure(sizeof(double) * 3 * std::max(N, 1)));
   CK(ctx->cx.ensure(sizeof(double) * std::max(N, 1)));
@@ -643,8 +639,6 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   const size_t nv = (size_t)N * NY;
   const int nd = std::max(ctx->prm.ndiis, 1);
   CK(ctx->pot.ensure(sizeof(double) * std::max(NP, 1LL)));
-  CK(ctx->xk.ensure(sizeof(double) * 2 * std::max(N, 1) *
-                    ((ctx->prm.lmax + 1) * (ctx->prm.lmax + 2) / 2)));
   CK(ctx->xig.ensure(sizeof(double) * std::max(NP, 1LL)));
   CK(ctx->uchi.ensure(sizeof(double) * std::max(NP, 1LL)));
   for (DBuf* b : {&ctx->rhs, &ctx->x, &ctx->y, &ctx->xn, &ctx->psi, &ctx->sigma, &ctx->s})
@@ -657,9 +651,12 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     CK(ctx->rcount.ensure(sizeof(unsigned)));
     CK(cudaMemsetAsync(ctx->rcount.p, 0, sizeof(unsigned), ctx->st));
   }
-  // the basis transposed to [Y][G] for the FP64 expansion xi = basis^T s
-  CK(ctx->basisT.ensure(sizeof(double) * G * NY));
-  CK(launch_transpose(L, G, NY, ctx->basis.as<double>(), ctx->basisT.as<double>()));
+  // the basis transposed to [Y][G] for the FP64 expansions xi = basis^T s
+  // (forces, zeta) and w xi = bw^T s (the operators)
+  for (auto t : {std::make_pair(&ctx->basis, &ctx->basisT), std::make_pair(&ctx->bw, &ctx->bwT)}) {
+    CK(t.second->ensure(sizeof(double) * G * NY));
+    CK(launch_transpose(L, G, NY, t.first->as<double>(), t.second->as<double>()));
+  }
   if (!ctx->hred) CK(cudaMallocHost(&ctx->hred, sizeof(double) * 2 * (kMaxHist + 1)));
   if (ctx->prm.igrad && !ctx->st2) {
     CK(cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking));
@@ -667,13 +664,8 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
   }
   if (ctx->prm.precision == DDC_PREC_MIXED) {
-    std::vector<float> gf(4 * (size_t)G);
-    for (size_t k = 0; k < gf.size(); k++) gf[k] = (float)ctx->h_grid[k];
-    CK(ctx->gridf.ensure(sizeof(float) * 4 * G));
-    CK(cudaMemcpyAsync(ctx->gridf.p, gf.data(), sizeof(float) * 4 * G, cudaMemcpyHostToDevice,
-                       ctx->st));
     // the two contractions run on the tensor cores (split TF32) up to 128
-    // harmonics (lmax 10), else as FP32 SIMT GEMMs on FP32 copies of the basis
+    // harmonics (lmax 10), else as FP32 SIMT GEMMs on an FP32 copy of bw
     // DDC_TC_OFF=1 in the environment selects the SIMT contractions (a
     // diagnostic switch: the tests compare the two paths' accuracy)
     const char* tc_off = std::getenv("DDC_TC_OFF");
@@ -682,35 +674,30 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     CK(ctx->pot_f.ensure(sizeof(float) * std::max<long long>((long long)N * ctx->ldp_f, 1LL)));
     CK(ctx->xi_f.ensure(sizeof(float) * std::max(NP, 1LL)));
     if (tc) {
-      CK(tc_plan(L, ctx->tc, ctx->basis.as<double>(), ctx->bw.as<double>(), N, NY, G,
+      CK(tc_plan(L, ctx->tc, ctx->bw.as<double>(), N, NY, G,
                  ctx->pot_f.as<float>(), ctx->ldp_f));
       // tile widths by measurement (x and y are free work vectors here)
       CK(tc_autotune(L, ctx->tc, ctx->x.as<double>(), ctx->y.as<double>(),
                      ctx->xi_f.as<float>()));
     } else {
       ctx->tc.on = false;
-      CK(ctx->basis_f.ensure(sizeof(float) * G * NY));
       CK(ctx->bw_f.ensure(sizeof(float) * G * NY));
-      CK(launch_to_float(L, (long long)G * NY, ctx->basis.as<double>(), ctx->basis_f.as<float>()));
       CK(launch_to_float(L, (long long)G * NY, ctx->bw.as<double>(), ctx->bw_f.as<float>()));
     }
     for (DBuf* b : {&ctx->rres, &ctx->dres, &ctx->eres})
       CK(b->ensure(sizeof(double) * std::max(nv, (size_t)1)));
     // the FP32 fused pass reads each triple's static geometry instead of
-    // recomputing it every iteration (24 bytes per triple)
+    // recomputing it every iteration (16 bytes per triple)
     ctx->tgeo_on = false;
     CK(ctx->tgeo4.ensure(sizeof(float4) * std::max<long long>(ctx->ntri, 1)));
-    CK(ctx->tgeo2.ensure(sizeof(float2) * std::max<long long>(ctx->ntri, 1)));
-    CK(launch_lxs_geo(L, ctx->tb, ctx->geo(), ctx->tgeo4.as<float4>(), ctx->tgeo2.as<float2>()));
+    CK(launch_lxs_geo(L, ctx->tb, ctx->geo(), ctx->tgeo4.as<float4>()));
     ctx->tgeo_on = true;
   }
   if (ctx->prm.precision != DDC_PREC_MIXED && ctx->prm.pair_solves) {
     // the FP64 fused pass of the paired solves reads each triple's static
-    // geometry (48 bytes per triple) instead of recomputing it
+    // geometry (32 bytes per triple) instead of recomputing it
     CK(ctx->tgeo4d.ensure(sizeof(double4) * std::max<long long>(ctx->ntri, 1)));
-    CK(ctx->tgeo2d.ensure(sizeof(double2) * std::max<long long>(ctx->ntri, 1)));
-    CK(launch_lxs_geo_f64(L, ctx->tb, ctx->geo(), ctx->tgeo4d.as<double4>(),
-                          ctx->tgeo2d.as<double2>()));
+    CK(launch_lxs_geo_f64(L, ctx->tb, ctx->geo(), ctx->tgeo4d.as<double4>()));
     ctx->tgeo64_on = true;
   }
   if (ctx->prm.igrad && ctx->prm.pair_solves) {
@@ -793,18 +780,19 @@ int gemm_proj_f32(ddc_ctx* ctx, float alpha, const float* pot, double* y) {
                             ctx->bw_f.as<float>(), pot, ctx->ldp_f, y));
   return DDC_OK;
 }
-// xi(n,i) = sum_lm basis(lm,n) s(lm,i)   (matvec.f90:189-204)
-int gemm_xi(ddc_ctx* ctx, const double* s, double* xig) {
-  CK(launch_dgemm_nn(ctx->L(), ctx->ngrid, ctx->nsph, ctx->nylm, 1.0, ctx->basisT.as<double>(),
-                     ctx->ngrid, s, ctx->nylm, xig, ctx->ngrid, ctx->sweep));
+// xi(n,i) = sum_lm basis(lm,n) s(lm,i)   (matvec.f90:189-204); weighted: w_n xi
+int gemm_xi(ddc_ctx* ctx, const double* s, double* xig, bool weighted) {
+  CK(launch_dgemm_nn(ctx->L(), ctx->ngrid, ctx->nsph, ctx->nylm, 1.0,
+                     (weighted ? ctx->bwT : ctx->basisT).as<double>(), ctx->ngrid, s, ctx->nylm,
+                     xig, ctx->ngrid, ctx->sweep));
   return DDC_OK;
 }
-// FP32 xi of the FP64 vector s
+// FP32 w_n xi of the FP64 vector s
 int gemm_xi_f32(ddc_ctx* ctx, const double* s, float* xig) {
   if (ctx->tc.on)
     CK(launch_xi_tc(ctx->L(), ctx->tc, s, xig, ctx->sweep));
   else
-    CK(launch_xi_f32_simt(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, ctx->basis_f.as<float>(),
+    CK(launch_xi_f32_simt(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, ctx->bw_f.as<float>(),
                           s, xig));
   return DDC_OK;
 }
@@ -818,20 +806,19 @@ int op_lx(ddc_ctx* ctx, const double* x, double* y) {
     // the lx part of the fused pass (one value per triple), then the sums
     // per grid point
     StageScope sc(ctx, ST_LX_POT);
-    CK(launch_lx_vals(ctx->L(), ctx->tb, g, x, ctx->xk.p, ctx->tval.as<double>(), false));
+    CK(launch_lx_vals(ctx->L(), ctx->tb, g, x, ctx->tval.as<double>()));
     CK(launch_lx_gather(ctx->L(), g, ctx->tval.as<double>(), ctx->pot.as<double>()));
   }
   StageScope sc(ctx, ST_PROJ);
   // y = -Bw pot   (intrhs then negate, matvec.f90:131-135)
   return gemm_proj(ctx, -1.0, ctx->pot.as<double>(), y);
 }
-int op_xi(ddc_ctx* ctx, const double* x, double* xig) {
-  // xi(n,i) = sum_lm basis(lm,n) x(lm,i)   (matvec.f90:189-204)
+int op_xi(ddc_ctx* ctx, const double* x, double* xig, bool weighted = false) {
   StageScope sc(ctx, ST_XI);
-  return gemm_xi(ctx, x, xig);
+  return gemm_xi(ctx, x, xig, weighted);
 }
 int op_lstarx(ddc_ctx* ctx, const double* x, double* y) {
-  CKI(op_xi(ctx, x, ctx->xig.as<double>()));
+  CKI(op_xi(ctx, x, ctx->xig.as<double>(), true));
   StageScope sc(ctx, ST_LSTARX);
   CK(launch_lstarx_acc(ctx->L(), ctx->tb, ctx->geo(), ctx->xig.as<double>(), y));
   return DDC_OK;
@@ -842,7 +829,7 @@ int op_lx_f32(ddc_ctx* ctx, const double* x, double* y) {
   {
     StageScope sc(ctx, ST_LX_POT);
     DevGeo g = ctx->geo();
-    CK(launch_lx_vals_f32(ctx->L(), ctx->tb, g, x, ctx->xk.p, ctx->tval.as<float>()));
+    CK(launch_lx_vals_f32(ctx->L(), ctx->tb, g, x, ctx->tval.as<float>()));
     CK(launch_lx_gather_f32(ctx->L(), g, ctx->tval.as<float>(), ctx->pot_f.as<float>(),
                             ctx->ldp_f));
   }
@@ -862,11 +849,10 @@ int op_lstarx_f32(ddc_ctx* ctx, const double* x, double* y) {
 // y = L x and z = L* s (off-diagonal parts) from one pass over the triples
 int op_pair(ddc_ctx* ctx, const double* x, double* y, const double* s, double* z) {
   DevGeo g = ctx->geo();
-  CKI(op_xi(ctx, s, ctx->xig.as<double>()));
+  CKI(op_xi(ctx, s, ctx->xig.as<double>(), true));
   {
     StageScope sc(ctx, ST_LXS);
-    CK(launch_lxs(ctx->L(), ctx->tb, g, x, ctx->xig.as<double>(), ctx->xk.p,
-                  ctx->tval.as<double>(), z));
+    CK(launch_lxs(ctx->L(), ctx->tb, g, x, ctx->xig.as<double>(), ctx->tval.as<double>(), z));
   }
   {
     StageScope sc(ctx, ST_GATHER);
@@ -883,8 +869,7 @@ int op_pair_f32(ddc_ctx* ctx, const double* x, double* y, const double* s, doubl
   }
   {
     StageScope sc(ctx, ST_LXS);
-    CK(launch_lxs_f32(ctx->L(), ctx->tb, g, x, ctx->xi_f.as<float>(), ctx->xk.p,
-                      ctx->tval.as<float>(), z));
+    CK(launch_lxs_f32(ctx->L(), ctx->tb, g, x, ctx->xi_f.as<float>(), ctx->tval.as<float>(), z));
   }
   {
     StageScope sc(ctx, ST_GATHER);
@@ -1481,11 +1466,11 @@ int forces_dev(ddc_ctx* ctx, const double* phi, const double* sigma, const doubl
   if (!xi_ready) CKI(op_xi(ctx, s, ctx->xig.as<double>()));
   {
     // u_chi(a, n) = sum over the neighbours b of chi(t) * intmlp(X_b): the
-    // chi-weighted lx sum, per triple then per grid point
+    // lx sum (weight chi / f) per triple, then per grid point times f
     StageScope sc(ctx, ST_UCHI);
     DevGeo g = ctx->geo();
-    CK(launch_lx_vals(ctx->L(), ctx->tb, g, sigma, ctx->xk.p, ctx->tval.as<double>(), true));
-    CK(launch_lx_gather(ctx->L(), g, ctx->tval.as<double>(), ctx->uchi.as<double>()));
+    CK(launch_lx_vals(ctx->L(), ctx->tb, g, sigma, ctx->tval.as<double>()));
+    CK(launch_lx_gather(ctx->L(), g, ctx->tval.as<double>(), ctx->uchi.as<double>(), true));
   }
   const double fep = 0.5 * (ctx->prm.eps - 1.0) / ctx->prm.eps;
   CK(ctx->fxa.ensure(sizeof(double) * 3 * std::max(ctx->nsph, 1)));

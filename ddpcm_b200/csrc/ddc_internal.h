@@ -11,7 +11,7 @@
 //   zi[N][G][3]          grad f (forces only)
 //   pn_ptr[P+1], pn[T]   per pair (i,j): grid points n of sphere i with
 //                        t_n^ij < 1 (point inside sphere j), ascending n
-//   ls_ptr[N+1], ls[T]   per sphere i: (j, n) for j in N_i (CSR order) and the
+//   ls_ptr[N+1], ls[T]   per sphere i: j * G + n for j in N_i (CSR order) and the
 //                        points n of sphere j inside sphere i (adjoint gather)
 //   ntri[N][G]           number of neighbours containing point (i,n)
 //   cavoff[N+1], cavidx[N][G], cavpt[ncav], ccav[ncav][3]
@@ -84,14 +84,21 @@ struct YlmTables {
   double K[DDC_NLM_CAP];          // facs / facl
   double A[DDC_NLM_CAP];          // (2l-1)/(l-m): Legendre recurrence
   double B[DDC_NLM_CAP];          // (l+m-1)/(l-m)
-  float Kf[DDC_NLM_CAP], Af[DDC_NLM_CAP], Bf[DDC_NLM_CAP];  // FP32 copies (mixed path)
   // normalised recurrence of the fused L / L* kernel: Pt_l^m = gam_lm Q_l^m with
   // Q_m = Pt_m^m, Q_{m+1} = c t Q_m, Q_l = c t Q_{l-1} - beta_lm t^2 Q_{l-2};
   // Kg = K * gam folds the scale into the contractions
   double Bn[DDC_NLM_CAP], Kg[DDC_NLM_CAP];
-  float Bnf[DDC_NLM_CAP];
+  // Kg times the signed (2m-1)!! of the prefix P_m^m: the scale of the monic
+  // recurrence in Cartesian powers (ddc_lxs.cu)
+  double Kp[DDC_NLM_CAP];
   double eta;
   int lmax, nylm, ngrid;
+};
+
+// What the operator kernels (ddc_lxs.cu) need of the tables.
+struct LxsTab {
+  double kp[DDC_NLM_CAP];
+  double eta, ie5;  // eta and eta^-5
 };
 
 // Device geometry handed to every kernel.
@@ -123,16 +130,13 @@ __device__ __forceinline__ bool sweep_skip_tile(const SweepMask& m, int i0, int 
 struct DevGeo {
   int nsph, ngrid, nylm, ncav, npair;
   int maxnb;  // largest neighbour count of a sphere
-  // FP32 geometry of each gather-list triple (mixed path; null if absent):
-  // (t cos theta, t^2, t sin theta, W) and (cos phi, sin phi)
+  // geometry (u, v, z, W) of each gather-list triple (ddc_lxs.cu): FP32 in
+  // the mixed path, FP64 in the FP64 path; null if absent
   const float4* tgeo4;
-  const float2* tgeo2;
-  const double4* tgeo4d;  // the same in FP64 (FP64 path)
-  const double2* tgeo2d;
+  const double4* tgeo4d;
   long long ntri;
   const double4* sph;
   const double4* grid;
-  const float4* gridf;  // FP32 copy of grid (mixed path)
   const double* basis;
   const double* bw;
   const double* fi;
@@ -145,7 +149,7 @@ struct DevGeo {
   const uint16_t* pn;
   const uint8_t* pn_pair;  // local index (within the sphere's CSR range) of each triple's pair
   const int* ls_ptr;
-  const int2* ls;
+  const int* ls;  // gather list: a * ngrid + n of each triple
   const int* lsstart;  // per CSR entry (j,i): start of that pair's block in i's gather list
   const uint8_t* ntri_pt;
   const int* cavoff;
@@ -239,8 +243,8 @@ cudaError_t launch_pair_fill(Launch L, int nsph, int npair, int ngrid, const dou
 cudaError_t launch_ls_count(Launch L, int nsph, const int* inl, const int* rev, const int* pn_ptr,
                             int* cnt);
 cudaError_t launch_ls_fill(Launch L, int nsph, const int* inl, const int* nl, const int* rev,
-                           const int* pn_ptr, const uint16_t* pn, const int* ls_ptr, int2* ls,
-                           int* lsstart);
+                           const int* pn_ptr, const uint16_t* pn, const int* ls_ptr, int ngrid,
+                           int* ls, int* lsstart);
 // exclusive scan of n ints (out[n] = total); temp is device scratch of temp_bytes
 cudaError_t scan_exclusive(Launch L, const int* in, int* out, int n, void* temp,
                            size_t temp_bytes);
@@ -248,34 +252,34 @@ size_t scan_temp_bytes(int n);
 // *out = sum of cnt[0..n) in 64 bits (out: device memory, overwritten)
 cudaError_t launch_sum_counts(Launch L, const int* cnt, int n, unsigned long long* out);
 
-// operators
-// xk: scratch of N*(lmax+1)(lmax+2)/2 double2 (K-scaled X in pair layout)
+// operators over the triples (ddc_lxs.cu): lx values, one per triple in
+// gather-list order, for k_lx_gather, and / or the L* rows.  xi holds the
+// weighted field w_n xi_a(n).  The FP32 variants are the mixed path's: xi and
+// val in FP32, X and y in FP64, geometry from g.tgeo4; the FP64 ones take
+// g.tgeo4d if there, else evaluate the geometry in the pass.
+cudaError_t launch_lxs(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
+                       const double* xi, double* val, double* y);
+cudaError_t launch_lx_vals(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
+                           double* val);
 cudaError_t launch_lstarx_acc(Launch L, const YlmTables& tb, const DevGeo& g, const double* xi,
                               double* y);
-// FP32 operator variants (mixed precision): pot/xi in FP32, y in FP64
-// fused L / L*: val (one lx value per triple, gather-list order) and y = L* rows
-cudaError_t launch_lxs(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                       const double* xi, void* xk, double* val, double* y);
-// the lx part of the fused pass alone: one value per triple (gather-list
-// order) for k_lx_gather; chi_only: weight chi(t) instead of chi(t)/f_a(n)
-// (the u_chi sum of the forces)
-cudaError_t launch_lx_vals(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                           void* xk, double* val, bool chi_only);
-cudaError_t launch_lx_vals_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                               void* xk, float* val);
-cudaError_t launch_lxs_geo(Launch L, const YlmTables& tb, const DevGeo& g, float4* tg4,
-                           float2* tg2);
-cudaError_t launch_lxs_geo_f64(Launch L, const YlmTables& tb, const DevGeo& g, double4* tg4,
-                               double2* tg2);
 cudaError_t launch_lxs_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                           const float* xi, void* xk, float* val, double* y);
-cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, double* pot);
+                           const float* xi, float* val, double* y);
+cudaError_t launch_lx_vals_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
+                               float* val);
+cudaError_t launch_lstarx_acc_f32(Launch L, const YlmTables& tb, const DevGeo& g,
+                                  const float* xi, double* y);
+// the triples' geometry (g.tgeo4, g.tgeo4d), once per molecule
+cudaError_t launch_lxs_geo(Launch L, const YlmTables& tb, const DevGeo& g, float4* tg);
+cudaError_t launch_lxs_geo_f64(Launch L, const YlmTables& tb, const DevGeo& g, double4* tg);
+// pot_a(n) = sum of the lx values of the triples of (a, n); chi: times
+// max(f_a(n), 1), the u_chi sum of the forces
+cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, double* pot,
+                             bool chi = false);
 // FP32 field rows are ldp >= ngrid floats apart (the tensor-core projection
 // reads them with TMA, which wants 16-byte row strides)
 cudaError_t launch_lx_gather_f32(Launch L, const DevGeo& g, const float* val, float* pot,
                                  int ldp);
-cudaError_t launch_lstarx_acc_f32(Launch L, const YlmTables& tb, const DevGeo& g,
-                                  const float* xi, double* y);
 cudaError_t launch_to_float(Launch L, long long n, const double* x, float* y);
 // r = rhs - y - x/facl ; d = facl*r (Jacobi increment at x), partial H-norm of d
 cudaError_t launch_residual(Launch L, const YlmTables& tb, long long n, const double* rhs,
@@ -293,7 +297,7 @@ cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const d
 // FP32 SIMT projection / expansion (mixed path, more than 128 harmonics)
 cudaError_t launch_proj_f32_simt(Launch L, int nylm, int nsph, int ngrid, float alpha,
                                  const float* bw_f, const float* pot, int ldp, double* y);
-cudaError_t launch_xi_f32_simt(Launch L, int nylm, int nsph, int ngrid, const float* basis_f,
+cudaError_t launch_xi_f32_simt(Launch L, int nylm, int nsph, int ngrid, const float* bw_f,
                                const double* s, float* xi);
 cudaError_t launch_wghpot(Launch L, const DevGeo& g, const double* phi, double* gbuf);
 cudaError_t launch_ldm1x(Launch L, const YlmTables& tb, long long n, const double* x, double* y);
@@ -302,11 +306,11 @@ cudaError_t launch_guess(Launch L, const YlmTables& tb, long long n, const doubl
                          double* x, int mode);
 
 // tensor-core contractions of the mixed-precision operators (ddc_tc.cu):
-// projection y = alpha * bw pot (FP64 out) and expansion xi = basis^T s (FP32
+// projection y = alpha * bw pot (FP64 out) and expansion w xi = bw^T s (FP32
 // out), split-TF32 on tcgen05 for nylm <= 128
 bool tc_supported(int nylm);
-cudaError_t tc_plan(Launch L, TcPlan& p, const double* basis, const double* bw, int nsph,
-                    int nylm, int ngrid, float* pot_f, int ldp);
+cudaError_t tc_plan(Launch L, TcPlan& p, const double* bw, int nsph, int nylm,
+                    int ngrid, float* pot_f, int ldp);
 // pick the tile widths of both kernels by timing the candidates (y, xi are
 // scratch; s is zeroed)
 cudaError_t tc_autotune(Launch L, TcPlan& p, const double* s, double* y, float* xi);

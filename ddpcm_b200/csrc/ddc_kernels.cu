@@ -23,17 +23,6 @@ namespace ddc {
 
 __host__ __device__ constexpr int lmi(int l, int m) { return l * (l + 1) / 2 + m; }
 
-// recurrence constants in the arithmetic type of the kernel
-template <class Rl> __device__ __forceinline__ Rl cA(const YlmTables& tb, int e);
-template <> __device__ __forceinline__ double cA<double>(const YlmTables& tb, int e) { return tb.A[e]; }
-template <> __device__ __forceinline__ float cA<float>(const YlmTables& tb, int e) { return tb.Af[e]; }
-template <class Rl> __device__ __forceinline__ Rl cB(const YlmTables& tb, int e);
-template <> __device__ __forceinline__ double cB<double>(const YlmTables& tb, int e) { return tb.B[e]; }
-template <> __device__ __forceinline__ float cB<float>(const YlmTables& tb, int e) { return tb.Bf[e]; }
-template <class Rl> __device__ __forceinline__ Rl cK(const YlmTables& tb, int e);
-template <> __device__ __forceinline__ double cK<double>(const YlmTables& tb, int e) { return tb.K[e]; }
-template <> __device__ __forceinline__ float cK<float>(const YlmTables& tb, int e) { return tb.Kf[e]; }
-
 
 // ---------------------------------------------------------------------------
 // exact geometry helpers
@@ -85,15 +74,6 @@ __device__ __forceinline__ double dfsw_exact(double x, double eta) {
   double xe = DADD(xm, eta);
   return DDIV(DMUL(DMUL(DMUL(DMUL(30.0, DSUB(1.0, x)), xm), xe), xe), eta5(eta));
 }
-// value-only versions (contracted); same branches
-__device__ __forceinline__ double fsw_fast(double x, double eta, double flow, double a, double b,
-                                           double ie5) {
-  if (x >= 1.0) return 0.0;
-  if (x <= flow) return 1.0;
-  double xm = x - 1.0;
-  return (xm * xm * (1.0 - x)) * ((6.0 * x + a) * x + b) * ie5;
-}
-
 // ---------------------------------------------------------------------------
 // reference spherical harmonics (init only): ylmbas ddcosmo.f90:830-895
 // ---------------------------------------------------------------------------
@@ -525,22 +505,22 @@ cudaError_t launch_ls_count(Launch L, int nsph, const int* inl, const int* rev, 
 __global__ void k_ls_fill(int nsph, const int* __restrict__ inl, const int* __restrict__ nl,
                           const int* __restrict__ rev, const int* __restrict__ pn_ptr,
                           const uint16_t* __restrict__ pn, const int* __restrict__ ls_ptr,
-                          int2* ls, int* lsstart) {
+                          int ngrid, int* ls, int* lsstart) {
   int i = blockIdx.x;
   int off = ls_ptr[i];
   for (int k = inl[i]; k < inl[i + 1]; k++) {
     int kk = rev[k], j = nl[k];
     int a = pn_ptr[kk], b = pn_ptr[kk + 1];
     if (threadIdx.x == 0) lsstart[kk] = off;  // where pair (j, i) sits in i's gather list
-    for (int q = a + threadIdx.x; q < b; q += blockDim.x) ls[off + (q - a)] = make_int2(j, pn[q]);
+    for (int q = a + threadIdx.x; q < b; q += blockDim.x) ls[off + (q - a)] = j * ngrid + pn[q];
     off += b - a;
   }
 }
 cudaError_t launch_ls_fill(Launch L, int nsph, const int* inl, const int* nl, const int* rev,
-                           const int* pn_ptr, const uint16_t* pn, const int* ls_ptr, int2* ls,
-                           int* lsstart) {
+                           const int* pn_ptr, const uint16_t* pn, const int* ls_ptr, int ngrid,
+                           int* ls, int* lsstart) {
   if (nsph == 0) return cudaSuccess;
-  k_ls_fill<<<nsph, 128, 0, L.st>>>(nsph, inl, nl, rev, pn_ptr, pn, ls_ptr, ls, lsstart);
+  k_ls_fill<<<nsph, 128, 0, L.st>>>(nsph, inl, nl, rev, pn_ptr, pn, ls_ptr, ngrid, ls, lsstart);
   ++*L.launches;
   return cudaGetLastError();
 }
@@ -572,110 +552,6 @@ cudaError_t scan_exclusive(Launch L, const int* in, int* out, int n, void* temp,
   return cub::DeviceScan::ExclusiveSum(temp, temp_bytes, in, out, n + 1, L.st);
 }
 
-// ---------------------------------------------------------------------------
-// Spherical-harmonic contraction for the matvecs.  m-outer / l-inner
-// Legendre recurrence (polleg, ddcosmo.f90:1056-1094) with t^l folded in:
-//   Pt_l^m = t^l P_l^m,  Pt_m^m = t^m P_m^m,
-//   Pt_{m+1}^m = (2m+1) c t Pt_m^m,  Pt_l^m = A c t Pt_{l-1}^m - B t^2 Pt_{l-2}^m
-// cos(m phi), sin(m phi) by the Chebyshev recurrence (trgev :1103-1125).
-// ---------------------------------------------------------------------------
-struct Angles {
-  double c, s, cp, sp;  // cos/sin theta, cos/sin phi
-};
-__device__ __forceinline__ Angles angles_of(double sx, double sy, double sz) {
-  Angles a;
-  a.c = sz;
-  a.s = sqrt(fmax(0.0, 1.0 - sz * sz));
-  if (a.s != 0.0) {
-    double r = 1.0 / a.s;
-    a.cp = sx * r;
-    a.sp = sy * r;
-  } else {  // pole: only m = 0 survives (P_l^m = 0 for m > 0)
-    a.cp = 1.0;
-    a.sp = 0.0;
-  }
-  return a;
-}
-
-// X of one sphere staged as pairs (X_{l,m}, X_{l,-m}) * K_lm, index lmi(l,m)
-template <int LMAX>
-__device__ __forceinline__ double ylm_dot(const YlmTables& tb, const Angles& a, double t,
-                                          const double2* __restrict__ xs) {
-  const double ct = a.c * t, st = a.s * t, t2 = t * t;
-  double acc = 0.0;
-  double pmm = 1.0;                     // Pt_m^m
-  double cm = 1.0, sm = 0.0, cmm1 = 1.0, smm1 = 0.0;
-#pragma unroll
-  for (int m = 0; m <= LMAX; ++m) {
-    if (m == 1) {
-      cm = a.cp;
-      sm = a.sp;
-    } else if (m >= 2) {
-      double cn = 2.0 * a.cp * cm - cmm1, sn = 2.0 * a.cp * sm - smm1;
-      cmm1 = cm; smm1 = sm; cm = cn; sm = sn;
-    }
-    double p0 = pmm, p1 = 0.0;
-#pragma unroll
-    for (int l = m; l <= LMAX; ++l) {
-      double P;
-      if (l == m) {
-        P = p0;
-      } else if (l == m + 1) {
-        p1 = (2.0 * m + 1.0) * ct * p0;
-        P = p1;
-      } else {
-        P = (tb.A[lmi(l, m)] * ct) * p1 - (tb.B[lmi(l, m)] * t2) * p0;
-        p0 = p1;
-        p1 = P;
-      }
-      double2 xv = xs[lmi(l, m)];
-      double q = (m == 0) ? xv.x : fma(cm, xv.x, sm * xv.y);
-      acc = fma(P, q, acc);
-    }
-    pmm = -pmm * (2.0 * m + 1.0) * st;
-  }
-  return acc;
-}
-
-// ---------------------------------------------------------------------------
-// lx, part 1 (calcv ddcosmo.f90:1671-1746 with intmlp :1140-1178), second
-// form, both precisions.  Block per sphere i:
-//   * K*X_j of every neighbour j (as (X_{l,m}, X_{l,-m}) pairs) and the
-//     centre differences c_i - c_j are staged in shared memory once;
-//   * the sphere's triples (pair-major list) are spread over all threads, a
-//     per-triple local pair index selects the staged neighbour;
-//   * contributions to the same grid point inside one warp instruction are
-//     combined in lane order (match_any) before the warp-private row update,
-//     so the sum order is fixed and the result bit-reproducible;
-//   * one accumulator per m column keeps independent FMA chains in flight.
-// ---------------------------------------------------------------------------
-template <class Rl> struct RT;
-template <> struct RT<double> {
-  typedef double2 V2;
-};
-template <> struct RT<float> {
-  typedef float2 V2;
-};
-template <class Rl> __device__ __forceinline__ typename RT<Rl>::V2 mk2(Rl a, Rl b);
-template <> __device__ __forceinline__ double2 mk2<double>(double a, double b) {
-  return make_double2(a, b);
-}
-template <> __device__ __forceinline__ float2 mk2<float>(float a, float b) {
-  return make_float2(a, b);
-}
-template <class Rl> struct GP {
-  Rl x, y, z, w;
-};
-__device__ __forceinline__ GP<double> grid_pt(const DevGeo& g, int n, double*) {
-  double4 v = g.grid[n];
-  return GP<double>{v.x, v.y, v.z, v.w};
-}
-__device__ __forceinline__ GP<float> grid_pt(const DevGeo& g, int n, float*) {
-  float4 v = g.gridf[n];
-  return GP<float>{v.x, v.y, v.z, v.w};
-}
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
-__device__ __forceinline__ float rsqrt_t(float x) { return rsqrtf(x); }
 // 1/sqrt(x) for a positive normal x (a squared distance between distinct
 // points) in the N-body sums: the hardware estimate rsqrt.approx.ftz.f64,
 // then one third-order Householder step y (1 + h/2 + 3h^2/8), h = 1 - x y^2
@@ -688,80 +564,12 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
   const double h = fma(-x, y * y, 1.0);
   return fma(y * h, fma(h, 0.375, 0.5), y);
 }
-__device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
-__device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
-
-// K-scaled copy of X in (X_{l,m}, X_{l,-m}) pair layout, [N][NLM]
-template <class Rl, bool GAM = false>
-__global__ void k_xk(const YlmTables tb, int nsph, const double* __restrict__ X,
-                     typename RT<Rl>::V2* XK) {
-  const int nlm = (tb.lmax + 1) * (tb.lmax + 2) / 2;
-  // 32-bit indices (nsph * nlm < 2^31, checked at launch)
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nsph * nlm) return;
-  const int i = e / nlm, le = e - i * nlm;
-  int l = 0;
-  while (lmi(l + 1, 0) <= le) ++l;
-  const int m = le - lmi(l, 0), ind = l * l + l;
-  const double* Xi = X + (size_t)i * tb.nylm;
-  const double kk = GAM ? tb.Kg[le] : tb.K[le];
-  XK[e] = mk2<Rl>((Rl)(kk * Xi[ind + m]), m ? (Rl)(kk * Xi[ind - m]) : Rl(0));
-}
-
 #define DDC_LMAX_CASES(X) \
   X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 
-// ---------------------------------------------------------------------------
-// lstarx (adjrhs ddcosmo.f90:1301-1384, matvec.f90:161-235):
-//   y_i,lm = - sum_{j in N_i} sum_{n: t_n^ji<1} w_n xi_j(n) W_ji(n)
-//                4pi/(2l+1) t^l Y_lm(s_n^ji)
-// Block per sphere i, one warp per "role".  A role owns the Legendre
-// columns m and lmax-m (and the middle column when lmax is even), which
-// balances the recurrence work (lmax+2 steps per role) and caps the
-// register accumulators at 2*lmax+4.  Per chunk of triples (one per thread):
-//   phase A: every thread computes one triple's geometry, weight and the
-//            prefix Pt_m^m (coef folded in), cos(m phi), sin(m phi) for all m
-//            into shared memory;
-//   phase B: each role warp runs its columns over the chunk, lanes over
-//            triples, accumulating in registers.
-// At the end each role reduces its accumulators across its 32 lanes with a
-// fixed shuffle tree.  No atomics: the result is bit-reproducible.
-// ---------------------------------------------------------------------------
-__host__ __device__ constexpr int ls_nroles(int L) { return L / 2 + 1; }
-__host__ __device__ constexpr int ls_col2(int L, int r) { return L - r; }  // second column
-__host__ __device__ constexpr bool ls_has2(int L, int r) { return L - r > r; }
 __host__ __device__ constexpr int ls_nvals_m(int L, int m) { return m == 0 ? L + 1 : 2 * (L + 1 - m); }
-__host__ __device__ constexpr int ls_role_nvals(int L, int r) {
-  return ls_nvals_m(L, r) + (ls_has2(L, r) ? ls_nvals_m(L, L - r) : 0);
-}
 // shared-memory fields per triple: ct, t2, then pmm[m], cos[m], sin[m]
 __host__ __device__ constexpr int ls_nfields(int L) { return 2 + 3 * (L + 1); }
-
-template <int LMAX, int M, int OFF, class Rl>
-__device__ __forceinline__ void ls_column(const YlmTables& tb, Rl ct, Rl t2, Rl p0, Rl cm, Rl sm,
-                                          Rl* acc) {
-  Rl p1 = 0;
-#pragma unroll
-  for (int l = M; l <= LMAX; ++l) {
-    Rl P;
-    if (l == M) {
-      P = p0;
-    } else if (l == M + 1) {
-      p1 = (Rl)(2 * M + 1) * ct * p0;
-      P = p1;
-    } else {
-      P = (cA<Rl>(tb, lmi(l, M)) * ct) * p1 - (cB<Rl>(tb, lmi(l, M)) * t2) * p0;
-      p0 = p1;
-      p1 = P;
-    }
-    if (M == 0) {
-      acc[OFF + (l - M)] += P;
-    } else {
-      acc[OFF + (l - M)] = fma(P, cm, acc[OFF + (l - M)]);
-      acc[OFF + (LMAX + 1 - M) + (l - M)] = fma(P, sm, acc[OFF + (LMAX + 1 - M) + (l - M)]);
-    }
-  }
-}
 
 // GAM: accumulators of the normalised recurrence (scale Kg instead of K)
 template <int LMAX, int M, int OFF, class Rl, bool GAM = false>
@@ -778,161 +586,6 @@ __device__ __forceinline__ void ls_store(const YlmTables& tb, const Rl* acc, dou
       yi[ind - M] = -k * (double)acc[OFF + (LMAX + 1 - M) + (l - M)];
     }
   }
-}
-
-// fields are stored [field][stride]; lanes take triples q < count
-template <int LMAX, int R, class Rl>
-__device__ __forceinline__ void ls_role(const YlmTables& tb, const Rl* sh, int stride,
-                                        int count, int lane, Rl* acc) {
-  constexpr int M1 = R, M2 = LMAX - R;
-  for (int q = lane; q < count; q += 32) {
-    const Rl ct = sh[q], t2 = sh[stride + q];
-    ls_column<LMAX, M1, 0, Rl>(tb, ct, t2, sh[(2 + 3 * M1) * stride + q],
-                               sh[(3 + 3 * M1) * stride + q], sh[(4 + 3 * M1) * stride + q], acc);
-    if constexpr (ls_has2(LMAX, R))
-      ls_column<LMAX, M2, ls_nvals_m(LMAX, M1), Rl>(tb, ct, t2, sh[(2 + 3 * M2) * stride + q],
-                                                     sh[(3 + 3 * M2) * stride + q],
-                                                     sh[(4 + 3 * M2) * stride + q], acc);
-  }
-}
-
-template <int LMAX, int R, class Rl, bool GAM = false>
-__device__ __forceinline__ void ls_role_finish(const YlmTables& tb, Rl* acc, double* yi,
-                                               int lane) {
-  constexpr int NV = ls_role_nvals(LMAX, R);
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
-  }
-  ls_store<LMAX, R, 0, Rl, GAM>(tb, acc, yi, lane);
-  if constexpr (ls_has2(LMAX, R))
-    ls_store<LMAX, LMAX - R, ls_nvals_m(LMAX, R), Rl, GAM>(tb, acc, yi, lane);
-}
-
-// dispatch a runtime role index to the compile-time role code
-template <int LMAX, int R, class Rl>
-__device__ __forceinline__ void ls_run_role(int role, const YlmTables& tb, const Rl* sh,
-                                            int stride, int count, int lane, Rl* acc) {
-  if (role == R) {
-    ls_role<LMAX, R, Rl>(tb, sh, stride, count, lane, acc);
-    return;
-  }
-  if constexpr (R + 1 < ls_nroles(LMAX))
-    ls_run_role<LMAX, R + 1, Rl>(role, tb, sh, stride, count, lane, acc);
-}
-template <int LMAX, int R, class Rl, bool GAM = false>
-__device__ __forceinline__ void ls_finish_role(int role, const YlmTables& tb, Rl* acc,
-                                               double* yi, int lane) {
-  if (role == R) {
-    ls_role_finish<LMAX, R, Rl, GAM>(tb, acc, yi, lane);
-    return;
-  }
-  if constexpr (R + 1 < ls_nroles(LMAX))
-    ls_finish_role<LMAX, R + 1, Rl, GAM>(role, tb, acc, yi, lane);
-}
-
-__host__ __device__ constexpr int ls_max_nvals(int L) {
-  int mx = 0;
-  for (int r = 0; r < ls_nroles(L); ++r) mx = ls_role_nvals(L, r) > mx ? ls_role_nvals(L, r) : mx;
-  return mx;
-}
-
-template <int LMAX>
-__global__ void __launch_bounds__(32 * ls_nroles(LMAX)) k_lstarx(const YlmTables tb,
-                                                                  const DevGeo g,
-                                                                  const double* __restrict__ xi,
-                                                                  double* y) {
-  constexpr int NR = ls_nroles(LMAX);
-  constexpr int NT = 32 * NR;  // threads per block
-  constexpr int CH = NT;       // triples per chunk (one per thread in phase A)
-  constexpr int NF = ls_nfields(LMAX);
-  constexpr int NVM = ls_max_nvals(LMAX);
-  extern __shared__ double sh[];  // [NF][CH]
-  const int i = blockIdx.x;
-  if (sweep_skip(g.act, i)) return;
-  const int role = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double4 ci = g.sph[i];
-  const int G = g.ngrid;
-  const double eta = tb.eta, flow = 1.0 - eta;
-  const double fa = 15.0 * eta - 12.0, fb = 10.0 * eta * eta - 15.0 * eta + 6.0;
-  const double ie5 = 1.0 / (eta * eta * eta * eta * eta);
-  const double iri = 1.0 / ci.w;
-  double acc[NVM];
-#pragma unroll
-  for (int v = 0; v < NVM; ++v) acc[v] = 0.0;
-  const int q0 = g.ls_ptr[i], q1 = g.ls_ptr[i + 1];
-  for (int c0 = q0; c0 < q1; c0 += CH) {
-    const int chunk = min(CH, q1 - c0);
-    // phase A: one triple per thread
-    for (int tt = threadIdx.x; tt < chunk; tt += NT) {
-      const int q = c0 + tt;
-      const int2 jn = g.ls[q];
-      const int j = jn.x, n = jn.y;
-      const double4 cj = g.sph[j];
-      const double4 gn = g.grid[n];
-      double vx = fma(cj.w, gn.x, cj.x) - ci.x;
-      double vy = fma(cj.w, gn.y, cj.y) - ci.y;
-      double vz = fma(cj.w, gn.z, cj.z) - ci.z;
-      double r2 = vx * vx + vy * vy + vz * vz;
-      double rinv = rsqrt(r2);
-      double t = r2 * rinv * iri;
-      Angles a = angles_of(vx * rinv, vy * rinv, vz * rinv);
-      const size_t pj = (size_t)j * G + n;
-      double chi = fsw_fast(t, eta, flow, fa, fb, ie5);
-      double f = g.fi[pj];
-      double W = f > 1.0 ? chi / f : chi;
-      const double st = a.s * t;
-      double* col = sh + tt;
-      col[0] = a.c * t;
-      col[CH] = t * t;
-      double pmm = gn.w * xi[pj] * W;
-      double cm = 1.0, sm = 0.0, cmm1 = 1.0, smm1 = 0.0;
-#pragma unroll
-      for (int m = 0; m <= LMAX; ++m) {
-        if (m == 1) {
-          cm = a.cp; sm = a.sp;
-        } else if (m >= 2) {
-          double cn = 2.0 * a.cp * cm - cmm1, sn = 2.0 * a.cp * sm - smm1;
-          cmm1 = cm; smm1 = sm; cm = cn; sm = sn;
-        }
-        col[(2 + 3 * m) * CH] = pmm;
-        col[(3 + 3 * m) * CH] = cm;
-        col[(4 + 3 * m) * CH] = sm;
-        pmm = -pmm * (2.0 * m + 1.0) * st;
-      }
-    }
-    __syncthreads();
-    // phase B: the role's columns over the chunk
-    ls_run_role<LMAX, 0, double>(role, tb, sh, CH, chunk, lane, acc);
-    __syncthreads();
-  }
-  ls_finish_role<LMAX, 0, double>(role, tb, acc, y + (size_t)i * tb.nylm, lane);
-}
-
-cudaError_t launch_lstarx_acc(Launch L, const YlmTables& tb, const DevGeo& g, const double* xi,
-                              double* y) {
-  if (g.nsph == 0) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-#define CASE(LV)                                                                              \
-  case LV: {                                                                                  \
-    constexpr int NR = ls_nroles(LV);                                                         \
-    size_t sm = sizeof(double) * ls_nfields(LV) * 32 * NR;                                    \
-    if (sm > 48 * 1024)                                                                       \
-      if ((e = cudaFuncSetAttribute(k_lstarx<LV>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                    (int)sm)))                                                \
-        return e;                                                                             \
-    k_lstarx<LV><<<g.nsph, 32 * NR, sm, L.st>>>(tb, g, xi, y);                                \
-    break;                                                                                    \
-  }
-  switch (tb.lmax) {
-    DDC_LMAX_CASES(CASE)
-    default:
-      return cudaErrorInvalidValue;
-  }
-#undef CASE
-  ++*L.launches;
-  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -1192,9 +845,9 @@ cudaError_t launch_proj_f32_simt(Launch L, int nylm, int nsph, int ngrid, float 
   return gemm2<false, float, float, double, float>(L, nylm, nsph, ngrid, alpha, bw_f, nylm, pot,
                                                    ldp, y, nylm);
 }
-cudaError_t launch_xi_f32_simt(Launch L, int nylm, int nsph, int ngrid, const float* basis_f,
+cudaError_t launch_xi_f32_simt(Launch L, int nylm, int nsph, int ngrid, const float* bw_f,
                                const double* s, float* xi) {
-  return gemm2<true, float, double, float, float>(L, ngrid, nsph, nylm, 1.f, basis_f, nylm, s,
+  return gemm2<true, float, double, float, float>(L, ngrid, nsph, nylm, 1.f, bw_f, nylm, s,
                                                   nylm, xi, ngrid);
 }
 
@@ -2307,11 +1960,9 @@ __global__ void __launch_bounds__(128) k_forces_a(const YlmTables tb, const DevG
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const double* si = sigma + (size_t)i * NY;
   for (int q = g.ls_ptr[i] + threadIdx.x; q < g.ls_ptr[i + 1]; q += blockDim.x) {
-    const int2 jn = g.ls[q];
-    const int j = jn.x, n = jn.y;
+    const int pj = g.ls[q], j = pj / G, n = pj - j * G;
     const double4 cj = g.sph[j];
     const double4 gn = g.grid[n];
-    const size_t pj = (size_t)j * G + n;
     Rel r = rel_exact(cj, gn, ci);
     double sx = r.vx / r.vv, sy = r.vy / r.vv, sz = r.vz / r.vv;
     double alp[3], beta;
@@ -2335,9 +1986,9 @@ __global__ void __launch_bounds__(128) k_forces_a(const YlmTables tb, const DevG
         fb = 0.0;
       }
       double fa = oij / ci.w;
-      double va0 = fa * alp[0] + beta * fb * g.zi[3 * pj];
-      double va1 = fa * alp[1] + beta * fb * g.zi[3 * pj + 1];
-      double va2 = fa * alp[2] + beta * fb * g.zi[3 * pj + 2];
+      double va0 = fa * alp[0] + beta * fb * g.zi[3 * (size_t)pj];
+      double va1 = fa * alp[1] + beta * fb * g.zi[3 * (size_t)pj + 1];
+      double va2 = fa * alp[2] + beta * fb * g.zi[3 * (size_t)pj + 2];
       if (r.t > tlow) {
         double f3 = beta * dsw / ci.w;
         if (fj > 1.0) f3 = f3 / fj;
@@ -2565,231 +2216,6 @@ cudaError_t launch_csph_pack(Launch L, int n, const double4* sph, double* csph, 
   return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------------------
-// FP32 operator (mixed precision).  Same work decomposition as the FP64
-// kernels; geometry differences are formed in FP64 and rounded once to FP32,
-// the recurrences, switch function and accumulations run in FP32.  The
-// result is an operator accurate to ~1e-6 relative, used only inside the
-// FP64 iterative refinement of the solver (the outer residual is FP64).
-// ---------------------------------------------------------------------------
-struct AnglesF {
-  float c, s, cp, sp;
-};
-__device__ __forceinline__ AnglesF angles_of_f(float sx, float sy, float sz) {
-  AnglesF a;
-  a.c = sz;
-  a.s = sqrtf(fmaxf(0.f, 1.f - sz * sz));
-  if (a.s != 0.f) {
-    float r = 1.f / a.s;
-    a.cp = sx * r;
-    a.sp = sy * r;
-  } else {
-    a.cp = 1.f;
-    a.sp = 0.f;
-  }
-  return a;
-}
-__device__ __forceinline__ float fsw_f(float x, float eta, float flow, float a, float b,
-                                       float ie5) {
-  if (x >= 1.f) return 0.f;
-  if (x <= flow) return 1.f;
-  float xm = x - 1.f;
-  return (xm * xm * (1.f - x)) * ((6.f * x + a) * x + b) * ie5;
-}
-
-template <int LMAX>
-__device__ __forceinline__ float ylm_dot_f(const YlmTables& tb, const AnglesF& a, float t,
-                                           const float2* __restrict__ xs) {
-  const float ct = a.c * t, st = a.s * t, t2 = t * t;
-  float acc = 0.f, pmm = 1.f;
-  float cm = 1.f, sm = 0.f, cmm1 = 1.f, smm1 = 0.f;
-#pragma unroll
-  for (int m = 0; m <= LMAX; ++m) {
-    if (m == 1) {
-      cm = a.cp;
-      sm = a.sp;
-    } else if (m >= 2) {
-      float cn = 2.f * a.cp * cm - cmm1, sn = 2.f * a.cp * sm - smm1;
-      cmm1 = cm; smm1 = sm; cm = cn; sm = sn;
-    }
-    float p0 = pmm, p1 = 0.f;
-#pragma unroll
-    for (int l = m; l <= LMAX; ++l) {
-      float P;
-      if (l == m) {
-        P = p0;
-      } else if (l == m + 1) {
-        p1 = (float)(2 * m + 1) * ct * p0;
-        P = p1;
-      } else {
-        P = (tb.Af[lmi(l, m)] * ct) * p1 - (tb.Bf[lmi(l, m)] * t2) * p0;
-        p0 = p1;
-        p1 = P;
-      }
-      float2 xv = xs[lmi(l, m)];
-      float q = (m == 0) ? xv.x : fmaf(cm, xv.x, sm * xv.y);
-      acc = fmaf(P, q, acc);
-    }
-    pmm = -pmm * (float)(2 * m + 1) * st;
-  }
-  return acc;
-}
-
-template <int LMAX>
-__global__ void __launch_bounds__(32 * ls_nroles(LMAX)) k_lstarx_f(const YlmTables tb,
-                                                                    const DevGeo g,
-                                                                    const float* __restrict__ xi,
-                                                                    double* y) {
-  constexpr int NR = ls_nroles(LMAX);
-  constexpr int NT = 32 * NR;
-  constexpr int CH = NT;
-  constexpr int NVM = ls_max_nvals(LMAX);
-  extern __shared__ float shf[];  // [NF][CH]
-  const int i = blockIdx.x;
-  if (sweep_skip(g.act, i)) return;
-  const int role = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double4 ci = g.sph[i];
-  const int G = g.ngrid;
-  const float eta = (float)tb.eta, flow = 1.f - eta;
-  const float fa = 15.f * eta - 12.f, fb = 10.f * eta * eta - 15.f * eta + 6.f;
-  const float ie5 = (float)(1.0 / (tb.eta * tb.eta * tb.eta * tb.eta * tb.eta));
-  const float iri = (float)(1.0 / ci.w);
-  float acc[NVM];
-#pragma unroll
-  for (int v = 0; v < NVM; ++v) acc[v] = 0.f;
-  const int q0 = g.ls_ptr[i], q1 = g.ls_ptr[i + 1];
-  for (int c0 = q0; c0 < q1; c0 += CH) {
-    const int chunk = min(CH, q1 - c0);
-    for (int tt = threadIdx.x; tt < chunk; tt += NT) {
-      const int q = c0 + tt;
-      const int2 jn = g.ls[q];
-      const int j = jn.x, n = jn.y;
-      const double4 cj = g.sph[j];
-      const float4 gn = g.gridf[n];
-      const float rj = (float)cj.w;
-      float vx = fmaf(rj, gn.x, (float)(cj.x - ci.x));
-      float vy = fmaf(rj, gn.y, (float)(cj.y - ci.y));
-      float vz = fmaf(rj, gn.z, (float)(cj.z - ci.z));
-      float r2 = vx * vx + vy * vy + vz * vz;
-      float rinv = rsqrtf(r2);
-      float t = r2 * rinv * iri;
-      AnglesF a = angles_of_f(vx * rinv, vy * rinv, vz * rinv);
-      const size_t pj = (size_t)j * G + n;
-      float chi = fsw_f(t, eta, flow, fa, fb, ie5);
-      float f = (float)g.fi[pj];
-      float W = f > 1.f ? chi / f : chi;
-      const float st = a.s * t;
-      float* col = shf + tt;
-      col[0] = a.c * t;
-      col[CH] = t * t;
-      float pmm = gn.w * xi[pj] * W;
-      float cm = 1.f, sm = 0.f, cmm1 = 1.f, smm1 = 0.f;
-#pragma unroll
-      for (int m = 0; m <= LMAX; ++m) {
-        if (m == 1) {
-          cm = a.cp; sm = a.sp;
-        } else if (m >= 2) {
-          float cn = 2.f * a.cp * cm - cmm1, sn = 2.f * a.cp * sm - smm1;
-          cmm1 = cm; smm1 = sm; cm = cn; sm = sn;
-        }
-        col[(2 + 3 * m) * CH] = pmm;
-        col[(3 + 3 * m) * CH] = cm;
-        col[(4 + 3 * m) * CH] = sm;
-        pmm = -pmm * (float)(2 * m + 1) * st;
-      }
-    }
-    __syncthreads();
-    ls_run_role<LMAX, 0, float>(role, tb, shf, CH, chunk, lane, acc);
-    __syncthreads();
-  }
-  ls_finish_role<LMAX, 0, float>(role, tb, acc, y + (size_t)i * tb.nylm, lane);
-}
-
-cudaError_t launch_lstarx_acc_f32(Launch L, const YlmTables& tb, const DevGeo& g,
-                                  const float* xi, double* y) {
-  if (g.nsph == 0) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-#define CASE(LV)                                                                              \
-  case LV: {                                                                                  \
-    constexpr int NR = ls_nroles(LV);                                                         \
-    size_t sm = sizeof(float) * ls_nfields(LV) * 32 * NR;                                     \
-    if (sm > 48 * 1024)                                                                       \
-      if ((e = cudaFuncSetAttribute(k_lstarx_f<LV>,                                           \
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))   \
-        return e;                                                                             \
-    k_lstarx_f<LV><<<g.nsph, 32 * NR, sm, L.st>>>(tb, g, xi, y);                              \
-    break;                                                                                    \
-  }
-  switch (tb.lmax) {
-    DDC_LMAX_CASES(CASE)
-    default:
-      return cudaErrorInvalidValue;
-  }
-#undef CASE
-  ++*L.launches;
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Fused application of L and L* (lx matvec.f90:94-148 with calcv
-// ddcosmo.f90:1671-1746; lstarx matvec.f90:161-235 with adjrhs
-// ddcosmo.f90:1301-1384).  Both operators run over the same triples
-// (a, n, b): grid point n of sphere a inside sphere b (t < 1).  They share
-// the weight W = chi(t) / f_a(n) and the values t^l Y_lm(s), s the unit
-// vector from c_b to c_a + r_a s_n:
-//   lx     (output a):  pot_a(n) += W sum_lm K_lm t^l Y_lm(s) X_b,lm
-//   lstarx (output b):  y_b,lm   -= K_lm w_n xi_a(n) W t^l Y_lm(s)
-// Block per sphere b over its gather list (the lstarx layout), in chunks
-// of one triple per thread, software pipelined over two shared buffers:
-// every thread issues the global loads of its triple of chunk k+1, then the
-// role warps (a role owns a set of Legendre columns, below) run the
-// normalised recurrence over chunk k and feed each value to
-// both contractions (registers accumulate the L* rows, the role's share of
-// each triple's lx value goes to shared memory), then the thread turns its
-// loaded inputs into chunk k+1's fields (prefix Q_m^m with W folded in,
-// cos m phi, sin m phi) in the other buffer.  One barrier per chunk; the
-// load latency hides behind the recurrences.  X_b (K-scaled pairs) sits in
-// the roles' registers.  The lx value of each triple (the roles' shares
-// summed in role order) goes to val[q] in gather-list order; k_lx_gather
-// then sums the triples of each point (a, n).  No atomics: the results are
-// bit-reproducible.
-// ---------------------------------------------------------------------------
-// Shared fields of a chunk, in units of Rl with CH triples: a 4-vector
-// (ct, t2, c = w_n xi_a(n), q0[0]) per triple, then per column m >= 1 the
-// prefix q0[m] (W and t^m folded in) and the pair (cos m phi, sin m phi).
-// A role reads a triple with one 4-vector load plus two loads per column
-// m >= 1 (column 0 has cos = 1, sin = 0 and its prefix in the 4-vector).
-__host__ __device__ constexpr int lxs_nfields(int L) { return 4 + 3 * L; }
-__host__ __device__ constexpr int lxs_q0(int CH, int m) { return 4 * CH + 3 * CH * (m - 1); }
-__host__ __device__ constexpr int lxs_cs(int CH, int m) { return 4 * CH + 3 * CH * (m - 1) + CH; }
-template <class Rl> struct V4T;
-template <> struct V4T<float> { typedef float4 T; };
-template <> struct V4T<double> { typedef double4 T; };
-
-// Roles of the fused pass: NR warps share the lmax+1 Legendre columns.  Per
-// triple a column m costs about 5 (m = 0) or 7 (m > 0) operations for each
-// of its lmax+1-m values (recurrence, L* and L contractions) plus a fixed
-// part.  FP64 passes keep the pairing m / lmax-m of k_lstarx (lmax/2+1
-// roles; their summation order, pinned to the oracle's results at 1e-13,
-// stays that of the pairing).  FP32 passes give the columns to the roles
-// greedily, the most expensive first, each to the least-loaded role (lowest
-// index on ties); a role runs its columns in increasing m and holds them in
-// that order in its register arrays.  At lmax 10 the FP32 pass runs four
-// roles of about three columns each (128 registers, four blocks of 128
-// threads per SM): per triple, each role's fixed cost (header load, loop,
-// lx share to shared memory) is paid four times instead of six, 1.25 ms
-// per launch at the 20,000-sphere workload against 1.35 ms for six roles
-// (paired or greedy alike: the SM is issue-bound, and other blocks fill the
-// barrier waits of an uneven role split).
-template <class Rl>
-__host__ __device__ constexpr int lxs_nroles(int L) {
-  return sizeof(Rl) == 4 && L == 10 ? 4 : L / 2 + 1;
-}
-// blocks per SM the pass is compiled for
-template <class Rl>
-__host__ __device__ constexpr int lxs_min_blocks(int L) {
-  return L > 10 ? 1 : sizeof(Rl) == 8 ? (L <= 8 ? 4 : 2) : L == 10 ? 4 : 3;
-}
 __host__ __device__ constexpr int lxs_cost(int L, int m) {
   return m == 0 ? 5 * (L + 1) + 4 : 7 * (L + 1 - m) + 4;
 }
@@ -2830,129 +2256,6 @@ __host__ __device__ constexpr int lxs_max_nvals(int L, int NR, bool g) {
     mx = lxs_role_nvals(L, NR, r, g) > mx ? lxs_role_nvals(L, NR, r, g) : mx;
   return mx;
 }
-__host__ __device__ constexpr int lxs_first_col(int L, int NR, int r, bool g) {
-  for (int c = 0; c <= L; ++c)
-    if (lxs_role_of(L, NR, c, g) == r) return c;
-  return -1;
-}
-
-template <class Rl> __device__ __forceinline__ Rl cBn(const YlmTables& tb, int e);
-template <> __device__ __forceinline__ double cBn<double>(const YlmTables& tb, int e) { return tb.Bn[e]; }
-template <> __device__ __forceinline__ float cBn<float>(const YlmTables& tb, int e) { return tb.Bnf[e]; }
-
-// LONLY: the lx part only (no L* accumulation)
-template <int LMAX, int M, int OFF, class Rl, bool LONLY = false>
-__device__ __forceinline__ Rl lxs_column(const YlmTables& tb, Rl ct, Rl t2, Rl q0, Rl cm, Rl sm,
-                                         Rl c, Rl* acc, const Rl* xr) {
-  constexpr int NM = LMAX + 1 - M;
-  Rl q1 = 0, dc = 0, ds = 0;
-  const Rl cmc = LONLY ? Rl(0) : cm * c, smc = LONLY ? Rl(0) : sm * c;
-#pragma unroll
-  for (int l = M; l <= LMAX; ++l) {
-    Rl Q;
-    if (l == M) {
-      Q = q0;
-    } else if (l == M + 1) {
-      q1 = ct * q0;
-      Q = q1;
-    } else {
-      Q = fma(ct, q1, -(cBn<Rl>(tb, lmi(l, M)) * t2) * q0);
-      q0 = q1;
-      q1 = Q;
-    }
-    if (M == 0) {
-      if (!LONLY) acc[OFF + l] = fma(Q, c, acc[OFF + l]);
-      dc = fma(Q, xr[OFF + l], dc);
-    } else {
-      if (!LONLY) {
-        acc[OFF + (l - M)] = fma(Q, cmc, acc[OFF + (l - M)]);
-        acc[OFF + NM + (l - M)] = fma(Q, smc, acc[OFF + NM + (l - M)]);
-      }
-      dc = fma(Q, xr[OFF + (l - M)], dc);
-      ds = fma(Q, xr[OFF + NM + (l - M)], ds);
-    }
-  }
-  if (M == 0) return dc;
-  return fma(cm, dc, sm * ds);
-}
-
-template <int LMAX, int M, int OFF, class Rl>
-__device__ __forceinline__ void lxs_load_col(const typename RT<Rl>::V2* __restrict__ xb, Rl* xr) {
-  constexpr int NM = LMAX + 1 - M;
-#pragma unroll
-  for (int l = M; l <= LMAX; ++l) {
-    const typename RT<Rl>::V2 v = xb[lmi(l, M)];
-    xr[OFF + (l - M)] = v.x;
-    if (M > 0) xr[OFF + NM + (l - M)] = v.y;
-  }
-}
-
-// X_b of role R's columns into its registers
-template <int LMAX, int NR, int R, int M, class Rl>
-__device__ __forceinline__ void lxs_load_cols(const typename RT<Rl>::V2* xb, Rl* xr) {
-  if constexpr (lxs_role_of(LMAX, NR, M, sizeof(Rl) == 4) == R)
-    lxs_load_col<LMAX, M, lxs_off_of(LMAX, NR, M, sizeof(Rl) == 4), Rl>(xb, xr);
-  if constexpr (M < LMAX) lxs_load_cols<LMAX, NR, R, M + 1, Rl>(xb, xr);
-}
-template <int LMAX, int NR, int R, class Rl>
-__device__ __forceinline__ void lxs_load_role(int role, const typename RT<Rl>::V2* xb, Rl* xr) {
-  if (role == R) {
-    lxs_load_cols<LMAX, NR, R, 0, Rl>(xb, xr);
-    return;
-  }
-  if constexpr (R + 1 < NR) lxs_load_role<LMAX, NR, R + 1, Rl>(role, xb, xr);
-}
-
-// role R's share of triple q: its columns in increasing m, the lx parts
-// summed in that order
-template <int LMAX, int NR, int R, int M, class Rl, bool LONLY>
-__device__ __forceinline__ void lxs_cols(const YlmTables& tb, const Rl* sh, int q,
-                                         const typename V4T<Rl>::T& h, Rl* acc, const Rl* xr,
-                                         Rl& part) {
-  typedef typename RT<Rl>::V2 V2;
-  constexpr int CH = 32 * NR;
-  if constexpr (lxs_role_of(LMAX, NR, M, sizeof(Rl) == 4) == R) {
-    constexpr int OFF = lxs_off_of(LMAX, NR, M, sizeof(Rl) == 4);
-    Rl v;
-    if constexpr (M == 0) {
-      v = lxs_column<LMAX, 0, OFF, Rl, LONLY>(tb, h.x, h.y, h.w, Rl(1), Rl(0), h.z, acc, xr);
-    } else {
-      const V2 c2 = reinterpret_cast<const V2*>(sh + lxs_cs(CH, M))[q];
-      v = lxs_column<LMAX, M, OFF, Rl, LONLY>(tb, h.x, h.y, sh[lxs_q0(CH, M) + q], c2.x, c2.y,
-                                              h.z, acc, xr);
-    }
-    if constexpr (M == lxs_first_col(LMAX, NR, R, sizeof(Rl) == 4)) part = v;
-    else part += v;
-  }
-  if constexpr (M < LMAX) lxs_cols<LMAX, NR, R, M + 1, Rl, LONLY>(tb, sh, q, h, acc, xr, part);
-}
-
-// lanes take triples q < count of the chunk's fields sh
-template <int LMAX, int NR, int R, class Rl, bool LONLY = false>
-__device__ __forceinline__ void lxs_role(const YlmTables& tb, const Rl* sh, int count, int lane,
-                                         Rl* acc, const Rl* xr, Rl* lxp) {
-  typedef typename V4T<Rl>::T V4;
-  constexpr int CH = 32 * NR;
-  const V4* hdr = reinterpret_cast<const V4*>(sh);
-  for (int q = lane; q < count; q += 32) {
-    const V4 h = hdr[q];
-    Rl part;
-    lxs_cols<LMAX, NR, R, 0, Rl, LONLY>(tb, sh, q, h, acc, xr, part);
-    lxp[R * CH + q] = part;
-  }
-}
-template <int LMAX, int NR, int R, class Rl, bool LONLY = false>
-__device__ __forceinline__ void lxs_run_role(int role, const YlmTables& tb, const Rl* sh,
-                                             int count, int lane, Rl* acc, const Rl* xr,
-                                             Rl* lxp) {
-  if (role == R) {
-    lxs_role<LMAX, NR, R, Rl, LONLY>(tb, sh, count, lane, acc, xr, lxp);
-    return;
-  }
-  if constexpr (R + 1 < NR)
-    lxs_run_role<LMAX, NR, R + 1, Rl, LONLY>(role, tb, sh, count, lane, acc, xr, lxp);
-}
-
 // the L* rows of role R: lane sums by a fixed shuffle tree, then its columns
 // G: the greedy column map (else the pairing); the fused pass's choice by
 // default
@@ -2980,371 +2283,6 @@ __device__ __forceinline__ void lxs_finish_role(int role, const YlmTables& tb, R
     lxs_finish_role<LMAX, NR, R + 1, Rl, GAM, G>(role, tb, acc, yi, lane);
 }
 
-// the inputs of one triple's shared fields, loaded one chunk ahead
-template <class Rl>
-struct LxsIn {
-  double4 ca;
-  GP<Rl> gn;
-  double f;
-  Rl xv;
-};
-template <class Rl>
-__device__ __forceinline__ LxsIn<Rl> lxs_load(const DevGeo& g, const Rl* __restrict__ xi, int q,
-                                               int2 an) {
-  const size_t pa = (size_t)an.x * g.ngrid + an.y;
-  LxsIn<Rl> in;
-  in.ca = g.sph[an.x];
-  in.gn = grid_pt(g, an.y, (Rl*)nullptr);
-  in.f = g.fi[pa];
-  in.xv = xi ? xi[pa] : Rl(0);
-  return in;
-}
-// the shared fields of one triple from its inputs (column col of the buffer)
-// FP32 path: approximate reciprocal square root and division (about 2 ulp;
-// the FP32 operator only has to be accurate to ~1e-6 for the FP64
-// refinement); FP64 path: IEEE operations
-__device__ __forceinline__ double div_t(double a, double b) { return a / b; }
-__device__ __forceinline__ float div_t(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double sin_from_cos(double c) { return sqrt(fmax(0.0, 1.0 - c * c)); }
-__device__ __forceinline__ float sin_from_cos(float c) {
-  const float u = 1.f - c * c;
-  return u > 0.f ? u * rsqrtf(u) : 0.f;
-}
-// The static geometry of one triple: t cos(theta), t^2, t sin(theta), the
-// weight W = chi(t) / f_a(n), cos(phi), sin(phi).
-template <class Rl>
-struct LxsGeo {
-  Rl ct, t2, st, W, cp, sp;
-};
-template <class Rl>
-__device__ __forceinline__ LxsGeo<Rl> lxs_geom(const YlmTables& tb, double4 ca, GP<Rl> gn,
-                                               double fd, double4 cb, Rl irb) {
-  constexpr bool D = sizeof(Rl) == 8;
-  const Rl eta = (Rl)tb.eta, flow = Rl(1) - eta;
-  const Rl fa = Rl(15) * eta - Rl(12), fb = Rl(10) * eta * eta - Rl(15) * eta + Rl(6);
-  Rl vx, vy, vz;
-  if constexpr (D) {
-    vx = fma(ca.w, gn.x, ca.x) - cb.x;
-    vy = fma(ca.w, gn.y, ca.y) - cb.y;
-    vz = fma(ca.w, gn.z, ca.z) - cb.z;
-  } else {
-    const float ra = (float)ca.w;
-    vx = fmaf(ra, gn.x, (float)(ca.x - cb.x));
-    vy = fmaf(ra, gn.y, (float)(ca.y - cb.y));
-    vz = fmaf(ra, gn.z, (float)(ca.z - cb.z));
-  }
-  const Rl r2 = vx * vx + vy * vy + vz * vz;
-  const Rl rinv = rsqrt_t(r2);
-  const Rl t = r2 * rinv * irb;
-  const Rl sz = vz * rinv;
-  const Rl sth = sin_from_cos(sz);
-  LxsGeo<Rl> o;
-  o.cp = 1;  // pole: only m = 0 survives
-  o.sp = 0;
-  if (sth != Rl(0)) {
-    const Rl rs = div_t(rinv, sth);
-    o.cp = vx * rs;
-    o.sp = vy * rs;
-  }
-  Rl chi;
-  if (t >= Rl(1)) chi = 0;
-  else if (t <= flow) chi = 1;
-  else {
-    const Rl xm = t - Rl(1);
-    const Rl ie5 = (Rl)(1.0 / (tb.eta * tb.eta * tb.eta * tb.eta * tb.eta));
-    chi = (xm * xm * (Rl(1) - t)) * ((Rl(6) * t + fa) * t + fb) * ie5;
-  }
-  const Rl f = (Rl)fd;
-  o.W = f > Rl(1) ? div_t(chi, f) : chi;
-  o.st = sth * t;
-  o.ct = sz * t;
-  o.t2 = t * t;
-  return o;
-}
-// the shared fields of one triple (column tt of the chunk's buffer) from its
-// geometry, grid weight and xi_a(n)
-template <int LMAX, int NR, class Rl>
-__device__ __forceinline__ void lxs_fields(const LxsGeo<Rl>& gm, Rl w, Rl xv, Rl* sh, int tt) {
-  constexpr int CH = 32 * NR;
-  typedef typename RT<Rl>::V2 V2;
-  typedef typename V4T<Rl>::T V4;
-  V4 h;
-  h.x = gm.ct;
-  h.y = gm.t2;
-  h.z = w * xv;
-  h.w = gm.W;  // q0[0]
-  reinterpret_cast<V4*>(sh)[tt] = h;
-  const Rl cp = gm.cp, sp = gm.sp, st = gm.st;
-  Rl pmm = -gm.W * Rl(1) * st, cm = cp, sm = sp, cmm1 = 1, smm1 = 0;
-#pragma unroll
-  for (int m = 1; m <= LMAX; ++m) {
-    if (m >= 2) {
-      const Rl cn = Rl(2) * cp * cm - cmm1, sn = Rl(2) * cp * sm - smm1;
-      cmm1 = cm; smm1 = sm; cm = cn; sm = sn;
-    }
-    sh[lxs_q0(CH, m) + tt] = pmm;
-    V2 c2;
-    c2.x = cm;
-    c2.y = sm;
-    reinterpret_cast<V2*>(sh + lxs_cs(CH, m))[tt] = c2;
-    pmm = -pmm * Rl(2 * m + 1) * st;
-  }
-}
-template <int LMAX, int NR, class Rl>
-__device__ __forceinline__ void lxs_fields(const YlmTables& tb, const LxsIn<Rl>& in, double4 cb,
-                                           Rl irb, Rl* sh, int tt) {
-  lxs_fields<LMAX, NR, Rl>(lxs_geom<Rl>(tb, in.ca, in.gn, in.f, cb, irb), in.gn.w, in.xv, sh, tt);
-}
-// the geometry precomputed at ddinit (DevGeo::tgeo4/tgeo2 in FP32,
-// tgeo4d/tgeo2d in FP64)
-template <class Rl>
-struct LxsInP {
-  typename V4T<Rl>::T g4;  // ct, t2, st, W
-  typename RT<Rl>::V2 g2;  // cp, sp
-  Rl w, xv;
-};
-__device__ __forceinline__ float4 tgeo4_of(const DevGeo& g, int q, float*) { return g.tgeo4[q]; }
-__device__ __forceinline__ double4 tgeo4_of(const DevGeo& g, int q, double*) { return g.tgeo4d[q]; }
-__device__ __forceinline__ float2 tgeo2_of(const DevGeo& g, int q, float*) { return g.tgeo2[q]; }
-__device__ __forceinline__ double2 tgeo2_of(const DevGeo& g, int q, double*) { return g.tgeo2d[q]; }
-template <class Rl>
-__device__ __forceinline__ LxsInP<Rl> lxs_load_pre(const DevGeo& g, const Rl* __restrict__ xi,
-                                                   int q, int2 an) {
-  LxsInP<Rl> in;
-  in.g4 = tgeo4_of(g, q, (Rl*)nullptr);
-  in.g2 = tgeo2_of(g, q, (Rl*)nullptr);
-  in.w = grid_pt(g, an.y, (Rl*)nullptr).w;
-  in.xv = xi ? xi[(size_t)an.x * g.ngrid + an.y] : Rl(0);
-  return in;
-}
-template <int LMAX, int NR, class Rl>
-__device__ __forceinline__ void lxs_fields_pre(const LxsInP<Rl>& in, Rl* sh, int tt) {
-  LxsGeo<Rl> gm;
-  gm.ct = in.g4.x;
-  gm.t2 = in.g4.y;
-  gm.st = in.g4.z;
-  gm.W = in.g4.w;
-  gm.cp = in.g2.x;
-  gm.sp = in.g2.y;
-  lxs_fields<LMAX, NR, Rl>(gm, in.w, in.xv, sh, tt);
-}
-// the geometry of every triple, block per sphere b over its gather list
-template <class Rl>
-__global__ void k_lxs_geo(const YlmTables tb, const DevGeo g, typename V4T<Rl>::T* tg4,
-                          typename RT<Rl>::V2* tg2) {
-  const int b = blockIdx.x;
-  const double4 cb = g.sph[b];
-  const Rl irb = (Rl)(1.0 / cb.w);
-  for (int q = g.ls_ptr[b] + threadIdx.x; q < g.ls_ptr[b + 1]; q += blockDim.x) {
-    const int2 an = g.ls[q];
-    const LxsGeo<Rl> gm = lxs_geom<Rl>(tb, g.sph[an.x], grid_pt(g, an.y, (Rl*)nullptr),
-                                       g.fi[(size_t)an.x * g.ngrid + an.y], cb, irb);
-    tg4[q].x = gm.ct;
-    tg4[q].y = gm.t2;
-    tg4[q].z = gm.st;
-    tg4[q].w = gm.W;
-    tg2[q].x = gm.cp;
-    tg2[q].y = gm.sp;
-  }
-}
-cudaError_t launch_lxs_geo(Launch L, const YlmTables& tb, const DevGeo& g, float4* tg4,
-                           float2* tg2) {
-  if (g.nsph == 0) return cudaSuccess;
-  k_lxs_geo<float><<<g.nsph, 128, 0, L.st>>>(tb, g, tg4, tg2);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-cudaError_t launch_lxs_geo_f64(Launch L, const YlmTables& tb, const DevGeo& g, double4* tg4,
-                               double2* tg2) {
-  if (g.nsph == 0) return cudaSuccess;
-  k_lxs_geo<double><<<g.nsph, 128, 0, L.st>>>(tb, g, tg4, tg2);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-
-// FP32 chunks are double-buffered (software pipeline); FP64 chunks use one
-// buffer so that two blocks fit in shared memory
-template <class Rl> __host__ __device__ constexpr bool lxs_piped() { return sizeof(Rl) == 4; }
-// Blocks per SM: lxs_min_blocks (FP32 at lmax 10: four of 128 threads, at
-// most 128 registers; other FP32 cases three; FP64 up to lmax 8 four, at
-// most 128 registers: 253 against 282 ms for the 256-globule batch solve at
-// lmax 6 with two; FP64 at lmax 9-10 two, at most 168)
-// MODE 0: L x (val) and L* xi (y) together; 1: L x only (xi, y unused);
-// 2: L x only with the weight chi(t) in place of chi(t)/f_a(n) (the u_chi sum
-// of the forces, on-the-fly geometry only)
-template <int LMAX, class Rl, bool PRE = false, int MODE = 0>
-__global__ void __launch_bounds__(32 * lxs_nroles<Rl>(LMAX), lxs_min_blocks<Rl>(LMAX))
-    k_lxs(const YlmTables tb, const DevGeo g, const typename RT<Rl>::V2* __restrict__ XK,
-          const Rl* __restrict__ xi, Rl* __restrict__ val, double* __restrict__ y) {
-  static_assert(!(PRE && MODE == 2), "chi-only weights need the on-the-fly geometry");
-  constexpr bool LONLY = MODE != 0;
-  constexpr int NR = lxs_nroles<Rl>(LMAX);
-  constexpr int CH = 32 * NR;  // triples per chunk = threads per block
-  constexpr int NF = lxs_nfields(LMAX);
-  constexpr int NVM = lxs_max_nvals(LMAX, NR, sizeof(Rl) == 4);
-  constexpr int NLM = (LMAX + 1) * (LMAX + 2) / 2;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  constexpr int NBUF = lxs_piped<Rl>() ? 2 : 1;
-  Rl* fld = reinterpret_cast<Rl*>(smraw);  // [NBUF][NF][CH]
-  Rl* lxp = fld + NBUF * NF * CH;          // [NBUF][NR][CH]
-  const int b = blockIdx.x, tid = threadIdx.x;
-  if (sweep_skip(g.act, b)) return;
-  const int role = tid >> 5, lane = tid & 31;
-  const int q0 = g.ls_ptr[b], q1 = g.ls_ptr[b + 1];
-  const int nch = (q1 - q0 + CH - 1) / CH;
-  const double4 cb = g.sph[b];
-  const Rl irb = (Rl)(1.0 / cb.w);
-  Rl acc[NVM], xr[NVM];
-#pragma unroll
-  for (int v = 0; v < NVM; ++v) acc[v] = xr[v] = 0;
-  lxs_load_role<LMAX, NR, 0, Rl>(role, XK + (size_t)b * NLM, xr);
-  // with the geometry precomputed at ddinit only xi_a(n) and the grid weight
-  // are read per triple besides the two geometry vectors
-  typedef typename std::conditional<PRE, LxsInP<Rl>, LxsIn<Rl>>::type In;
-  // an: the triple's gather-list entry (a, n), loaded a chunk earlier than
-  // the inputs that depend on it
-  auto load = [&](int q, int2 an) -> In {
-    if constexpr (PRE) {
-      return lxs_load_pre<Rl>(g, LONLY ? nullptr : xi, q, an);
-    } else {
-      In in = lxs_load<Rl>(g, LONLY ? nullptr : xi, q, an);
-      if constexpr (MODE == 2) in.f = 1.0;  // W = chi(t)
-      return in;
-    }
-  };
-  auto fields = [&](const In& in, Rl* buf) {
-    if constexpr (PRE) lxs_fields_pre<LMAX, NR, Rl>(in, buf, tid);
-    else lxs_fields<LMAX, NR, Rl>(tb, in, cb, irb, buf, tid);
-  };
-  if constexpr (!lxs_piped<Rl>()) {
-    // FP64: one buffer (two blocks per SM fit), two barriers per chunk; the
-    // inputs of chunk k+1 are loaded while the roles work on chunk k
-    In cur;
-    int2 an1 = make_int2(0, 0);
-    if (nch > 0 && tid < min(CH, q1 - q0)) cur = load(q0 + tid, g.ls[q0 + tid]);
-    if (nch > 1 && tid < min(CH, q1 - q0 - CH)) an1 = g.ls[q0 + CH + tid];
-    for (int k = 0; k < nch; ++k) {
-      const int c0 = q0 + k * CH, cnt = min(CH, q1 - c0);
-      if (tid < cnt) fields(cur, fld);
-      __syncthreads();
-      const int n1 = k + 1 < nch ? min(CH, q1 - c0 - CH) : 0;
-      const int n2 = k + 2 < nch ? min(CH, q1 - c0 - 2 * CH) : 0;
-      if (tid < n1) cur = load(c0 + CH + tid, an1);
-      if (tid < n2) an1 = g.ls[c0 + 2 * CH + tid];
-      lxs_run_role<LMAX, NR, 0, Rl, LONLY>(role, tb, fld, cnt, lane, acc, xr, lxp);
-      __syncthreads();
-      if (tid < cnt) {
-        Rl sv = lxp[tid];
-#pragma unroll
-        for (int r = 1; r < NR; ++r) sv += lxp[r * CH + tid];
-        val[c0 + tid] = sv;
-      }
-    }
-    if constexpr (!LONLY)
-      lxs_finish_role<LMAX, NR, 0, Rl, true>(role, tb, acc, y + (size_t)b * tb.nylm, lane);
-    return;
-  }
-  if constexpr (PRE && lxs_piped<Rl>()) {
-    // FP32 with the geometry precomputed at ddinit: each thread copies its
-    // triple's two geometry vectors (24 bytes) to its own shared slot with
-    // cp.async two chunks ahead of their use (two chunks of role work cover
-    // the latency, and no registers hold them meanwhile; a thread reads only
-    // the slot it wrote, after its own wait_group).  The grid weight and
-    // xi_a(n) come through registers one chunk ahead, the gather-list entry
-    // that addresses them two chunks ahead.  (xi_a(n) by cp.async as well
-    // was slower: the copy's issue waits for its gather-list entry.)
-    typename V4T<Rl>::T* gs4 = reinterpret_cast<typename V4T<Rl>::T*>(lxp + NBUF * NR * CH);
-    typename RT<Rl>::V2* gs2 = reinterpret_cast<typename RT<Rl>::V2*>(gs4 + 2 * CH);
-    auto geo_copy = [&](int k) {  // chunk k's geometry into stage k & 1
-      const int q = q0 + k * CH + tid;
-      if (k < nch && q < q1) {
-        cp_async16(gs4 + (k & 1) * CH + tid, g.tgeo4 + q);
-        cp_async8(gs2 + (k & 1) * CH + tid, g.tgeo2 + q, true);
-      }
-      cp_async_commit();
-    };
-    auto wx = [&](int2 an, Rl& w, Rl& xv) {
-      w = grid_pt(g, an.y, (Rl*)nullptr).w;
-      xv = LONLY ? Rl(0) : xi[(size_t)an.x * g.ngrid + an.y];
-    };
-    auto fields_at = [&](int k, Rl w, Rl xv) {
-      LxsInP<Rl> in;
-      in.g4 = gs4[(k & 1) * CH + tid];
-      in.g2 = gs2[(k & 1) * CH + tid];
-      in.w = w;
-      in.xv = xv;
-      lxs_fields_pre<LMAX, NR, Rl>(in, fld + (k & 1) * NF * CH, tid);
-    };
-    geo_copy(0);
-    geo_copy(1);
-    Rl w1 = 0, xv1 = 0;
-    int2 an1 = make_int2(0, 0);
-    if (nch > 0 && tid < min(CH, q1 - q0)) wx(g.ls[q0 + tid], w1, xv1);
-    if (nch > 1 && tid < min(CH, q1 - q0 - CH)) an1 = g.ls[q0 + CH + tid];
-    cp_async_wait<1>();
-    if (nch > 0 && tid < min(CH, q1 - q0)) fields_at(0, w1, xv1);
-    __syncthreads();
-    for (int k = 0; k < nch; ++k) {
-      const int c0 = q0 + k * CH, cnt = min(CH, q1 - c0);
-      const int n1 = k + 1 < nch ? min(CH, q1 - c0 - CH) : 0;
-      const int n2 = k + 2 < nch ? min(CH, q1 - c0 - 2 * CH) : 0;
-      geo_copy(k + 2);
-      if (tid < n1) wx(an1, w1, xv1);
-      int2 an2 = make_int2(0, 0);
-      if (tid < n2) an2 = g.ls[c0 + 2 * CH + tid];
-      lxs_run_role<LMAX, NR, 0, Rl, LONLY>(role, tb, fld + (k & 1) * NF * CH, cnt, lane, acc,
-                                           xr, lxp + (k & 1) * NR * CH);
-      cp_async_wait<1>();  // chunk k+1's copies done (chunk k+2's may be in flight)
-      if (tid < n1) fields_at(k + 1, w1, xv1);
-      __syncthreads();
-      if (tid < cnt) {
-        const Rl* lp = lxp + (k & 1) * NR * CH;
-        Rl sv = lp[tid];
-#pragma unroll
-        for (int r = 1; r < NR; ++r) sv += lp[r * CH + tid];
-        val[c0 + tid] = sv;
-      }
-      an1 = an2;
-    }
-    cp_async_wait<0>();
-    if constexpr (!LONLY)
-      lxs_finish_role<LMAX, NR, 0, Rl, true>(role, tb, acc, y + (size_t)b * tb.nylm, lane);
-    return;
-  }
-  if (nch > 0 && tid < min(CH, q1 - q0)) fields(load(q0 + tid, g.ls[q0 + tid]), fld);
-  int2 an1 = make_int2(0, 0);
-  if (nch > 1 && tid < min(CH, q1 - q0 - CH)) an1 = g.ls[q0 + CH + tid];
-  __syncthreads();
-  // chunk k: loads of chunk k+1 (and the gather-list entries of chunk k+2)
-  // in flight while the roles work on chunk k, then chunk k+1's fields go to
-  // the other buffer; one barrier per chunk
-  for (int k = 0; k < nch; ++k) {
-    const int c0 = q0 + k * CH, cnt = min(CH, q1 - c0);
-    const int n1 = k + 1 < nch ? min(CH, q1 - c0 - CH) : 0;
-    const int n2 = k + 2 < nch ? min(CH, q1 - c0 - 2 * CH) : 0;
-    In nxt;
-    if (tid < n1) nxt = load(c0 + CH + tid, an1);
-    int2 an2 = make_int2(0, 0);
-    if (tid < n2) an2 = g.ls[c0 + 2 * CH + tid];
-    lxs_run_role<LMAX, NR, 0, Rl, LONLY>(role, tb, fld + (k & 1) * NF * CH, cnt, lane, acc, xr,
-                                     lxp + (k & 1) * NR * CH);
-    if (tid < n1) fields(nxt, fld + ((k + 1) & 1) * NF * CH);
-    __syncthreads();
-    // lx values of chunk k: the roles' shares in role order (buffer k&1 of
-    // lxp is next written two chunks on, after the next barrier)
-    if (tid < cnt) {
-      const Rl* lp = lxp + (k & 1) * NR * CH;
-      Rl sv = lp[tid];
-#pragma unroll
-      for (int r = 1; r < NR; ++r) sv += lp[r * CH + tid];
-      val[c0 + tid] = sv;
-    }
-    an1 = an2;
-  }
-  if constexpr (!LONLY)
-    lxs_finish_role<LMAX, NR, 0, Rl, true>(role, tb, acc, y + (size_t)b * tb.nylm, lane);
-}
-
 // pot_a(n) = sum over a's CSR pairs (a, b), in CSR order, of the lx values
 // of the triples (a, n, b), read from b's gather list at the pair's block
 // (lsstart).  Warp per sphere a, with a private shared row of ngrid values
@@ -3352,12 +2290,13 @@ __global__ void __launch_bounds__(32 * lxs_nroles<Rl>(LMAX), lxs_min_blocks<Rl>(
 // points (distinct within a pair, so no two lanes touch one entry), four
 // strided loads per lane, and the next pair's first loads are issued before
 // the current pair's adds; a __syncwarp between pairs orders the updates of
-// a point by its pairs.  No block barriers (each warp runs its sphere from
+// a point by its pairs.  chi: the sums times max(f_a(n), 1), i.e. with the
+// weight chi(t) of u_chi in place of chi(t) / f_a(n).  No block barriers (each warp runs its sphere from
 // start to end) and no atomics: a fixed summation order.
 constexpr int kGatherWarps = 4;  // spheres per block
 template <class Rl>
 __global__ void __launch_bounds__(32 * kGatherWarps)
-    k_lx_gather(const DevGeo g, const Rl* __restrict__ val, Rl* pot, int ldp) {
+    k_lx_gather(const DevGeo g, const Rl* __restrict__ val, Rl* pot, int ldp, bool chi) {
   constexpr int U = 4;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int G = g.ngrid;
@@ -3415,50 +2354,16 @@ __global__ void __launch_bounds__(32 * kGatherWarps)
       }
     }
   }
-  for (int n = lane; n < G; n += 32) pot[(size_t)a * ldp + n] = row[n];
+  for (int n = lane; n < G; n += 32) {
+    Rl v = row[n];
+    if (chi) v *= (Rl)fmax(g.fi[(size_t)a * G + n], 1.0);
+    pot[(size_t)a * ldp + n] = v;
+  }
 }
 
-template <class Rl, int MODE>
-static cudaError_t lxs_launch(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                              const Rl* xi, void* xk, Rl* val, double* y) {
-  if (g.nsph == 0) return cudaSuccess;
-  typedef typename RT<Rl>::V2 V2;
-  const long long nk = (long long)g.nsph * ((tb.lmax + 1) * (tb.lmax + 2) / 2);
-  if (nk >= INT_MAX) return cudaErrorInvalidValue;
-  V2* XK = static_cast<V2*>(xk);
-  k_xk<Rl, true><<<(unsigned)((nk + 255) / 256), 256, 0, L.st>>>(tb, g.nsph, X, XK);
-  ++*L.launches;
-  cudaError_t e = cudaGetLastError();
-  if (e) return e;
-#define CASE(LV)                                                                              \
-  case LV: {                                                                                  \
-    constexpr int NR = lxs_nroles<Rl>(LV);                                                    \
-    const bool pre = MODE != 2 && (sizeof(Rl) == 4 ? g.tgeo4 != nullptr : g.tgeo4d != nullptr); \
-    const size_t sm = sizeof(Rl) * (lxs_piped<Rl>() ? 2 : 1) * (lxs_nfields(LV) + NR) * 32 * NR + \
-                      (pre && lxs_piped<Rl>() ? 2 * 32 * NR * 6 * sizeof(Rl) : 0);             \
-    auto kfn = pre ? k_lxs<LV, Rl, MODE != 2, MODE> : k_lxs<LV, Rl, false, MODE>;             \
-    if (sm > 48 * 1024) {                                                                     \
-      if ((e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
-                                    (int)sm)))                                                \
-        return e;                                                                             \
-      if ((e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout,      \
-                                    100)))                                                    \
-        return e;                                                                             \
-    }                                                                                         \
-    kfn<<<g.nsph, 32 * NR, sm, L.st>>>(tb, g, XK, xi, val, y);                                \
-    break;                                                                                    \
-  }
-  switch (tb.lmax) {
-    DDC_LMAX_CASES(CASE)
-    default:
-      return cudaErrorInvalidValue;
-  }
-#undef CASE
-  ++*L.launches;
-  return cudaGetLastError();
-}
 template <class Rl>
-static cudaError_t gather_launch(Launch L, const DevGeo& g, const Rl* val, Rl* pot, int ldp) {
+static cudaError_t gather_launch(Launch L, const DevGeo& g, const Rl* val, Rl* pot, int ldp,
+                                 bool chi) {
   if (g.nsph == 0) return cudaSuccess;
   const int mb = (g.maxnb + 3) & ~3;
   const size_t sm = kGatherWarps * (sizeof(int) * (2 * mb + 4) + sizeof(Rl) * g.ngrid);
@@ -3468,33 +2373,17 @@ static cudaError_t gather_launch(Launch L, const DevGeo& g, const Rl* val, Rl* p
                                   (int)sm)))
       return e;
   k_lx_gather<Rl><<<(g.nsph + kGatherWarps - 1) / kGatherWarps, 32 * kGatherWarps, sm, L.st>>>(
-      g, val, pot, ldp);
+      g, val, pot, ldp, chi);
   ++*L.launches;
   return cudaGetLastError();
 }
-cudaError_t launch_lxs(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                       const double* xi, void* xk, double* val, double* y) {
-  return lxs_launch<double, 0>(L, tb, g, X, xi, xk, val, y);
-}
-cudaError_t launch_lxs_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                           const float* xi, void* xk, float* val, double* y) {
-  return lxs_launch<float, 0>(L, tb, g, X, xi, xk, val, y);
-}
-cudaError_t launch_lx_vals(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                           void* xk, double* val, bool chi_only) {
-  return chi_only ? lxs_launch<double, 2>(L, tb, g, X, nullptr, xk, val, nullptr)
-                  : lxs_launch<double, 1>(L, tb, g, X, nullptr, xk, val, nullptr);
-}
-cudaError_t launch_lx_vals_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
-                               void* xk, float* val) {
-  return lxs_launch<float, 1>(L, tb, g, X, nullptr, xk, val, nullptr);
-}
-cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, double* pot) {
-  return gather_launch<double>(L, g, val, pot, g.ngrid);
+cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, double* pot,
+                             bool chi) {
+  return gather_launch<double>(L, g, val, pot, g.ngrid, chi);
 }
 cudaError_t launch_lx_gather_f32(Launch L, const DevGeo& g, const float* val, float* pot,
                                  int ldp) {
-  return gather_launch<float>(L, g, val, pot, ldp);
+  return gather_launch<float>(L, g, val, pot, ldp, false);
 }
 
 __global__ void k_to_float(long long n, const double* __restrict__ x, float* y) {

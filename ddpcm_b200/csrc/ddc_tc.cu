@@ -3,15 +3,15 @@
 //
 //   projection (intrhs inside lx, matvec.f90:131-135; ddcosmo.f90:789-821):
 //       y(lm, i) = alpha * sum_n bw(lm, n) pot(n, i)         M = lm, K = n
-//   expansion (xi = basis^T s, matvec.f90:189-204):
-//       xi(n, i) = sum_lm basis(lm, n) s(lm, i)               M = n,  K = lm
+//   expansion (w xi = bw^T s, matvec.f90:189-204, with the weights of :216):
+//       w_n xi(n, i) = sum_lm bw(lm, n) s(lm, i)              M = n,  K = lm
 //
 // Both run as TF32 tensor-core GEMMs with the three-term split that recovers
 // FP32 accuracy: every operand v is carried as hi = tf32(v) and
 // lo = tf32(v - hi), and each k-step issues A_hi*B_hi + A_hi*B_lo + A_lo*B_hi
 // into one FP32 accumulator in tensor memory (the dropped A_lo*B_lo term and
 // the truncation of the lo parts are below 2^-20 of each product).  The
-// static operand (bw or basis) is split once, at set-up, from its FP64 values
+// static operand (bw) is split once, at set-up, from its FP64 values
 // into a packed image whose 16 KB chunks are the exact shared-memory tiles the
 // MMA reads (K-major, 128-byte swizzle), so a chunk arrives with one bulk copy.
 // The per-call operand is split on the way in: the grid field pot (FP32, row
@@ -212,7 +212,7 @@ __host__ __device__ constexpr uint32_t tmem_cols(int n) {
 // ---------------------------------------------------------------------------
 // packed image of a static operand: A(m, k) for m < M, k < K (zero beyond),
 // chunk (mt, kc) at ((mt*KC + kc)*2 + part) * kChunk bytes, part 0 = hi, 1 = lo.
-// src is [G][Y] FP64 (basis or bw): trans = false reads A(m, k) = src[k*ld + m]
+// src is [G][Y] FP64 (bw): trans = false reads A(m, k) = src[k*ld + m]
 // (projection: m = lm, k = grid point), trans = true reads src[m*ld + k]
 // (expansion: m = grid point, k = lm).
 // ---------------------------------------------------------------------------
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 }
 
 // ---------------------------------------------------------------------------
-// expansion: xi(n, i) = sum_lm basis(lm, n) s(lm, i), FP32 out (ld = ngrid)
+// expansion: w_n xi(n, i) = sum_lm bw(lm, n) s(lm, i), FP32 out (ld = ngrid)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_xi_tc(const double* __restrict__ s, const float* __restrict__ aimg, int nsph, int nylm,
@@ -667,7 +667,7 @@ cudaError_t cfg_proj(TcPlan& p, int bn) {
                               p.smem_proj);
 }
 // tile width of the expansion: the split coefficients of bn spheres stay
-// resident, the basis chunks stream through a ring of at least two stages
+// resident, the bw chunks stream through a ring of at least two stages
 cudaError_t cfg_xi(TcPlan& p, int bn) {
   if (bn % 32 != 0 || bn > kMaxBn) return cudaErrorInvalidValue;
   const int bsz = p.kc_xi * 2 * bn * 128;
@@ -688,7 +688,7 @@ std::vector<int> bn_candidates(int nsph) {
 
 }  // namespace
 
-cudaError_t tc_plan(Launch L, TcPlan& p, const double* basis, const double* bw, int nsph,
+cudaError_t tc_plan(Launch L, TcPlan& p, const double* bw, int nsph,
                     int nylm, int ngrid, float* pot_f, int ldp) {
   p.on = false;
   if (!tc_supported(nylm) || nsph <= 0) return cudaSuccess;
@@ -723,7 +723,7 @@ cudaError_t tc_plan(Launch L, TcPlan& p, const double* basis, const double* bw, 
     ++*L.launches;
     const long long tot2 = (long long)p.mt_xi * p.kc_xi * 128 * 32;
     k_pack_static<<<(unsigned)((tot2 + 255) / 256), 256, 0, L.st>>>(
-        basis, nylm, true, ngrid, nylm, p.mt_xi, p.kc_xi, p.img_xi.as<float>());
+        bw, nylm, true, ngrid, nylm, p.mt_xi, p.kc_xi, p.img_xi.as<float>());
     ++*L.launches;
     if ((e = cudaGetLastError())) return e;
   }
