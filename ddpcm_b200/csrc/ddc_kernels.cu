@@ -1291,9 +1291,9 @@ __device__ __forceinline__ SrcRange block_src_range(const int2* trange, int t, i
       r.hi = s0;
     }
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {  // an empty range unless a thread has sources
     b_lo = s1;
-    b_hi = s0;
+    b_hi = min(s0, s1);
   }
   __syncthreads();
   if (r.lo < r.hi) {
@@ -1634,6 +1634,7 @@ cudaError_t launch_efield_f32(Launch L, int nsrc, const double* q, const double*
   int chunk = (nsrc + nchunk - 1) / max(nchunk, 1);
   chunk = ((chunk + kNbTile - 1) / kNbTile) * kNbTile;
   if (chunk == 0) chunk = kNbTile;
+  nchunk = max(1, (nsrc + chunk - 1) / chunk);  // rounding up may leave chunks without sources
   double* out = nchunk == 1 ? ef : scratch;
   const int tiles2 = (ntrg + 2 * kNbTile - 1) / (2 * kNbTile);
   if (!trange && (long long)tiles2 * nchunk >= 148 * 8) {  // enough blocks to fill the GPU
@@ -1658,6 +1659,7 @@ cudaError_t launch_efield(Launch L, int nsrc, const double* q, const double* csr
   int chunk = (nsrc + nchunk - 1) / max(nchunk, 1);
   chunk = ((chunk + kNbTile - 1) / kNbTile) * kNbTile;
   if (chunk == 0) chunk = kNbTile;
+  nchunk = max(1, (nsrc + chunk - 1) / chunk);  // rounding up may leave chunks without sources
   dim3 grid((ntrg + kNbTile - 1) / kNbTile, nchunk);
   double* out = nchunk == 1 ? ef : scratch;
   k_efield<<<grid, kNbTile, 0, L.st>>>(nsrc, q, csrc, ntrg, ctrg, chunk, out, trange);
