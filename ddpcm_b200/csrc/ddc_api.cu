@@ -132,26 +132,27 @@ struct ddc_ctx {
   // batched molecules: partition, per-target N-body ranges, per-molecule DIIS state
   int nmol = 1;
   bool batch_init = false;  // set while ddc_batch_energy_forces initialises
-  bool capturing = false;   // stream capture in progress: no stage events
+  bool batch = false;       // the solve belongs to ddc_batch_energy_forces
   std::vector<int> h_off;
-  DBuf b_cmol, b_cfirst, b_part, b_cnt, b_coef, b_ext;  // chunked batched Jacobi/DIIS
   DBuf b_sphmol;        // molecule of each sphere (batched solves)
-  DBuf b_tolk, b_maxk;  // per-molecule tolerance and budget of the inner solves
-  DBuf b_run, b_upd, b_onorm;  // mixed refinement of a batch: outer status, update mask, norms
-  SweepMask sweep{};    // set while the batched sweeps are captured
-  DBuf d_off, mrange, tr_cav, tr_nuc, b_nmat, b_slot, b_B, b_status, b_iters, b_restarts, b_norm,
-      b_out;
+  DBuf b_cmol, b_cfirst;  // molecule of each solver chunk, first chunk of each molecule
+  // state of the Jacobi/DIIS solves (SolverSys), both systems side by side
+  DBuf s_int, s_dbl, s_slot, s_gram, s_coef, s_part, s_log;
+  int* hstop = nullptr;  // mapped host memory: [2] stop reports, [2] active counts
+  int* dstop = nullptr;
+  cudaEvent_t ev_sweep[4] = {};
+  SweepMask sweep{};    // set while a solver sweep is launched
+  DBuf d_off, mrange, tr_cav, tr_nuc, b_out;
   const int2* mrange_ptr() const { return nmol > 1 ? mrange.as<int2>() : nullptr; }
   int maxnb = 0;
   DBuf cavoff, cavidx, cavpt, ccav, cnt, scan_tmp;
   DBuf csph, cx, cy, cz;  // csph(3,n) and SoA centres
   // work
-  DBuf pot, xig, gbuf, rhs, x, y, xn, partials, red, hist_x, hist_e;
-  DBuf rcount;  // arrival counter of the solver kernels' last-block sums (kept zero)
+  DBuf pot, xig, gbuf, rhs, y, partials, red, hist_x, hist_e;
   DBuf phi, psi, sigma, s, q, fx, zeta, ef1, ef2, ef_scratch, uchi;
   DBuf in1, in2, in3, in4, out1;  // staging for host-pointer calls
   // mixed precision: FP32 basis copy, FP32 grid fields, refinement vectors
-  DBuf bw_f, pot_f, xi_f, rres, dres, eres;
+  DBuf bw_f, pot_f, xi_f, rres, eres;
   // static geometry of the gather-list triples: FP32 (mixed path)
   DBuf tgeo4;
   bool tgeo_on = false;
@@ -160,7 +161,7 @@ struct ddc_ctx {
   bool tgeo64_on = false;
   // second solve set (direct and adjoint solved together) and the fused
   // operator's per-triple lx values
-  DBuf y2, xn2, hist_x2, hist_e2, rres2, dres2, eres2, tval;
+  DBuf y2, hist_x2, hist_e2, rres2, eres2, tval;
   // the two dense contractions of every operator application (projection
   // onto the harmonics, expansion to the grid): basisT[Y][G] is the basis
   // transposed for the FP64 expansion, bwT[Y][G] with the weights; tc plans the tensor-core kernels of
@@ -335,7 +336,7 @@ struct StageScope {
   cudaStream_t on;
   StageScope(ddc_ctx* ctx, int s, cudaStream_t stream = nullptr)
       : c(ctx), stage(s), on(stream ? stream : ctx->st) {
-    if (!c->prm.timing || c->capturing || !((c->stage_mask >> s) & 1u)) return;
+    if (!c->prm.timing || !((c->stage_mask >> s) & 1u)) return;
     a = take();
     b = take();
     if (a && b) cudaEventRecord(a, on);
@@ -641,16 +642,12 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   CK(ctx->pot.ensure(sizeof(double) * std::max(NP, 1LL)));
   CK(ctx->xig.ensure(sizeof(double) * std::max(NP, 1LL)));
   CK(ctx->uchi.ensure(sizeof(double) * std::max(NP, 1LL)));
-  for (DBuf* b : {&ctx->rhs, &ctx->x, &ctx->y, &ctx->xn, &ctx->psi, &ctx->sigma, &ctx->s})
+  for (DBuf* b : {&ctx->rhs, &ctx->y, &ctx->psi, &ctx->sigma, &ctx->s})
     CK(b->ensure(sizeof(double) * std::max(nv, (size_t)1)));
   CK(ctx->hist_x.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
   CK(ctx->hist_e.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
   CK(ctx->partials.ensure(sizeof(double) * reduce_blocks() * (kMaxHist + 1)));
   CK(ctx->red.ensure(sizeof(double) * 2 * (kMaxHist + 1)));
-  if (!ctx->rcount.p) {
-    CK(ctx->rcount.ensure(sizeof(unsigned)));
-    CK(cudaMemsetAsync(ctx->rcount.p, 0, sizeof(unsigned), ctx->st));
-  }
   // the basis transposed to [Y][G] for the FP64 expansions xi = basis^T s
   // (forces, zeta) and w xi = bw^T s (the operators)
   for (auto t : {std::make_pair(&ctx->basis, &ctx->basisT), std::make_pair(&ctx->bw, &ctx->bwT)}) {
@@ -676,15 +673,15 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     if (tc) {
       CK(tc_plan(L, ctx->tc, ctx->bw.as<double>(), N, NY, G,
                  ctx->pot_f.as<float>(), ctx->ldp_f));
-      // tile widths by measurement (x and y are free work vectors here)
-      CK(tc_autotune(L, ctx->tc, ctx->x.as<double>(), ctx->y.as<double>(),
+      // tile widths by measurement (rhs and y are free work vectors here)
+      CK(tc_autotune(L, ctx->tc, ctx->rhs.as<double>(), ctx->y.as<double>(),
                      ctx->xi_f.as<float>()));
     } else {
       ctx->tc.on = false;
       CK(ctx->bw_f.ensure(sizeof(float) * G * NY));
       CK(launch_to_float(L, (long long)G * NY, ctx->bw.as<double>(), ctx->bw_f.as<float>()));
     }
-    for (DBuf* b : {&ctx->rres, &ctx->dres, &ctx->eres})
+    for (DBuf* b : {&ctx->rres, &ctx->eres})
       CK(b->ensure(sizeof(double) * std::max(nv, (size_t)1)));
     // the FP32 fused pass reads each triple's static geometry instead of
     // recomputing it every iteration (16 bytes per triple)
@@ -701,12 +698,11 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     ctx->tgeo64_on = true;
   }
   if (ctx->prm.igrad && ctx->prm.pair_solves) {
-    for (DBuf* b : {&ctx->y2, &ctx->xn2})
-      CK(b->ensure(sizeof(double) * std::max(nv, (size_t)1)));
+    CK(ctx->y2.ensure(sizeof(double) * std::max(nv, (size_t)1)));
     CK(ctx->hist_x2.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
     CK(ctx->hist_e2.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
     if (ctx->prm.precision == DDC_PREC_MIXED)
-      for (DBuf* b : {&ctx->rres2, &ctx->dres2, &ctx->eres2})
+      for (DBuf* b : {&ctx->rres2, &ctx->eres2})
         CK(b->ensure(sizeof(double) * std::max(nv, (size_t)1)));
   }
   // per-triple lx values of the fused passes (FP64 size: the mixed path also
@@ -880,489 +876,345 @@ int op_pair_f32(ddc_ctx* ctx, const double* x, double* y, const double* s, doubl
   return gemm_proj_f32(ctx, -1.f, ctx->pot_f.as<float>(), y);
 }
 
-// gjinv (jacobi_diis.f90:272-360): Gauss-Jordan, full pivoting, one rhs.
-bool gjinv(int n, std::vector<double>& a, std::vector<double>& b) {
-  std::vector<int> indxc(n + 1), indxr(n + 1), piv(n + 1, 0);
-  auto A = [&](int j, int k) -> double& { return a[(size_t)(k - 1) * n + (j - 1)]; };
-  int irow = 0, icol = 0;
-  for (int i = 1; i <= n; i++) {
-    double big = 0.0;
-    for (int j = 1; j <= n; j++)
-      if (piv[j] != 1)
-        for (int k = 1; k <= n; k++)
-          if (piv[k] == 0 && std::fabs(A(j, k)) > big) {
-            big = std::fabs(A(j, k));
-            irow = j;
-            icol = k;
-          }
-    if (icol == 0) return false;
-    piv[icol] += 1;
-    if (piv[icol] > 1) return false;
-    if (irow != icol) {
-      for (int k = 1; k <= n; k++) std::swap(A(irow, k), A(icol, k));
-      std::swap(b[irow - 1], b[icol - 1]);
-    }
-    indxr[i] = irow;
-    indxc[i] = icol;
-    if (A(icol, icol) == 0.0) return false;
-    double pinv = 1.0 / A(icol, icol);
-    A(icol, icol) = 1.0;
-    for (int k = 1; k <= n; k++) A(icol, k) *= pinv;
-    b[icol - 1] *= pinv;
-    for (int j = 1; j <= n; j++)
-      if (j != icol) {
-        double dum = A(j, icol);
-        A(j, icol) = 0.0;
-        for (int k = 1; k <= n; k++) A(j, k) -= A(icol, k) * dum;
-        b[j - 1] -= b[icol - 1] * dum;
-      }
-  }
-  for (int j = n; j >= 1; j--)
-    if (indxr[j] != indxc[j])
-      for (int k = 1; k <= n; k++) std::swap(A(k, indxr[j]), A(k, indxc[j]));
-  return true;
-}
-
-typedef int (*OpFn)(ddc_ctx*, const double*, double*);
-
-// Work vectors of one solve: set 0 is the context's, set 1 the second set
-// used when the direct and adjoint systems are solved together.
-struct SolveBufs {
-  double *y, *xn, *hx, *he, *r, *d, *e;
-};
-SolveBufs solve_bufs(ddc_ctx* ctx, int set) {
-  if (set == 0)
-    return SolveBufs{ctx->y.as<double>(),      ctx->xn.as<double>(),   ctx->hist_x.as<double>(),
-                     ctx->hist_e.as<double>(), ctx->rres.as<double>(), ctx->dres.as<double>(),
-                     ctx->eres.as<double>()};
-  return SolveBufs{ctx->y2.as<double>(),      ctx->xn2.as<double>(),   ctx->hist_x2.as<double>(),
-                   ctx->hist_e2.as<double>(), ctx->rres2.as<double>(), ctx->dres2.as<double>(),
-                   ctx->eres2.as<double>()};
-}
-
-// jacobi_diis (jacobi_diis.f90:1-176), norm mode 4 (hnorm), as a resumable
-// state: the caller applies the operator to x into y, then jd_step performs
-// the rest of the iteration (Jacobi step, DIIS extrapolation, increment
-// norm and convergence test).  x holds the initial guess on entry and the
-// solution on exit (device).  The log of increment norms continues at
-// inf->norms[*logpos].
-struct JDState {
-  const double* rhs = nullptr;
-  double* x = nullptr;
-  double tol = 0.0;
-  int max_iter = 0;
-  double *y = nullptr, *hx = nullptr, *he = nullptr, *xjac = nullptr;
-  std::vector<double> B;
-  std::vector<int> map;
-  int lenb = 0, nmat = 1, it = 0, restarts = 0;
-  double rms = 0.0;
-  bool done = false, ok = false;
-  bool f32 = false;  // history vectors in FP32 (inner solves of the mixed path)
-  ddc_solve_info* inf = nullptr;
-  int* logpos = nullptr;
-  int set = 0;  // which device row / pinned row of the reductions (0 direct, 1 adjoint)
-  // between the three host steps of an iteration (jd_a, jd_b, jd_c)
-  int p_nm = 0;
-  bool p_shift = false;
-  std::vector<int> p_map;
-  void* p_xnew = nullptr;
-  // history slot k of hx / he in the history precision
-  void* slot(double* base, int k, long long n) const {
-    return reinterpret_cast<char*>(base) + (size_t)k * n * (f32 ? sizeof(float) : sizeof(double));
-  }
-};
-
+// ---------------------------------------------------------------------------
+// Jacobi/DIIS (jacobi_diis.f90) over one system, or the direct and the adjoint
+// one together with one fused L / L* pass per sweep; one molecule or a batch.
+// The iteration itself lives on the device (ddc_solver.cu); the host launches
+// sweeps a little ahead of the device and stops when no molecule runs.
+//
+// Mixed precision: iterative refinement.  Each outer step forms in FP64 the
+// residual r = rhs - L x and the Jacobi increment d = D^-1 r at x; its H-norm
+// is the reference's convergence test (jacobi_diis.f90:143-150), so a molecule
+// stops exactly when its FP64 Jacobi increment is below 10^-iconv.  Otherwise
+// the correction equation L e = r is solved with Jacobi/DIIS on the FP32
+// operator (from e = d, to 1e-4 relative, FP32 history) and x += e.  From the
+// reference or the zero start the first residual (at a start that is never
+// converged) comes from the FP32 operator, and the test runs from the second
+// refinement on.
+// ---------------------------------------------------------------------------
 // DIIS history length: the reference's ndiis (jacobi_diis.f90) for the FP64
 // solves; at most kInnerDiis for the FP32 inner solves of the mixed
-// refinement, whose Jacobi step and extrapolation read the whole history
-// from HBM every iteration (20k workload: 15 instead of 25 entries keeps the
-// 88 / 85 iterations and takes 6 ms off the 190 ms step)
+// refinement, whose kernels read the whole history from HBM every iteration
+// (20k workload: 15 instead of 25 entries keeps the 88 / 85 iterations and
+// took 6 ms off a 190 ms step)
 constexpr int kInnerDiis = 15;
-int jd_ndiis(const ddc_ctx* ctx, bool f32) {
-  return f32 ? std::min(ctx->prm.ndiis, kInnerDiis) : ctx->prm.ndiis;
-}
 
-void jd_begin(ddc_ctx* ctx, JDState& s, const double* rhs, double* x, double tol, int max_iter,
-              const SolveBufs& b, ddc_solve_info* inf, int* logpos, bool f32 = false,
-              int set = 0) {
-  s.set = set;
-  const int ndiis = jd_ndiis(ctx, f32);
-  s.rhs = rhs;
-  s.x = x;
-  s.tol = tol;
-  s.max_iter = max_iter;
-  s.y = b.y;
-  s.hx = b.hx;
-  s.he = b.he;
-  s.xjac = b.xn;
-  s.lenb = ndiis + 1;
-  s.B.assign((size_t)s.lenb * s.lenb, 0.0);
-  s.map.resize(std::max(ndiis, 1));
-  for (int k = 0; k < (int)s.map.size(); k++) s.map[k] = k;
-  s.nmat = 1;
-  s.it = 0;
-  s.restarts = 0;
-  s.rms = 0.0;
-  s.ok = false;
-  s.done = max_iter <= 0;
-  s.f32 = f32;
-  s.inf = inf;
-  s.logpos = logpos;
-}
-
-// One iteration after y = op(x) (jacobi_diis.f90:120-160 with diis
-// :183-230), in three host steps so that two systems solved together share
-// their synchronisations: jd_a launches the Jacobi step with the Gram row
-// and queues the row's copy to pinned memory; jd_b (after a synchronisation)
-// updates the bordered system (makeb), solves it (gjinv) and launches the
-// extrapolation with the increment norm, its copy queued; jd_c (after a
-// synchronisation) reads the norm and applies the stop test.
-double* red_row(ddc_ctx* ctx, int set) { return ctx->red.as<double>() + set * (kMaxHist + 1); }
-double* hred_row(ddc_ctx* ctx, int set) { return ctx->hred + set * (kMaxHist + 1); }
-
-int jd_a(ddc_ctx* ctx, JDState& s) {
-  const long long n = (long long)ctx->nsph * ctx->nylm;
-  const int ndiis = jd_ndiis(ctx, s.f32);
-  const int nblk = reduce_blocks();
-  ++s.it;
-  HistPtrs hist{};
-  double* out = red_row(ctx, s.set);
-  if (ndiis != 0) {
-    const int phys_new = s.map[s.nmat - 1];
-    int nm = s.nmat;
-    std::vector<int> pmap = s.map;
-    const bool shift = s.nmat >= ndiis;
-    if (shift) {  // drop the 10 oldest (jacobi_diis.f90:196-205)
-      std::vector<int> r(s.map.begin() + 10, s.map.end());
-      r.insert(r.end(), s.map.begin(), s.map.begin() + 10);
-      pmap = r;
-      nm = s.nmat - 10;
-    }
-    hist.n = nm - 1;
-    for (int k = 0; k < nm - 1; k++) hist.p[k] = s.slot(s.he, pmap[k], n);
-    void* xnew = s.slot(s.hx, phys_new, n);
-    void* enew = s.slot(s.he, phys_new, n);
-    {
-      StageScope sc(ctx, ST_JACOBI);
-      int jblk = nblk;
-      CK(launch_jacobi_step(ctx->L(), ctx->tb, n, s.rhs, s.y, s.x, xnew, enew, hist,
-                            ctx->partials.as<double>(), nblk, s.f32, &jblk,
-                            ctx->rcount.as<unsigned>(), out));
-    }
-    CK(cudaMemcpyAsync(hred_row(ctx, s.set), out, sizeof(double) * nm, cudaMemcpyDeviceToHost,
-                       ctx->st));
-    s.p_nm = nm;
-    s.p_shift = shift;
-    s.p_map = pmap;
-    s.p_xnew = xnew;
-  } else {
-    hist.n = 0;
-    StageScope sc(ctx, ST_JACOBI);
-    CK(launch_jacobi_step(ctx->L(), ctx->tb, n, s.rhs, s.y, s.x, s.hx, s.he, hist,
-                          ctx->partials.as<double>(), nblk, s.f32, nullptr,
-                          ctx->rcount.as<unsigned>(), out));
-  }
-  return DDC_OK;
-}
-
-int jd_b(ddc_ctx* ctx, JDState& s) {
-  const long long n = (long long)ctx->nsph * ctx->nylm;
-  const int ndiis = jd_ndiis(ctx, s.f32);
-  const int lenb = s.lenb;
-  auto Bm = [&](int j, int k) -> double& { return s.B[(size_t)(k - 1) * lenb + (j - 1)]; };
-  HistPtrs comb{};
-  const void* xj = s.hx;
-  double* out = red_row(ctx, s.set);
-  if (ndiis != 0) {
-    const double* row = hred_row(ctx, s.set);
-    if (s.p_shift) {
-      for (int j = 2; j <= s.nmat - 10; j++)
-        for (int k = 2; k <= s.nmat - 10; k++) Bm(j, k) = Bm(j + 10, k + 10);
-      s.map = s.p_map;
-    }
-    s.nmat = s.p_nm;
-    // makeb (jacobi_diis.f90:232-270)
-    if (s.nmat == 1) {
-      Bm(1, 1) = 0.0;
-      Bm(1, 2) = 1.0;
-      Bm(2, 1) = 1.0;
-      Bm(2, 2) = row[0];
-    } else {
-      Bm(s.nmat + 1, 1) = 1.0;
-      Bm(1, s.nmat + 1) = 1.0;
-      for (int i = 1; i <= s.nmat - 1; i++) {
-        Bm(s.nmat + 1, i + 1) = row[i - 1];
-        Bm(i + 1, s.nmat + 1) = row[i - 1];
-      }
-      Bm(s.nmat + 1, s.nmat + 1) = row[s.nmat - 1];
-    }
-    const int nmat1 = s.nmat + 1;
-    std::vector<double> bloc((size_t)nmat1 * nmat1), cex(nmat1, 0.0);
-    for (int k = 1; k <= nmat1; k++)
-      for (int j = 1; j <= nmat1; j++) bloc[(size_t)(k - 1) * nmat1 + (j - 1)] = Bm(j, k);
-    cex[0] = 1.0;
-    if (gjinv(nmat1, bloc, cex)) {
-      comb.n = s.nmat;
-      for (int k = 0; k < s.nmat; k++) {
-        comb.p[k] = s.slot(s.hx, s.map[k], n);
-        comb.c[k] = cex[k + 1];
-      }
-      s.nmat = s.nmat + 1;
-    } else {  // singular: restart the history (jacobi_diis.f90:214-217)
-      s.nmat = 1;
-      s.restarts++;
-      comb.n = 0;
-    }
-    xj = s.p_xnew;
-  }
-  {
-    StageScope sc(ctx, ST_COMBINE);
-    CK(launch_diis_combine(ctx->L(), ctx->tb, n, comb, xj, s.x, ctx->partials.as<double>(),
-                           reduce_blocks(), s.f32, ctx->rcount.as<unsigned>(), out));
-  }
-  CK(cudaMemcpyAsync(hred_row(ctx, s.set), out, sizeof(double), cudaMemcpyDeviceToHost,
-                     ctx->st));
-  return DDC_OK;
-}
-
-int jd_c(ddc_ctx* ctx, JDState& s) {
-  const double ss = hred_row(ctx, s.set)[0];
-  s.rms = std::sqrt(ss / (double)std::max(ctx->nsph, 1));
-  if (*s.logpos < 256) s.inf->norms[*s.logpos] = s.rms;
-  ++*s.logpos;
-  if (ctx->prm.iprint > 0) printf("  iter=%4d residual norm: %14.4E\n", *s.logpos, s.rms);
-  if (!std::isfinite(s.rms)) {
-    s.done = true;
-    return fail(ctx, DDC_ERR_NUMERIC, "non-finite increment norm");
-  }
-  s.ok = s.rms < s.tol;
-  s.done = s.ok || s.it >= s.max_iter;
-  return DDC_OK;
-}
-
-int jd_step(ddc_ctx* ctx, JDState& s) {
-  CKI(jd_a(ctx, s));
-  CKI(sync(ctx));
-  CKI(jd_b(ctx, s));
-  CKI(sync(ctx));
-  return jd_c(ctx, s);
-}
-
-// FP64 solve: the reference's Jacobi/DIIS on the FP64 operator.
-// Mixed solve: iterative refinement.  Each outer step forms in FP64 the
-// residual r = rhs - L x and the Jacobi increment d = D^-1 r at x; its
-// H-norm is the reference's convergence test (jacobi_diis.f90:143-150), so
-// the solve stops exactly when the FP64 Jacobi increment is below
-// 10^-iconv.  Otherwise the correction equation L e = r is solved with
-// Jacobi/DIIS on the FP32 operator (from e = d, to 1e-4 relative) and x += e.
-// A SolveTask is one such solve as a resumable state; solve_tasks advances
-// one or two of them, one operator application each per round.
-enum OpKind { OP_NONE = 0, OP_F64 = 1, OP_F32 = 2 };
-struct SolveTask {
-  bool adjoint = false, mixed = false;
+struct System {
+  bool adjoint = false;
   const double* rhs = nullptr;
-  double* x = nullptr;
+  double* x = nullptr;               // start in, solution out (device)
+  int* iters = nullptr;              // per molecule (host), or null
   ddc_solve_info* inf = nullptr;
-  SolveBufs b{};
-  double tol = 0.0, t0 = 0.0, last = 0.0;
-  int phase = 0;  // mixed: 0 = FP64 residual at x next, 1 = inner solve running
-  JDState jd;
-  int logpos = 0, its = 0, restarts = 0, budget = 0, outer = 0;
-  bool done = false, ok = false;
-  // mixed, from the reference or the zero start: the first residual (at a
-  // start that is never converged) comes from the FP32 operator, like the
-  // inner iterations; the convergence test runs from the second refinement on
-  bool f32_first = false;
-  int set = 0;  // work-vector set and reduction row (0 direct, 1 adjoint)
 };
 
-void task_begin(ddc_ctx* ctx, SolveTask& t, bool adjoint, const double* rhs, double* x,
-                ddc_solve_info* inf, int set) {
-  t.adjoint = adjoint;
-  t.mixed = ctx->prm.precision == DDC_PREC_MIXED;
-  t.rhs = rhs;
-  t.x = x;
-  t.inf = inf;
-  memset(inf, 0, sizeof(*inf));
-  t.b = solve_bufs(ctx, set);
-  t.set = set;
-  t.tol = std::pow(10.0, -(double)ctx->prm.iconv);
-  t.t0 = now_s();
-  t.phase = 0;
-  t.logpos = t.its = t.restarts = t.outer = 0;
-  t.budget = ctx->prm.max_iter;
-  t.last = 0.0;
-  t.done = t.ok = false;
-  t.f32_first = t.mixed && !ctx->guess_preset &&
-                (ctx->prm.guess == DDC_GUESS_REFERENCE || ctx->prm.guess == DDC_GUESS_ZERO);
-  if (!t.mixed)
-    jd_begin(ctx, t.jd, rhs, x, t.tol, ctx->prm.max_iter, t.b, inf, &t.logpos, false, set);
-  if (!t.mixed && t.jd.done) t.done = true;
-}
+// integer and double state arrays of a system, nmol entries each
+enum { SI_NMAT, SI_STATUS, SI_ITERS, SI_RESTARTS, SI_EXT, SI_MAXK, SI_RUN, SI_ITS, SI_OUTER, SI_RST,
+       SI_UPD, SI_CNT, SI_N };
+enum { SD_NORM, SD_LAST, SD_TOLK, SD_N };
 
-// operator application the task needs next: kind, input, output
-OpKind task_next(const SolveTask& t, const double** in, double** out) {
-  if (t.done) return OP_NONE;
-  if (!t.mixed || t.phase == 1) {
-    *in = t.jd.x;
-    *out = t.jd.y;
-    return t.mixed ? OP_F32 : OP_F64;
+int solver_setup(ddc_ctx* ctx, SolverArgs& a, const System* sys, int ns, bool mixed) {
+  const int nmol = ctx->nmol, nylm = ctx->nylm;
+  memset(&a, 0, sizeof(a));
+  a.nmol = nmol;
+  a.nsph = ctx->nsph;
+  a.nylm = nylm;
+  a.ndiis = mixed ? std::min(ctx->prm.ndiis, kInnerDiis) : ctx->prm.ndiis;
+  a.max_iter = ctx->prm.max_iter;
+  a.tol = std::pow(10.0, -(double)ctx->prm.iconv);
+  a.n_total = (long long)ctx->nsph * nylm;
+  a.chunk = solver_chunk(a.n_total, nmol == 1);
+  for (int l = 0; l <= ctx->prm.lmax; l++) {
+    a.facl[l] = ctx->tb.facl[l];
+    a.hw[l] = 1.0 / (1.0 + l);
   }
-  *in = t.x;
-  *out = t.b.y;
-  return t.f32_first && t.outer == 0 ? OP_F32 : OP_F64;
-}
-
-// the task's next step is a Jacobi/DIIS iteration (FP64 solve, or an inner
-// solve of the mixed refinement)
-bool task_in_jd(const SolveTask& t) { return !t.mixed || t.phase == 1; }
-
-// the task's bookkeeping after a Jacobi/DIIS iteration
-int task_after_jd(ddc_ctx* ctx, SolveTask& t) {
-  if (!t.jd.done) return DDC_OK;
-  if (!t.mixed) {
-    t.done = true;
-    t.ok = t.jd.ok;
-    t.its = t.jd.ok ? t.jd.it : ctx->prm.max_iter;
-    t.restarts += t.jd.restarts;
-    t.last = t.jd.rms;
-    return DDC_OK;
+  if (nmol == 1) {
+    a.nchunk = (int)((a.n_total + a.chunk - 1) / a.chunk);
+    a.nonempty = ctx->nsph > 0;
+  } else {
+    std::vector<int> cfirst(nmol + 1, 0), cmol, sphmol(ctx->nsph);
+    for (int k = 0; k < nmol; k++) {
+      const int n = ctx->h_off[k + 1] - ctx->h_off[k];
+      const int nc = (int)(((long long)n * nylm + a.chunk - 1) / a.chunk);
+      cmol.insert(cmol.end(), nc, k);
+      cfirst[k + 1] = cfirst[k] + nc;
+      a.nonempty += n > 0;
+      std::fill(sphmol.begin() + ctx->h_off[k], sphmol.begin() + ctx->h_off[k + 1], k);
+    }
+    a.nchunk = cfirst[nmol];
+    CK(ctx->b_cmol.ensure(sizeof(int) * std::max(a.nchunk, 1)));
+    CK(ctx->b_cfirst.ensure(sizeof(int) * (nmol + 1)));
+    CK(ctx->b_sphmol.ensure(sizeof(int) * std::max(ctx->nsph, 1)));
+    if (a.nchunk)
+      CK(cudaMemcpyAsync(ctx->b_cmol.p, cmol.data(), sizeof(int) * a.nchunk,
+                         cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaMemcpyAsync(ctx->b_cfirst.p, cfirst.data(), sizeof(int) * (nmol + 1),
+                       cudaMemcpyHostToDevice, ctx->st));
+    if (ctx->nsph)
+      CK(cudaMemcpyAsync(ctx->b_sphmol.p, sphmol.data(), sizeof(int) * ctx->nsph,
+                         cudaMemcpyHostToDevice, ctx->st));
+    CKI(sync(ctx));  // the host vectors go out of scope
+    a.off = ctx->d_off.as<int>();
+    a.cmol = ctx->b_cmol.as<int>();
+    a.cfirst = ctx->b_cfirst.as<int>();
   }
-  const long long n = (long long)ctx->nsph * ctx->nylm;
-  const int done = t.jd.ok ? t.jd.it : t.jd.max_iter;
-  t.its += done;
-  t.budget -= done;
-  t.restarts += t.jd.restarts;
-  CK(launch_axpy(ctx->L(), n, 1.0, t.b.e, t.x));
-  t.phase = 0;
-  if (t.outer >= 64) t.done = true;
+  const int nd = std::max(a.ndiis, 1);
+  CK(ctx->s_int.ensure(sizeof(int) * 2 * (SI_N * (size_t)nmol + 1)));
+  CK(ctx->s_dbl.ensure(sizeof(double) * 2 * SD_N * nmol));
+  CK(ctx->s_slot.ensure(sizeof(int) * 2 * (size_t)nmol * nd));
+  CK(ctx->s_gram.ensure(sizeof(double) * 2 * (size_t)nmol * nd * nd));
+  CK(ctx->s_coef.ensure(sizeof(double) * 2 * (size_t)nmol * kMaxHist));
+  CK(ctx->s_part.ensure(sizeof(double) * 2 * (size_t)std::max(a.nchunk, 1) * (kMaxHist + 1)));
+  if (nmol == 1) CK(ctx->s_log.ensure(sizeof(double) * 2 * (size_t)ctx->prm.max_iter));
+  if (!ctx->hstop) {
+    CK(cudaHostAlloc(&ctx->hstop, sizeof(int) * 4, cudaHostAllocMapped));
+    CK(cudaHostGetDevicePointer(&ctx->dstop, ctx->hstop, 0));
+  }
+  if (!ctx->ev_sweep[0])
+    for (cudaEvent_t& e : ctx->ev_sweep)
+      CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  a.active = ctx->s_int.as<int>() + 2 * SI_N * (size_t)nmol;
+  a.hstop = ctx->dstop;
+  for (int q = 0; q < ns; q++) {
+    SolverSys& s = a.sys[q];
+    int* si = ctx->s_int.as<int>() + (size_t)q * SI_N * nmol;
+    double* sd = ctx->s_dbl.as<double>() + (size_t)q * SD_N * nmol;
+    s.nmat = si + (size_t)SI_NMAT * nmol;
+    s.status = si + (size_t)SI_STATUS * nmol;
+    s.iters = si + (size_t)SI_ITERS * nmol;
+    s.restarts = si + (size_t)SI_RESTARTS * nmol;
+    s.ext = si + (size_t)SI_EXT * nmol;
+    s.maxk = si + (size_t)SI_MAXK * nmol;
+    s.run = si + (size_t)SI_RUN * nmol;
+    s.its = si + (size_t)SI_ITS * nmol;
+    s.outer = si + (size_t)SI_OUTER * nmol;
+    s.rst = si + (size_t)SI_RST * nmol;
+    s.upd = si + (size_t)SI_UPD * nmol;
+    s.cnt = reinterpret_cast<unsigned*>(si + (size_t)SI_CNT * nmol);
+    s.norm = sd + (size_t)SD_NORM * nmol;
+    s.last = sd + (size_t)SD_LAST * nmol;
+    s.tolk = sd + (size_t)SD_TOLK * nmol;
+    s.slot = ctx->s_slot.as<int>() + (size_t)q * nmol * nd;
+    s.gram = ctx->s_gram.as<double>() + (size_t)q * nmol * nd * nd;
+    s.coef = ctx->s_coef.as<double>() + (size_t)q * nmol * kMaxHist;
+    s.part = ctx->s_part.as<double>() + (size_t)q * std::max(a.nchunk, 1) * (kMaxHist + 1);
+    s.log = nmol == 1 ? ctx->s_log.as<double>() + (size_t)q * ctx->prm.max_iter : nullptr;
+    s.hx = (q ? ctx->hist_x2 : ctx->hist_x).p;
+    s.he = (q ? ctx->hist_e2 : ctx->hist_e).p;
+    s.y = (q ? ctx->y2 : ctx->y).as<double>();
+    s.orhs = sys[q].rhs;
+    s.ox = sys[q].x;
+    s.r = mixed ? (q ? ctx->rres2 : ctx->rres).as<double>() : nullptr;
+    s.rhs = mixed ? s.r : s.orhs;
+    s.x = mixed ? (q ? ctx->eres2 : ctx->eres).as<double>() : s.ox;
+  }
   return DDC_OK;
 }
 
-int task_after(ddc_ctx* ctx, SolveTask& t) {
-  if (task_in_jd(t)) {
-    CKI(jd_step(ctx, t.jd));
-    return task_after_jd(ctx, t);
-  }
-  const long long n = (long long)ctx->nsph * ctx->nylm;
-  // phase 0: y = L x in FP64 is ready
-  ++t.outer;
-  {
-    StageScope sc(ctx, ST_JACOBI);
-    CK(launch_residual(ctx->L(), ctx->tb, n, t.rhs, t.b.y, t.x, t.b.r, t.b.d,
-                       ctx->partials.as<double>(), reduce_blocks()));
-  }
-  double ss = 0.0;
-  CKI(reduce_to_host(ctx, 1, &ss));
-  t.last = std::sqrt(ss / (double)std::max(ctx->nsph, 1));
-  const bool f32_res = t.f32_first && t.outer == 1;
-  if (ctx->prm.iprint > 0)
-    printf("  refinement %d: %s increment norm %14.4E\n", t.outer, f32_res ? "FP32" : "FP64",
-           t.last);
-  if (!std::isfinite(t.last)) {
-    t.done = true;
-    return fail(ctx, DDC_ERR_NUMERIC, "non-finite increment norm");
-  }
-  if (t.last < t.tol && !f32_res) {
-    t.done = t.ok = true;
-    return DDC_OK;
-  }
-  if (t.budget <= 0) {
-    t.done = true;
-    return DDC_OK;
-  }
-  // correction: (D + O32) e = r from e = D^-1 r
-  CK(cudaMemcpyAsync(t.b.e, t.b.d, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->st));
-  // Each inner solve reduces its increment by rho (floor 0.3 tol).  Every
-  // restart of the inner DIIS costs about ten iterations before the
-  // extrapolation has a subspace again, so the split between the two inner
-  // solves matters: at the 20,000-sphere workload rho = 1e-5 takes 88 / 86
-  // iterations, 3e-5 86 / 80, 1e-4 80 / 79 (Esolv 2e-10 from the FP64
-  // oracle; at most 3.9e-10 over eight smaller molecules, as with 1e-5), and
-  // 3e-4 84 / 71 but 1.7e-9 on the 600-sphere configuration.
-  // The correction is wanted to 1e-4 relative: FP32 history vectors suffice.
-  const double rho = 1e-4;
-  const double itol = std::max(rho * t.last, 0.3 * t.tol);
-  jd_begin(ctx, t.jd, t.b.r, t.b.e, itol, t.budget, t.b, t.inf, &t.logpos, true, t.set);
-  t.phase = 1;
-  return DDC_OK;
-}
-
-int op_single(ddc_ctx* ctx, OpKind k, bool adjoint, const double* in, double* out) {
-  if (k == OP_F64) return adjoint ? op_lstarx(ctx, in, out) : op_lx(ctx, in, out);
+int op_single(ddc_ctx* ctx, bool f32, bool adjoint, const double* in, double* out) {
+  if (!f32) return adjoint ? op_lstarx(ctx, in, out) : op_lx(ctx, in, out);
   return adjoint ? op_lstarx_f32(ctx, in, out) : op_lx_f32(ctx, in, out);
 }
+// y = O x for the systems [q0, q1), skipping the molecules whose state (mask)
+// is not zero in every one of them; outer: at the outer iterate
+int solver_op(ddc_ctx* ctx, const SolverArgs& a, const System* sys, int q0, int q1, bool f32,
+              bool outer) {
+  auto mask = [&](int q) { return outer ? a.sys[q].run : a.sys[q].status; };
+  auto in = [&](int q) { return outer ? a.sys[q].ox : a.sys[q].x; };
+  auto out = [&](int q) { return const_cast<double*>(a.sys[q].y); };
+  ctx->sweep = SweepMask{a.cmol ? ctx->b_sphmol.as<int>() : nullptr, mask(q0),
+                         q1 - q0 == 2 ? mask(q0 + 1) : nullptr};
+  int rc;
+  if (q1 - q0 == 2) {
+    const int d = sys[0].adjoint ? 1 : 0, j = 1 - d;
+    rc = f32 ? op_pair_f32(ctx, in(d), out(d), in(j), out(j))
+             : op_pair(ctx, in(d), out(d), in(j), out(j));
+  } else {
+    rc = op_single(ctx, f32, sys[q0].adjoint, in(q0), out(q0));
+  }
+  ctx->sweep = SweepMask{};
+  return rc;
+}
 
-// Advance the tasks in lockstep.  When a direct and an adjoint task need an
-// operator of the same precision in the same round, both come from one
-// fused pass over the triples (op_pair / op_pair_f32).
-int solve_tasks(ddc_ctx* ctx, SolveTask* t, int nt) {
-  for (;;) {
-    const double* in[2] = {nullptr, nullptr};
-    double* out[2] = {nullptr, nullptr};
-    OpKind k[2] = {OP_NONE, OP_NONE};
-    int active = 0;
-    for (int q = 0; q < nt; q++) {
-      k[q] = task_next(t[q], &in[q], &out[q]);
-      if (k[q] != OP_NONE) active++;
+// Sweeps until every molecule of every system has stopped.  The device
+// reports the sweep in which a system's last molecule stopped through mapped
+// memory; the host reads it `ahead` sweeps later, so that it stays ahead of
+// the device, and then leaves the system out (or ends).  A stopped molecule's
+// blocks return at once, so the sweeps launched too many are cheap; the
+// decision depends on finished sweeps alone, so the launches of a solve are
+// always the same.
+int solver_sweeps(ddc_ctx* ctx, SolverArgs& a, const System* sys, int q0, int q1, bool f32) {
+  // one sweep ahead where a sweep takes a few hundred microseconds, else two
+  const int ahead = ctx->ntri * ctx->nylm > 200000000LL ? 1 : 2;
+  constexpr int NE = sizeof(ctx->ev_sweep) / sizeof(ctx->ev_sweep[0]);
+  volatile int* stop = ctx->hstop;
+  stop[0] = stop[1] = 0;
+  for (int it = 1; q0 < q1; it++) {
+    CKI(solver_op(ctx, a, sys, q0, q1, f32, false));
+    a.first = q0;
+    a.sweep = it;
+    {
+      StageScope sc(ctx, ST_JACOBI);
+      CK(launch_solver_step(ctx->L(), a, q1 - q0, f32, 0));
     }
-    if (!active) break;
-    // A task that needs an FP64 step (mixed refinement) while the other
-    // runs FP32 inner iterations waits a round: the other reaches its own
-    // FP64 step or finishes, and the FP64 steps then share a fused pass.
-    // This only reorders the tasks' rounds; each keeps its own arithmetic.
-    if (nt == 2 && k[0] != OP_NONE && k[1] != OP_NONE && k[0] != k[1]) {
-      const int wait = k[0] == OP_F64 ? 0 : 1;
-      k[wait] = OP_NONE;
+    {
+      StageScope sc(ctx, ST_COMBINE);
+      CK(launch_solver_step(ctx->L(), a, q1 - q0, f32, 1));
     }
-    if (nt == 2 && k[0] != OP_NONE && k[0] == k[1] && t[0].adjoint != t[1].adjoint) {
-      const int dq = t[0].adjoint ? 1 : 0, aq = 1 - dq;
-      if (k[0] == OP_F64) CKI(op_pair(ctx, in[dq], out[dq], in[aq], out[aq]));
-      else CKI(op_pair_f32(ctx, in[dq], out[dq], in[aq], out[aq]));
-    } else {
-      for (int q = 0; q < nt; q++)
-        if (k[q] != OP_NONE) CKI(op_single(ctx, k[q], t[q].adjoint, in[q], out[q]));
+    CK(cudaEventRecord(ctx->ev_sweep[it % NE], ctx->st));
+    const int done = it - ahead;
+    if (done < 1) continue;
+    CK(cudaEventSynchronize(ctx->ev_sweep[done % NE]));
+    auto stopped = [&](int q) { return stop[q] != 0 && stop[q] <= done; };
+    while (q0 < q1 && stopped(q0)) q0++;
+    while (q1 > q0 && stopped(q1 - 1)) q1--;
+    if (done > ctx->prm.max_iter)  // every molecule's budget is spent by now
+      return fail(ctx, DDC_ERR_STATE, "the solver did not stop within its budget");
+  }
+  a.first = 0;
+  return DDC_OK;
+}
+
+// increment norms of iterations [from[q], to[q]) (iprint), interleaved as the
+// systems iterate
+int print_log(ddc_ctx* ctx, const SolverArgs& a, int ns, const int* from, const int* to) {
+  std::vector<double> log[2];
+  int most = 0;
+  for (int q = 0; q < ns; q++) {
+    log[q].resize(std::max(to[q] - from[q], 0));
+    most = std::max(most, (int)log[q].size());
+    if (!log[q].empty())
+      CK(cudaMemcpyAsync(log[q].data(), a.sys[q].log + from[q], sizeof(double) * log[q].size(),
+                         cudaMemcpyDeviceToHost, ctx->st));
+  }
+  CKI(sync(ctx));
+  for (int i = 0; i < most; i++)
+    for (int q = 0; q < ns; q++)
+      if (i < (int)log[q].size())
+        printf("  iter=%4d residual norm: %14.4E\n", from[q] + i + 1, log[q][i]);
+  return DDC_OK;
+}
+
+// Solves the systems; reports go to sys[q].inf and .iters.  One molecule that
+// does not converge: DDC_ERR_NOCONV with the last iterate in x; a non-finite
+// increment: DDC_ERR_NUMERIC.
+int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
+  const double t0 = now_s();
+  const bool mixed = ctx->prm.precision == DDC_PREC_MIXED;
+  const bool one = ctx->nmol == 1 && !ctx->batch;
+  const bool log = ctx->prm.iprint > 0 && one;
+  const int nmol = ctx->nmol;
+  if (ctx->batch && ctx->prm.ndiis == 0)
+    return fail(ctx, DDC_ERR_UNSUPPORTED, "batched solves need DIIS");
+  for (int q = 0; q < ns; q++) memset(sys[q].inf, 0, sizeof(*sys[q].inf));
+  SolverArgs a;
+  CKI(solver_setup(ctx, a, sys, ns, mixed));
+  CK(launch_solver_begin(ctx->L(), a, ns, mixed));
+  std::vector<int> si(2 * (SI_N * (size_t)nmol + 1));
+  std::vector<double> sd(2 * SD_N * (size_t)nmol);
+  auto read_state = [&]() -> int {
+    CK(cudaMemcpyAsync(si.data(), ctx->s_int.p, sizeof(int) * si.size(), cudaMemcpyDeviceToHost,
+                       ctx->st));
+    CK(cudaMemcpyAsync(sd.data(), ctx->s_dbl.p, sizeof(double) * sd.size(),
+                       cudaMemcpyDeviceToHost, ctx->st));
+    return sync(ctx);
+  };
+  auto I = [&](int q, int w, int k) { return si[((size_t)q * SI_N + w) * nmol + k]; };
+  auto D = [&](int q, int w, int k) { return sd[((size_t)q * SD_N + w) * nmol + k]; };
+  if (!mixed) {
+    if (a.nonempty) CKI(solver_sweeps(ctx, a, sys, 0, ns, false));
+    if (log) {
+      CKI(read_state());
+      const int from[2] = {0, 0}, to[2] = {I(0, SI_ITERS, 0), ns > 1 ? I(1, SI_ITERS, 0) : 0};
+      CKI(print_log(ctx, a, ns, from, to));
     }
-    if (nt == 2 && k[0] != OP_NONE && k[1] != OP_NONE && task_in_jd(t[0]) && task_in_jd(t[1])) {
-      // both systems take a Jacobi/DIIS iteration: one synchronisation for
-      // both Gram rows and one for both increment norms (each system keeps
-      // its own state, history and reduction row)
-      CKI(jd_a(ctx, t[0].jd));
-      CKI(jd_a(ctx, t[1].jd));
+  } else {
+    const bool f32_first = !ctx->guess_preset && (ctx->prm.guess == DDC_GUESS_REFERENCE ||
+                                                   ctx->prm.guess == DDC_GUESS_ZERO);
+    int printed[2] = {0, 0};
+    for (int round = 0; round < 64 && a.nonempty; round++) {
+      const bool f32_res = f32_first && round == 0;
+      CKI(solver_op(ctx, a, sys, 0, ns, f32_res, true));
+      {
+        StageScope sc(ctx, ST_JACOBI);
+        CK(launch_solver_residual(ctx->L(), a, ns, f32_res));
+      }
+      CK(cudaMemcpyAsync(ctx->hstop + 2, a.active, sizeof(int) * 2, cudaMemcpyDeviceToHost,
+                         ctx->st));
       CKI(sync(ctx));
-      CKI(jd_b(ctx, t[0].jd));
-      CKI(jd_b(ctx, t[1].jd));
-      CKI(sync(ctx));
-      CKI(jd_c(ctx, t[0].jd));
-      CKI(jd_c(ctx, t[1].jd));
-      CKI(task_after_jd(ctx, t[0]));
-      CKI(task_after_jd(ctx, t[1]));
-    } else {
-      for (int q = 0; q < nt; q++)
-        if (k[q] != OP_NONE) CKI(task_after(ctx, t[q]));
+      if (log) {
+        CKI(read_state());
+        for (int q = 0; q < ns; q++)
+          if (I(q, SI_OUTER, 0) == round + 1)
+            printf("  refinement %d: %s increment norm %14.4E\n", round + 1,
+                   f32_res ? "FP32" : "FP64", D(q, SD_LAST, 0));
+      }
+      const bool run0 = ctx->hstop[2] != 0, run1 = ns > 1 && ctx->hstop[3] != 0;
+      if (!run0 && !run1) break;
+      // the systems that have molecules left
+      CKI(solver_sweeps(ctx, a, sys, run0 ? 0 : 1, run1 ? 2 : 1, true));
+      CK(launch_solver_update(ctx->L(), a, ns));
+      if (log) {
+        CKI(read_state());
+        const int to[2] = {I(0, SI_ITS, 0), ns > 1 ? I(1, SI_ITS, 0) : 0};
+        CKI(print_log(ctx, a, ns, printed, to));
+        printed[0] = to[0];
+        printed[1] = to[1];
+      }
     }
   }
+  CKI(read_state());
   int rc = DDC_OK;
-  for (int q = 0; q < nt; q++) {
-    ddc_solve_info* inf = t[q].inf;
-    inf->iterations = t[q].its;
-    inf->refinements = t[q].mixed ? t[q].outer : 0;
-    inf->converged = t[q].ok ? 1 : 0;
-    inf->diis_restarts = t[q].restarts;
-    inf->final_norm = t[q].last;
-    inf->seconds = now_s() - t[q].t0;
-    if (!t[q].ok && rc == DDC_OK)
-      rc = fail(ctx, DDC_ERR_NOCONV, t[q].adjoint ? "adjoint ddCOSMO did not converge"
-                                                  : "ddCOSMO did not converge");
+  for (int q = 0; q < ns; q++) {
+    ddc_solve_info& f = *sys[q].inf;
+    int maxit = 0, maxout = 0, nfail = 0, restarts = 0;
+    double worst = 0.0;
+    bool finite = true;
+    for (int k = 0; k < nmol; k++) {
+      const bool empty = one ? ctx->nsph == 0 : ctx->h_off[k + 1] == ctx->h_off[k];
+      const int state = I(q, mixed ? SI_RUN : SI_STATUS, k);
+      const int it = mixed ? I(q, SI_ITS, k) : I(q, SI_ITERS, k);
+      if (sys[q].iters) sys[q].iters[k] = it;
+      maxit = std::max(maxit, it);
+      maxout = std::max(maxout, mixed ? I(q, SI_OUTER, k) : 0);
+      restarts += mixed ? I(q, SI_RST, k) : I(q, SI_RESTARTS, k);
+      if (state != 1 && !empty) nfail++;
+      if (state == 3) finite = false;
+      if (!empty) worst = std::max(worst, D(q, mixed ? SD_LAST : SD_NORM, k));
+    }
+    f.iterations = maxit;
+    f.refinements = maxout;
+    f.converged = nfail == 0;
+    f.diis_restarts = restarts;
+    f.final_norm = worst;
+    if (one) {
+      const int n = std::min({maxit, 256, ctx->prm.max_iter});
+      if (n > 0)
+        CK(cudaMemcpyAsync(f.norms, a.sys[q].log, sizeof(double) * n, cudaMemcpyDeviceToHost,
+                           ctx->st));
+    }
+    if (rc != DDC_OK || !nfail) continue;
+    if (!one)
+      rc = fail(ctx, DDC_ERR_NOCONV, std::to_string(nfail) + " molecule(s) did not converge" +
+                                         (sys[q].adjoint ? " (adjoint)" : ""));
+    else if (!finite)
+      rc = fail(ctx, DDC_ERR_NUMERIC, "non-finite increment norm");
+    else
+      rc = fail(ctx, DDC_ERR_NOCONV, sys[q].adjoint ? "adjoint ddCOSMO did not converge"
+                                                    : "ddCOSMO did not converge");
   }
+  CKI(sync(ctx));
+  for (int q = 0; q < ns; q++) sys[q].inf->seconds = now_s() - t0;
   return rc;
 }
 
 int solve(ddc_ctx* ctx, bool adjoint, const double* rhs, double* x, ddc_solve_info* info) {
   ddc_solve_info loc{};
-  SolveTask t;
-  task_begin(ctx, t, adjoint, rhs, x, info ? info : &loc, 0);
-  return solve_tasks(ctx, &t, 1);
+  System s;
+  s.adjoint = adjoint;
+  s.rhs = rhs;
+  s.x = x;
+  s.inf = info ? info : &loc;
+  return solve_systems(ctx, &s, 1);
 }
 
 int need_ready(ddc_ctx* ctx) {
@@ -1486,397 +1338,6 @@ int forces_dev(ddc_ctx* ctx, const double* phi, const double* sigma, const doubl
 
 }  // namespace
 
-// Batched Jacobi/DIIS: every molecule runs the reference's algorithm on its
-// own segment of the concatenated vectors (own history, Gram matrix,
-// restarts and convergence test); per iteration two kernels over element
-// chunks do the Jacobi step and Gram row, then the bordered solve (the
-// molecule's last chunk), the extrapolation and the norm for all molecules;
-// a stopped molecule's chunks return at once.  iters receives the
-// per-molecule iteration counts.
-// One system of a batched solve: its right-hand side, iterate, operator
-// output and per-molecule Jacobi/DIIS state on the device.  The state arrays
-// of the two systems of a paired solve sit side by side in the same buffers
-// (set 0, set 1).
-struct BatchSys {
-  bool adjoint = false;
-  const double* rhs = nullptr;
-  double* x = nullptr;
-  double* y = nullptr;
-  BatchState bs{};
-  int* iters = nullptr;
-  ddc_solve_info* inf = nullptr;
-};
-
-// f32: an inner solve of the mixed refinement (FP32 history of at most
-// kInnerDiis vectors); status0 (host, or null: every non-empty molecule
-// runs), tolk and maxk (host, or null: the parameters' tolerance and budget)
-// give the molecules' starting status, tolerance and iteration budget.
-int batch_setup(ddc_ctx* ctx, BatchSys& b, bool adjoint, const double* rhs, double* x,
-                int* iters, ddc_solve_info* inf, int set, bool f32 = false,
-                const int* status0 = nullptr, const double* tolk = nullptr,
-                const int* maxk = nullptr) {
-  const int nmol = ctx->nmol;
-  const int nd = std::max(f32 ? std::min(ctx->prm.ndiis, kInnerDiis) : ctx->prm.ndiis, 11);
-  if (ctx->prm.ndiis == 0) return fail(ctx, DDC_ERR_UNSUPPORTED, "batched solves need DIIS");
-  std::vector<int> nmat(nmol, 1), slot((size_t)nmol * nd);
-  for (int k = 0; k < nmol; k++)
-    for (int j = 0; j < nd; j++) slot[(size_t)k * nd + j] = j;
-  std::vector<int> status(nmol, 0);
-  for (int k = 0; k < nmol; k++)
-    if (ctx->h_off[k + 1] == ctx->h_off[k]) status[k] = 1;  // empty molecule
-    else if (status0) status[k] = status0[k];
-  const size_t lenb = nd + 1, lb2 = lenb * lenb;
-  // room for both sets
-  CK(ctx->b_nmat.ensure(sizeof(int) * 2 * nmol));
-  CK(ctx->b_slot.ensure(sizeof(int) * 2 * nmol * nd));
-  CK(ctx->b_B.ensure(sizeof(double) * 2 * nmol * lb2));
-  CK(ctx->b_status.ensure(sizeof(int) * 2 * nmol));
-  CK(ctx->b_iters.ensure(sizeof(int) * 2 * nmol));
-  CK(ctx->b_restarts.ensure(sizeof(int) * 2 * nmol));
-  CK(ctx->b_norm.ensure(sizeof(double) * 2 * nmol));
-  // element chunks of each molecule (the same for both sets)
-  std::vector<int> cfirst(nmol + 1, 0), cmol;
-  for (int k = 0; k < nmol; k++) {
-    const long long len = (long long)(ctx->h_off[k + 1] - ctx->h_off[k]) * ctx->nylm;
-    const int nc = (int)((len + kBatchChunk - 1) / kBatchChunk);
-    for (int c = 0; c < nc; c++) cmol.push_back(k);
-    cfirst[k + 1] = cfirst[k] + nc;
-  }
-  const int nchunk = cfirst[nmol];
-  CK(ctx->b_cmol.ensure(sizeof(int) * std::max(nchunk, 1)));
-  CK(ctx->b_cfirst.ensure(sizeof(int) * (nmol + 1)));
-  CK(ctx->b_part.ensure(sizeof(double) * 2 * (size_t)std::max(nchunk, 1) * (kMaxHist + 1)));
-  CK(ctx->b_cnt.ensure(sizeof(unsigned) * 2 * nmol));
-  CK(ctx->b_coef.ensure(sizeof(double) * 2 * (size_t)nmol * kMaxHist));
-  CK(ctx->b_ext.ensure(sizeof(int) * 2 * nmol));
-  BatchState& bs = b.bs;
-  bs.nchunk = nchunk;
-  bs.cmol = ctx->b_cmol.as<int>();
-  bs.cfirst = ctx->b_cfirst.as<int>();
-  bs.part = ctx->b_part.as<double>() + (size_t)set * std::max(nchunk, 1) * (kMaxHist + 1);
-  bs.cnt = ctx->b_cnt.as<unsigned>() + (size_t)set * nmol;
-  bs.coef = ctx->b_coef.as<double>() + (size_t)set * nmol * kMaxHist;
-  bs.ext = ctx->b_ext.as<int>() + (size_t)set * nmol;
-  if (nchunk)
-    CK(cudaMemcpyAsync(ctx->b_cmol.p, cmol.data(), sizeof(int) * nchunk, cudaMemcpyHostToDevice,
-                       ctx->st));
-  CK(cudaMemcpyAsync(ctx->b_cfirst.p, cfirst.data(), sizeof(int) * (nmol + 1),
-                     cudaMemcpyHostToDevice, ctx->st));
-  CK(cudaMemsetAsync(bs.cnt, 0, sizeof(unsigned) * nmol, ctx->st));
-  {
-    std::vector<int> sphmol(ctx->nsph);
-    for (int k = 0; k < nmol; k++)
-      for (int i = ctx->h_off[k]; i < ctx->h_off[k + 1]; i++) sphmol[i] = k;
-    CK(ctx->b_sphmol.ensure(sizeof(int) * std::max(ctx->nsph, 1)));
-    CK(cudaMemcpyAsync(ctx->b_sphmol.p, sphmol.data(), sizeof(int) * ctx->nsph,
-                       cudaMemcpyHostToDevice, ctx->st));
-  }
-  bs.nmol = nmol;
-  bs.ndiis = nd;
-  bs.max_iter = ctx->prm.max_iter;
-  bs.tol = std::pow(10.0, -(double)ctx->prm.iconv);
-  bs.n_total = (long long)ctx->nsph * ctx->nylm;
-  bs.off = ctx->d_off.as<int>();
-  bs.nmat = ctx->b_nmat.as<int>() + (size_t)set * nmol;
-  bs.slot = ctx->b_slot.as<int>() + (size_t)set * nmol * nd;
-  bs.B = ctx->b_B.as<double>() + (size_t)set * nmol * lb2;
-  bs.status = ctx->b_status.as<int>() + (size_t)set * nmol;
-  bs.iters = ctx->b_iters.as<int>() + (size_t)set * nmol;
-  bs.restarts = ctx->b_restarts.as<int>() + (size_t)set * nmol;
-  bs.norm = ctx->b_norm.as<double>() + (size_t)set * nmol;
-  const SolveBufs sb = solve_bufs(ctx, set);
-  bs.hx = sb.hx;
-  bs.he = sb.he;
-  bs.f32 = f32 ? 1 : 0;
-  bs.tolk = nullptr;
-  bs.maxk = nullptr;
-  if (tolk) {
-    CK(ctx->b_tolk.ensure(sizeof(double) * 2 * nmol));
-    double* dt = ctx->b_tolk.as<double>() + (size_t)set * nmol;
-    CK(cudaMemcpyAsync(dt, tolk, sizeof(double) * nmol, cudaMemcpyHostToDevice, ctx->st));
-    bs.tolk = dt;
-  }
-  if (maxk) {
-    CK(ctx->b_maxk.ensure(sizeof(int) * 2 * nmol));
-    int* dm = ctx->b_maxk.as<int>() + (size_t)set * nmol;
-    CK(cudaMemcpyAsync(dm, maxk, sizeof(int) * nmol, cudaMemcpyHostToDevice, ctx->st));
-    bs.maxk = dm;
-  }
-  CK(cudaMemcpyAsync(bs.nmat, nmat.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice, ctx->st));
-  CK(cudaMemcpyAsync(bs.slot, slot.data(), sizeof(int) * nmol * nd, cudaMemcpyHostToDevice,
-                     ctx->st));
-  CK(cudaMemsetAsync(bs.B, 0, sizeof(double) * nmol * lb2, ctx->st));
-  CK(cudaMemcpyAsync(bs.status, status.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice,
-                     ctx->st));
-  CK(cudaMemsetAsync(bs.iters, 0, sizeof(int) * nmol, ctx->st));
-  CK(cudaMemsetAsync(bs.restarts, 0, sizeof(int) * nmol, ctx->st));
-  b.adjoint = adjoint;
-  b.rhs = rhs;
-  b.x = x;
-  b.y = sb.y;
-  b.iters = iters;
-  b.inf = inf;
-  // the host copy of status must not be read before these copies land
-  CKI(sync(ctx));
-  return DDC_OK;
-}
-
-// Copies one system's per-molecule results back and fills its report.
-int batch_finish(ddc_ctx* ctx, const BatchSys& b, double t0) {
-  const int nmol = ctx->nmol;
-  std::vector<int> status(nmol), its(nmol), rst(nmol);
-  std::vector<double> nrm(nmol);
-  CK(cudaMemcpyAsync(status.data(), b.bs.status, sizeof(int) * nmol, cudaMemcpyDeviceToHost,
-                     ctx->st));
-  CK(cudaMemcpyAsync(its.data(), b.bs.iters, sizeof(int) * nmol, cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaMemcpyAsync(rst.data(), b.bs.restarts, sizeof(int) * nmol, cudaMemcpyDeviceToHost,
-                     ctx->st));
-  CK(cudaMemcpyAsync(nrm.data(), b.bs.norm, sizeof(double) * nmol, cudaMemcpyDeviceToHost,
-                     ctx->st));
-  CKI(sync(ctx));
-  int maxit = 0, nfail = 0, restarts = 0;
-  double worst = 0.0;
-  for (int k = 0; k < nmol; k++) {
-    if (b.iters) b.iters[k] = its[k];
-    maxit = std::max(maxit, its[k]);
-    restarts += rst[k];
-    if (status[k] != 1) nfail++;
-    if (ctx->h_off[k + 1] > ctx->h_off[k]) worst = std::max(worst, nrm[k]);
-  }
-  if (b.inf) {
-    memset(b.inf, 0, sizeof(*b.inf));
-    b.inf->iterations = maxit;
-    b.inf->converged = nfail == 0;
-    b.inf->diis_restarts = restarts;
-    b.inf->final_norm = worst;
-    b.inf->seconds = now_s() - t0;
-  }
-  if (nfail)
-    return fail(ctx, DDC_ERR_NOCONV,
-                std::to_string(nfail) + " molecule(s) did not converge" +
-                    (b.adjoint ? " (adjoint)" : ""));
-  return DDC_OK;
-}
-
-// Batched Jacobi/DIIS over one system, or over a direct and an adjoint
-// system together (one fused L / L* pass per sweep).  A CUDA graph of
-// `check` sweeps (operator kernels + the fused per-molecule DIIS kernels)
-// is captured once and replayed until every molecule of every system has
-// stopped; a stopped molecule's DIIS block returns at once, so extra sweeps
-// are harmless.
-int batch_sweeps(ddc_ctx* ctx, BatchSys* sys, int ns) {
-  const int nmol = ctx->nmol;
-  const bool f32 = sys[0].bs.f32 != 0;
-  const int check = 4;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  CK(cudaStreamSynchronize(ctx->st));
-  ctx->capturing = true;
-  // the sweeps skip the spheres of molecules whose systems have all stopped
-  ctx->sweep = SweepMask{ctx->b_sphmol.as<int>(), sys[0].bs.status,
-                         ns == 2 ? sys[1].bs.status : nullptr};
-  cudaError_t ce = cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal);
-  int orc = DDC_OK;
-  if (ce == cudaSuccess) {
-    for (int r = 0; r < check && orc == DDC_OK; r++) {
-      if (ns == 2) {
-        const int dq = sys[0].adjoint ? 1 : 0, aq = 1 - dq;
-        orc = f32 ? op_pair_f32(ctx, sys[dq].x, sys[dq].y, sys[aq].x, sys[aq].y)
-                  : op_pair(ctx, sys[dq].x, sys[dq].y, sys[aq].x, sys[aq].y);
-      } else {
-        orc = op_single(ctx, f32 ? OP_F32 : OP_F64, sys[0].adjoint, sys[0].x, sys[0].y);
-      }
-      for (int q = 0; q < ns && orc == DDC_OK; q++)
-        if (launch_batch_diis(ctx->L(), ctx->tb, sys[q].bs, sys[q].rhs, sys[q].y, sys[q].x) !=
-            cudaSuccess)
-          orc = DDC_ERR_CUDA;
-    }
-    cudaError_t ee = cudaStreamEndCapture(ctx->st, &graph);
-    if (ce == cudaSuccess) ce = ee;
-  }
-  ctx->capturing = false;
-  ctx->sweep = SweepMask{};
-  if (orc != DDC_OK) {
-    if (graph) cudaGraphDestroy(graph);
-    cudaGetLastError();
-    return orc;
-  }
-  CK(ce);
-  CK(cudaGraphInstantiate(&exec, graph, 0));
-  std::vector<int> status(nmol);
-  int it = 0, active = 1;
-  cudaError_t ge = cudaSuccess;
-  while (it < ctx->prm.max_iter && active > 0) {
-    {
-      StageScope sc(ctx, ST_COMBINE);
-      ge = cudaGraphLaunch(exec, ctx->st);
-    }
-    if (ge != cudaSuccess) break;
-    it += check;
-    active = 0;
-    for (int q = 0; q < ns; q++) {
-      CK(cudaMemcpyAsync(status.data(), sys[q].bs.status, sizeof(int) * nmol,
-                         cudaMemcpyDeviceToHost, ctx->st));
-      CKI(sync(ctx));
-      for (int k = 0; k < nmol; k++) active += status[k] == 0;
-    }
-  }
-  cudaGraphExecDestroy(exec);
-  cudaGraphDestroy(graph);
-  CK(ge);
-  return DDC_OK;
-}
-
-int batch_run(ddc_ctx* ctx, BatchSys* sys, int ns) {
-  const double t0 = now_s();
-  CKI(batch_sweeps(ctx, sys, ns));
-  int rc = DDC_OK;
-  for (int q = 0; q < ns; q++) {
-    const int r = batch_finish(ctx, sys[q], t0);
-    if (r != DDC_OK && rc == DDC_OK) rc = r;
-  }
-  return rc;
-}
-
-// Mixed-precision batched solve: the single-molecule refinement (FP64
-// residual and convergence test, inner FP32 Jacobi/DIIS solve of the
-// correction to rho = 1e-4 of its increment, x += e) with every molecule on
-// its own schedule, the molecules in lockstep per phase: one FP64 operator
-// pass for all molecules still refining (converged ones are skipped), the
-// batched residual with per-molecule norms, then one batched inner solve
-// whose molecules each carry their own tolerance and remaining budget.
-// sys[q].rhs / .x are the systems' right-hand sides and iterates.
-int batch_run_mixed(ddc_ctx* ctx, BatchSys* sys, int ns) {
-  const double t0 = now_s();
-  const int nmol = ctx->nmol;
-  const double tol = std::pow(10.0, -(double)ctx->prm.iconv);
-  const bool f32_first = !ctx->guess_preset && (ctx->prm.guess == DDC_GUESS_REFERENCE ||
-                                                 ctx->prm.guess == DDC_GUESS_ZERO);
-  CK(ctx->b_run.ensure(sizeof(int) * 2 * nmol));
-  CK(ctx->b_upd.ensure(sizeof(int) * 2 * nmol));
-  CK(ctx->b_onorm.ensure(sizeof(double) * 2 * nmol));
-  // per system and molecule: outer status (0 refining, 1 converged, 2 budget
-  // spent, 3 non-finite), iterations, refinements, restarts, last norm
-  std::vector<int> run(2 * nmol, 0), its(2 * nmol, 0), outer(2 * nmol, 0), rst(2 * nmol, 0);
-  std::vector<double> last(2 * nmol, 0.0);
-  for (int q = 0; q < ns; q++)
-    for (int k = 0; k < nmol; k++)
-      if (ctx->h_off[k + 1] == ctx->h_off[k]) run[q * nmol + k] = 1;
-  int* drun = ctx->b_run.as<int>();
-  int* dupd = ctx->b_upd.as<int>();
-  double* dnorm = ctx->b_onorm.as<double>();
-  BatchSys in[2];  // the inner systems: L e = r from e = d
-  for (int round = 0; round < 64; round++) {
-    int nrun = 0;
-    for (int q = 0; q < ns; q++)
-      for (int k = 0; k < nmol; k++) nrun += run[q * nmol + k] == 0;
-    if (!nrun) break;
-    CK(cudaMemcpyAsync(drun, run.data(), sizeof(int) * 2 * nmol, cudaMemcpyHostToDevice, ctx->st));
-    // y = L x for the molecules still refining (FP32 at a reference or zero
-    // start, whose first residual is never tested)
-    const bool f32_res = f32_first && round == 0;
-    ctx->sweep = SweepMask{ctx->b_sphmol.as<int>(), drun, ns == 2 ? drun + nmol : nullptr};
-    int orc;
-    if (ns == 2) {
-      const int dq = sys[0].adjoint ? 1 : 0, aq = 1 - dq;
-      const SolveBufs bd = solve_bufs(ctx, dq), ba = solve_bufs(ctx, aq);
-      orc = f32_res ? op_pair_f32(ctx, sys[dq].x, bd.y, sys[aq].x, ba.y)
-                    : op_pair(ctx, sys[dq].x, bd.y, sys[aq].x, ba.y);
-    } else {
-      orc = op_single(ctx, f32_res ? OP_F32 : OP_F64, sys[0].adjoint, sys[0].x,
-                      solve_bufs(ctx, 0).y);
-    }
-    ctx->sweep = SweepMask{};
-    CKI(orc);
-    for (int q = 0; q < ns; q++) {
-      const SolveBufs b = solve_bufs(ctx, q);
-      StageScope sc(ctx, ST_JACOBI);
-      CK(launch_batch_residual(ctx->L(), ctx->tb, sys[q].bs, drun + q * nmol, sys[q].rhs, b.y,
-                               sys[q].x, b.r, b.d, b.e, dnorm + q * nmol));
-    }
-    std::vector<double> nrm(2 * nmol, 0.0);
-    CK(cudaMemcpyAsync(nrm.data(), dnorm, sizeof(double) * 2 * nmol, cudaMemcpyDeviceToHost,
-                       ctx->st));
-    CKI(sync(ctx));
-    // per molecule: converged, out of budget, or an inner solve
-    std::vector<int> ist(2 * nmol, 1), maxk(2 * nmol, 1), upd(2 * nmol, 0);
-    std::vector<double> tolk(2 * nmol, tol);
-    int ninner = 0;
-    for (int q = 0; q < ns; q++)
-      for (int k = 0; k < nmol; k++) {
-        const int j = q * nmol + k;
-        if (run[j] != 0) continue;
-        ++outer[j];
-        last[j] = nrm[j];
-        if (!std::isfinite(nrm[j])) {
-          run[j] = 3;
-        } else if (nrm[j] < tol && !f32_res) {
-          run[j] = 1;
-        } else if (its[j] >= ctx->prm.max_iter) {
-          run[j] = 2;
-        } else {
-          ist[j] = 0;
-          upd[j] = 1;
-          maxk[j] = ctx->prm.max_iter - its[j];
-          tolk[j] = std::max(1e-4 * nrm[j], 0.3 * tol);
-          ++ninner;
-        }
-      }
-    if (!ninner) break;
-    for (int q = 0; q < ns; q++) {
-      const SolveBufs b = solve_bufs(ctx, q);
-      CKI(batch_setup(ctx, in[q], sys[q].adjoint, b.r, b.e, nullptr, nullptr, q, true,
-                      ist.data() + q * nmol, tolk.data() + q * nmol, maxk.data() + q * nmol));
-    }
-    CKI(batch_sweeps(ctx, in, ns));
-    // account the inner solves and apply their corrections
-    CK(cudaMemcpyAsync(dupd, upd.data(), sizeof(int) * 2 * nmol, cudaMemcpyHostToDevice, ctx->st));
-    std::vector<int> iit(2 * nmol, 0), irs(2 * nmol, 0);
-    for (int q = 0; q < ns; q++) {
-      CK(launch_batch_update(ctx->L(), in[q].bs, ctx->nylm, dupd + q * nmol,
-                             solve_bufs(ctx, q).e, sys[q].x));
-      CK(cudaMemcpyAsync(iit.data() + q * nmol, in[q].bs.iters, sizeof(int) * nmol,
-                         cudaMemcpyDeviceToHost, ctx->st));
-      CK(cudaMemcpyAsync(irs.data() + q * nmol, in[q].bs.restarts, sizeof(int) * nmol,
-                         cudaMemcpyDeviceToHost, ctx->st));
-    }
-    CKI(sync(ctx));
-    for (int j = 0; j < 2 * nmol; j++)
-      if (upd[j]) {
-        its[j] += iit[j];
-        rst[j] += irs[j];
-      }
-  }
-  int rc = DDC_OK;
-  for (int q = 0; q < ns; q++) {
-    int maxit = 0, maxout = 0, nfail = 0, restarts = 0;
-    double worst = 0.0;
-    for (int k = 0; k < nmol; k++) {
-      const int j = q * nmol + k;
-      if (sys[q].iters) sys[q].iters[k] = its[j];
-      maxit = std::max(maxit, its[j]);
-      maxout = std::max(maxout, outer[j]);
-      restarts += rst[j];
-      if (run[j] != 1 && ctx->h_off[k + 1] > ctx->h_off[k]) nfail++;
-      if (ctx->h_off[k + 1] > ctx->h_off[k]) worst = std::max(worst, last[j]);
-    }
-    if (sys[q].inf) {
-      memset(sys[q].inf, 0, sizeof(*sys[q].inf));
-      sys[q].inf->iterations = maxit;
-      sys[q].inf->refinements = maxout;
-      sys[q].inf->converged = nfail == 0;
-      sys[q].inf->diis_restarts = restarts;
-      sys[q].inf->final_norm = worst;
-      sys[q].inf->seconds = now_s() - t0;
-    }
-    if (nfail && rc == DDC_OK)
-      rc = fail(ctx, DDC_ERR_NOCONV,
-                std::to_string(nfail) + " molecule(s) did not converge" +
-                    (sys[q].adjoint ? " (adjoint)" : ""));
-  }
-  return rc;
-}
-
 // ===========================================================================
 // C ABI
 // ===========================================================================
@@ -1956,6 +1417,9 @@ int ddc_destroy(ddc_ctx* c) {
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   tc_release(c->tc);
   if (c->hred) cudaFreeHost(c->hred);
+  if (c->hstop) cudaFreeHost(c->hstop);
+  for (cudaEvent_t e : c->ev_sweep)
+    if (e) cudaEventDestroy(e);
   if (c->st2) cudaStreamSynchronize(c->st2);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -2394,10 +1858,9 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
       CK(launch_guess(ctx->L(), ctx->tb, (long long)nv, rhs, dsig, gmode));
       CK(launch_guess(ctx->L(), ctx->tb, (long long)nv, dpsi, ds, gmode));
     }
-    SolveTask task[2];
-    task_begin(ctx, task[0], false, rhs, dsig, &inf->direct, 0);
-    task_begin(ctx, task[1], true, dpsi, ds, &inf->adjoint, 1);
-    CKI(solve_tasks(ctx, task, 2));
+    const System sys[2] = {{false, rhs, dsig, nullptr, &inf->direct},
+                           {true, dpsi, ds, nullptr, &inf->adjoint}};
+    CKI(solve_systems(ctx, sys, 2));
     double d = 0.0;
     CKI(dot_dev(ctx, (long long)nv, dsig, dpsi, &d));
     *esolv = 0.5 * ((ctx->prm.eps - 1.0) / ctx->prm.eps) * d;
@@ -2571,35 +2034,29 @@ int ddc_batch_energy_forces(ddc_ctx* ctx, int nmol, const int* off, const double
   double* ds = ctx->s.as<double>();
   const long long n = (long long)nv;
   const bool paired = ctx->prm.igrad && ctx->prm.pair_solves;
+  auto batch_solve = [&](const System* sys, int ns) {
+    ctx->batch = true;
+    const int r = solve_systems(ctx, sys, ns);
+    ctx->batch = false;
+    return r;
+  };
   // direct solve (and the adjoint with it when paired)
   {
     double* rhs = ctx->rhs.as<double>();
-    CK(ctx->gbuf.ensure(sizeof(double) * std::max<long long>((long long)N * ctx->ngrid, 1)));
-    {
-      StageScope sc(ctx, ST_RHS);
-      CK(launch_wghpot(ctx->L(), ctx->geo(), dphi, ctx->gbuf.as<double>()));
-      CK(launch_dgemm_nn(ctx->L(), ctx->nylm, N, ctx->ngrid, 1.0, ctx->bw.as<double>(),
-                         ctx->nylm, ctx->gbuf.as<double>(), ctx->ngrid, rhs, ctx->nylm));
-    }
+    CKI(direct_rhs(ctx, dphi, rhs));
     const bool learned = ctx->prm.guess == DDC_GUESS_LEARNED;
     if (learned)
       CKI(learned_guess(ctx, rhs, dpsi, dsig, ctx->prm.igrad ? ds : nullptr));
     else
       CK(launch_guess(ctx->L(), ctx->tb, n, rhs, dsig, ctx->prm.guess == DDC_GUESS_ZERO ? 1 : 0));
     std::vector<int> it(nmol), ita(nmol);
-    BatchSys sys[2];
-    CKI(batch_setup(ctx, sys[0], false, rhs, dsig, it.data(), &inf->direct, 0));
-    if (paired) {
-      // the adjoint right-hand side psi is known already: both systems share
-      // each sweep's fused L / L* pass
-      if (!learned)
-        CK(launch_guess(ctx->L(), ctx->tb, n, dpsi, ds, ctx->prm.guess == DDC_GUESS_ZERO ? 1 : 0));
-      CKI(batch_setup(ctx, sys[1], true, dpsi, ds, ita.data(), &inf->adjoint, 1));
-    }
-    if (ctx->prm.precision == DDC_PREC_MIXED)
-      CKI(batch_run_mixed(ctx, sys, paired ? 2 : 1));
-    else
-      CKI(batch_run(ctx, sys, paired ? 2 : 1));
+    // the adjoint right-hand side psi is known already: paired systems share
+    // each sweep's fused L / L* pass
+    if (paired && !learned)
+      CK(launch_guess(ctx->L(), ctx->tb, n, dpsi, ds, ctx->prm.guess == DDC_GUESS_ZERO ? 1 : 0));
+    const System sys[2] = {{false, rhs, dsig, it.data(), &inf->direct},
+                           {true, dpsi, ds, ita.data(), &inf->adjoint}};
+    CKI(batch_solve(sys, paired ? 2 : 1));
     if (iters)
       for (int k = 0; k < nmol; k++) {
         iters[2 * k] = it[k];
@@ -2619,12 +2076,8 @@ int ddc_batch_energy_forces(ddc_ctx* ctx, int nmol, const int* off, const double
       if (ctx->prm.guess != DDC_GUESS_LEARNED)
         CK(launch_guess(ctx->L(), ctx->tb, n, dpsi, ds, ctx->prm.guess == DDC_GUESS_ZERO ? 1 : 0));
       std::vector<int> it(nmol);
-      BatchSys sys;
-      CKI(batch_setup(ctx, sys, true, dpsi, ds, it.data(), &inf->adjoint, 0));
-      if (ctx->prm.precision == DDC_PREC_MIXED)
-        CKI(batch_run_mixed(ctx, &sys, 1));
-      else
-        CKI(batch_run(ctx, &sys, 1));
+      const System sys{true, dpsi, ds, it.data(), &inf->adjoint};
+      CKI(batch_solve(&sys, 1));
       if (iters)
         for (int k = 0; k < nmol; k++) iters[2 * k + 1] = it[k];
     }

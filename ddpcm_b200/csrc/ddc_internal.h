@@ -102,26 +102,26 @@ struct LxsTab {
 };
 
 // Device geometry handed to every kernel.
-// Spheres a batched sweep may skip: those of molecules whose systems have
-// all stopped (their operator outputs are not read again).  mol == null:
+// Spheres a solver sweep may skip: those of molecules whose systems have
+// all stopped (their operator outputs are not read again).  st0 == null:
 // every sphere is computed.
 struct SweepMask {
-  const int* mol;  // [nsph] molecule of each sphere
-  const int* st0;  // [nmol] Jacobi/DIIS status of the first system (0: running)
+  const int* mol;  // [nsph] molecule of each sphere, or null: one molecule
+  const int* st0;  // [nmol] status of the first system (0: running)
   const int* st1;  // [nmol] status of the second system, or null
 };
 
 #ifdef __CUDACC__
-// True for a sphere of a batched molecule whose systems have all stopped.
+// True for a sphere of a molecule whose systems have all stopped.
 __device__ __forceinline__ bool sweep_skip(const SweepMask& m, int sph) {
-  if (!m.mol) return false;
-  const int k = m.mol[sph];
+  if (!m.st0) return false;
+  const int k = m.mol ? m.mol[sph] : 0;
   return m.st0[k] != 0 && (!m.st1 || m.st1[k] != 0);
 }
 // True for every thread of the block when the spheres [i0, i0 + w) are all
 // skipped (a block barrier: call it from every thread, w <= blockDim.x)
 __device__ __forceinline__ bool sweep_skip_tile(const SweepMask& m, int i0, int w, int nsph) {
-  if (!m.mol) return false;
+  if (!m.st0) return false;
   const int i = i0 + (int)threadIdx.x;
   return __syncthreads_and((int)threadIdx.x >= w || i >= nsph || sweep_skip(m, i)) != 0;
 }
@@ -166,44 +166,55 @@ enum Stage {
   ST_GATHER, ST_N
 };
 
-// History of DIIS vectors for the fused Jacobi step / extrapolation.
+// Longest DIIS history.
 constexpr int kMaxHist = 32;
-// elements per chunk of the batched Jacobi/DIIS kernels
-constexpr int kBatchChunk = 2048;
-// The vectors are FP64, or FP32 for the inner solves of the mixed path.
-struct HistPtrs {
-  const void* p[kMaxHist];
-  double c[kMaxHist];
-  int n;
+// State of one system (direct or adjoint) of a Jacobi/DIIS solve: device
+// arrays, one entry per molecule unless noted.
+struct SolverSys {
+  const double* rhs;   // what the iteration solves for: the system's
+  const double* y;     //   right-hand side, its operator output (O x) and its
+  double* x;           //   iterate; mixed: the inner system r, O e, e
+  const double* orhs;  // mixed: the outer right-hand side and iterate, and r
+  double* ox;
+  double* r;
+  void* hx;  // [ndiis][n_total] history of iterates and increments, FP64 or
+  void* he;  //   FP32 (inner solves of the mixed refinement)
+  int* nmat;      // next history position, 1-based
+  int* slot;      // [nmol][ndiis] logical -> physical history slot
+  int* status;    // 0 running, 1 converged, 2 budget spent, 3 non-finite
+  int* iters;     // iterations of this (inner) solve
+  int* restarts;  // singular DIIS systems of this (inner) solve
+  int* ext;       // terms of the extrapolation; negative: take the Jacobi iterate
+  int* maxk;      // iteration budget
+  int* run;       // mixed, outer: 0 refining, 1 converged, 2 budget spent, 3 non-finite
+  int* its;       // mixed, outer: iterations, refinements and restarts so far
+  int* outer;
+  int* rst;
+  int* upd;       // the inner solve ran
+  unsigned* cnt;  // arrival counters, zero between kernels
+  double* norm;   // last increment norm
+  double* last;   // last outer increment norm
+  double* tolk;   // tolerance
+  double* coef;   // [nmol][kMaxHist] extrapolation coefficients
+  double* gram;   // [nmol][ndiis][ndiis] inner products by physical slot
+  double* part;   // [nchunk][kMaxHist+1] per-chunk partial sums
+  double* log;    // increment norm of every iteration (one molecule), or null
 };
-
-// Per-molecule Jacobi/DIIS state of a batched solve (device arrays).
-struct BatchState {
-  int nmol, ndiis, max_iter;
+struct SolverArgs {
+  int nmol, nonempty, nsph, nylm, ndiis, max_iter;
+  int nchunk, chunk;  // chunks of `chunk` elements
+  int first;          // system of grid row 0
+  int sweep;          // number of the sweep, from 1
   double tol;
-  long long n_total;  // length of the concatenated vectors
-  const int* off;     // [nmol+1] sphere offsets
-  int* nmat;          // [nmol]
-  int* slot;          // [nmol][ndiis] logical -> physical history slot
-  double* B;          // [nmol][(ndiis+1)^2] column-major bordered Gram matrix
-  int* status;        // [nmol]: 0 active, 1 converged, 2 max_iter, 3 non-finite
-  int* iters;         // [nmol]
-  int* restarts;      // [nmol]
-  double* norm;       // [nmol] last increment norm
-  void* hx;           // [ndiis][n_total], FP64 or (f32) FP32
-  void* he;           // [ndiis][n_total]
-  int f32;            // history vectors in FP32 (inner solves of the mixed refinement)
-  const double* tolk; // [nmol] per-molecule tolerance, or null: tol
-  const int* maxk;    // [nmol] per-molecule iteration budget, or null: max_iter
-  // element chunks of the per-molecule kernels: chunk c holds up to
-  // kBatchChunk consecutive elements of molecule cmol[c]
-  int nchunk;
-  const int* cmol;    // [nchunk]
+  long long n_total;
+  const int* off;     // [nmol+1] sphere offsets of the molecules; with cmol
+  const int* cmol;    // [nchunk] molecule of each chunk, or null: one molecule
   const int* cfirst;  // [nmol+1] first chunk of each molecule
-  double* part;       // [nchunk][kMaxHist+1] per-chunk partial sums
-  unsigned* cnt;      // [nmol] arrival counters, zero between kernels
-  double* coef;       // [nmol][kMaxHist] extrapolation coefficients
-  int* ext;           // [nmol] terms of the extrapolation; negative after a singular solve
+  int* active;        // [2] molecules still running
+  int* hstop;         // [2] mapped host memory: the sweep that stopped the system
+  double facl[DDC_MAX_LMAX + 1];  // D^-1 of degree l
+  double hw[DDC_MAX_LMAX + 1];    // 1 / (1 + l): weights of the increment norm
+  SolverSys sys[2];
 };
 
 // ---------------------------------------------------------------------------
@@ -281,11 +292,6 @@ cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, doubl
 cudaError_t launch_lx_gather_f32(Launch L, const DevGeo& g, const float* val, float* pot,
                                  int ldp);
 cudaError_t launch_to_float(Launch L, long long n, const double* x, float* y);
-// r = rhs - y - x/facl ; d = facl*r (Jacobi increment at x), partial H-norm of d
-cudaError_t launch_residual(Launch L, const YlmTables& tb, long long n, const double* rhs,
-                            const double* y, const double* x, double* r, double* d,
-                            double* partials, int nblk);
-cudaError_t launch_axpy(Launch L, long long n, double a, const double* x, double* y);
 // dst[c*rows + r] = src[r*cols + c] (FP64)
 cudaError_t launch_transpose(Launch L, int rows, int cols, const double* src, double* dst);
 // C[n*ldc + m] = alpha * sum_k A[k*lda + m] B[n*ldb + k] (FP64, pipelined);
@@ -301,7 +307,6 @@ cudaError_t launch_xi_f32_simt(Launch L, int nylm, int nsph, int ngrid, const fl
                                const double* s, float* xi);
 cudaError_t launch_wghpot(Launch L, const DevGeo& g, const double* phi, double* gbuf);
 cudaError_t launch_ldm1x(Launch L, const YlmTables& tb, long long n, const double* x, double* y);
-cudaError_t launch_scale(Launch L, long long n, double a, const double* x, double* y);
 cudaError_t launch_guess(Launch L, const YlmTables& tb, long long n, const double* rhs,
                          double* x, int mode);
 
@@ -337,21 +342,16 @@ cudaError_t launch_guess_targets(Launch L, const YlmTables& tb, int nsph, int no
 cudaError_t guess_infer(Launch L, ddc_guess* m, const YlmTables& tb, int nsph, const float* feat,
                         const double* g, const double* psi, double* x, double* s);
 
-// solver
-// xnew = facl*(rhs - y); e = xnew - x; dots e.h_k (k < hist.n) and e.e.
-// xnew, e and the history are FP32 when f32 (mixed-path inner solves), else FP64.
-// The block partials go to partials; the last block sums them into out[0..hist.n]
-// (counter: a zeroed device word, left zeroed).
-cudaError_t launch_jacobi_step(Launch L, const YlmTables& tb, long long n, const double* rhs,
-                               const double* y, const double* x, void* xnew, void* e,
-                               const HistPtrs& hist, double* partials, int nblk, bool f32,
-                               int* nblk_used,  // blocks launched (<= nblk): partial rows
-                               unsigned* counter, double* out);
-// xout = sum c_k p_k (or xjac if hist.n == 0); sum_l 1/(l+1) (xout-x)^2 into
-// out[0] (through partials and counter as above); x = xout
-cudaError_t launch_diis_combine(Launch L, const YlmTables& tb, long long n, const HistPtrs& hist,
-                                const void* xjac, double* x, double* partials, int nblk,
-                                bool f32, unsigned* counter, double* out);
+// Jacobi/DIIS on the device (ddc_solver.cu), over the first ns systems of a
+// (from a.first on): starting state; one half of an iteration after
+// y = O x (which 0: Jacobi step and Gram solve, 1: extrapolation and stop
+// test); the mixed refinement's residual at ox with y = O ox, and x += e
+int solver_chunk(long long n_total, bool one);
+cudaError_t launch_solver_begin(Launch L, const SolverArgs& a, int ns, bool mixed);
+cudaError_t launch_solver_step(Launch L, const SolverArgs& a, int ns, bool f32, int which);
+cudaError_t launch_solver_residual(Launch L, const SolverArgs& a, int ns, bool f32_res);
+cudaError_t launch_solver_update(Launch L, const SolverArgs& a, int ns);
+
 cudaError_t launch_hnorm_partial(Launch L, const YlmTables& tb, long long n, const double* x,
                                  double* partials, int nblk);
 cudaError_t launch_dot_partial(Launch L, long long n, const double* a, const double* b,
@@ -462,17 +462,6 @@ cudaError_t launch_zeta_efld_contract(Launch L, const DevGeo& g, const double* z
 cudaError_t launch_charge_efld_contract(Launch L, int n, const double* q, const double* ef,
                                         double* fx);
 // batched solves
-cudaError_t launch_batch_diis(Launch L, const YlmTables& tb, const BatchState& bs,
-                              const double* rhs, const double* y, double* x);
-// Mixed refinement of a batch, per molecule with run[k] == 0: r = rhs - y -
-// x/facl, d = facl r (the FP64 Jacobi increment at x), e = d, and the
-// increment's H-norm into norm[k] (chunk map and partials of bs).
-cudaError_t launch_batch_residual(Launch L, const YlmTables& tb, const BatchState& bs,
-                                  const int* run, const double* rhs, const double* y,
-                                  const double* x, double* r, double* d, double* e, double* norm);
-// x += e over the molecules with upd[k] != 0
-cudaError_t launch_batch_update(Launch L, const BatchState& bs, int nylm, const int* upd,
-                                const double* e, double* x);
 cudaError_t launch_batch_dot(Launch L, int nmol, const int* off, int nylm, const double* a,
                              const double* b, double scale, double* out);
 cudaError_t launch_batch_ranges(Launch L, int nsph, int ngrid, int ncav, const int2* mrange,

@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(256, 3) k_dgemm_dmma(int M, int N, int K, doub
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   // columns are spheres: a batched sweep skips a tile whose spheres all belong
   // to stopped molecules
-  if (act.mol && __syncthreads_and(tid >= BN || n0 + tid >= N || sweep_skip(act, n0 + tid)))
+  if (act.st0 && __syncthreads_and(tid >= BN || n0 + tid >= N || sweep_skip(act, n0 + tid)))
     return;
   auto load = [&](int buf, int k0) {
 #pragma unroll
@@ -908,16 +908,6 @@ cudaError_t launch_ldm1x(Launch L, const YlmTables& tb, long long n, const doubl
   ++*L.launches;
   return cudaGetLastError();
 }
-__global__ void k_scale(long long n, double a, const double* __restrict__ x, double* y) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < n) y[e] = a * x[e];
-}
-cudaError_t launch_scale(Launch L, long long n, double a, const double* x, double* y) {
-  if (n == 0) return cudaSuccess;
-  k_scale<<<(unsigned)((n + 255) / 256), 256, 0, L.st>>>(n, a, x, y);
-  ++*L.launches;
-  return cudaGetLastError();
-}
 // mode 0: x = facl * rhs (cosmo.f90:136-138), 1: x = 0
 __global__ void k_guess(const YlmTables tb, long long n, const double* __restrict__ rhs, double* x,
                         int mode) {
@@ -956,254 +946,6 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], int nv, double*
     for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) s += sh[threadIdx.x][ww];
     partials[(size_t)blockIdx.x * STRIDE + threadIdx.x] = s;
   }
-}
-
-// The last block of a grid to finish (an arrival counter) sums the per-block
-// partials of all blocks, in block order, into out[k] for k < nv and resets
-// the counter: the solver kernels hand their final sums to the host without
-// a separate reduction launch.  A fixed order: reproducible.
-__device__ __forceinline__ void last_block_reduce(const double* partials, int stride, int nv,
-                                                  unsigned* counter, double* out) {
-  __shared__ unsigned s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = w; k < nv; k += nw) {
-    double v = 0.0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) v += __ldcg(partials + (size_t)b * stride + k);
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) out[k] = v;
-  }
-  if (threadIdx.x == 0) *counter = 0u;
-}
-
-// Element tiles of the solver kernels: a block takes 4 x 256 consecutive
-// elements per step, thread t the elements t, t+256, t+512, t+768, so that
-// each thread has four independent loads of every vector in flight.
-constexpr int kSolU = 4, kSolT = 256;
-__device__ __forceinline__ int lm_first(long long q, int nylm) { return (int)(q % nylm); }
-__device__ __forceinline__ int lm_add(int lm, int d, int nylm) {
-  lm += d;
-  return lm >= nylm ? lm - nylm : lm;
-}
-
-// Jacobi step + DIIS Gram row: xnew = D^-1 (rhs - Ox) (jacobi_diis.f90:105-110),
-// e = xnew - x (:117), dots e.h_k for the history and e.e (makeb :232-270).
-// A block takes tiles of 8 x 256 consecutive elements: each thread forms
-// eight elements of xnew and e and leaves e in shared memory; then warp w
-// takes the history vectors k = w, w + 8, ... and reads the tile of h_k
-// (sixteen loads per lane in flight) against e from shared memory.  Per
-// history vector a lane accumulates in FP64 over the tiles in order, and the
-// warp's shuffle tree gives the block's partial, so the row is reproducible.
-// The partial row keeps the stride kMaxHist + 1 that the host-side
-// reduction expects.
-template <class H>
-__global__ void __launch_bounds__(kSolT, 4) k_jacobi_step(const YlmTables tb, long long n,
-                                                       const double* __restrict__ rhs,
-                                                       const double* __restrict__ y,
-                                                       const double* __restrict__ x, H* xnew,
-                                                       H* e, const HistPtrs hist,
-                                                       double* partials, unsigned* counter, double* out) {
-  constexpr int U = 2 * kSolU;  // eight elements per thread and tile
-  constexpr int TILE = U * kSolT;
-  constexpr int NW = kSolT / 32;
-  constexpr int KS = (kMaxHist + NW - 1) / NW;  // history vectors per warp
-  constexpr int HL = 16;                        // loads per lane in flight
-  __shared__ H es[TILE];
-  __shared__ double red[kMaxHist + 1 + NW];
-  double d[KS];
-#pragma unroll
-  for (int s = 0; s < KS; ++s) d[s] = 0.0;
-  double ee = 0.0;
-  const int nh = hist.n, nylm = tb.nylm;
-  const int dt = kSolT % nylm;
-  const int nn = (int)n;  // vectors hold fewer than 2^31 elements (checked at launch)
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int b0 = blockIdx.x * TILE; b0 < nn; b0 += gridDim.x * TILE) {
-    const int q0 = b0 + threadIdx.x;
-    int lm = lm_first(q0, nylm);
-#pragma unroll
-    for (int h = 0; h < U; h += kSolU) {  // two halves of four elements
-      double rv[kSolU], yv[kSolU], xv[kSolU];
-#pragma unroll
-      for (int u = 0; u < kSolU; ++u) {
-        const int q = q0 + (h + u) * kSolT;
-        rv[u] = q < nn ? rhs[q] : 0.0;
-        yv[u] = q < nn ? y[q] : 0.0;
-        xv[u] = q < nn ? x[q] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < kSolU; ++u) {
-        const int q = q0 + (h + u) * kSolT;
-        const double xn = tb.facl[l_of(lm)] * (rv[u] - yv[u]);
-        const H ev = q < nn ? (H)(xn - xv[u]) : H(0);
-        if (q < nn) {
-          xnew[q] = (H)xn;
-          e[q] = ev;
-        }
-        es[threadIdx.x + (h + u) * kSolT] = ev;
-        ee = fma((double)ev, (double)ev, ee);
-        lm = lm_add(lm, dt, nylm);
-      }
-    }
-    __syncthreads();
-    const int cnt = min(TILE, nn - b0);
-#pragma unroll
-    for (int s = 0; s < KS; ++s) {
-      const int k = w + NW * s;
-      if (k < nh) {
-        const H* hk = static_cast<const H*>(hist.p[k]) + b0;
-        for (int j0 = 0; j0 < TILE; j0 += 32 * HL) {
-          H hv[HL];
-#pragma unroll
-          for (int u = 0; u < HL; ++u) {
-            const int j = j0 + u * 32 + lane;
-            hv[u] = j < cnt ? hk[j] : H(0);
-          }
-#pragma unroll
-          for (int u = 0; u < HL; ++u)
-            d[s] = fma((double)es[j0 + u * 32 + lane], (double)hv[u], d[s]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  // partial row [e.h_0 .. e.h_{nh-1}, e.e]
-#pragma unroll
-  for (int s = 0; s < KS; ++s) {
-    double v = d[s];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int k = w + NW * s;
-    if (lane == 0 && k < nh) red[k] = v;
-  }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) ee += __shfl_xor_sync(0xffffffffu, ee, o);
-  if (lane == 0) red[kMaxHist + 1 + w] = ee;
-  __syncthreads();
-  if (threadIdx.x < nh) {
-    partials[(size_t)blockIdx.x * (kMaxHist + 1) + threadIdx.x] = red[threadIdx.x];
-  } else if (threadIdx.x == nh) {
-    double t = 0.0;
-    for (int ww = 0; ww < NW; ++ww) t += red[kMaxHist + 1 + ww];
-    partials[(size_t)blockIdx.x * (kMaxHist + 1) + nh] = t;
-  }
-  last_block_reduce(partials, kMaxHist + 1, nh + 1, counter, out);
-}
-// One wave: as many blocks as fit on the device at once (at most nblk, the
-// partial-row capacity).
-template <class KFN>
-static int one_wave_blocks(KFN kfn, int nblk) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
-  }
-  int per = 0;
-  if (sms <= 0 ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, kSolT, 0) != cudaSuccess ||
-      per <= 0) {
-    cudaGetLastError();
-    return nblk;
-  }
-  return std::min(nblk, sms * per);
-}
-template <class H>
-static int jacobi_launch(Launch L, const YlmTables& tb, long long n, const double* rhs,
-                         const double* y, const double* x, H* xnew, H* e, const HistPtrs& hist,
-                         double* partials, int nblk, unsigned* counter, double* out) {
-  const int used = one_wave_blocks(k_jacobi_step<H>, nblk);
-  k_jacobi_step<H><<<used, kSolT, 0, L.st>>>(tb, n, rhs, y, x, xnew, e, hist, partials, counter,
-                                             out);
-  return used;
-}
-cudaError_t launch_jacobi_step(Launch L, const YlmTables& tb, long long n, const double* rhs,
-                               const double* y, const double* x, void* xnew, void* e,
-                               const HistPtrs& hist, double* partials, int nblk, bool f32,
-                               int* nblk_used, unsigned* counter, double* out) {
-  if (hist.n > kMaxHist - 1 || n >= (1LL << 31)) return cudaErrorInvalidValue;
-  int used;
-  if (f32)
-    used = jacobi_launch<float>(L, tb, n, rhs, y, x, static_cast<float*>(xnew),
-                                static_cast<float*>(e), hist, partials, nblk, counter, out);
-  else
-    used = jacobi_launch<double>(L, tb, n, rhs, y, x, static_cast<double*>(xnew),
-                                 static_cast<double*>(e), hist, partials, nblk, counter, out);
-  if (nblk_used) *nblk_used = used;
-  ++*L.launches;
-  return cudaGetLastError();
-}
-
-// DIIS extrapolation (jacobi_diis.f90:222-226) + increment norm (hnorm,
-// matvec.f90:281-323: sum over spheres of sum_l 1/(l+1) |u_l|^2) + update.
-template <class H>
-__global__ void __launch_bounds__(kSolT) k_diis_combine(const YlmTables tb, long long n,
-                                                        const HistPtrs hist,
-                                                        const H* __restrict__ xjac, double* x,
-                                                        double* partials, unsigned* counter, double* out) {
-  double acc = 0.0;
-  const int nh = hist.n, nylm = tb.nylm;
-  const int dt = kSolT % nylm;
-  const long long tile = (long long)kSolU * kSolT;
-  for (long long b0 = (long long)blockIdx.x * tile; b0 < n; b0 += (long long)gridDim.x * tile) {
-    long long q[kSolU];
-    bool ok[kSolU];
-    double xo[kSolU], xold[kSolU];
-#pragma unroll
-    for (int u = 0; u < kSolU; ++u) {
-      q[u] = b0 + u * kSolT + threadIdx.x;
-      ok[u] = q[u] < n;
-      xold[u] = ok[u] ? x[q[u]] : 0.0;
-      xo[u] = 0.0;
-    }
-    if (nh == 0) {
-#pragma unroll
-      for (int u = 0; u < kSolU; ++u) xo[u] = ok[u] ? (double)xjac[q[u]] : 0.0;
-    } else {
-#pragma unroll 4
-      for (int k = 0; k < nh; ++k) {
-        const H* hk = static_cast<const H*>(hist.p[k]);
-        const double ck = hist.c[k];
-        H hv[kSolU];
-#pragma unroll
-        for (int u = 0; u < kSolU; ++u) hv[u] = ok[u] ? hk[q[u]] : H(0);
-#pragma unroll
-        for (int u = 0; u < kSolU; ++u) xo[u] = fma(ck, (double)hv[u], xo[u]);
-      }
-    }
-    int lm = lm_first(b0 + threadIdx.x, nylm);
-#pragma unroll
-    for (int u = 0; u < kSolU; ++u) {
-      if (ok[u]) {
-        const double dd = xo[u] - xold[u];
-        acc = fma(dd * dd, 1.0 / (1.0 + l_of(lm)), acc);
-        x[q[u]] = xo[u];
-      }
-      lm = lm_add(lm, dt, nylm);
-    }
-  }
-  double v[1] = {acc};
-  block_sum_store<1>(v, 1, partials);
-  last_block_reduce(partials, 1, 1, counter, out);
-}
-cudaError_t launch_diis_combine(Launch L, const YlmTables& tb, long long n, const HistPtrs& hist,
-                                const void* xjac, double* x, double* partials, int nblk,
-                                bool f32, unsigned* counter, double* out) {
-  if (f32)
-    k_diis_combine<float><<<nblk, kSolT, 0, L.st>>>(tb, n, hist, static_cast<const float*>(xjac),
-                                                    x, partials, counter, out);
-  else
-    k_diis_combine<double><<<nblk, kSolT, 0, L.st>>>(tb, n, hist,
-                                                     static_cast<const double*>(xjac), x,
-                                                     partials, counter, out);
-  ++*L.launches;
-  return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(256) k_hnorm_partial(const YlmTables tb, long long n,
@@ -2398,476 +2140,9 @@ cudaError_t launch_to_float(Launch L, long long n, const double* x, float* y) {
   ++*L.launches;
   return cudaGetLastError();
 }
-// FP64 residual of the full operator L = D + O at x (y = O x):
-//   r = rhs - y - x / facl,  d = facl * r  (the Jacobi increment at x)
-// plus the partial sum of the increment's H-norm (hnorm, matvec.f90:281-323)
-__global__ void __launch_bounds__(256) k_residual(const YlmTables tb, long long n,
-                                                  const double* __restrict__ rhs,
-                                                  const double* __restrict__ y,
-                                                  const double* __restrict__ x, double* r,
-                                                  double* d, double* partials) {
-  double acc = 0.0;
-  for (LmWalk w(tb.nylm); w.q < n; w.next()) {
-    const long long q = w.q;
-    int l = l_of(w.lm);
-    double fl = tb.facl[l];
-    double rv = rhs[q] - y[q] - x[q] / fl;
-    double dv = fl * rv;
-    r[q] = rv;
-    d[q] = dv;
-    acc = fma(dv * dv, 1.0 / (1.0 + l), acc);
-  }
-  double v[1] = {acc};
-  block_sum_store<1>(v, 1, partials);
-}
-cudaError_t launch_residual(Launch L, const YlmTables& tb, long long n, const double* rhs,
-                            const double* y, const double* x, double* r, double* d,
-                            double* partials, int nblk) {
-  k_residual<<<nblk, 256, 0, L.st>>>(tb, n, rhs, y, x, r, d, partials);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-__global__ void k_axpy(long long n, double a, const double* __restrict__ x, double* y) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < n) y[e] = fma(a, x[e], y[e]);
-}
-cudaError_t launch_axpy(Launch L, long long n, double a, const double* x, double* y) {
-  if (n == 0) return cudaSuccess;
-  k_axpy<<<(unsigned)((n + 255) / 256), 256, 0, L.st>>>(n, a, x, y);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------
-// Batched solves: many molecules concatenated into one system.  The
-// operators act per sphere and need no change; the Jacobi/DIIS driver
-// (jacobi_diis.f90) runs per molecule over element chunks (below).
+// batches of molecules
 // ---------------------------------------------------------------------------
-// Gauss-Jordan with full pivoting (gjinv, jacobi_diis.f90:272-360), one warp,
-// lane j owns row j.  a is n x n column-major in shared memory, b the rhs.
-// Pivot: the first maximum of |a| over free rows/columns in the reference's
-// scan order (rows outer, columns inner).  Returns false when singular.
-__device__ bool gjinv_warp(int n, double* a, double* b, int* piv) {
-  const int lane = threadIdx.x & 31;
-  if (lane < n) piv[lane] = 0;
-  __syncwarp();
-  for (int i = 0; i < n; ++i) {
-    double bv = 0.0;
-    int bk = -1;
-    if (lane < n && piv[lane] != 1) {
-      for (int k = 0; k < n; ++k)
-        if (piv[k] == 0) {
-          double v = fabs(a[k * n + lane]);
-          if (v > bv) {
-            bv = v;
-            bk = k;
-          }
-        }
-    }
-    int bj = bk >= 0 ? lane : 1 << 30;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-      int ok = __shfl_xor_sync(0xffffffffu, bk, o);
-      if (ov > bv || (ov == bv && oj < bj)) {
-        bv = ov;
-        bj = oj;
-        bk = ok;
-      }
-    }
-    if (bk < 0) return false;  // no non-zero free entry
-    const int irow = bj, icol = bk;
-    __syncwarp();
-    if (lane == 0) piv[icol] += 1;
-    __syncwarp();
-    if (piv[icol] > 1) return false;
-    if (irow != icol) {
-      for (int k = lane; k < n; k += 32) {
-        double t = a[k * n + irow];
-        a[k * n + irow] = a[k * n + icol];
-        a[k * n + icol] = t;
-      }
-      if (lane == 0) {
-        double t = b[irow];
-        b[irow] = b[icol];
-        b[icol] = t;
-      }
-    }
-    __syncwarp();
-    const double piv_v = a[icol * n + icol];
-    if (piv_v == 0.0) return false;
-    const double pinv = 1.0 / piv_v;
-    __syncwarp();
-    if (lane == 0) a[icol * n + icol] = 1.0;
-    __syncwarp();
-    for (int k = lane; k < n; k += 32) a[k * n + icol] *= pinv;
-    if (lane == 0) b[icol] *= pinv;
-    __syncwarp();
-    double dum = 0.0;
-    if (lane < n && lane != icol) dum = a[icol * n + lane];
-    __syncwarp();
-    if (lane < n && lane != icol) {
-      a[icol * n + lane] = 0.0;
-      for (int k = 0; k < n; ++k) a[k * n + lane] -= a[k * n + icol] * dum;
-      b[lane] -= b[icol] * dum;
-    }
-    __syncwarp();
-  }
-  return true;
-}
-
-// The per-molecule Jacobi/DIIS step runs over element chunks of kBChunk
-// consecutive elements (a molecule owns one or more chunks), so that a
-// large molecule's vectors are read by many blocks at once.  Two kernels:
-// k_batch_gram forms the Jacobi iterate, the increment and the chunk's Gram
-// partials, and the molecule's last chunk to finish sums the partials in
-// chunk order, updates the bordered matrix and solves it (one warp);
-// k_batch_extrap forms the extrapolated iterate and the chunk's part of the
-// increment norm, and the molecule's last chunk sets its norm, iteration
-// count and status.  The history reads are spread over the whole device.
-constexpr int kBChunk = kBatchChunk;
-static_assert(kBChunk % (kSolU * kSolT) == 0 && kBChunk % (32 * 16) == 0, "chunk tiling");
-
-// Logical-to-physical history slots of molecule k for this step: after
-// `nmat` reaches ndiis the ten oldest are dropped (jacobi_diis.f90:196-205).
-__device__ __forceinline__ int batch_hist_perm(const BatchState& bs, int k, int* pm) {
-  const int nd = bs.ndiis, nm_old = bs.nmat[k];
-  const bool shift = nm_old >= nd;
-  const int* sl = bs.slot + (size_t)k * nd;
-  for (int j = threadIdx.x; j < nd; j += blockDim.x) pm[j] = shift ? sl[(j + 10) % nd] : sl[j];
-  return shift ? nm_old - 10 : nm_old;
-}
-
-// Last arriving chunk of molecule k (the counter is reset for the next
-// kernel).  Every block of the molecule calls it after writing its partials.
-__device__ __forceinline__ bool batch_last_chunk(const BatchState& bs, int k) {
-  __shared__ unsigned s_last;
-  __threadfence();
-  __syncthreads();
-  const unsigned nc = (unsigned)(bs.cfirst[k + 1] - bs.cfirst[k]);
-  if (threadIdx.x == 0) {
-    s_last = atomicAdd(bs.cnt + k, 1u) == nc - 1 ? 1u : 0u;
-    if (s_last) bs.cnt[k] = 0u;
-  }
-  __syncthreads();
-  if (s_last) __threadfence();
-  return s_last != 0;
-}
-
-// Sums entries [0, nv) of molecule k's chunk partials in chunk order.
-__device__ __forceinline__ void batch_sum_parts(const BatchState& bs, int k, int nv,
-                                                double* out) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int c0 = bs.cfirst[k], c1 = bs.cfirst[k + 1];
-  for (int h = w; h < nv; h += nw) {
-    double v = 0.0;
-    for (int c = c0 + lane; c < c1; c += 32) v += __ldcg(bs.part + (size_t)c * (kMaxHist + 1) + h);
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) out[h] = v;
-  }
-  __syncthreads();
-}
-
-template <class H>
-__global__ void __launch_bounds__(kSolT) k_batch_gram(const YlmTables tb, BatchState bs,
-                                                      const double* __restrict__ rhs,
-                                                      const double* __restrict__ y,
-                                                      const double* __restrict__ x) {
-  constexpr int U = kBChunk / kSolT;
-  constexpr int NW = kSolT / 32;
-  constexpr int KS = (kMaxHist + NW - 1) / NW;
-  constexpr int HL = 16;
-  const int c = blockIdx.x, k = bs.cmol[c];
-  if (bs.status[k] != 0) return;
-  __shared__ int pm[kMaxHist];
-  __shared__ double es[kBChunk];
-  __shared__ double red[kMaxHist + 1 + NW];
-  __shared__ double row[kMaxHist + 1];
-  const int nm = batch_hist_perm(bs, k, pm), nh = nm - 1;
-  __syncthreads();
-  const int nylm = tb.nylm, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long N = bs.n_total;
-  const long long b0 = (long long)bs.off[k] * nylm + (long long)(c - bs.cfirst[k]) * kBChunk;
-  const int cnt = (int)min((long long)kBChunk, (long long)bs.off[k + 1] * nylm - b0);
-  H* xnew = static_cast<H*>(bs.hx) + (size_t)pm[nm - 1] * N;
-  H* enew = static_cast<H*>(bs.he) + (size_t)pm[nm - 1] * N;
-  double ee = 0.0;
-  {
-    const int dt = kSolT % nylm;
-    int lm = (int)((b0 + threadIdx.x) % nylm);
-    double rv[U], yv[U], xv[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = threadIdx.x + u * kSolT;
-      rv[u] = j < cnt ? rhs[b0 + j] : 0.0;
-      yv[u] = j < cnt ? y[b0 + j] : 0.0;
-      xv[u] = j < cnt ? x[b0 + j] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = threadIdx.x + u * kSolT;
-      double ev = 0.0;
-      if (j < cnt) {
-        const double xn = tb.facl[l_of(lm)] * (rv[u] - yv[u]);
-        const H eh = (H)(xn - xv[u]);
-        ev = (double)eh;
-        xnew[b0 + j] = (H)xn;
-        enew[b0 + j] = eh;
-      }
-      es[j] = ev;
-      ee = fma(ev, ev, ee);
-      lm = lm_add(lm, dt, nylm);
-    }
-  }
-  __syncthreads();
-  double d[KS];
-#pragma unroll
-  for (int s = 0; s < KS; ++s) {
-    d[s] = 0.0;
-    const int kk = w + NW * s;
-    if (kk < nh) {
-      const H* hk = static_cast<const H*>(bs.he) + (size_t)pm[kk] * N + b0;
-      for (int j0 = 0; j0 < kBChunk; j0 += 32 * HL) {
-        H hv[HL];
-#pragma unroll
-        for (int u = 0; u < HL; ++u) {
-          const int j = j0 + u * 32 + lane;
-          hv[u] = j < cnt ? hk[j] : H(0);
-        }
-#pragma unroll
-        for (int u = 0; u < HL; ++u) d[s] = fma(es[j0 + u * 32 + lane], (double)hv[u], d[s]);
-      }
-    }
-  }
-#pragma unroll
-  for (int s = 0; s < KS; ++s) {
-    double v = d[s];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int kk = w + NW * s;
-    if (lane == 0 && kk < nh) red[kk] = v;
-  }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) ee += __shfl_xor_sync(0xffffffffu, ee, o);
-  if (lane == 0) red[kMaxHist + 1 + w] = ee;
-  __syncthreads();
-  double* part = bs.part + (size_t)c * (kMaxHist + 1);
-  if (threadIdx.x < nh) {
-    part[threadIdx.x] = red[threadIdx.x];
-  } else if (threadIdx.x == nh) {
-    double t = 0.0;
-    for (int ww = 0; ww < NW; ++ww) t += red[kMaxHist + 1 + ww];
-    part[nh] = t;
-  }
-  if (!batch_last_chunk(bs, k)) return;
-  batch_sum_parts(bs, k, nh + 1, row);
-  if (threadIdx.x >= 32) return;
-  // bordered Gram matrix (makeb, jacobi_diis.f90:232-270) and its solve
-  __shared__ double ga[(kMaxHist + 1) * (kMaxHist + 1)], gb[kMaxHist + 1];
-  __shared__ int gpiv[kMaxHist + 1];
-  const int nd = bs.ndiis, lenb = nd + 1, nm_old = bs.nmat[k];
-  double* B = bs.B + (size_t)k * lenb * lenb;
-  auto Bm = [&](int j, int kk) -> double& { return B[(size_t)(kk - 1) * lenb + (j - 1)]; };
-  if (threadIdx.x == 0) {
-    if (nm_old >= nd) {
-      for (int j = 2; j <= nm_old - 10; ++j)
-        for (int kk = 2; kk <= nm_old - 10; ++kk) Bm(j, kk) = Bm(j + 10, kk + 10);
-    }
-    if (nm == 1) {
-      Bm(1, 1) = 0.0;
-      Bm(1, 2) = 1.0;
-      Bm(2, 1) = 1.0;
-      Bm(2, 2) = row[0];
-    } else {
-      Bm(nm + 1, 1) = 1.0;
-      Bm(1, nm + 1) = 1.0;
-      for (int i = 1; i <= nm - 1; ++i) {
-        Bm(nm + 1, i + 1) = row[i - 1];
-        Bm(i + 1, nm + 1) = row[i - 1];
-      }
-      Bm(nm + 1, nm + 1) = row[nm - 1];
-    }
-    const int n1 = nm + 1;
-    for (int kk = 1; kk <= n1; ++kk)
-      for (int j = 1; j <= n1; ++j) ga[(kk - 1) * n1 + (j - 1)] = Bm(j, kk);
-    for (int j = 0; j < n1; ++j) gb[j] = 0.0;
-    gb[0] = 1.0;
-  }
-  __syncwarp();
-  const bool ok = gjinv_warp(nm + 1, ga, gb, gpiv);
-  if (threadIdx.x == 0) {
-    int* sl = bs.slot + (size_t)k * nd;
-    if (nm_old >= nd)
-      for (int j = 0; j < nd; ++j) sl[j] = pm[j];
-    double* cf = bs.coef + (size_t)k * kMaxHist;
-    if (ok) {
-      for (int h = 0; h < nm; ++h) cf[h] = gb[h + 1];
-      bs.nmat[k] = nm + 1;
-    } else {  // singular: restart the history (jacobi_diis.f90:214-217)
-      bs.nmat[k] = 1;
-      bs.restarts[k] += 1;
-    }
-    bs.ext[k] = ok ? nm : -nm;
-  }
-}
-
-// DIIS extrapolation (jacobi_diis.f90:222-226) or, after a singular Gram
-// system, the Jacobi iterate; increment H-norm (hnorm) and update.
-template <class H>
-__global__ void __launch_bounds__(kSolT) k_batch_extrap(const YlmTables tb, BatchState bs,
-                                                        double* x) {
-  const int c = blockIdx.x, k = bs.cmol[c];
-  if (bs.status[k] != 0) return;
-  __shared__ int pm[kMaxHist];
-  __shared__ double cf[kMaxHist];
-  __shared__ double tot[1];
-  const int ext = bs.ext[k], nm = ext > 0 ? ext : -ext;
-  const bool ok = ext > 0;
-  if (threadIdx.x < nm) {
-    pm[threadIdx.x] = bs.slot[(size_t)k * bs.ndiis + threadIdx.x];
-    cf[threadIdx.x] = ok ? bs.coef[(size_t)k * kMaxHist + threadIdx.x] : 0.0;
-  }
-  __syncthreads();
-  const int nylm = tb.nylm;
-  const long long N = bs.n_total;
-  const long long b0 = (long long)bs.off[k] * nylm + (long long)(c - bs.cfirst[k]) * kBChunk;
-  const int cnt = (int)min((long long)kBChunk, (long long)bs.off[k + 1] * nylm - b0);
-  const H* xjac = static_cast<const H*>(bs.hx) + (size_t)pm[nm - 1] * N + b0;
-  const int dt = kSolT % nylm;
-  double acc = 0.0;
-#pragma unroll
-  for (int u0 = 0; u0 < kBChunk / kSolT; u0 += kSolU) {
-    double xo[kSolU];
-    bool in[kSolU];
-#pragma unroll
-    for (int u = 0; u < kSolU; ++u) {
-      in[u] = threadIdx.x + (u0 + u) * kSolT < cnt;
-      xo[u] = 0.0;
-    }
-    if (ok) {
-#pragma unroll 4
-      for (int h = 0; h < nm; ++h) {
-        const H* hk = static_cast<const H*>(bs.hx) + (size_t)pm[h] * N + b0;
-        H hv[kSolU];
-#pragma unroll
-        for (int u = 0; u < kSolU; ++u)
-          hv[u] = in[u] ? hk[threadIdx.x + (u0 + u) * kSolT] : H(0);
-#pragma unroll
-        for (int u = 0; u < kSolU; ++u) xo[u] = fma(cf[h], (double)hv[u], xo[u]);
-      }
-    } else {
-#pragma unroll
-      for (int u = 0; u < kSolU; ++u)
-        xo[u] = in[u] ? (double)xjac[threadIdx.x + (u0 + u) * kSolT] : 0.0;
-    }
-    int lm = (int)((b0 + threadIdx.x + u0 * kSolT) % nylm);
-#pragma unroll
-    for (int u = 0; u < kSolU; ++u) {
-      if (in[u]) {
-        const long long q = b0 + threadIdx.x + (u0 + u) * kSolT;
-        const double dd = xo[u] - x[q];
-        acc = fma(dd * dd, 1.0 / (1.0 + l_of(lm)), acc);
-        x[q] = xo[u];
-      }
-      lm = lm_add(lm, dt, nylm);
-    }
-  }
-  double v[1] = {acc};
-  block_sum_store<1, kMaxHist + 1>(v, 1, bs.part);  // chunk c is block c
-  if (!batch_last_chunk(bs, k)) return;
-  batch_sum_parts(bs, k, 1, tot);
-  if (threadIdx.x == 0) {
-    const int nsph = bs.off[k + 1] - bs.off[k];
-    const double nrm = sqrt(tot[0] / (double)max(nsph, 1));
-    bs.norm[k] = nrm;
-    const int it = bs.iters[k] + 1;
-    bs.iters[k] = it;
-    const double tol = bs.tolk ? bs.tolk[k] : bs.tol;
-    const int mx = bs.maxk ? bs.maxk[k] : bs.max_iter;
-    bs.status[k] = (nrm < tol) ? 1 : (it >= mx ? 2 : (isfinite(nrm) ? 0 : 3));
-  }
-}
-cudaError_t launch_batch_diis(Launch L, const YlmTables& tb, const BatchState& bs,
-                              const double* rhs, const double* y, double* x) {
-  if (bs.nchunk == 0) return cudaSuccess;
-  if (bs.f32) {
-    k_batch_gram<float><<<bs.nchunk, kSolT, 0, L.st>>>(tb, bs, rhs, y, x);
-    k_batch_extrap<float><<<bs.nchunk, kSolT, 0, L.st>>>(tb, bs, x);
-  } else {
-    k_batch_gram<double><<<bs.nchunk, kSolT, 0, L.st>>>(tb, bs, rhs, y, x);
-    k_batch_extrap<double><<<bs.nchunk, kSolT, 0, L.st>>>(tb, bs, x);
-  }
-  *L.launches += 2;
-  return cudaGetLastError();
-}
-
-__global__ void __launch_bounds__(kSolT) k_batch_residual(const YlmTables tb, BatchState bs,
-                                                          const int* __restrict__ run,
-                                                          const double* __restrict__ rhs,
-                                                          const double* __restrict__ y,
-                                                          const double* __restrict__ x,
-                                                          double* r, double* d, double* e,
-                                                          double* norm) {
-  const int c = blockIdx.x, k = bs.cmol[c];
-  if (run[k] != 0) return;
-  __shared__ double tot[1];
-  const int nylm = tb.nylm, dt = kSolT % nylm;
-  const long long b0 = (long long)bs.off[k] * nylm + (long long)(c - bs.cfirst[k]) * kBChunk;
-  const int cnt = (int)min((long long)kBChunk, (long long)bs.off[k + 1] * nylm - b0);
-  int lm = (int)((b0 + threadIdx.x) % nylm);
-  double acc = 0.0;
-#pragma unroll 2
-  for (int j = threadIdx.x; j < kBChunk; j += kSolT) {
-    if (j < cnt) {
-      const long long q = b0 + j;
-      const int l = l_of(lm);
-      const double rr = rhs[q] - y[q] - x[q] / tb.facl[l];
-      const double dd = tb.facl[l] * rr;
-      r[q] = rr;
-      d[q] = dd;
-      e[q] = dd;
-      acc = fma(dd * dd, 1.0 / (1.0 + l), acc);
-    }
-    lm = lm_add(lm, dt, nylm);
-  }
-  double v[1] = {acc};
-  block_sum_store<1, kMaxHist + 1>(v, 1, bs.part);
-  if (!batch_last_chunk(bs, k)) return;
-  batch_sum_parts(bs, k, 1, tot);
-  if (threadIdx.x == 0) {
-    const int nsph = bs.off[k + 1] - bs.off[k];
-    norm[k] = sqrt(tot[0] / (double)max(nsph, 1));
-  }
-}
-cudaError_t launch_batch_residual(Launch L, const YlmTables& tb, const BatchState& bs,
-                                  const int* run, const double* rhs, const double* y,
-                                  const double* x, double* r, double* d, double* e,
-                                  double* norm) {
-  if (bs.nchunk == 0) return cudaSuccess;
-  k_batch_residual<<<bs.nchunk, kSolT, 0, L.st>>>(tb, bs, run, rhs, y, x, r, d, e, norm);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-
-__global__ void __launch_bounds__(kSolT) k_batch_update(const BatchState bs, int nylm,
-                                                        const int* __restrict__ upd,
-                                                        const double* __restrict__ e, double* x) {
-  const int c = blockIdx.x, k = bs.cmol[c];
-  if (upd[k] == 0) return;
-  const long long b0 = (long long)bs.off[k] * nylm + (long long)(c - bs.cfirst[k]) * kBChunk;
-  const int cnt = (int)min((long long)kBChunk, (long long)bs.off[k + 1] * nylm - b0);
-  for (int j = threadIdx.x; j < cnt; j += kSolT) x[b0 + j] += e[b0 + j];
-}
-cudaError_t launch_batch_update(Launch L, const BatchState& bs, int nylm, const int* upd,
-                                const double* e, double* x) {
-  if (bs.nchunk == 0) return cudaSuccess;
-  k_batch_update<<<bs.nchunk, kSolT, 0, L.st>>>(bs, nylm, upd, e, x);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-
 // per-molecule <a, b> (energy: fep * <X, psi>, cosmo.f90:155)
 __global__ void k_batch_dot(const int* __restrict__ off, int nylm, const double* __restrict__ a,
                             const double* __restrict__ b, double scale, double* out) {
