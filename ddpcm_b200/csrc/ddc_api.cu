@@ -168,6 +168,7 @@ struct ddc_ctx {
   // the mixed path, whose FP32 grid field pot_f has rows ldp_f floats apart
   DBuf basisT, bwT;
   TcPlan tc;
+  bool dmma_f32 = false;  // mixed: both contractions on the FP64 tensor cores
   int ldp_f = 0;
   // learned initial guess: the attached model, its feature rows, and flags
   // for the flows (rhs/psi/sigma/s of the last flow are valid; the initial
@@ -443,6 +444,10 @@ int check_count_total(ddc_ctx* ctx, const int* cnt, int n, const char* what) {
   return DDC_OK;
 }
 
+// most products (harmonics x spheres x grid points) of a contraction that the
+// mixed operators run on the FP64 tensor cores
+constexpr long long kDmmaProducts = 50000000;
+
 // ---------------------------------------------------------------------------
 // ddinit (ddcosmo.f90:159-483) on device buffers
 // ---------------------------------------------------------------------------
@@ -666,7 +671,13 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     // DDC_TC_OFF=1 in the environment selects the SIMT contractions (a
     // diagnostic switch: the tests compare the two paths' accuracy)
     const char* tc_off = std::getenv("DDC_TC_OFF");
-    const bool tc = tc_supported(NY) && !(tc_off && tc_off[0] == '1');
+    const bool tc_env = !(tc_off && tc_off[0] == '1');
+    // smaller molecules run them on the FP64 tensor cores instead, where the
+    // set-up of a tcgen05 tile is the larger part: 2,000 spheres, lmax 8, 302
+    // points (4.9e7 products) 15 / 16 us against 19 / 17 us; 5,000 spheres,
+    // lmax 6 (7.4e7) 21 / 22 against 21 / 19 us
+    ctx->dmma_f32 = tc_env && (long long)NY * NP <= kDmmaProducts;
+    const bool tc = tc_supported(NY) && tc_env && !ctx->dmma_f32;
     ctx->ldp_f = tc ? (G + 3) / 4 * 4 : G;
     CK(ctx->pot_f.ensure(sizeof(float) * std::max<long long>((long long)N * ctx->ldp_f, 1LL)));
     CK(ctx->xi_f.ensure(sizeof(float) * std::max(NP, 1LL)));
@@ -676,6 +687,8 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
       // tile widths by measurement (rhs and y are free work vectors here)
       CK(tc_autotune(L, ctx->tc, ctx->rhs.as<double>(), ctx->y.as<double>(),
                      ctx->xi_f.as<float>()));
+    } else if (ctx->dmma_f32) {
+      ctx->tc.on = false;
     } else {
       ctx->tc.on = false;
       CK(ctx->bw_f.ensure(sizeof(float) * G * NY));
@@ -769,7 +782,11 @@ int gemm_proj(ddc_ctx* ctx, double alpha, const double* pot, double* y) {
 }
 // projection of the FP32 field (rows ldp_f apart) into the FP64 vector y
 int gemm_proj_f32(ddc_ctx* ctx, float alpha, const float* pot, double* y) {
-  if (ctx->tc.on)
+  if (ctx->dmma_f32)
+    CK(launch_dgemm_nn(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, (double)alpha,
+                       ctx->bw.as<double>(), ctx->nylm, pot, ctx->ldp_f, y, ctx->nylm,
+                       ctx->sweep));
+  else if (ctx->tc.on)
     CK(launch_proj_tc(ctx->L(), ctx->tc, alpha, y, ctx->sweep));
   else
     CK(launch_proj_f32_simt(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, alpha,
@@ -785,7 +802,10 @@ int gemm_xi(ddc_ctx* ctx, const double* s, double* xig, bool weighted) {
 }
 // FP32 w_n xi of the FP64 vector s
 int gemm_xi_f32(ddc_ctx* ctx, const double* s, float* xig) {
-  if (ctx->tc.on)
+  if (ctx->dmma_f32)
+    CK(launch_dgemm_nn(ctx->L(), ctx->ngrid, ctx->nsph, ctx->nylm, 1.0, ctx->bwT.as<double>(),
+                       ctx->ngrid, s, ctx->nylm, xig, ctx->ngrid, ctx->sweep));
+  else if (ctx->tc.on)
     CK(launch_xi_tc(ctx->L(), ctx->tc, s, xig, ctx->sweep));
   else
     CK(launch_xi_f32_simt(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, ctx->bw_f.as<float>(),

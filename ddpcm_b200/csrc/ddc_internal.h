@@ -294,11 +294,17 @@ cudaError_t launch_lx_gather_f32(Launch L, const DevGeo& g, const float* val, fl
 cudaError_t launch_to_float(Launch L, long long n, const double* x, float* y);
 // dst[c*rows + r] = src[r*cols + c] (FP64)
 cudaError_t launch_transpose(Launch L, int rows, int cols, const double* src, double* dst);
-// C[n*ldc + m] = alpha * sum_k A[k*lda + m] B[n*ldb + k] (FP64, pipelined);
-// with act.mol set the N columns are spheres and tiles of skipped spheres
+// C[n*ldc + m] = alpha * sum_k A[k*lda + m] B[n*ldb + k] in FP64 arithmetic;
+// with act set the N columns are spheres and tiles of skipped spheres
 // are left alone
 cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
                             int lda, const double* B, int ldb, double* C, int ldc,
+                            const SweepMask& act = SweepMask{});
+cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
+                            int lda, const float* B, int ldb, double* C, int ldc,
+                            const SweepMask& act = SweepMask{});
+cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
+                            int lda, const double* B, int ldb, float* C, int ldc,
                             const SweepMask& act = SweepMask{});
 // FP32 SIMT projection / expansion (mixed path, more than 128 harmonics)
 cudaError_t launch_proj_f32_simt(Launch L, int nylm, int nsph, int ngrid, float alpha,

@@ -41,3 +41,25 @@ def test_operators_at_chunk_edges(oracle, kind, ngrid, lmax):
                 assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
         if kind == "pair":  # the lone sphere has no triples
             assert np.all(pair[0][-1] == 0.0) and np.all(pair[1][-1] == 0.0)
+
+
+@pytest.mark.parametrize("n,lmax,ngrid", [
+    (9, 8, 110),      # eight slices of k, the last block of spheres nearly empty
+    (1603, 8, 110),   # projection: 16 spheres per block; expansion: two slices
+    (1190, 10, 110),  # fewer points than harmonics
+    (14305, 2, 26)])  # staged 128 x 64 tiles
+def test_contractions_by_shape(oracle, n, lmax, ngrid):
+    """The projection and expansion GEMMs of every dispatch branch (remainders
+    in all three dimensions), through lx and lstarx."""
+    from ddpcm_b200 import molecules as M
+    from ddpcm_b200.ddcosmo import DDCosmo, PREC_FP64, PREC_MIXED
+    m = M.to_bohr(M.make_molecule(n, 900))
+    rng = np.random.default_rng(n)
+    x, s = rng.normal(size=(2, n, (lmax + 1) ** 2))
+    ref = oracle.RefDD(lmax, ngrid, 10, 1, 78.3553, 0.1).init(m["x"], m["y"], m["z"], m["r"])
+    want = ref.lx(x), ref.lstarx(s)
+    for prec, tol in ((PREC_FP64, 1e-13), (PREC_MIXED, 64 * 2.0 ** -24)):
+        with DDCosmo(lmax=lmax, ngrid=ngrid, iconv=10, eta=0.1, precision=prec) as dd:
+            dd.ddinit(m["x"], m["y"], m["z"], m["r"])
+            for a, b in zip(dd.lx_lstarx(x, s), want):
+                assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
