@@ -123,10 +123,10 @@ struct ddc_ctx {
   int nsph = 0, ncav = 0, nylm = 0, ngrid = 0, npair = 0;
   long long ntri = 0;
   std::vector<double> h_grid;  // x,y,z,w per point
-  std::vector<int> h_gord;     // grid points in patch order (k_fiui)
-  DBuf gord;
+  DBuf gpos;                   // position of each Lebedev point in the patch-ordered grid
   // geometry
-  DBuf sph, grid, basis, bw, fi, ui, zi, inl, nl, rev, pn_ptr, pn, pn_pair, ls_ptr, ls, ntri_pt;
+  DBuf sph, grid, basis, bw, fi, ui, zi, inl, nl, rev, pn_ptr, pn, ls_ptr, ls, ntri_pt, pt_ptr,
+      pt_idx;
   DBuf lsstart, fxa, fda, fvec;
   DBuf pn_bits;  // per pair, which grid points lie inside the neighbour (ddinit scratch)
   // batched molecules: partition, per-target N-body ranges, per-molecule DIIS state
@@ -144,7 +144,6 @@ struct ddc_ctx {
   SweepMask sweep{};    // set while a solver sweep is launched
   DBuf d_off, mrange, tr_cav, tr_nuc, b_out;
   const int2* mrange_ptr() const { return nmol > 1 ? mrange.as<int2>() : nullptr; }
-  int maxnb = 0;
   DBuf cavoff, cavidx, cavpt, ccav, cnt, scan_tmp;
   DBuf csph, cx, cy, cz;  // csph(3,n) and SoA centres
   // work
@@ -215,8 +214,8 @@ struct ddc_ctx {
     g.rev = rev.as<int>();
     g.pn_ptr = pn_ptr.as<int>();
     g.pn = pn.as<uint16_t>();
-    g.pn_pair = pn_pair.as<uint8_t>();
-    g.maxnb = maxnb;
+    g.pt_ptr = pt_ptr.as<int>();
+    g.pt_idx = pt_idx.as<int>();
     g.tgeo4 = tgeo_on ? tgeo4.as<float4>() : nullptr;
     g.tgeo4d = tgeo64_on ? tgeo4d.as<double4>() : nullptr;
     g.ls_ptr = ls_ptr.as<int>();
@@ -475,13 +474,13 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   else if (dsph != ctx->sph.as<double4>())
     CK(cudaMemcpyAsync(ctx->sph.p, dsph, sizeof(double4) * N, cudaMemcpyDeviceToDevice, ctx->st));
   CK(ctx->grid.ensure(sizeof(double4) * G));
-  CK(cudaMemcpyAsync(ctx->grid.p, ctx->h_grid.data(), sizeof(double4) * G, cudaMemcpyHostToDevice,
-                     ctx->st));
+  CK(ctx->gpos.ensure(sizeof(int) * G));
   {
-    // grid points in Morton order of their directions: 32 consecutive
-    // entries form a compact patch of the sphere, so that the warps of the
-    // per-point neighbour loop (k_fiui) skip whole neighbours whose cap
-    // misses their patch
+    // the grid in Morton order of the points' directions: 32 consecutive
+    // points form a compact patch of the sphere, so that a warp's points lie
+    // inside nearly the same neighbours (k_fiui skips together those that
+    // miss the patch; the triple values, the fields and the point lists that
+    // consecutive threads read are adjacent)
     std::vector<std::pair<uint64_t, int>> key(G);
     for (int k = 0; k < G; k++) {
       uint64_t m = 0;
@@ -493,10 +492,15 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
       key[k] = {m, k};
     }
     std::sort(key.begin(), key.end());
-    ctx->h_gord.resize(G);
-    for (int k = 0; k < G; k++) ctx->h_gord[k] = key[k].second;
-    CK(ctx->gord.ensure(sizeof(int) * G));
-    CK(cudaMemcpyAsync(ctx->gord.p, ctx->h_gord.data(), sizeof(int) * G, cudaMemcpyHostToDevice,
+    std::vector<double> g4(4 * (size_t)G);
+    std::vector<int> gpos(G);
+    for (int k = 0; k < G; k++) {
+      gpos[key[k].second] = k;
+      for (int d = 0; d < 4; d++) g4[4 * k + d] = ctx->h_grid[4 * key[k].second + d];
+    }
+    CK(cudaMemcpyAsync(ctx->grid.p, g4.data(), sizeof(double4) * G, cudaMemcpyHostToDevice,
+                       ctx->st));
+    CK(cudaMemcpyAsync(ctx->gpos.p, gpos.data(), sizeof(int) * G, cudaMemcpyHostToDevice,
                        ctx->st));
   }
   CK(ctx->basis.ensure(sizeof(double) * G * NY));
@@ -556,8 +560,7 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
     CKI(sync(ctx));
     int mx = 0;
     for (int i = 0; i < N; i++) mx = std::max(mx, h_inl[i + 1] - h_inl[i]);
-    ctx->maxnb = mx;
-    // the lx kernel indexes a sphere's neighbours with 8 bits (the reference
+    // a point's triples are counted with 8 bits (the reference
     // caps the list at nngmax = 100 per sphere on average, ddcosmo.f90:87)
     const size_t smem = 32 * (size_t)mx + 4 * (size_t)mx + 32 * (size_t)G;
     if (mx > 255 || smem > 200 * 1024)
@@ -580,7 +583,7 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   if (ctx->prm.igrad) CK(ctx->zi.ensure(sizeof(double) * 3 * std::max(NP, 1LL)));
   else ctx->zi.release();
   CK(launch_fiui(L, ctx->tb, N, ctx->sph.as<double4>(), ctx->grid.as<double4>(),
-                 ctx->gord.as<int>(), ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->fi.as<double>(),
+                 ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->fi.as<double>(),
                  ctx->ui.as<double>(),
                  ctx->prm.igrad ? ctx->zi.as<double>() : nullptr, ctx->ntri_pt.as<uint8_t>()));
   // cavity
@@ -596,7 +599,7 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   CK(ctx->cavidx.ensure(sizeof(int) * std::max(NP, 1LL)));
   CK(ctx->cavpt.ensure(sizeof(int) * std::max(ncav, 1)));
   CK(ctx->ccav.ensure(sizeof(double) * 3 * std::max(ncav, 1)));
-  CK(launch_cav_fill(L, N, G, ctx->ui.as<double>(), ctx->sph.as<double4>(),
+  CK(launch_cav_fill(L, N, G, ctx->gpos.as<int>(), ctx->ui.as<double>(), ctx->sph.as<double4>(),
                      ctx->grid.as<double4>(), ctx->cavoff.as<int>(), ctx->cavidx.as<int>(),
                      ctx->cavpt.as<int>(), ctx->ccav.as<double>()));
   // pair-major triple lists
@@ -619,10 +622,9 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   CKI(sync(ctx));
   ctx->ntri = ntri;
   CK(ctx->pn.ensure(sizeof(uint16_t) * std::max(ntri, 1)));
-  CK(ctx->pn_pair.ensure(std::max(ntri, 1)));
   CK(launch_pair_fill(L, N, npair, G, ctx->sph.as<double4>(), ctx->grid.as<double4>(),
                       ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->pn_bits.as<unsigned>(),
-                      ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>(), ctx->pn_pair.as<uint8_t>()));
+                      ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>()));
   CK(ctx->ls_ptr.ensure(sizeof(int) * (N + 1)));
   CK(cudaMemsetAsync(ctx->cnt.p, 0, sizeof(int) * (N + 1), ctx->st));
   CK(launch_ls_count(L, N, ctx->inl.as<int>(), ctx->rev.as<int>(), ctx->pn_ptr.as<int>(),
@@ -634,6 +636,11 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   CK(launch_ls_fill(L, N, ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->rev.as<int>(),
                     ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>(), ctx->ls_ptr.as<int>(), G,
                     ctx->ls.as<int>(), ctx->lsstart.as<int>()));
+  CK(ctx->pt_ptr.ensure(sizeof(int) * (size_t)(NP + 1)));
+  CK(ctx->pt_idx.ensure(sizeof(int) * std::max(ntri, 1)));
+  CK(launch_pt_fill(L, N, G, ctx->inl.as<int>(), ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>(),
+                    ctx->lsstart.as<int>(), ctx->ntri_pt.as<uint8_t>(), ctx->pt_ptr.as<int>(),
+                    ctx->pt_idx.as<int>()));
   // centres for the electrostatics
   CK(ctx->csph.ensure(sizeof(double) * 3 * std::max(N, 1)));
   CK(ctx->cx.ensure(sizeof(double) * std::max(N, 1)));
@@ -1593,7 +1600,15 @@ int ddc_get_ccav(ddc_ctx* ctx, double* ccav) {
 }
 int ddc_get_ui(ddc_ctx* ctx, double* ui) {
   CKI(need_ready(ctx));
-  return get_dev_array(ctx, ui, ctx->ui.p, (size_t)ctx->nsph * ctx->ngrid);
+  if (!ui) return fail(ctx, DDC_ERR_PARAM, "null output");
+  cudaSetDevice(ctx->prm.device);
+  const size_t np = (size_t)ctx->nsph * ctx->ngrid;
+  double* d;
+  CKI(out_ptr(ctx, ui, np, ctx->out1, &d));
+  CK(launch_grid_order(ctx->L(), ctx->nsph, ctx->ngrid, ctx->gpos.as<int>(), ctx->ui.as<double>(),
+                       d));
+  CKI(finish_out(ctx, ui, d, np));
+  return sync(ctx);
 }
 int ddc_get_csph(ddc_ctx* ctx, double* csph) {
   CKI(need_ready(ctx));

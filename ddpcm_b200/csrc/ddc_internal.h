@@ -3,7 +3,10 @@
 // Layout in HBM (one molecule per context, sizes for N spheres, G grid
 // points, Y = (lmax+1)^2 harmonics, P neighbour pairs, T triples):
 //   sph[N]         double4 {x, y, z, r} (bohr)
-//   grid[G]        double4 {sx, sy, sz, w} (unit vectors, 4pi-scaled weights)
+//   grid[G]        double4 {sx, sy, sz, w} (unit vectors, 4pi-scaled weights), in
+//                  patch (Morton) order: every grid index n below is in this
+//                  order; the cavity and the arrays that cross the interface
+//                  follow the Lebedev order (gpos)
 //   basis[G][Y]    Y_lm(s_n); bw[G][Y] = basis * w  (the intrhs operator)
 //   inl[N+1], nl[P]      CSR neighbour list, 0-based, ascending j (ddinit)
 //   rev[P]               index of (j,i) for the entry (i,j)
@@ -14,6 +17,7 @@
 //   ls_ptr[N+1], ls[T]   per sphere i: j * G + n for j in N_i (CSR order) and the
 //                        points n of sphere j inside sphere i (adjoint gather)
 //   ntri[N][G]           number of neighbours containing point (i,n)
+//   pt_ptr[N*G+1], pt_idx[T]  per point: where its triples sit in the gather lists
 //   cavoff[N+1], cavidx[N][G], cavpt[ncav], ccav[ncav][3]
 // Vectors X(nylm,nsph) live as X[i*nylm + lm], like the reference.
 #pragma once
@@ -129,7 +133,6 @@ __device__ __forceinline__ bool sweep_skip_tile(const SweepMask& m, int i0, int 
 
 struct DevGeo {
   int nsph, ngrid, nylm, ncav, npair;
-  int maxnb;  // largest neighbour count of a sphere
   // geometry (u, v, z, W) of each gather-list triple (ddc_lxs.cu): FP32 in
   // the mixed path, FP64 in the FP64 path; null if absent
   const float4* tgeo4;
@@ -147,9 +150,10 @@ struct DevGeo {
   const int* rev;
   const int* pn_ptr;
   const uint16_t* pn;
-  const uint8_t* pn_pair;  // local index (within the sphere's CSR range) of each triple's pair
   const int* ls_ptr;
   const int* ls;  // gather list: a * ngrid + n of each triple
+  const int* pt_ptr;   // per point (a, n): its entries of pt_idx
+  const int* pt_idx;   // positions of its triples in the gather lists, CSR order
   const int* lsstart;  // per CSR entry (j,i): start of that pair's block in i's gather list
   const uint8_t* ntri_pt;
   const int* cavoff;
@@ -235,27 +239,30 @@ cudaError_t launch_csr_count(Launch L, int nsph, const double4* sph, int* cnt,
 cudaError_t launch_csr_fill(Launch L, int nsph, const double4* sph, const int* inl, int* nl,
                             const int2* mrange);
 cudaError_t launch_csr_rev(Launch L, int nsph, const int* inl, const int* nl, int* rev);
-// gord: the grid points in patch order (the threads of a warp take 32
-// consecutive entries of one sphere)
 cudaError_t launch_fiui(Launch L, const YlmTables& tb, int nsph, const double4* sph,
-                        const double4* grid, const int* gord, const int* inl, const int* nl,
+                        const double4* grid, const int* inl, const int* nl,
                         double* fi, double* ui, double* zi, uint8_t* ntri);
 cudaError_t launch_cav_count(Launch L, int nsph, int ngrid, const double* ui, int* cnt);
-cudaError_t launch_cav_fill(Launch L, int nsph, int ngrid, const double* ui, const double4* sph,
-                            const double4* grid, const int* cavoff, int* cavidx, int* cavpt,
-                            double* ccav);
+// gpos: position of each Lebedev point in the grid (which is in patch order)
+cudaError_t launch_cav_fill(Launch L, int nsph, int ngrid, const int* gpos, const double* ui,
+                            const double4* sph, const double4* grid, const int* cavoff,
+                            int* cavidx, int* cavpt, double* ccav);
+cudaError_t launch_grid_order(Launch L, int nsph, int ngrid, const int* gpos, const double* f,
+                              double* out);
 cudaError_t launch_pair_count(Launch L, int nsph, int npair, int ngrid, const double4* sph,
                               const double4* grid, const int* inl, const int* nl, int* cnt,
                               unsigned* bits);  // bits: [npair][ceil(ngrid / 32)] words
 cudaError_t launch_pair_fill(Launch L, int nsph, int npair, int ngrid, const double4* sph,
                              const double4* grid, const int* inl, const int* nl,
-                             const unsigned* bits, const int* pn_ptr, uint16_t* pn,
-                             uint8_t* pn_pair);
+                             const unsigned* bits, const int* pn_ptr, uint16_t* pn);
 cudaError_t launch_ls_count(Launch L, int nsph, const int* inl, const int* rev, const int* pn_ptr,
                             int* cnt);
 cudaError_t launch_ls_fill(Launch L, int nsph, const int* inl, const int* nl, const int* rev,
                            const int* pn_ptr, const uint16_t* pn, const int* ls_ptr, int ngrid,
                            int* ls, int* lsstart);
+cudaError_t launch_pt_fill(Launch L, int nsph, int ngrid, const int* inl, const int* pn_ptr,
+                           const uint16_t* pn, const int* lsstart, const uint8_t* ntri,
+                           int* pt_ptr, int* pt_idx);
 // exclusive scan of n ints (out[n] = total); temp is device scratch of temp_bytes
 cudaError_t scan_exclusive(Launch L, const int* in, int* out, int n, void* temp,
                            size_t temp_bytes);

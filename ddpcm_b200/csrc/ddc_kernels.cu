@@ -287,22 +287,21 @@ cudaError_t launch_csr_rev(Launch L, int nsph, const int* inl, const int* nl, in
 
 // ---------------------------------------------------------------------------
 // fi, ui, zi (ddcosmo.f90:363-411) and the per-point count of containing
-// neighbours.  Thread per (sphere, grid point); a sphere's points are taken
-// in patch order, padded to whole warps, so that a warp's 32 points lie
+// neighbours.  Thread per (sphere, grid point); a sphere's points (in patch
+// order, as the whole grid is kept) are padded to whole warps, so that a warp's 32 points lie
 // close together on the sphere and skip together the neighbours whose cap
 // they all miss (rel_outside: those add exactly nothing).  Each point sums
 // its neighbours in CSR order, as the reference does.
 // ---------------------------------------------------------------------------
 __global__ void k_fiui(const YlmTables tb, int nsph, const double4* __restrict__ sph,
-                       const double4* __restrict__ grid, const int* __restrict__ gord,
+                       const double4* __restrict__ grid,
                        const int* __restrict__ inl, const int* __restrict__ nl, double* fi,
                        double* ui, double* zi, uint8_t* ntri) {
   const int G = tb.ngrid, GP = (G + 31) & ~31;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)nsph * GP) return;
-  const int i = (int)(t / GP), slot = (int)(t - (long long)i * GP);
-  if (slot >= G) return;
-  const int n = gord[slot];
+  const int i = (int)(t / GP), n = (int)(t - (long long)i * GP);
+  if (n >= G) return;
   const long long p = (long long)i * G + n;
   double4 ci = sph[i], g = grid[n];
   double f = 0.0, zx = 0.0, zy = 0.0, zz = 0.0;
@@ -332,11 +331,11 @@ __global__ void k_fiui(const YlmTables tb, int nsph, const double4* __restrict__
   }
 }
 cudaError_t launch_fiui(Launch L, const YlmTables& tb, int nsph, const double4* sph,
-                        const double4* grid, const int* gord, const int* inl, const int* nl,
+                        const double4* grid, const int* inl, const int* nl,
                         double* fi, double* ui, double* zi, uint8_t* ntri) {
   const long long nt = (long long)nsph * ((tb.ngrid + 31) & ~31);
   if (nt == 0) return cudaSuccess;
-  k_fiui<<<(unsigned)((nt + 255) / 256), 256, 0, L.st>>>(tb, nsph, sph, grid, gord, inl, nl, fi,
+  k_fiui<<<(unsigned)((nt + 255) / 256), 256, 0, L.st>>>(tb, nsph, sph, grid, inl, nl, fi,
                                                          ui, zi, ntri);
   ++*L.launches;
   return cudaGetLastError();
@@ -361,7 +360,7 @@ cudaError_t launch_cav_count(Launch L, int nsph, int ngrid, const double* ui, in
   return cudaGetLastError();
 }
 
-__global__ void k_cav_fill(int ngrid, const double* __restrict__ ui,
+__global__ void k_cav_fill(int ngrid, const int* __restrict__ gpos, const double* __restrict__ ui,
                            const double4* __restrict__ sph, const double4* __restrict__ grid,
                            const int* __restrict__ cavoff, int* cavidx, int* cavpt, double* ccav) {
   int i = blockIdx.x;
@@ -371,8 +370,9 @@ __global__ void k_cav_fill(int ngrid, const double* __restrict__ ui,
   if (threadIdx.x == 0) carry = cavoff[i];
   __syncthreads();
   double4 ci = sph[i];
+  // the cavity is numbered in the Lebedev order: point o sits at gpos[o]
   for (int n0 = 0; n0 < ngrid; n0 += 256) {
-    int n = n0 + threadIdx.x;
+    const int o = n0 + threadIdx.x, n = o < ngrid ? gpos[o] : ngrid;
     size_t p = (size_t)i * ngrid + n;
     int flag = (n < ngrid && ui[p] > 0.0) ? 1 : 0;
     int pos, tot;
@@ -396,11 +396,28 @@ __global__ void k_cav_fill(int ngrid, const double* __restrict__ ui,
     __syncthreads();
   }
 }
-cudaError_t launch_cav_fill(Launch L, int nsph, int ngrid, const double* ui, const double4* sph,
-                            const double4* grid, const int* cavoff, int* cavidx, int* cavpt,
-                            double* ccav) {
+cudaError_t launch_cav_fill(Launch L, int nsph, int ngrid, const int* gpos, const double* ui,
+                            const double4* sph, const double4* grid, const int* cavoff,
+                            int* cavidx, int* cavpt, double* ccav) {
   if (nsph == 0) return cudaSuccess;
-  k_cav_fill<<<nsph, 256, 0, L.st>>>(ngrid, ui, sph, grid, cavoff, cavidx, cavpt, ccav);
+  k_cav_fill<<<nsph, 256, 0, L.st>>>(ngrid, gpos, ui, sph, grid, cavoff, cavidx, cavpt, ccav);
+  ++*L.launches;
+  return cudaGetLastError();
+}
+
+// out(o, i) = ui(gpos[o], i): a grid field in the Lebedev order
+__global__ void k_grid_order(long long np, int ngrid, const int* __restrict__ gpos,
+                             const double* __restrict__ f, double* out) {
+  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= np) return;
+  const int o = (int)(p % ngrid);
+  out[p] = f[p - o + gpos[o]];
+}
+cudaError_t launch_grid_order(Launch L, int nsph, int ngrid, const int* gpos, const double* f,
+                              double* out) {
+  const long long np = (long long)nsph * ngrid;
+  if (np == 0) return cudaSuccess;
+  k_grid_order<<<(unsigned)((np + 255) / 256), 256, 0, L.st>>>(np, ngrid, gpos, f, out);
   ++*L.launches;
   return cudaGetLastError();
 }
@@ -417,7 +434,7 @@ template <bool FILL>
 __global__ void k_pairs(int nsph, int npair, int ngrid, const double4* __restrict__ sph,
                         const double4* __restrict__ grid, const int* __restrict__ inl,
                         const int* __restrict__ nl, int* cnt, unsigned* __restrict__ bits,
-                        const int* pn_ptr, uint16_t* pn, uint8_t* pn_pair) {
+                        const int* pn_ptr, uint16_t* pn) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= npair) return;
   const int k = warp;
@@ -443,19 +460,12 @@ __global__ void k_pairs(int nsph, int npair, int ngrid, const double4* __restric
     }
     if (lane == 0) cnt[k] = total;
   } else {
-    int lo = 0, hi = nsph - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (inl[mid] <= k) lo = mid; else hi = mid - 1;
-    }
-    const int i = lo;
     int base = pn_ptr[k];
     for (int w = 0; w < nw; ++w) {
       const unsigned mask = kb[w];
       if ((mask >> lane) & 1u) {
         const int pos = base + __popc(mask & ((1u << lane) - 1u));
         pn[pos] = (uint16_t)(32 * w + lane);
-        pn_pair[pos] = (uint8_t)(k - inl[i]);
       }
       base += __popc(mask);
     }
@@ -466,18 +476,17 @@ cudaError_t launch_pair_count(Launch L, int nsph, int npair, int ngrid, const do
                               unsigned* bits) {
   if (npair == 0) return cudaSuccess;
   k_pairs<false><<<(npair + 7) / 8, 256, 0, L.st>>>(nsph, npair, ngrid, sph, grid, inl, nl, cnt,
-                                                    bits, nullptr, nullptr, nullptr);
+                                                    bits, nullptr, nullptr);
   ++*L.launches;
   return cudaGetLastError();
 }
 cudaError_t launch_pair_fill(Launch L, int nsph, int npair, int ngrid, const double4* sph,
                              const double4* grid, const int* inl, const int* nl,
-                             const unsigned* bits, const int* pn_ptr, uint16_t* pn,
-                             uint8_t* pn_pair) {
+                             const unsigned* bits, const int* pn_ptr, uint16_t* pn) {
   if (npair == 0) return cudaSuccess;
   k_pairs<true><<<(npair + 7) / 8, 256, 0, L.st>>>(nsph, npair, ngrid, sph, grid, inl, nl,
                                                    nullptr, const_cast<unsigned*>(bits), pn_ptr,
-                                                   pn, pn_pair);
+                                                   pn);
   ++*L.launches;
   return cudaGetLastError();
 }
@@ -2169,81 +2178,126 @@ __device__ __forceinline__ void lxs_finish_role(int role, const YlmTables& tb, R
     lxs_finish_role<LMAX, NR, R + 1, Rl, GAM, G>(role, tb, acc, yi, lane);
 }
 
-// pot_a(n) = sum over a's CSR pairs (a, b), in CSR order, of the lx values
-// of the triples (a, n, b), read from b's gather list at the pair's block
-// (lsstart).  Warp per sphere a, with a private shared row of ngrid values
-// and the pairs' bounds staged in shared memory: lanes take the pair's
-// points (distinct within a pair, so no two lanes touch one entry), four
-// strided loads per lane, and the next pair's first loads are issued before
-// the current pair's adds; a __syncwarp between pairs orders the updates of
-// a point by its pairs.  chi: the sums times max(f_a(n), 1), i.e. with the
-// weight chi(t) of u_chi in place of chi(t) / f_a(n).  No block barriers (each warp runs its sphere from
-// start to end) and no atomics: a fixed summation order.
-constexpr int kGatherWarps = 4;  // spheres per block
-template <class Rl>
-__global__ void __launch_bounds__(32 * kGatherWarps)
-    k_lx_gather(const DevGeo g, const Rl* __restrict__ val, Rl* pot, int ldp, bool chi) {
-  constexpr int U = 4;
+// ---------------------------------------------------------------------------
+// point lists: for every (a, n) the positions, in the neighbours' gather
+// lists, of the triples (a, n, b), in a's CSR order.  Sphere a's entries take
+// the range of its pair lists; pt_ptr counts through it point by point.
+// Warp per sphere: prefix sums of the points' triple counts, then the pairs
+// one after the other (a pair's points are distinct).
+// ---------------------------------------------------------------------------
+constexpr int kPtWarps = 4;
+__global__ void __launch_bounds__(32 * kPtWarps)
+    k_pt_fill(int nsph, int ngrid, const int* __restrict__ inl, const int* __restrict__ pn_ptr,
+              const uint16_t* __restrict__ pn, const int* __restrict__ lsstart,
+              const uint8_t* __restrict__ ntri, int* pt_ptr, int* pt_idx) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int G = g.ngrid;
-  const int mb = (g.maxnb + 3) & ~3;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int a = blockIdx.x * kGatherWarps + w;
-  // warp-uniform; the kernel has no block barriers
-  if (a >= g.nsph || sweep_skip(g.act, a)) return;
-  // per warp: pst[mb + 4] (pn_ptr of the pairs), dl[mb] (lsstart - pn_ptr),
-  // then the row (16-byte aligned: mb is a multiple of four)
-  int* pst = reinterpret_cast<int*>(smraw) + (size_t)w * (2 * mb + 4);
-  int* dl = pst + mb + 4;
-  Rl* row = reinterpret_cast<Rl*>(reinterpret_cast<int*>(smraw) + kGatherWarps * (2 * mb + 4)) +
-            (size_t)w * G;
-  const int k0 = g.inl[a], nn = g.inl[a + 1] - k0;
-  for (int k = lane; k <= nn; k += 32) pst[k] = g.pn_ptr[k0 + k];
-  for (int k = lane; k < nn; k += 32) dl[k] = g.lsstart[k0 + k] - g.pn_ptr[k0 + k];
-  for (int n = lane; n < G; n += 32) row[n] = Rl(0);
-  __syncwarp();
-  auto load = [&](int base, int q1, int d, int* n, Rl* v) {
+  const int a = blockIdx.x * kPtWarps + w;
+  if (a >= nsph) return;  // warp-uniform; no block barriers
+  int* cur = reinterpret_cast<int*>(smraw) + (size_t)w * ngrid;
+  const size_t p0 = (size_t)a * ngrid;
+  int run = pn_ptr[inl[a]];
+  for (int n0 = 0; n0 < ngrid; n0 += 32) {
+    const int n = n0 + lane, c = n < ngrid ? ntri[p0 + n] : 0;
+    int v = c;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int q = base + 32 * u;
-      n[u] = q < q1 ? (int)g.pn[q] : -1;
-      v[u] = q < q1 ? val[q + d] : Rl(0);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
     }
-  };
-  auto add = [&](const int* n, const Rl* v) {
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (n[u] >= 0) row[n[u]] += v[u];
-  };
-  int cn[U];
-  Rl cv[U];
-  if (nn > 0) load(pst[0] + lane, pst[1], dl[0], cn, cv);
-  for (int p = 0; p < nn; ++p) {
-    const int q0 = pst[p], q1 = pst[p + 1], d = dl[p];
-    int nn1[U];
-    Rl nv1[U];
-    const bool more = p + 1 < nn;
-    if (more) load(pst[p + 1] + lane, pst[p + 2], dl[p + 1], nn1, nv1);
-    add(cn, cv);
-    for (int base = q0 + lane + 32 * U; base < q1; base += 32 * U) {
-      int n2[U];
-      Rl v2[U];
-      load(base, q1, d, n2, v2);
-      add(n2, v2);
+    if (n < ngrid) {
+      cur[n] = run + v - c;
+      pt_ptr[p0 + n] = run + v - c;
+    }
+    run += __shfl_sync(0xffffffffu, v, 31);
+  }
+  if (a == nsph - 1 && lane == 0) pt_ptr[p0 + ngrid] = run;
+  __syncwarp();
+  for (int k = inl[a]; k < inl[a + 1]; ++k) {
+    const int q0 = pn_ptr[k], q1 = pn_ptr[k + 1], base = lsstart[k] - q0;
+    for (int q = q0 + lane; q < q1; q += 32) {
+      const int n = pn[q], at = cur[n];
+      cur[n] = at + 1;
+      pt_idx[at] = base + q;
     }
     __syncwarp();
-    if (more) {
+  }
+}
+cudaError_t launch_pt_fill(Launch L, int nsph, int ngrid, const int* inl, const int* pn_ptr,
+                           const uint16_t* pn, const int* lsstart, const uint8_t* ntri,
+                           int* pt_ptr, int* pt_idx) {
+  if (nsph == 0) return cudaSuccess;
+  const size_t sm = sizeof(int) * kPtWarps * ngrid;
+  if (sm > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_pt_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e) return e;
+  }
+  k_pt_fill<<<(nsph + kPtWarps - 1) / kPtWarps, 32 * kPtWarps, sm, L.st>>>(
+      nsph, ngrid, inl, pn_ptr, pn, lsstart, ntri, pt_ptr, pt_idx);
+  ++*L.launches;
+  return cudaGetLastError();
+}
+
+// pot_a(n) = sum of the lx values of the triples of (a, n), in CSR order.
+// Thread per point: a list has 3 entries on average, and consecutive threads
+// (neighbouring points: the grid is in patch order) lie inside nearly the
+// same neighbours, whose values are adjacent.  chi: the sums times
+// max(f_a(n), 1), i.e. with the weight chi(t) of u_chi in place of
+// chi(t) / f_a(n).  Fixed order, no atomics.  Bound: latency of the chain
+// list bounds -> positions -> values for few points, HBM for many (0.4 GB at
+// 20,000 spheres, lmax 10, 590 points).  Two points per thread: one is 123
+// us there, two 83 us, four 84 us.  The warp-per-sphere form that this
+// replaces walked a sphere's 20 or so pairs one after the other: 113 us there
+// (FP64 151, now 102), 37 us at 5,000 spheres and 302 points (now 19), 21 us
+// at 600 spheres (now 9).
+constexpr int kPtPoints = 2;
+template <class Rl>
+__global__ void __launch_bounds__(256)
+    k_lx_gather(const DevGeo g, const Rl* __restrict__ val, Rl* pot, int ldp, bool chi) {
+  constexpr int P = kPtPoints;
+  constexpr int U = 4;  // triples of a point in flight
+  const int np = g.nsph * g.ngrid;
+  int q[P], q1[P];
+  Rl v[P];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        cn[u] = nn1[u];
-        cv[u] = nv1[u];
-      }
+  for (int i = 0; i < P; ++i) {
+    const int p = (blockIdx.x * P + i) * 256 + threadIdx.x;
+    q[i] = q1[i] = 0;
+    v[i] = 0;
+    if (p < np && !sweep_skip(g.act, p / g.ngrid)) {
+      q[i] = g.pt_ptr[p];
+      q1[i] = g.pt_ptr[p + 1];
     }
   }
-  for (int n = lane; n < G; n += 32) {
-    Rl v = row[n];
-    if (chi) v *= (Rl)fmax(g.fi[(size_t)a * G + n], 1.0);
-    pot[(size_t)a * ldp + n] = v;
+  for (bool more = true; more;) {
+    int at[P][U];
+    Rl x[P][U];
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+#pragma unroll
+      for (int u = 0; u < U; ++u) at[i][u] = q[i] + u < q1[i] ? g.pt_idx[q[i] + u] : -1;
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[i][u] = at[i][u] >= 0 ? val[at[i][u]] : Rl(0);
+    more = false;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[i] += x[i][u];
+      q[i] += U;
+      more |= q[i] < q1[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const int p = (blockIdx.x * P + i) * 256 + threadIdx.x;
+    if (p >= np) continue;
+    const int a = p / g.ngrid;
+    if (sweep_skip(g.act, a)) continue;
+    if (chi) v[i] *= (Rl)fmax(g.fi[p], 1.0);
+    pot[(size_t)a * ldp + (p - a * g.ngrid)] = v[i];
   }
 }
 
@@ -2251,14 +2305,8 @@ template <class Rl>
 static cudaError_t gather_launch(Launch L, const DevGeo& g, const Rl* val, Rl* pot, int ldp,
                                  bool chi) {
   if (g.nsph == 0) return cudaSuccess;
-  const int mb = (g.maxnb + 3) & ~3;
-  const size_t sm = kGatherWarps * (sizeof(int) * (2 * mb + 4) + sizeof(Rl) * g.ngrid);
-  cudaError_t e;
-  if (sm > 48 * 1024)
-    if ((e = cudaFuncSetAttribute(k_lx_gather<Rl>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sm)))
-      return e;
-  k_lx_gather<Rl><<<(g.nsph + kGatherWarps - 1) / kGatherWarps, 32 * kGatherWarps, sm, L.st>>>(
+  const long long np = (long long)g.nsph * g.ngrid;
+  k_lx_gather<Rl><<<(unsigned)((np + 256 * kPtPoints - 1) / (256 * kPtPoints)), 256, 0, L.st>>>(
       g, val, pot, ldp, chi);
   ++*L.launches;
   return cudaGetLastError();
