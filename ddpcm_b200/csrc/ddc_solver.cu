@@ -128,68 +128,58 @@ __device__ __forceinline__ void sum_parts(const SolverArgs& a, const SolverSys& 
 // n x n system, n <= 32, by the whole block: thread (w, lane) holds column
 // `lane` of the rows w, w + 8, w + 16, w + 24 in a[], the rows' right-hand
 // sides in b[] (every lane).  The pivot is the largest |a| over free rows and
-// columns, the first in the reference's scan order (rows outer, columns
-// inner) on ties; rows stay in place (row[c] is the row that column c was
-// pivoted in) instead of being swapped, which changes no value.  Each warp
-// offers its best candidate with that row, one barrier, and every warp
-// eliminates in its own rows.  Solution in x[0..n); false when singular.
+// columns, compared by its high word (to 20 bits of the mantissa), the first
+// in the reference's scan order (rows outer, columns inner) among equals;
+// rows stay in place (myrow: the row that column `lane` was pivoted in)
+// instead of being swapped, which changes no value.  A chain of n dependent
+// pivots, each some hundred cycles of latency: one barrier per pivot, the
+// rows mirrored in shared memory as they are updated, so that every warp
+// reads the pivot row of whichever warp offers it; 650 cycles per pivot
+// (1,500 when the warps compared and handed over FP64 candidates).  Solution
+// in x[0..n); false when singular.
 __device__ bool gauss_jordan(int n, double (&a)[4], double (&b)[4], double* x) {
-  __shared__ double crow[2][kW][32], cb[2][kW];
-  __shared__ double cv[2][kW];
-  __shared__ int crc[2][kW];
+  __shared__ double mir[2][32][33];  // the matrix and (column 32) the right-hand side
+  __shared__ uint2 cand[2][kW];      // high word and position of each warp's candidate
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned rused = 0, cused = 0;  // pivoted rows and columns
-  int myrow = -1;                 // the row column `lane` was pivoted in
+  unsigned rfree = 0;  // rows of this warp (bit u) not pivoted yet
+#pragma unroll
+  for (int u = 0; u < 4; ++u) rfree |= (w + 8 * u < n ? 1u : 0u) << u;
+  bool cfree = lane < n;
+  int myrow = -1;  // the row column `lane` was pivoted in
   for (int i = 0; i < n; ++i) {
     const int buf = i & 1;
-    double best = 0.0;
-    int code = INT_MAX;  // row * 32 + column
-    if (lane < n && !((cused >> lane) & 1u)) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int r = w + 8 * u;
-        const double v = fabs(a[u]);
-        if (r < n && !((rused >> r) & 1u) && v > best) {
-          best = v;
-          code = r * 32 + lane;
-        }
-      }
-    }
-    // the warp's maximum: high words, low words, then the first position
-    const unsigned hi = (unsigned)__double2hiint(best);
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned lo = hi == mh ? (unsigned)__double2loint(best) : 0u;
-    const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-    const int pos = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? code : INT_MAX);
-    const double wv = __hiloint2double((int)mh, (int)ml);
-    if (pos != INT_MAX) {
-      const int u = (pos >> 5) >> 3;
-      crow[buf][w][lane] = u == 0 ? a[0] : u == 1 ? a[1] : u == 2 ? a[2] : a[3];
-      if (lane == 0) cb[buf][w] = u == 0 ? b[0] : u == 1 ? b[1] : u == 2 ? b[2] : b[3];
-    }
-    if (lane == 0) {
-      cv[buf][w] = wv;
-      crc[buf][w] = pos;
-    }
-    __syncthreads();
-    int wb = 0;
-#pragma unroll
-    for (int q = 1; q < kW; ++q)
-      if (cv[buf][q] > cv[buf][wb] || (cv[buf][q] == cv[buf][wb] && crc[buf][q] < crc[buf][wb]))
-        wb = q;
-    const int rc = crc[buf][wb];
-    if (rc == INT_MAX) return false;  // no non-zero free entry (NaN included)
-    const int r = rc >> 5, c = rc & 31;
-    const double pinv = 1.0 / crow[buf][wb][c];
-    const double pr = crow[buf][wb][lane] * pinv, pb = cb[buf][wb] * pinv;
-    rused |= 1u << r;
-    cused |= 1u << c;
-    if (lane == c) myrow = r;
+    unsigned key = 0, code = 0xffffffffu;  // position: row * 32 + column
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int row = w + 8 * u;
-      const double dum = __shfl_sync(0xffffffffu, a[u], c);
-      if (row == r) {
+      mir[buf][w + 8 * u][lane] = a[u];
+      if (lane == 0) mir[buf][w + 8 * u][32] = b[u];
+      const unsigned h = (rfree >> u) & 1u ? (unsigned)__double2hiint(a[u]) & 0x7fffffffu : 0u;
+      if (h > key) {
+        key = h;
+        code = (w + 8 * u) * 32 + lane;
+      }
+    }
+    if (!cfree) key = 0;
+    const unsigned mk = __reduce_max_sync(0xffffffffu, key);
+    const unsigned pos = __reduce_min_sync(0xffffffffu, key == mk && key ? code : 0xffffffffu);
+    if (lane == 0) cand[buf][w] = make_uint2(mk, pos);
+    __syncthreads();
+    const uint2 cd = cand[buf][lane & (kW - 1)];
+    const unsigned bk = __reduce_max_sync(0xffffffffu, cd.x);
+    if (!bk) return false;  // no non-zero free entry
+    const unsigned rc = __reduce_min_sync(0xffffffffu, cd.x == bk ? cd.y : 0xffffffffu);
+    const int r = rc >> 5, c = rc & 31;
+    const double pinv = 1.0 / mir[buf][r][c];
+    const double pr = mir[buf][r][lane] * pinv, pb = mir[buf][r][32] * pinv;
+    if ((r & (kW - 1)) == w) rfree &= ~(1u << (r >> 3));
+    if (lane == c) {
+      cfree = false;
+      myrow = r;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double dum = mir[buf][w + 8 * u][c];
+      if (w + 8 * u == r) {
         a[u] = pr;
         b[u] = pb;
       } else {
