@@ -120,6 +120,7 @@ struct ddc_ctx {
   long long st_calls[ST_N] = {0};
   std::string err;
   bool ready = false;
+  bool lxs_ready = false;  // attributes of the triple kernels are set
   int nsph = 0, ncav = 0, nylm = 0, ngrid = 0, npair = 0;
   long long ntri = 0;
   std::vector<double> h_grid;  // x,y,z,w per point
@@ -458,6 +459,10 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   ctx->nylm = (ctx->prm.lmax + 1) * (ctx->prm.lmax + 1);
   ctx->ngrid = snap_ngrid(ctx->prm.ngrid);
   build_tables(ctx);
+  if (!ctx->lxs_ready) {
+    CK(prepare_lxs(ctx->prm.lmax));
+    ctx->lxs_ready = true;
+  }
   if (!lebedev(ctx->ngrid, ctx->h_grid)) return fail(ctx, DDC_ERR_PARAM, "bad Lebedev size");
   const int N = n, G = ctx->ngrid, NY = ctx->nylm;
   const long long NP = (long long)N * G;

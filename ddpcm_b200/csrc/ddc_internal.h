@@ -116,6 +116,31 @@ struct SweepMask {
 };
 
 #ifdef __CUDACC__
+// The kernels of a solver sweep follow one another with a dependency on all
+// of the previous kernel.  Launched with launch_chained they are scheduled
+// while that kernel still runs (programmatic dependent launch) and begin with
+// chain_wait, which every thread of them executes before anything else: it
+// returns when the previous kernel has finished and its writes are visible.
+// Saves about 1 us between two kernels.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kfn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                           A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kfn, static_cast<P>(args)...);
+}
 // True for a sphere of a molecule whose systems have all stopped.
 __device__ __forceinline__ bool sweep_skip(const SweepMask& m, int sph) {
   if (!m.st0) return false;
@@ -287,6 +312,8 @@ cudaError_t launch_lx_vals_f32(Launch L, const YlmTables& tb, const DevGeo& g, c
                                float* val);
 cudaError_t launch_lstarx_acc_f32(Launch L, const YlmTables& tb, const DevGeo& g,
                                   const float* xi, double* y);
+// attributes of those kernels for one degree, once per context and device
+cudaError_t prepare_lxs(int lmax);
 // the triples' geometry (g.tgeo4, g.tgeo4d), once per molecule
 cudaError_t launch_lxs_geo(Launch L, const YlmTables& tb, const DevGeo& g, float4* tg);
 cudaError_t launch_lxs_geo_f64(Launch L, const YlmTables& tb, const DevGeo& g, double4* tg);

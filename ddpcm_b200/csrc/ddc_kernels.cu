@@ -737,6 +737,7 @@ __global__ void __launch_bounds__(256) k_dmma(int M, int N, int K, double alpha,
                                               const double* __restrict__ A, int lda,
                                               const TB* __restrict__ B, int ldb,
                                               TC* __restrict__ C, int ldc, const SweepMask act) {
+  chain_wait();
   constexpr int MT = 4, MG = 8 / KS;  // 8-row tiles per warp, row groups per block
   constexpr int TS = MT * NB * 64;    // values of a warp's tile
   extern __shared__ __align__(16) double dm_smem[];  // [KS - 1][MG][TS]
@@ -838,9 +839,8 @@ static cudaError_t dmma_launch(Launch L, int M, int N, int K, double alpha, cons
     if (e) return e;
   }
   const dim3 grid((N + 8 * NB - 1) / (8 * NB), (M + 32 * MG - 1) / (32 * MG));
-  kfn<<<grid, 256, sm, L.st>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
   ++*L.launches;
-  return cudaGetLastError();
+  return launch_chained(kfn, grid, 256, sm, L.st, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
 }
 // The same product for shapes of many tiles (B and C in FP64):
 // 128 x 64 tiles, 8 warps of 32 x 32 (4 x 4 MMA tiles of 8 x 8), 16-deep k
@@ -865,6 +865,7 @@ __global__ void __launch_bounds__(256, 3) k_dgemm_dmma(int M, int N, int K, doub
                                                        const double* __restrict__ B, int ldb,
                                                        double* __restrict__ C, int ldc,
                                                        const SweepMask act) {
+  chain_wait();
   using namespace dgp;
   extern __shared__ __align__(16) double dg_smem[];
   double* As = dg_smem;                // [2][BK][AS]
@@ -974,9 +975,9 @@ cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const d
   cudaError_t e = cudaFuncSetAttribute(k_dgemm_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        dgp::SMEM);
   if (e) return e;
-  k_dgemm_dmma<<<grid, 256, dgp::SMEM, L.st>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
   ++*L.launches;
-  return cudaGetLastError();
+  return launch_chained(k_dgemm_dmma, grid, 256, dgp::SMEM, L.st, M, N, K, alpha, A, lda, B, ldb, C,
+                        ldc, act);
 }
 cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
                             int lda, const float* B, int ldb, double* C, int ldc,
@@ -2255,6 +2256,7 @@ constexpr int kPtPoints = 2;
 template <class Rl>
 __global__ void __launch_bounds__(256)
     k_lx_gather(const DevGeo g, const Rl* __restrict__ val, Rl* pot, int ldp, bool chi) {
+  chain_wait();
   constexpr int P = kPtPoints;
   constexpr int U = 4;  // triples of a point in flight
   const int np = g.nsph * g.ngrid;
@@ -2306,10 +2308,9 @@ static cudaError_t gather_launch(Launch L, const DevGeo& g, const Rl* val, Rl* p
                                  bool chi) {
   if (g.nsph == 0) return cudaSuccess;
   const long long np = (long long)g.nsph * g.ngrid;
-  k_lx_gather<Rl><<<(unsigned)((np + 256 * kPtPoints - 1) / (256 * kPtPoints)), 256, 0, L.st>>>(
-      g, val, pot, ldp, chi);
   ++*L.launches;
-  return cudaGetLastError();
+  return launch_chained(k_lx_gather<Rl>, dim3((unsigned)((np + 256 * kPtPoints - 1) / (256 * kPtPoints))),
+                        256, 0, L.st, g, val, pot, ldp, chi);
 }
 cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, double* pot,
                              bool chi) {

@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(32 * nroles<Rl>(LMAX), min_blocks<Rl>(LMAX))
     k_lxs(const __grid_constant__ LxsTab tb, const DevGeo g,
           const typename Slot<Rl>::G4* __restrict__ tg, const double* __restrict__ X,
           const Rl* __restrict__ xi, Rl* __restrict__ val, double* __restrict__ y) {
+  chain_wait();
   typedef Slot<Rl> S;
   typedef typename S::V V;
   typedef typename S::G4 G4;
@@ -616,14 +617,8 @@ cudaError_t lxs_launch(Launch L, const YlmTables& tb, const DevGeo& g,
   cudaError_t e = cudaSuccess;
 #define CASE(LV)                                                                               \
   case LV: {                                                                                   \
-    constexpr size_t sm = lxs_smem<LV, Rl>(PRE);                                               \
-    auto kfn = k_lxs<LV, Rl, PRE, MODE>;                                                       \
-    if (sm > 48 * 1024)                                                                        \
-      if ((e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm))) \
-        return e;                                                                              \
-    if ((e = cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, 100)))  \
-      return e;                                                                                \
-    kfn<<<g.nsph, 32 * nroles<Rl>(LV), sm, L.st>>>(t, g, tg, X, xi, val, y);                   \
+    e = launch_chained(k_lxs<LV, Rl, PRE, MODE>, g.nsph, 32 * nroles<Rl>(LV),                  \
+                       lxs_smem<LV, Rl>(PRE), L.st, t, g, tg, X, xi, val, y);                  \
     break;                                                                                     \
   }
   switch (tb.lmax) {
@@ -633,7 +628,22 @@ cudaError_t lxs_launch(Launch L, const YlmTables& tb, const DevGeo& g,
   }
 #undef CASE
   ++*L.launches;
-  return cudaGetLastError();
+  return e ? e : cudaGetLastError();
+}
+template <int LV, class Rl, bool PRE, int MODE>
+cudaError_t lxs_attributes() {
+  constexpr size_t sm = lxs_smem<LV, Rl>(PRE);
+  auto kfn = k_lxs<LV, Rl, PRE, MODE>;
+  cudaError_t e = cudaSuccess;
+  if (sm > 48 * 1024)
+    e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  return e ? e : cudaFuncSetAttribute(kfn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+template <int LV, int MODE>
+cudaError_t lxs_attributes_mode() {
+  cudaError_t e = lxs_attributes<LV, double, true, MODE>();
+  if (!e) e = lxs_attributes<LV, double, false, MODE>();
+  return e ? e : lxs_attributes<LV, float, true, MODE>();
 }
 // FP64: with the stored geometry when there is one
 template <int MODE>
@@ -645,6 +655,18 @@ cudaError_t lxs_launch64(Launch L, const YlmTables& tb, const DevGeo& g, const d
 
 }  // namespace
 
+cudaError_t prepare_lxs(int lmax) {
+  cudaError_t e = cudaErrorInvalidValue;
+#define CASE(LV)                                       \
+  case LV:                                             \
+    e = lxs_attributes_mode<LV, 0>();                  \
+    if (!e) e = lxs_attributes_mode<LV, 1>();          \
+    if (!e) e = lxs_attributes_mode<LV, 2>();          \
+    break;
+  switch (lmax) { DDC_LMAX_CASES(CASE) }
+#undef CASE
+  return e;
+}
 cudaError_t launch_lxs(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
                        const double* xi, double* val, double* y) {
   return lxs_launch64<0>(L, tb, g, X, xi, val, y);

@@ -200,6 +200,7 @@ __device__ bool gauss_jordan(int n, double (&a)[4], double (&b)[4], double* x) {
 
 template <class H, int CK>
 __global__ void __launch_bounds__(kT, 4) k_gram(const __grid_constant__ SolverArgs a) {
+  chain_wait();
   constexpr int TILE = CK < 2048 ? CK : 2048;
   constexpr int U = TILE / kT;
   constexpr int KS = (kMaxHist + kW - 1) / kW;  // history vectors per warp
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(kT, 4) k_gram(const __grid_constant__ SolverAr
 // and update.
 template <class H, int CK>
 __global__ void __launch_bounds__(kT) k_extrap(const __grid_constant__ SolverArgs a) {
+  chain_wait();
   constexpr int U = CK / kT < 4 ? CK / kT : 4;  // elements per thread and step
   const int q = a.first + blockIdx.y;
   const SolverSys& s = a.sys[q];
@@ -561,11 +563,9 @@ cudaError_t launch_solver_step(Launch L, const SolverArgs& a, int ns, bool f32, 
   return by_chunk(a, [&](auto ck) {
     constexpr int CK = decltype(ck)::value;
     if (which == 0) {
-      if (f32) k_gram<float, CK><<<g, kT, 0, L.st>>>(a);
-      else k_gram<double, CK><<<g, kT, 0, L.st>>>(a);
+      launch_chained(f32 ? k_gram<float, CK> : k_gram<double, CK>, g, kT, 0, L.st, a);
     } else {
-      if (f32) k_extrap<float, CK><<<g, kT, 0, L.st>>>(a);
-      else k_extrap<double, CK><<<g, kT, 0, L.st>>>(a);
+      launch_chained(f32 ? k_extrap<float, CK> : k_extrap<double, CK>, g, kT, 0, L.st, a);
     }
   });
 }
