@@ -120,7 +120,8 @@ struct ddc_ctx {
   long long st_calls[ST_N] = {0};
   std::string err;
   bool ready = false;
-  bool lxs_ready = false;  // attributes of the triple kernels are set
+  bool tables_ready = false;  // static_tables done
+  bool far_tables = false;    // farBT, farDT built
   int nsph = 0, ncav = 0, nylm = 0, ngrid = 0, npair = 0;
   long long ntri = 0;
   std::vector<double> h_grid;  // x,y,z,w per point
@@ -129,6 +130,7 @@ struct ddc_ctx {
   DBuf sph, grid, basis, bw, fi, ui, zi, inl, nl, rev, pn_ptr, pn, ls_ptr, ls, ntri_pt, pt_ptr,
       pt_idx;
   DBuf lsstart, fxa, fda, fvec;
+  DBuf pcnt;     // triples per pair (ddinit scratch)
   DBuf pn_bits;  // per pair, which grid points lie inside the neighbour (ddinit scratch)
   // batched molecules: partition, per-target N-body ranges, per-molecule DIIS state
   int nmol = 1;
@@ -429,15 +431,8 @@ int reduce_to_host(ddc_ctx* ctx, int nvals, double* host, int stride = 1, int nb
   return DDC_OK;
 }
 
-// The per-item counts that are about to be scanned into 32-bit offsets must
-// total less than 2^31: summed in 64 bits on the device first.
-int check_count_total(ddc_ctx* ctx, const int* cnt, int n, const char* what) {
-  if (n <= 0) return DDC_OK;
-  unsigned long long* d = reinterpret_cast<unsigned long long*>(ctx->red.p);
-  CK(launch_sum_counts(ctx->L(), cnt, n, d));
-  unsigned long long total = 0;
-  CK(cudaMemcpyAsync(&total, d, sizeof(total), cudaMemcpyDeviceToHost, ctx->st));
-  CKI(sync(ctx));
+// The per-item counts scanned into 32-bit offsets must total less than 2^31.
+int check_count_total(ddc_ctx* ctx, unsigned long long total, const char* what) {
   if (total >= (unsigned long long)INT_MAX)
     return fail(ctx, DDC_ERR_UNSUPPORTED,
                 std::string("more than 2^31 - 1 ") + what + " (" + std::to_string(total) + ")");
@@ -448,36 +443,15 @@ int check_count_total(ddc_ctx* ctx, const int* cnt, int n, const char* what) {
 // mixed operators run on the FP64 tensor cores
 constexpr long long kDmmaProducts = 50000000;
 
-// ---------------------------------------------------------------------------
-// ddinit (ddcosmo.f90:159-483) on device buffers
-// ---------------------------------------------------------------------------
-int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4* dsph) {
-  ctx->ready = false;
-  ctx->tgeo_on = false;
-  ctx->tgeo64_on = false;
-  ctx->nsph = n;
-  ctx->nylm = (ctx->prm.lmax + 1) * (ctx->prm.lmax + 1);
-  ctx->ngrid = snap_ngrid(ctx->prm.ngrid);
-  build_tables(ctx);
-  if (!ctx->lxs_ready) {
-    CK(prepare_lxs(ctx->prm.lmax));
-    ctx->lxs_ready = true;
-  }
-  if (!lebedev(ctx->ngrid, ctx->h_grid)) return fail(ctx, DDC_ERR_PARAM, "bad Lebedev size");
-  const int N = n, G = ctx->ngrid, NY = ctx->nylm;
-  const long long NP = (long long)N * G;
-  // grid fields, cavity and triple lists are indexed with 32-bit integers
-  if (NP >= (long long)INT_MAX)
-    return fail(ctx, DDC_ERR_UNSUPPORTED, "nsph * ngrid exceeds 2^31 - 1 grid points");
-  // two rows (the direct and adjoint solves' reductions); also the count checks' scratch
-  CK(ctx->red.ensure(sizeof(double) * 2 * (kMaxHist + 1)));
+// What depends on the parameters alone (degree, grid, eta), once per context:
+// the constants, the grid, the basis with its transposes and weights.
+int static_tables(ddc_ctx* ctx) {
+  if (ctx->tables_ready) return DDC_OK;
+  const int G = ctx->ngrid, NY = ctx->nylm;
   auto L = ctx->L();
-  CK(ctx->sph.ensure(sizeof(double4) * std::max(N, 1)));
-  if (hsph)
-    CK(cudaMemcpyAsync(ctx->sph.p, hsph->data(), sizeof(double4) * N, cudaMemcpyHostToDevice,
-                       ctx->st));
-  else if (dsph != ctx->sph.as<double4>())
-    CK(cudaMemcpyAsync(ctx->sph.p, dsph, sizeof(double4) * N, cudaMemcpyDeviceToDevice, ctx->st));
+  build_tables(ctx);
+  CK(prepare_lxs(ctx->prm.lmax));
+  if (!lebedev(G, ctx->h_grid)) return fail(ctx, DDC_ERR_PARAM, "bad Lebedev size");
   CK(ctx->grid.ensure(sizeof(double4) * G));
   CK(ctx->gpos.ensure(sizeof(int) * G));
   {
@@ -512,6 +486,42 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   CK(ctx->bw.ensure(sizeof(double) * G * NY));
   CK(launch_basis(L, ctx->tb, ctx->grid.as<double4>(), ctx->basis.as<double>(),
                   ctx->bw.as<double>()));
+  // the basis transposed to [Y][G] for the FP64 expansions xi = basis^T s
+  // (forces, zeta) and w xi = bw^T s (the operators)
+  for (auto t : {std::make_pair(&ctx->basis, &ctx->basisT), std::make_pair(&ctx->bw, &ctx->bwT)}) {
+    CK(t.second->ensure(sizeof(double) * G * NY));
+    CK(launch_transpose(L, G, NY, t.first->as<double>(), t.second->as<double>()));
+  }
+  ctx->tables_ready = true;
+  return DDC_OK;
+}
+
+// ---------------------------------------------------------------------------
+// ddinit (ddcosmo.f90:159-483) on device buffers
+// ---------------------------------------------------------------------------
+int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
+  ctx->ready = false;
+  ctx->tgeo_on = false;
+  ctx->tgeo64_on = false;
+  ctx->nsph = n;
+  ctx->nylm = (ctx->prm.lmax + 1) * (ctx->prm.lmax + 1);
+  ctx->ngrid = snap_ngrid(ctx->prm.ngrid);
+  const int N = n, G = ctx->ngrid, NY = ctx->nylm;
+  const long long NP = (long long)N * G;
+  // grid fields, cavity and triple lists are indexed with 32-bit integers
+  if (NP >= (long long)INT_MAX)
+    return fail(ctx, DDC_ERR_UNSUPPORTED, "nsph * ngrid exceeds 2^31 - 1 grid points");
+  if (!ctx->hred) CK(cudaMallocHost(&ctx->hred, sizeof(double) * 2 * (kMaxHist + 1)));
+  CK(ctx->red.ensure(sizeof(double) * 2 * (kMaxHist + 1)));
+  // red holds the counts' totals during ddinit: [0] pairs, [1] cavity points,
+  // [2] triples
+  CountStats* stats = ctx->red.as<CountStats>();
+  CountStats* hstats = reinterpret_cast<CountStats*>(ctx->hred);
+  auto L = ctx->L();
+  CK(ctx->sph.ensure(sizeof(double4) * std::max(N, 1)));
+  CK(cudaMemcpyAsync(ctx->sph.p, hsph.data(), sizeof(double4) * N, cudaMemcpyHostToDevice,
+                     ctx->st));
+  CKI(static_tables(ctx));
   // cell groups of one large molecule: candidates for the neighbour list,
   // the near lists of the cavity far field and the groups of the field of
   // zeta (DDC_CELLS_OFF=1 keeps the all-pairs scans: a diagnostic switch)
@@ -531,16 +541,13 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
       z.gcen = ctx->zg_cen.as<double4>();
       z.gnpt = nullptr;
       z.gptr = nullptr;
-      if (!ctx->hred) CK(cudaMallocHost(&ctx->hred, sizeof(double) * 2 * (kMaxHist + 1)));
       CK(launch_zgroups_cells(L, N, ctx->sph.as<double4>(), z, ctx->zg_cnt.as<int>(),
                               reinterpret_cast<int*>(ctx->hred)));
     }
   }
   // neighbour list
-  size_t scan_n = (size_t)std::max<long long>(N, 1);
-  CK(ctx->cnt.ensure(sizeof(int) * (scan_n + 1)));
+  CK(ctx->cnt.ensure(sizeof(int) * (N + 1)));
   CK(ctx->inl.ensure(sizeof(int) * (N + 1)));
-  CK(cudaMemsetAsync(ctx->cnt.p, 0, sizeof(int) * (N + 1), ctx->st));
   if (N > 0) {
     if (ctx->zg_on)
       CK(launch_csr_count_cells(L, N, ctx->sph.as<double4>(), ctx->zg, ctx->cnt.as<int>()));
@@ -549,24 +556,18 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   }
   size_t tb_bytes = scan_temp_bytes(N);
   CK(ctx->scan_tmp.ensure(tb_bytes));
-  CKI(check_count_total(ctx, ctx->cnt.as<int>(), N, "neighbour pairs"));
-  CK(scan_exclusive(L, ctx->cnt.as<int>(), ctx->inl.as<int>(), N, ctx->scan_tmp.p, tb_bytes));
-  int npair = 0;
-  CK(cudaMemcpyAsync(&npair, ctx->inl.as<int>() + N, sizeof(int), cudaMemcpyDeviceToHost,
-                     ctx->st));
+  CK(scan_counts(L, ctx->cnt.as<int>(), ctx->inl.as<int>(), N, ctx->scan_tmp.p, tb_bytes, stats));
+  CK(cudaMemcpyAsync(hstats, stats, sizeof(CountStats), cudaMemcpyDeviceToHost, ctx->st));
   CKI(sync(ctx));
+  CKI(check_count_total(ctx, hstats[0].total, "neighbour pairs"));
+  const int npair = (int)hstats[0].total;
   ctx->npair = npair;
   CK(ctx->nl.ensure(sizeof(int) * std::max(npair, 1)));
   CK(ctx->rev.ensure(sizeof(int) * std::max(npair, 1)));
   {
-    std::vector<int> h_inl(N + 1);
-    CK(cudaMemcpyAsync(h_inl.data(), ctx->inl.p, sizeof(int) * (N + 1), cudaMemcpyDeviceToHost,
-                       ctx->st));
-    CKI(sync(ctx));
-    int mx = 0;
-    for (int i = 0; i < N; i++) mx = std::max(mx, h_inl[i + 1] - h_inl[i]);
     // a point's triples are counted with 8 bits (the reference
     // caps the list at nngmax = 100 per sphere on average, ddcosmo.f90:87)
+    const int mx = hstats[0].largest;
     const size_t smem = 32 * (size_t)mx + 4 * (size_t)mx + 32 * (size_t)G;
     if (mx > 255 || smem > 200 * 1024)
       return fail(ctx, DDC_ERR_UNSUPPORTED, "a sphere has too many neighbours (" +
@@ -591,51 +592,42 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
                  ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->fi.as<double>(),
                  ctx->ui.as<double>(),
                  ctx->prm.igrad ? ctx->zi.as<double>() : nullptr, ctx->ntri_pt.as<uint8_t>()));
-  // cavity
+  // cavity counts, and the pair-major triple lists' counts
   CK(ctx->cavoff.ensure(sizeof(int) * (N + 1)));
-  CK(cudaMemsetAsync(ctx->cnt.p, 0, sizeof(int) * (N + 1), ctx->st));
   CK(launch_cav_count(L, N, G, ctx->ui.as<double>(), ctx->cnt.as<int>()));
-  CK(scan_exclusive(L, ctx->cnt.as<int>(), ctx->cavoff.as<int>(), N, ctx->scan_tmp.p, tb_bytes));
-  int ncav = 0;
-  CK(cudaMemcpyAsync(&ncav, ctx->cavoff.as<int>() + N, sizeof(int), cudaMemcpyDeviceToHost,
+  CK(scan_counts(L, ctx->cnt.as<int>(), ctx->cavoff.as<int>(), N, ctx->scan_tmp.p, tb_bytes,
+                 stats + 1));
+  CK(ctx->pcnt.ensure(sizeof(int) * ((size_t)npair + 1)));
+  CK(ctx->pn_ptr.ensure(sizeof(int) * ((size_t)npair + 1)));
+  CK(ctx->pn_bits.ensure(sizeof(unsigned) * std::max(npair, 1) * (size_t)((G + 31) / 32)));
+  CK(launch_pair_count(L, N, npair, G, ctx->sph.as<double4>(), ctx->grid.as<double4>(),
+                       ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->pcnt.as<int>(),
+                       ctx->pn_bits.as<unsigned>()));
+  CK(ctx->scan_tmp.ensure(std::max(tb_bytes, scan_temp_bytes(npair))));
+  CK(scan_counts(L, ctx->pcnt.as<int>(), ctx->pn_ptr.as<int>(), npair, ctx->scan_tmp.p,
+                 ctx->scan_tmp.bytes, stats + 2));
+  CK(cudaMemcpyAsync(hstats + 1, stats + 1, 2 * sizeof(CountStats), cudaMemcpyDeviceToHost,
                      ctx->st));
   CKI(sync(ctx));
+  CKI(check_count_total(ctx, hstats[2].total, "(sphere, point, neighbour) triples"));
+  const int ncav = (int)hstats[1].total, ntri = (int)hstats[2].total;
   ctx->ncav = ncav;
+  ctx->ntri = ntri;
   CK(ctx->cavidx.ensure(sizeof(int) * std::max(NP, 1LL)));
   CK(ctx->cavpt.ensure(sizeof(int) * std::max(ncav, 1)));
   CK(ctx->ccav.ensure(sizeof(double) * 3 * std::max(ncav, 1)));
   CK(launch_cav_fill(L, N, G, ctx->gpos.as<int>(), ctx->ui.as<double>(), ctx->sph.as<double4>(),
                      ctx->grid.as<double4>(), ctx->cavoff.as<int>(), ctx->cavidx.as<int>(),
                      ctx->cavpt.as<int>(), ctx->ccav.as<double>()));
-  // pair-major triple lists
-  size_t pscan = (size_t)std::max(npair, 1);
-  CK(ctx->cnt.ensure(sizeof(int) * (std::max(scan_n, pscan) + 1)));
-  CK(ctx->pn_ptr.ensure(sizeof(int) * (npair + 1)));
-  CK(cudaMemsetAsync(ctx->cnt.p, 0, sizeof(int) * (npair + 1), ctx->st));
-  CK(ctx->pn_bits.ensure(sizeof(unsigned) * std::max(npair, 1) * (size_t)((G + 31) / 32)));
-  CK(launch_pair_count(L, N, npair, G, ctx->sph.as<double4>(), ctx->grid.as<double4>(),
-                       ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->cnt.as<int>(),
-                       ctx->pn_bits.as<unsigned>()));
-  CKI(check_count_total(ctx, ctx->cnt.as<int>(), npair, "(sphere, point, neighbour) triples"));
-  size_t tb2 = scan_temp_bytes(npair);
-  CK(ctx->scan_tmp.ensure(std::max(tb_bytes, tb2)));
-  CK(scan_exclusive(L, ctx->cnt.as<int>(), ctx->pn_ptr.as<int>(), npair, ctx->scan_tmp.p,
-                    ctx->scan_tmp.bytes));
-  int ntri = 0;
-  CK(cudaMemcpyAsync(&ntri, ctx->pn_ptr.as<int>() + npair, sizeof(int), cudaMemcpyDeviceToHost,
-                     ctx->st));
-  CKI(sync(ctx));
-  ctx->ntri = ntri;
   CK(ctx->pn.ensure(sizeof(uint16_t) * std::max(ntri, 1)));
   CK(launch_pair_fill(L, N, npair, G, ctx->sph.as<double4>(), ctx->grid.as<double4>(),
                       ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->pn_bits.as<unsigned>(),
                       ctx->pn_ptr.as<int>(), ctx->pn.as<uint16_t>()));
   CK(ctx->ls_ptr.ensure(sizeof(int) * (N + 1)));
-  CK(cudaMemsetAsync(ctx->cnt.p, 0, sizeof(int) * (N + 1), ctx->st));
   CK(launch_ls_count(L, N, ctx->inl.as<int>(), ctx->rev.as<int>(), ctx->pn_ptr.as<int>(),
                      ctx->cnt.as<int>()));
-  CK(scan_exclusive(L, ctx->cnt.as<int>(), ctx->ls_ptr.as<int>(), N, ctx->scan_tmp.p,
-                    ctx->scan_tmp.bytes));
+  CK(scan_counts(L, ctx->cnt.as<int>(), ctx->ls_ptr.as<int>(), N, ctx->scan_tmp.p,
+                 ctx->scan_tmp.bytes, stats));
   CK(ctx->ls.ensure(sizeof(int) * std::max(ntri, 1)));
   CK(ctx->lsstart.ensure(sizeof(int) * std::max(npair, 1)));
   CK(launch_ls_fill(L, N, ctx->inl.as<int>(), ctx->nl.as<int>(), ctx->rev.as<int>(),
@@ -665,13 +657,6 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
   CK(ctx->hist_e.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
   CK(ctx->partials.ensure(sizeof(double) * reduce_blocks() * (kMaxHist + 1)));
   CK(ctx->red.ensure(sizeof(double) * 2 * (kMaxHist + 1)));
-  // the basis transposed to [Y][G] for the FP64 expansions xi = basis^T s
-  // (forces, zeta) and w xi = bw^T s (the operators)
-  for (auto t : {std::make_pair(&ctx->basis, &ctx->basisT), std::make_pair(&ctx->bw, &ctx->bwT)}) {
-    CK(t.second->ensure(sizeof(double) * G * NY));
-    CK(launch_transpose(L, G, NY, t.first->as<double>(), t.second->as<double>()));
-  }
-  if (!ctx->hred) CK(cudaMallocHost(&ctx->hred, sizeof(double) * 2 * (kMaxHist + 1)));
   if (ctx->prm.igrad && !ctx->st2) {
     CK(cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
@@ -754,8 +739,10 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>* hsph, const double4
       CK(ctx->farBT.ensure(sizeof(double) * YP * G));
       CK(ctx->farDT.ensure(sizeof(double) * 3 * YP * G));
       CK(ctx->farA.ensure(sizeof(double) * (size_t)YP * N));
-      CK(launch_far_tables(L, ctx->tbP, ctx->grid.as<double4>(), G, ctx->farBT.as<double>(),
-                           ctx->farDT.as<double>()));
+      if (!ctx->far_tables)
+        CK(launch_far_tables(L, ctx->tbP, ctx->grid.as<double4>(), G, ctx->farBT.as<double>(),
+                             ctx->farDT.as<double>()));
+      ctx->far_tables = true;
     }
     // the field of zeta at the nuclei of one large molecule in the mixed
     // flow: spheres grouped for the multipole far field (DDC_ZFAR_OFF=1, or
@@ -1574,7 +1561,7 @@ int ddc_init(ddc_ctx* ctx, int n, const double* x, const double* y, const double
   int rc;
   {
     StageScope sc(ctx, ST_INIT);
-    rc = do_init(ctx, n, &hs, nullptr);
+    rc = do_init(ctx, n, hs);
   }
   if (rc == DDC_OK) CKI(sync(ctx));
   return rc;

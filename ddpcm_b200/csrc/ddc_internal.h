@@ -64,6 +64,7 @@ struct DBuf {
 // mapped host memory that a kernel sets when one of its bounded waits runs out.
 struct TcPlan {
   bool on = false;
+  bool packed = false;       // the static images are built (they depend on bw alone)
   bool tuned = false;        // tile widths measured for tune_key's shape
   long long tune_key = 0;
   int tuned_bn_proj = 0, tuned_bn_xi = 0;
@@ -288,12 +289,17 @@ cudaError_t launch_ls_fill(Launch L, int nsph, const int* inl, const int* nl, co
 cudaError_t launch_pt_fill(Launch L, int nsph, int ngrid, const int* inl, const int* pn_ptr,
                            const uint16_t* pn, const int* lsstart, const uint8_t* ntri,
                            int* pt_ptr, int* pt_idx);
-// exclusive scan of n ints (out[n] = total); temp is device scratch of temp_bytes
-cudaError_t scan_exclusive(Launch L, const int* in, int* out, int n, void* temp,
-                           size_t temp_bytes);
+// exclusive scan of n ints (out[n] = total; in[n] is overwritten); temp is
+// device scratch of temp_bytes
+cudaError_t scan_exclusive(Launch L, int* in, int* out, int n, void* temp, size_t temp_bytes);
 size_t scan_temp_bytes(int n);
-// *out = sum of cnt[0..n) in 64 bits (out: device memory, overwritten)
-cudaError_t launch_sum_counts(Launch L, const int* cnt, int n, unsigned long long* out);
+// the same with the total in 64 bits and the largest count
+struct CountStats {
+  unsigned long long total;
+  int largest;
+};
+cudaError_t scan_counts(Launch L, int* cnt, int* out, int n, void* temp, size_t temp_bytes,
+                        CountStats* st);
 
 // operators over the triples (ddc_lxs.cu): lx values, one per triple in
 // gather-list order, for k_lx_gather, and / or the L* rows.  xi holds the

@@ -713,10 +713,10 @@ cudaError_t tc_plan(Launch L, TcPlan& p, const double* bw, int nsph,
   bn = pick_bn(nsph, kMaxBn);
   while ((e = cfg_xi(p, bn)) == cudaErrorInvalidValue && bn > 32) bn -= 32;
   if (e) return e;
-  // static operands, split once
-  if ((e = p.img_proj.ensure((size_t)p.kc_proj * 2 * kChunk))) return e;
-  if ((e = p.img_xi.ensure((size_t)p.mt_xi * p.kc_xi * 2 * kChunk))) return e;
-  {
+  // static operands, split once (bw does not change in a context)
+  if (!p.packed) {
+    if ((e = p.img_proj.ensure((size_t)p.kc_proj * 2 * kChunk))) return e;
+    if ((e = p.img_xi.ensure((size_t)p.mt_xi * p.kc_xi * 2 * kChunk))) return e;
     const long long tot = (long long)p.kc_proj * 128 * 32;
     k_pack_static<<<(unsigned)((tot + 255) / 256), 256, 0, L.st>>>(
         bw, nylm, false, nylm, ngrid, 1, p.kc_proj, p.img_proj.as<float>());
@@ -726,6 +726,7 @@ cudaError_t tc_plan(Launch L, TcPlan& p, const double* bw, int nsph,
         bw, nylm, true, ngrid, nylm, p.mt_xi, p.kc_xi, p.img_xi.as<float>());
     ++*L.launches;
     if ((e = cudaGetLastError())) return e;
+    p.packed = true;
   }
   if (!p.err_h) {
     if ((e = cudaHostAlloc(&p.err_h, sizeof(int), cudaHostAllocMapped))) return e;
