@@ -2123,7 +2123,8 @@ int ddc_batch_energy_forces(ddc_ctx* ctx, int nmol, const int* off, const double
     double t5 = now_s();
     inf->t_forces = t5 - t4;
     CK(ctx->ef2.ensure(sizeof(double) * 3 * std::max(N, 1)));
-    CK(ctx->ef_scratch.ensure(sizeof(double) * 3 * std::max((size_t)NC, (size_t)N)));
+    const int parts = efield_parts(N);
+    CK(ctx->ef_scratch.ensure(sizeof(double) * 3 * (size_t)std::max(N, 1) * parts));
     {
       StageScope sc(ctx, ST_EFIELD);
       // each nucleus from the cavity points of its own molecule; in mixed
@@ -2131,7 +2132,7 @@ int ddc_batch_energy_forces(ddc_ctx* ctx, int nmol, const int* off, const double
       // single-molecule flow does for this force-only field
       auto efield = ctx->prm.precision == DDC_PREC_MIXED ? launch_efield_f32 : launch_efield;
       CK(efield(ctx->L(), NC, ctx->zeta.as<double>(), ctx->ccav.as<double>(), N,
-                ctx->csph.as<double>(), ctx->ef2.as<double>(), ctx->ef_scratch.as<double>(), 1,
+                ctx->csph.as<double>(), ctx->ef2.as<double>(), ctx->ef_scratch.as<double>(), parts,
                 ctx->tr_nuc.as<int2>()));
     }
     {

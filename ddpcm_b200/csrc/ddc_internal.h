@@ -487,6 +487,7 @@ cudaError_t launch_efield(Launch L, int nsrc, const double* q, const double* csr
                           const double* ctrg, double* ef, double* scratch, int nchunk,
                           const int2* trange);
 int efield_chunks(int nsrc, int ntrg);
+int efield_parts(int ntrg);  // nchunk where every target has its own range
 // load k_efield / k_efield_reduce on the current device (one-time set-up)
 cudaError_t preload_efield();
 int efield_chunks_f32(int nsrc, int ntrg);

@@ -20,3 +20,29 @@ def test_field_with_rounded_chunks(oracle, nsrc, ntrg):
         got = dd.efld(src, csrc, ctrg)
     want = oracle.efld(src, csrc, ctrg)
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("nsrc,ntrg", [(587, 12), (64, 1), (65, 1), (1023, 300), (1025, 257),
+                                       (16385, 3)])
+def test_field_at_few_targets(oracle, nsrc, ntrg):
+    """Chunks shorter than a tile (64 sources), up to 16 of them."""
+    test_field_with_rounded_chunks(oracle, nsrc, ntrg)
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-8), (1, 1e-6)])
+def test_field_of_a_batch_in_parts(precision, tol):
+    """Blocks of 256 nuclei with one, two and three molecules, their sources
+    split over parts: forces of the batch against one molecule at a time
+    (iconv 10: solutions to 1e-10, taken 100-fold; FP32 pair field 2^-24, taken
+    16-fold)."""
+    from ddpcm_b200 import molecules as M
+    from ddpcm_b200.ddcosmo import DDCosmo
+    mols = [M.to_bohr(M.make_molecule(n, 40 + n)) for n in (300, 12, 350)]
+    kw = dict(lmax=4, ngrid=50, iconv=10, eta=0.1, precision=precision)
+    with DDCosmo(**kw) as dd:
+        got = dd.batch_energy_forces(mols)
+    with DDCosmo(**kw) as dd:
+        for i, m in enumerate(mols):
+            one = dd.energy_forces(m["q"], m["x"], m["y"], m["z"], m["r"])
+            f = got["fx"][i]
+            assert np.linalg.norm(f - one["fx"]) <= tol * np.linalg.norm(one["fx"])
