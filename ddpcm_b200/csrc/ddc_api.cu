@@ -11,7 +11,6 @@
 #include <string>
 #include <vector>
 
-
 #include "ddc_internal.h"
 #include "lebedev_orbits.inc"
 
@@ -19,9 +18,22 @@ using namespace ddc;
 
 namespace {
 
-// ---------------------------------------------------------------------------
-// device buffer
-// ---------------------------------------------------------------------------
+struct HBuf {  // pinned host memory
+  void* p = nullptr;
+  size_t bytes = 0;
+  ~HBuf() {
+    if (p) cudaFreeHost(p);
+  }
+  cudaError_t ensure(size_t b) {
+    if (b <= bytes) return cudaSuccess;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    bytes = 0;
+    const cudaError_t e = cudaMallocHost(&p, b);
+    if (e == cudaSuccess) bytes = b;
+    return e;
+  }
+};
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch())
       .count();
@@ -141,6 +153,7 @@ struct ddc_ctx {
   DBuf b_cmol, b_cfirst;  // molecule of each solver chunk, first chunk of each molecule
   // state of the Jacobi/DIIS solves (SolverSys), both systems side by side
   DBuf s_int, s_dbl, s_slot, s_gram, s_coef, s_part, s_log;
+  HBuf hstate;           // the solver's state on the host
   int* hstop = nullptr;  // mapped host memory: [2] stop reports, [2] active counts
   int* dstop = nullptr;
   cudaEvent_t ev_sweep[4] = {};
@@ -194,6 +207,8 @@ struct ddc_ctx {
   // beside the force kernels (events: fork after zeta, join before its use)
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t st_out = nullptr;  // results to the host beside the force kernels
+  cudaEvent_t ev_mark[3] = {};    // ends of the phases of a run
   unsigned int stage_mask = ~0u;  // stages timed when prm.timing is set
 
   Launch L() { return Launch{st, &launches}; }
@@ -415,7 +430,7 @@ void build_tables(ddc_ctx* c) {
 // stride: the partial row length of the producing kernel (kMaxHist + 1 for the
 // Jacobi step's Gram row, whatever its current length; 1 for single sums).
 // nblk: the producing kernel's block count (partial rows).
-int reduce_to_host(ddc_ctx* ctx, int nvals, double* host, int stride = 1, int nblk = 0) {
+int reduce_to_pinned(ddc_ctx* ctx, int nvals, int stride = 1, int nblk = 0) {
   if (nvals > kMaxHist + 1 || !ctx->hred)
     return fail(ctx, DDC_ERR_STATE, "reduction read beyond the pinned buffer");
   {
@@ -426,6 +441,10 @@ int reduce_to_host(ddc_ctx* ctx, int nvals, double* host, int stride = 1, int nb
   }
   CK(cudaMemcpyAsync(ctx->hred, ctx->red.p, sizeof(double) * nvals, cudaMemcpyDeviceToHost,
                      ctx->st));
+  return DDC_OK;
+}
+int reduce_to_host(ddc_ctx* ctx, int nvals, double* host, int stride = 1, int nblk = 0) {
+  CKI(reduce_to_pinned(ctx, nvals, stride, nblk));
   CKI(sync(ctx));
   memcpy(host, ctx->hred, sizeof(double) * nvals);
   return DDC_OK;
@@ -661,6 +680,7 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
     CK(cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithFlags(&ctx->st_out, cudaStreamNonBlocking));
   }
   if (ctx->prm.precision == DDC_PREC_MIXED) {
     // the two contractions run on the tensor cores (split TF32) up to 128
@@ -764,7 +784,6 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
       CK(ctx->zg_scr.ensure(sizeof(double) * 3 * (size_t)zgroups_nchunk(z) * N));
     }
   }
-  CKI(sync(ctx));
   ctx->ready = true;
   return DDC_OK;
 }
@@ -1128,13 +1147,20 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
   SolverArgs a;
   CKI(solver_setup(ctx, a, sys, ns, mixed));
   CK(launch_solver_begin(ctx->L(), a, ns, mixed));
-  std::vector<int> si(2 * (SI_N * (size_t)nmol + 1));
-  std::vector<double> sd(2 * SD_N * (size_t)nmol);
-  auto read_state = [&]() -> int {
-    CK(cudaMemcpyAsync(si.data(), ctx->s_int.p, sizeof(int) * si.size(), cudaMemcpyDeviceToHost,
-                       ctx->st));
-    CK(cudaMemcpyAsync(sd.data(), ctx->s_dbl.p, sizeof(double) * sd.size(),
-                       cudaMemcpyDeviceToHost, ctx->st));
+  // the state comes back in one go, through pinned memory: the integers, the
+  // doubles, and one molecule's norms
+  const size_t nsi = 2 * (SI_N * (size_t)nmol + 1), nsd = 2 * SD_N * (size_t)nmol;
+  const int nlog = one ? std::max(std::min(256, ctx->prm.max_iter), 0) : 0;
+  CK(ctx->hstate.ensure(sizeof(double) * (nsd + 2 * (size_t)nlog) + sizeof(int) * nsi));
+  double* sd = static_cast<double*>(ctx->hstate.p);
+  double* slog = sd + nsd;
+  int* si = reinterpret_cast<int*>(slog + 2 * nlog);
+  auto read_state = [&](bool norms) -> int {
+    CK(cudaMemcpyAsync(si, ctx->s_int.p, sizeof(int) * nsi, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(sd, ctx->s_dbl.p, sizeof(double) * nsd, cudaMemcpyDeviceToHost, ctx->st));
+    for (int q = 0; norms && nlog && q < ns; q++)
+      CK(cudaMemcpyAsync(slog + (size_t)q * nlog, a.sys[q].log, sizeof(double) * nlog,
+                         cudaMemcpyDeviceToHost, ctx->st));
     return sync(ctx);
   };
   auto I = [&](int q, int w, int k) { return si[((size_t)q * SI_N + w) * nmol + k]; };
@@ -1142,7 +1168,7 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
   if (!mixed) {
     if (a.nonempty) CKI(solver_sweeps(ctx, a, sys, 0, ns, false));
     if (log) {
-      CKI(read_state());
+      CKI(read_state(false));
       const int from[2] = {0, 0}, to[2] = {I(0, SI_ITERS, 0), ns > 1 ? I(1, SI_ITERS, 0) : 0};
       CKI(print_log(ctx, a, ns, from, to));
     }
@@ -1161,7 +1187,7 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
                          ctx->st));
       CKI(sync(ctx));
       if (log) {
-        CKI(read_state());
+        CKI(read_state(false));
         for (int q = 0; q < ns; q++)
           if (I(q, SI_OUTER, 0) == round + 1)
             printf("  refinement %d: %s increment norm %14.4E\n", round + 1,
@@ -1173,7 +1199,7 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
       CKI(solver_sweeps(ctx, a, sys, run0 ? 0 : 1, run1 ? 2 : 1, true));
       CK(launch_solver_update(ctx->L(), a, ns));
       if (log) {
-        CKI(read_state());
+        CKI(read_state(false));
         const int to[2] = {I(0, SI_ITS, 0), ns > 1 ? I(1, SI_ITS, 0) : 0};
         CKI(print_log(ctx, a, ns, printed, to));
         printed[0] = to[0];
@@ -1181,7 +1207,7 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
       }
     }
   }
-  CKI(read_state());
+  CKI(read_state(true));
   int rc = DDC_OK;
   for (int q = 0; q < ns; q++) {
     ddc_solve_info& f = *sys[q].inf;
@@ -1206,10 +1232,8 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
     f.diis_restarts = restarts;
     f.final_norm = worst;
     if (one) {
-      const int n = std::min({maxit, 256, ctx->prm.max_iter});
-      if (n > 0)
-        CK(cudaMemcpyAsync(f.norms, a.sys[q].log, sizeof(double) * n, cudaMemcpyDeviceToHost,
-                           ctx->st));
+      const int n = std::min(maxit, nlog);
+      if (n > 0) memcpy(f.norms, slog + (size_t)q * nlog, sizeof(double) * n);
     }
     if (rc != DDC_OK || !nfail) continue;
     if (!one)
@@ -1221,7 +1245,6 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
       rc = fail(ctx, DDC_ERR_NOCONV, sys[q].adjoint ? "adjoint ddCOSMO did not converge"
                                                     : "ddCOSMO did not converge");
   }
-  CKI(sync(ctx));
   for (int q = 0; q < ns; q++) sys[q].inf->seconds = now_s() - t0;
   return rc;
 }
@@ -1440,6 +1463,9 @@ int ddc_destroy(ddc_ctx* c) {
   for (cudaEvent_t e : c->ev_sweep)
     if (e) cudaEventDestroy(e);
   if (c->st2) cudaStreamSynchronize(c->st2);
+  if (c->st_out) cudaStreamDestroy(c->st_out);
+  for (cudaEvent_t e : c->ev_mark)
+    if (e) cudaEventDestroy(e);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->st2) cudaStreamDestroy(c->st2);
@@ -1536,8 +1562,9 @@ extern "C" {
 int ddc_fp64_peak(int device, double* gflops) { return fma_peak(device, false, gflops); }
 int ddc_fp32_peak(int device, double* gflops) { return fma_peak(device, true, gflops); }
 
-int ddc_init(ddc_ctx* ctx, int n, const double* x, const double* y, const double* z,
-             const double* r) {
+// ddc_init without the wait at its end
+static int init_spheres(ddc_ctx* ctx, int n, const double* x, const double* y, const double* z,
+                        const double* r) {
   if (!ctx) return DDC_ERR_PARAM;
   if (n < 0 || (n > 0 && (!x || !y || !z || !r))) return fail(ctx, DDC_ERR_PARAM, "bad input");
   cudaSetDevice(ctx->prm.device);
@@ -1558,12 +1585,14 @@ int ddc_init(ddc_ctx* ctx, int n, const double* x, const double* y, const double
     if (!(hs[i].w > 0.0)) return fail(ctx, DDC_ERR_PARAM, "radii must be positive");
   if (!ctx->batch_init) ctx->nmol = 1;
   ctx->have_flow = false;
-  int rc;
-  {
-    StageScope sc(ctx, ST_INIT);
-    rc = do_init(ctx, n, hs);
-  }
-  if (rc == DDC_OK) CKI(sync(ctx));
+  StageScope sc(ctx, ST_INIT);
+  return do_init(ctx, n, hs);
+}
+int ddc_init(ddc_ctx* ctx, int n, const double* x, const double* y, const double* z,
+             const double* r) {
+  CKI(init_spheres(ctx, n, x, y, z, r));
+  const int rc = sync(ctx);
+  if (rc != DDC_OK) ctx->ready = false;
   return rc;
 }
 
@@ -1831,6 +1860,43 @@ int ddc_hnorm(ddc_ctx* ctx, const double* x, double* norm) {
   return DDC_OK;
 }
 
+// What a run hands back without waiting for it: the times of its phases, from
+// events at their ends, and the energy's sum in pinned memory.  Both are taken
+// when the call returns, whatever it returns.
+struct RunEnd {
+  ddc_ctx* ctx;
+  ddc_run_info* inf;
+  double t0, t3 = 0.0;  // start; end of the solve, where mark 2 lies
+  int marks = 0;
+  double* esolv = nullptr;
+  double fac = 0.0;
+  int mark() {
+    cudaEvent_t& e = ctx->ev_mark[marks];
+    if (!e) CK(cudaEventCreate(&e));
+    CK(cudaEventRecord(e, ctx->st));
+    ++marks;
+    return DDC_OK;
+  }
+  ~RunEnd() {
+    if (marks == 0) return;
+    if (marks < 3) {  // ended early: the end is now
+      if (cudaStreamSynchronize(ctx->st) != cudaSuccess) return;
+      t3 = now_s();
+      while (marks < 3)
+        if (mark() != DDC_OK) return;
+    }
+    if (cudaStreamSynchronize(ctx->st) != cudaSuccess) return;
+    if (esolv) *esolv = fac * ctx->hred[0];
+    float a = 0.0f, b = 0.0f;
+    if (cudaEventElapsedTime(&a, ctx->ev_mark[0], ctx->ev_mark[2]) != cudaSuccess ||
+        cudaEventElapsedTime(&b, ctx->ev_mark[1], ctx->ev_mark[2]) != cudaSuccess)
+      return;
+    inf->t_init = t3 - 1e-3 * a - t0;
+    inf->t_mkrhs = 1e-3 * (a - b);
+    inf->t_direct = 1e-3 * b;
+  }
+};
+
 int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x,
                       const double* y, const double* z, const double* rvdw, double* esolv,
                       double* sigma, double* s, double* fx, ddc_run_info* info) {
@@ -1839,10 +1905,9 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
   ddc_run_info loc{};
   ddc_run_info* inf = info ? info : &loc;
   memset(inf, 0, sizeof(*inf));
-  double t0 = now_s();
-  CKI(ddc_init(ctx, n, x, y, z, rvdw));
-  double t1 = now_s();
-  inf->t_init = t1 - t0;
+  RunEnd run{ctx, inf, now_s()};
+  CKI(init_spheres(ctx, n, x, y, z, rvdw));
+  CKI(run.mark());
   const int N = ctx->nsph, NC = ctx->ncav;
   const size_t nv = (size_t)N * ctx->nylm;
   const double* dq;
@@ -1857,9 +1922,7 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
   CKI(solute_pot_field(ctx, dq, dphi, ctx->prm.igrad ? ctx->ef1.as<double>() : nullptr,
                        nullptr));
   CK(launch_psi(ctx->L(), N, ctx->nylm, dq, dpsi));
-  CKI(sync(ctx));
-  double t2 = now_s();
-  inf->t_mkrhs = t2 - t1;
+  CKI(run.mark());
   double* dsig = ctx->sigma.as<double>();
   double* ds = ctx->s.as<double>();
   if (ctx->prm.guess == DDC_GUESS_USER) {
@@ -1888,9 +1951,13 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
     const System sys[2] = {{false, rhs, dsig, nullptr, &inf->direct},
                            {true, dpsi, ds, nullptr, &inf->adjoint}};
     CKI(solve_systems(ctx, sys, 2));
-    double d = 0.0;
-    CKI(dot_dev(ctx, (long long)nv, dsig, dpsi, &d));
-    *esolv = 0.5 * ((ctx->prm.eps - 1.0) / ctx->prm.eps) * d;
+    run.t3 = now_s();
+    CKI(run.mark());
+    CK(launch_dot_partial(ctx->L(), (long long)nv, dsig, dpsi, ctx->partials.as<double>(),
+                          reduce_blocks()));
+    CKI(reduce_to_pinned(ctx, 1));
+    run.esolv = esolv;
+    run.fac = 0.5 * ((ctx->prm.eps - 1.0) / ctx->prm.eps);
   } else {
     if (ctx->prm.guess == DDC_GUESS_LEARNED) {
       // both starts from the model before the solves (cosmo_dev recomputes
@@ -1903,8 +1970,10 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
     if (rc != DDC_OK || !ctx->prm.igrad) ctx->guess_preset = false;
     if (rc != DDC_OK) return rc;
   }
-  double t3 = now_s();
-  inf->t_direct = t3 - t2;
+  if (!paired) {
+    run.t3 = now_s();
+    CKI(run.mark());
+  }
   double* dfx = nullptr;
   if (ctx->prm.igrad) {
     if (!paired) {
@@ -1912,8 +1981,8 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
       ctx->guess_preset = false;
       if (rc != DDC_OK) return rc;
     }
-    double t4 = now_s();
-    inf->t_adjoint = t4 - t3;
+    const double t4 = now_s();
+    inf->t_adjoint = t4 - run.t3;
     CK(ctx->fx.ensure(sizeof(double) * 3 * std::max(N, 1)));
     dfx = ctx->fx.as<double>();
     // zeta first (ddmkzeta, ddcosmo.f90:1758-1806): the field of zeta at the
@@ -1977,14 +2046,28 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
       StageScope sc(ctx, ST_CONTRACT);
       CK(launch_charge_efld_contract(ctx->L(), N, dq, ctx->ef2.as<double>(), dfx));
     }
+    if (!ctx->prm.device_pointers) {
+      // the solutions go to the host while the force kernels run (5,000
+      // spheres: 2 x 4.8 MB into memory that is touched for the first time,
+      // 3.7 ms beside 4.1 ms of kernels); the solves have ended, so no event
+      // is needed
+      cudaError_t e = cudaSuccess;
+      for (auto o : {std::make_pair(sigma, dsig), std::make_pair(s, ds)})
+        if (e == cudaSuccess && o.first && nv)
+          e = cudaMemcpyAsync(o.first, o.second, sizeof(double) * nv, cudaMemcpyDeviceToHost,
+                              ctx->st_out);
+      const cudaError_t w = cudaStreamSynchronize(ctx->st_out);
+      CK(e);
+      CK(w);
+    }
     CKI(sync(ctx));
     const double t5 = now_s();
     inf->t_forces = t5 - t4;  // forces and both field contractions, overlapped
     inf->t_efld = 0.0;
   }
-  CKI(finish_out(ctx, sigma, dsig, nv));
+  if (!ctx->prm.igrad || ctx->prm.device_pointers) CKI(finish_out(ctx, sigma, dsig, nv));
   if (ctx->prm.igrad) {
-    CKI(finish_out(ctx, s, ds, nv));
+    if (ctx->prm.device_pointers) CKI(finish_out(ctx, s, ds, nv));
     CKI(finish_out(ctx, fx, dfx, 3 * (size_t)N));
   }
   CKI(sync(ctx));
