@@ -1001,7 +1001,8 @@ int solver_setup(ddc_ctx* ctx, SolverArgs& a, const System* sys, int ns, bool mi
   CK(ctx->s_slot.ensure(sizeof(int) * 2 * (size_t)nmol * nd));
   CK(ctx->s_gram.ensure(sizeof(double) * 2 * (size_t)nmol * nd * nd));
   CK(ctx->s_coef.ensure(sizeof(double) * 2 * (size_t)nmol * kMaxHist));
-  CK(ctx->s_part.ensure(sizeof(double) * 2 * (size_t)std::max(a.nchunk, 1) * (kMaxHist + 1)));
+  const size_t parts = (size_t)std::max(solver_parts(a.nchunk, a.chunk), 1) * (kMaxHist + 1);
+  CK(ctx->s_part.ensure(sizeof(double) * 2 * parts));
   if (nmol == 1) CK(ctx->s_log.ensure(sizeof(double) * 2 * (size_t)ctx->prm.max_iter));
   if (!ctx->hstop) {
     CK(cudaHostAlloc(&ctx->hstop, sizeof(int) * 4, cudaHostAllocMapped));
@@ -1034,7 +1035,7 @@ int solver_setup(ddc_ctx* ctx, SolverArgs& a, const System* sys, int ns, bool mi
     s.slot = ctx->s_slot.as<int>() + (size_t)q * nmol * nd;
     s.gram = ctx->s_gram.as<double>() + (size_t)q * nmol * nd * nd;
     s.coef = ctx->s_coef.as<double>() + (size_t)q * nmol * kMaxHist;
-    s.part = ctx->s_part.as<double>() + (size_t)q * std::max(a.nchunk, 1) * (kMaxHist + 1);
+    s.part = ctx->s_part.as<double>() + (size_t)q * parts;
     s.log = nmol == 1 ? ctx->s_log.as<double>() + (size_t)q * ctx->prm.max_iter : nullptr;
     s.hx = (q ? ctx->hist_x2 : ctx->hist_x).p;
     s.he = (q ? ctx->hist_e2 : ctx->hist_e).p;

@@ -393,6 +393,8 @@ cudaError_t guess_infer(Launch L, ddc_guess* m, const YlmTables& tb, int nsph, c
 // y = O x (which 0: Jacobi step and Gram solve, 1: extrapolation and stop
 // test); the mixed refinement's residual at ox with y = O ox, and x += e
 int solver_chunk(long long n_total, bool one);
+// rows of the partial sums
+int solver_parts(int nchunk, int chunk);
 cudaError_t launch_solver_begin(Launch L, const SolverArgs& a, int ns, bool mixed);
 cudaError_t launch_solver_step(Launch L, const SolverArgs& a, int ns, bool f32, int which);
 cudaError_t launch_solver_residual(Launch L, const SolverArgs& a, int ns, bool f32_res);

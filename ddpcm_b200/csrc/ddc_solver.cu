@@ -53,6 +53,12 @@ struct Segment {
   long long b0;  // first element
   int cnt;       // elements
 };
+// Blocks per chunk in k_extrap: its blocks want short segments, as many loads at
+// once as there are vectors, while k_gram's wait longer for a short segment
+// than they work on it.  5,000 spheres, lmax 10, FP64, both systems: k_gram
+// 67 us by 512 elements and 53 by 2,048, k_extrap 41 and 70.
+template <int CK>
+constexpr int kSub = CK == 2048 ? 4 : 1;
 template <int CK>
 __device__ __forceinline__ Segment segment_of(const SolverArgs& a, int c, int k) {
   const int2 sp = spheres_of(a, k), ch = chunks_of(a, k);
@@ -64,13 +70,13 @@ __device__ __forceinline__ Segment segment_of(const SolverArgs& a, int c, int k)
 
 // Last arriving chunk of molecule k (the counter is reset for the next
 // kernel).  Every block of the molecule calls it after writing its parts.
-__device__ __forceinline__ bool last_chunk(const SolverArgs& a, const SolverSys& s, int k) {
+__device__ __forceinline__ bool last_chunk(const SolverArgs& a, const SolverSys& s, int k, int sub = 1) {
   __shared__ unsigned s_last;
   __threadfence();
   __syncthreads();
   const int2 ch = chunks_of(a, k);
   if (threadIdx.x == 0) {
-    s_last = atomicAdd(s.cnt + k, 1u) == (unsigned)(ch.y - ch.x) - 1 ? 1u : 0u;
+    s_last = atomicAdd(s.cnt + k, 1u) == (unsigned)((ch.y - ch.x) * sub) - 1 ? 1u : 0u;
     if (s_last) s.cnt[k] = 0u;
   }
   __syncthreads();
@@ -95,14 +101,14 @@ __device__ __forceinline__ double block_sum(double v) {
 // chunks w, w + 8, ... (a lane per entry), then the warps in order; a single
 // entry by thread.
 __device__ __forceinline__ void sum_parts(const SolverArgs& a, const SolverSys& s, int k, int nv,
-                                          double* out) {
+                                          double* out, int sub = 1) {
   __shared__ double acc[kW][kMaxHist + 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int2 ch = chunks_of(a, k);
   if (nv == 1) {
     double v = 0.0;
 #pragma unroll 4
-    for (int c = ch.x + (int)threadIdx.x; c < ch.y; c += kT)
+    for (int c = ch.x * sub + (int)threadIdx.x; c < ch.y * sub; c += kT)
       v += __ldcg(s.part + (size_t)c * (kMaxHist + 1));
     v = block_sum(v);
     if (threadIdx.x == 0) out[0] = v;
@@ -341,10 +347,16 @@ __global__ void __launch_bounds__(kT, 4) k_gram(const __grid_constant__ SolverAr
 template <class H, int CK>
 __global__ void __launch_bounds__(kT) k_extrap(const __grid_constant__ SolverArgs a) {
   chain_wait();
-  constexpr int U = CK / kT < 4 ? CK / kT : 4;  // elements per thread and step
+  constexpr int SUB = kSub<CK>, LEN = CK / SUB;
+  constexpr int U = LEN / kT < 4 ? LEN / kT : 4;  // elements per thread and step
+  // history vectors loaded at a time, unconditionally: 4 to 16 loads of a
+  // thread in flight.  With loads behind the range test one at a time went out
+  // (5,000 spheres FP64 54 us, 41 now; 20,000 FP32 by 8,192 73 and 58; a read of
+  // the history at the copy rate 34 and 60); 2 at a time 42 and 57, 8: 45 and 77
+  constexpr int B = 4;
   const int q = a.first + blockIdx.y;
   const SolverSys& s = a.sys[q];
-  const int c = blockIdx.x, k = mol_of(a, c), tid = threadIdx.x;
+  const int c = blockIdx.x, k = mol_of(a, c / SUB), tid = threadIdx.x;
   __shared__ int pm[kMaxHist];
   __shared__ double cf[kMaxHist];
   __shared__ double tot[1];
@@ -359,50 +371,67 @@ __global__ void __launch_bounds__(kT) k_extrap(const __grid_constant__ SolverArg
   if (tid < kMaxHist) cf[tid] = cv;
   __syncthreads();
   const long long N = a.n_total;
-  const Segment sg = segment_of<CK>(a, c, k);
+  Segment sg = segment_of<CK>(a, c / SUB, k);
+  sg.b0 += (c % SUB) * LEN;
+  sg.cnt = min(sg.cnt - (c % SUB) * LEN, LEN);  // zero or less: nothing here
   const H* hx = static_cast<const H*>(s.hx) + sg.b0;
   const int dt = kT % a.nylm;
   int lm = (int)((sg.b0 + tid) % a.nylm);
   double acc = 0.0;
   for (int u0 = 0; u0 * kT < sg.cnt; u0 += U) {
     double xo[U], xold[U];
-    bool in[U];
+    int j[U];  // past the end: the last element again, not stored
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int j = tid + (u0 + u) * kT;
-      in[u] = j < sg.cnt;
-      xold[u] = in[u] ? s.x[sg.b0 + j] : 0.0;
+      j[u] = min(tid + (u0 + u) * kT, sg.cnt - 1);
+      xold[u] = s.x[sg.b0 + j[u]];
       xo[u] = 0.0;
     }
     if (ok) {
-#pragma unroll 8
-      for (int h = 0; h < nm; ++h) {
-        const H* hk = hx + (size_t)pm[h] * N;
-        H hv[U];
+      int h = 0;
+      for (; h + B <= nm; h += B) {
+        H hv[B][U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) hv[u] = in[u] ? hk[tid + (u0 + u) * kT] : H(0);
+        for (int g = 0; g < B; ++g)
 #pragma unroll
-        for (int u = 0; u < U; ++u) xo[u] = fma(cf[h], (double)hv[u], xo[u]);
+          for (int u = 0; u < U; ++u) hv[g][u] = hx[(size_t)pm[h + g] * N + j[u]];
+#pragma unroll
+        for (int g = 0; g < B; ++g)
+#pragma unroll
+          for (int u = 0; u < U; ++u) xo[u] = fma(cf[h + g], (double)hv[g][u], xo[u]);
+      }
+      if (h < nm) {
+        H hv[B][U];
+#pragma unroll
+        for (int g = 0; g < B; ++g)
+#pragma unroll
+          for (int u = 0; u < U; ++u) hv[g][u] = hx[(size_t)pm[min(h + g, nm - 1)] * N + j[u]];
+#pragma unroll
+        for (int g = 0; g < B; ++g)
+          if (h + g < nm) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) xo[u] = fma(cf[h + g], (double)hv[g][u], xo[u]);
+          }
       }
     } else {
       const H* xjac = hx + (size_t)pm[nm - 1] * N;
 #pragma unroll
-      for (int u = 0; u < U; ++u) xo[u] = in[u] ? (double)xjac[tid + (u0 + u) * kT] : 0.0;
+      for (int u = 0; u < U; ++u) xo[u] = (double)xjac[j[u]];
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (in[u]) {
+      if (tid + (u0 + u) * kT < sg.cnt) {
         const double dd = xo[u] - xold[u];
         acc = fma(dd * dd, a.hw[l_of(lm)], acc);
-        s.x[sg.b0 + tid + (u0 + u) * kT] = xo[u];
+        s.x[sg.b0 + j[u]] = xo[u];
       }
       lm = lm_add(lm, dt, a.nylm);
     }
   }
   acc = block_sum(acc);
   if (tid == 0) s.part[(size_t)c * (kMaxHist + 1)] = acc;
-  if (!last_chunk(a, s, k)) return;
-  sum_parts(a, s, k, 1, tot);
+  if (!last_chunk(a, s, k, SUB)) return;
+  sum_parts(a, s, k, 1, tot, SUB);
   if (tid == 0) {
     const int2 sp = spheres_of(a, k);
     const double nrm = sqrt(tot[0] / (double)max(sp.y - sp.x, 1));
@@ -542,12 +571,15 @@ cudaError_t by_chunk(const SolverArgs& a, F&& f) {
 
 }  // namespace
 
-// Chunk length: 512 elements while longer chunks would leave the device short
-// of blocks (fewer than 296 chunks of 2,048, two per SM); 8,192 for one
-// molecule that fills it with those, so that the last chunk sums few parts
-// (20,000 spheres, lmax 10: k_gram 140 us with 1,182 chunks, 88 us with 296)
+// Rows of the partial sums: a block of k_extrap each
+int solver_parts(int nchunk, int chunk) { return nchunk * (chunk == 2048 ? kSub<2048> : 1); }
+// Chunk length of k_gram's blocks (k_gram us, both systems, FP64): 512 elements
+// while 2,048 would leave half of the SMs without a block per system (154,000
+// elements 33.4 by 512 and 32.8 by 2,048, 250,000 42.9 and 38.9, 605,000 67 and
+// 53); 8,192 for one molecule that fills the device with those, so that the
+// last chunk sums few parts (2.4 million, FP32: 140 by 2,048 and 83 by 8,192)
 int solver_chunk(long long n_total, bool one) {
-  return n_total < 296LL * 2048 ? 512 : one && n_total >= 148LL * 8192 ? 8192 : 2048;
+  return n_total < 148LL * 1024 ? 512 : one && n_total >= 148LL * 8192 ? 8192 : 2048;
 }
 
 cudaError_t launch_solver_begin(Launch L, const SolverArgs& a, int ns, bool mixed) {
@@ -558,10 +590,10 @@ cudaError_t launch_solver_begin(Launch L, const SolverArgs& a, int ns, bool mixe
 }
 cudaError_t launch_solver_step(Launch L, const SolverArgs& a, int ns, bool f32, int which) {
   if (a.nchunk == 0) return cudaSuccess;
-  const dim3 g(a.nchunk, ns);
   ++*L.launches;
   return by_chunk(a, [&](auto ck) {
     constexpr int CK = decltype(ck)::value;
+    const dim3 g(a.nchunk * (which == 0 ? 1 : kSub<CK>), ns);
     if (which == 0) {
       launch_chained(f32 ? k_gram<float, CK> : k_gram<double, CK>, g, kT, 0, L.st, a);
     } else {

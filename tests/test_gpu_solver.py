@@ -52,3 +52,12 @@ def test_budget_runs_out():
             with pytest.raises(DDCosmoError) as e:
                 dd.energy_forces(m["q"], m["x"], m["y"], m["z"], m["r"])
             assert e.value.status == DDC_ERR_NOCONV
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("n", [3092, 3093, 3135, 3136])
+def test_where_the_chunks_grow(n, prec):
+    """49 elements per sphere: 151,508 elements by 512 and 151,557 by 2,048, the
+    last chunk with 5 elements (k_extrap's other three blocks of it have none);
+    75 chunks and 15 elements, 64 more."""
+    test_solution_meets_the_stop_test(n, 6, 110, {}, prec)
