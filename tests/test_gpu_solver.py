@@ -61,3 +61,21 @@ def test_where_the_chunks_grow(n, prec):
     last chunk with 5 elements (k_extrap's other three blocks of it have none);
     75 chunks and 15 elements, 64 more."""
     test_solution_meets_the_stop_test(n, 6, 110, {}, prec)
+
+
+def test_no_early_stop():
+    """Small molecules to 1e-12: the coefficients of the late extrapolations
+    must not be rounding noise, which stops some solves with errors of 1e-10 to
+    3e-9.  With exact coefficients the largest error of 40 molecules is 7e-12
+    of a solution of norm about 1; the increment of the returned solution
+    stays within 50 times the tolerance."""
+    from ddpcm_b200 import molecules as M
+    from ddpcm_b200.ddcosmo import DDCosmo
+    with DDCosmo(lmax=6, ngrid=110, iconv=12, eta=0.1) as dd:
+        for seed in range(20, 50):
+            m = M.to_bohr(M.make_molecule(12, seed, globule=False))
+            out = dd.energy_forces(m["q"], m["x"], m["y"], m["z"], m["r"])
+            dd.ddinit(m["x"], m["y"], m["z"], m["r"])
+            phi, psi = dd.mkrhs(m["q"], m["x"], m["y"], m["z"])
+            assert _increment(dd, out["sigma"], dd.rhs(phi), dd.lx) <= 5e-11
+            assert _increment(dd, out["s"], psi, dd.lstarx) <= 5e-11
