@@ -178,12 +178,13 @@ struct ddc_ctx {
   // operator's per-triple lx values
   DBuf y2, hist_x2, hist_e2, rres2, eres2, tval;
   // the two dense contractions of every operator application (projection
-  // onto the harmonics, expansion to the grid): basisT[Y][G] is the basis
-  // transposed for the FP64 expansion, bwT[Y][G] with the weights; tc plans the tensor-core kernels of
-  // the mixed path, whose FP32 grid field pot_f has rows ldp_f floats apart
-  DBuf basisT, bwT;
+  // onto the harmonics, expansion to the grid): the folded kernels' tables;
+  // tc plans the tensor-core kernels of the mixed path, whose FP32 grid field
+  // pot_f has rows ldp_f floats apart
+  FoldTab fold{};
+  DBuf fold_img, fold_first, fold_lm, fold_p, fold_xw, fold_xb;
   TcPlan tc;
-  bool dmma_f32 = false;  // mixed: both contractions on the FP64 tensor cores
+  bool fold_f32 = false;  // mixed: the folded kernels too
   int ldp_f = 0;
   // learned initial guess: the attached model, its feature rows, and flags
   // for the flows (rhs/psi/sigma/s of the last flow are valid; the initial
@@ -459,8 +460,8 @@ int check_count_total(ddc_ctx* ctx, unsigned long long total, const char* what) 
 }
 
 // most products (harmonics x spheres x grid points) of a contraction that the
-// mixed operators run on the FP64 tensor cores
-constexpr long long kDmmaProducts = 50000000;
+// mixed operators fold
+constexpr long long kFoldProducts = 200000000;
 
 // What depends on the parameters alone (degree, grid, eta), once per context:
 // the constants, the grid, the basis with its transposes and weights.
@@ -474,17 +475,21 @@ int static_tables(ddc_ctx* ctx) {
   CK(ctx->grid.ensure(sizeof(double4) * G));
   CK(ctx->gpos.ensure(sizeof(int) * G));
   {
-    // the grid in Morton order of the points' directions: 32 consecutive
-    // points form a compact patch of the sphere, so that a warp's points lie
-    // inside nearly the same neighbours (k_fiui skips together those that
-    // miss the patch; the triple values, the fields and the point lists that
-    // consecutive threads read are adjacent)
+    // the grid octant by octant, in each by the Morton order of the points'
+    // absolute coordinates: 32 consecutive points form a compact patch of the
+    // sphere, so that a warp's points lie inside nearly the same neighbours
+    // (k_fiui skips together those that miss the patch; the triple values, the
+    // fields and the point lists that consecutive threads read are adjacent),
+    // and the mirror images of consecutive points are consecutive
     std::vector<std::pair<uint64_t, int>> key(G);
     for (int k = 0; k < G; k++) {
       uint64_t m = 0;
       uint32_t c[3];
-      for (int d = 0; d < 3; d++)
-        c[d] = (uint32_t)std::min(1023.0, std::floor((ctx->h_grid[4 * k + d] + 1.0) * 511.75));
+      for (int d = 0; d < 3; d++) {
+        const double x = ctx->h_grid[4 * k + d];
+        if (x < 0.0) m |= 1u << d;
+        c[d] = (uint32_t)std::min(1023.0, std::floor(std::fabs(x) * 1023.5));
+      }
       for (int b = 9; b >= 0; b--)
         for (int d = 0; d < 3; d++) m = (m << 1) | ((c[d] >> b) & 1u);
       key[k] = {m, k};
@@ -500,17 +505,35 @@ int static_tables(ddc_ctx* ctx) {
                        ctx->st));
     CK(cudaMemcpyAsync(ctx->gpos.p, gpos.data(), sizeof(int) * G, cudaMemcpyHostToDevice,
                        ctx->st));
+    std::vector<short> img, lm;
+    std::vector<uint8_t> first;
+    if (!fold_tables(g4, ctx->prm.lmax, ctx->fold, img, first, lm))
+      return fail(ctx, DDC_ERR_STATE, "the grid is not symmetric under reflections");
+    auto upload = [&](DBuf& b, const auto& v) -> int {
+      CK(b.ensure(v.size() * sizeof(v[0])));
+      CK(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, ctx->st));
+      return DDC_OK;
+    };
+    CKI(upload(ctx->fold_img, img));
+    CKI(upload(ctx->fold_first, first));
+    CKI(upload(ctx->fold_lm, lm));
+    ctx->fold.img = ctx->fold_img.as<short>();
+    ctx->fold.first = ctx->fold_first.as<uint8_t>();
+    ctx->fold.lm = ctx->fold_lm.as<short>();
   }
   CK(ctx->basis.ensure(sizeof(double) * G * NY));
   CK(ctx->bw.ensure(sizeof(double) * G * NY));
   CK(launch_basis(L, ctx->tb, ctx->grid.as<double4>(), ctx->basis.as<double>(),
                   ctx->bw.as<double>()));
-  // the basis transposed to [Y][G] for the FP64 expansions xi = basis^T s
-  // (forces, zeta) and w xi = bw^T s (the operators)
-  for (auto t : {std::make_pair(&ctx->basis, &ctx->basisT), std::make_pair(&ctx->bw, &ctx->bwT)}) {
-    CK(t.second->ensure(sizeof(double) * G * NY));
-    CK(launch_transpose(L, G, NY, t.first->as<double>(), t.second->as<double>()));
-  }
+  CK(ctx->fold_p.ensure(sizeof(double) * ctx->fold.psize));
+  CK(ctx->fold_xw.ensure(sizeof(double) * ctx->fold.xsize));
+  CK(ctx->fold_xb.ensure(sizeof(double) * ctx->fold.xsize));
+  CK(launch_fold_pack(L, ctx->fold, ctx->basis.as<double>(), ctx->bw.as<double>(),
+                      ctx->fold_p.as<double>(), ctx->fold_xw.as<double>(),
+                      ctx->fold_xb.as<double>()));
+  ctx->fold.pf = ctx->fold_p.as<double>();
+  ctx->fold.xfw = ctx->fold_xw.as<double>();
+  ctx->fold.xfb = ctx->fold_xb.as<double>();
   ctx->tables_ready = true;
   return DDC_OK;
 }
@@ -689,12 +712,13 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
     // diagnostic switch: the tests compare the two paths' accuracy)
     const char* tc_off = std::getenv("DDC_TC_OFF");
     const bool tc_env = !(tc_off && tc_off[0] == '1');
-    // smaller molecules run them on the FP64 tensor cores instead, where the
-    // set-up of a tcgen05 tile is the larger part: 2,000 spheres, lmax 8, 302
-    // points (4.9e7 products) 15 / 16 us against 19 / 17 us; 5,000 spheres,
-    // lmax 6 (7.4e7) 21 / 22 against 21 / 19 us
-    ctx->dmma_f32 = tc_env && (long long)NY * NP <= kDmmaProducts;
-    const bool tc = tc_supported(NY) && tc_env && !ctx->dmma_f32;
+    // up to 2e8 products (harmonics x points) the folded FP64 kernels instead,
+    // whose blocks are short (projection / expansion us, folded against
+    // tcgen05): 5,000 spheres, lmax 6, 302 points (7.4e7) 13 / 19 against 21 /
+    // 20, 8,000 (1.2e8) 15 / 20 against 21 / 20; 48 molecules, 18,000 spheres,
+    // lmax 8 (4.5e8) 22 / 32 against 24 / 24
+    ctx->fold_f32 = tc_env && (long long)NY * NP <= kFoldProducts;
+    const bool tc = tc_supported(NY) && tc_env && !ctx->fold_f32;
     ctx->ldp_f = tc ? (G + 3) / 4 * 4 : G;
     CK(ctx->pot_f.ensure(sizeof(float) * std::max<long long>((long long)N * ctx->ldp_f, 1LL)));
     CK(ctx->xi_f.ensure(sizeof(float) * std::max(NP, 1LL)));
@@ -704,7 +728,7 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
       // tile widths by measurement (rhs and y are free work vectors here)
       CK(tc_autotune(L, ctx->tc, ctx->rhs.as<double>(), ctx->y.as<double>(),
                      ctx->xi_f.as<float>()));
-    } else if (ctx->dmma_f32) {
+    } else if (ctx->fold_f32) {
       ctx->tc.on = false;
     } else {
       ctx->tc.on = false;
@@ -794,16 +818,14 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
 // y(lm,i) = alpha sum_n bw(lm,n) pot(n,i): intrhs over every sphere
 // (matvec.f90:131-135, bw = w_n Y_lm(s_n))
 int gemm_proj(ddc_ctx* ctx, double alpha, const double* pot, double* y) {
-  CK(launch_dgemm_nn(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, alpha, ctx->bw.as<double>(),
-                     ctx->nylm, pot, ctx->ngrid, y, ctx->nylm, ctx->sweep));
+  CK(launch_fold_proj(ctx->L(), ctx->fold, ctx->nsph, alpha, pot, ctx->ngrid, y, ctx->sweep));
   return DDC_OK;
 }
 // projection of the FP32 field (rows ldp_f apart) into the FP64 vector y
 int gemm_proj_f32(ddc_ctx* ctx, float alpha, const float* pot, double* y) {
-  if (ctx->dmma_f32)
-    CK(launch_dgemm_nn(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, (double)alpha,
-                       ctx->bw.as<double>(), ctx->nylm, pot, ctx->ldp_f, y, ctx->nylm,
-                       ctx->sweep));
+  if (ctx->fold_f32)
+    CK(launch_fold_proj(ctx->L(), ctx->fold, ctx->nsph, (double)alpha, pot, ctx->ldp_f, y,
+                        ctx->sweep));
   else if (ctx->tc.on)
     CK(launch_proj_tc(ctx->L(), ctx->tc, alpha, y, ctx->sweep));
   else
@@ -813,16 +835,13 @@ int gemm_proj_f32(ddc_ctx* ctx, float alpha, const float* pot, double* y) {
 }
 // xi(n,i) = sum_lm basis(lm,n) s(lm,i)   (matvec.f90:189-204); weighted: w_n xi
 int gemm_xi(ddc_ctx* ctx, const double* s, double* xig, bool weighted) {
-  CK(launch_dgemm_nn(ctx->L(), ctx->ngrid, ctx->nsph, ctx->nylm, 1.0,
-                     (weighted ? ctx->bwT : ctx->basisT).as<double>(), ctx->ngrid, s, ctx->nylm,
-                     xig, ctx->ngrid, ctx->sweep));
+  CK(launch_fold_xi(ctx->L(), ctx->fold, weighted, ctx->nsph, s, xig, ctx->ngrid, ctx->sweep));
   return DDC_OK;
 }
 // FP32 w_n xi of the FP64 vector s
 int gemm_xi_f32(ddc_ctx* ctx, const double* s, float* xig) {
-  if (ctx->dmma_f32)
-    CK(launch_dgemm_nn(ctx->L(), ctx->ngrid, ctx->nsph, ctx->nylm, 1.0, ctx->bwT.as<double>(),
-                       ctx->ngrid, s, ctx->nylm, xig, ctx->ngrid, ctx->sweep));
+  if (ctx->fold_f32)
+    CK(launch_fold_xi(ctx->L(), ctx->fold, true, ctx->nsph, s, xig, ctx->ngrid, ctx->sweep));
   else if (ctx->tc.on)
     CK(launch_xi_tc(ctx->L(), ctx->tc, s, xig, ctx->sweep));
   else
@@ -1302,8 +1321,8 @@ int direct_rhs(ddc_ctx* ctx, const double* phi, double* rhs) {
   CK(ctx->gbuf.ensure(sizeof(double) * std::max<long long>((long long)ctx->nsph * ctx->ngrid, 1)));
   StageScope sc(ctx, ST_RHS);
   CK(launch_wghpot(ctx->L(), ctx->geo(), phi, ctx->gbuf.as<double>()));
-  CK(launch_dgemm_nn(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, 1.0, ctx->bw.as<double>(),
-                     ctx->nylm, ctx->gbuf.as<double>(), ctx->ngrid, rhs, ctx->nylm));
+  CK(launch_fold_proj(ctx->L(), ctx->fold, ctx->nsph, 1.0, ctx->gbuf.as<double>(), ctx->ngrid,
+                      rhs, SweepMask{}));
   return DDC_OK;
 }
 
@@ -1681,8 +1700,8 @@ int ddc_rhs(ddc_ctx* ctx, const double* phi, double* g) {
   CKI(out_ptr(ctx, g, (size_t)ctx->nsph * ctx->nylm, ctx->out1, &dg));
   CK(ctx->gbuf.ensure(sizeof(double) * std::max<long long>((long long)ctx->nsph * ctx->ngrid, 1)));
   CK(launch_wghpot(ctx->L(), ctx->geo(), dphi, ctx->gbuf.as<double>()));
-  CK(launch_dgemm_nn(ctx->L(), ctx->nylm, ctx->nsph, ctx->ngrid, 1.0, ctx->bw.as<double>(),
-                     ctx->nylm, ctx->gbuf.as<double>(), ctx->ngrid, dg, ctx->nylm));
+  CK(launch_fold_proj(ctx->L(), ctx->fold, ctx->nsph, 1.0, ctx->gbuf.as<double>(), ctx->ngrid, dg,
+                      SweepMask{}));
   CKI(finish_out(ctx, g, dg, (size_t)ctx->nsph * ctx->nylm));
   return sync(ctx);
 }

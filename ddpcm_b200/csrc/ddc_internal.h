@@ -116,6 +116,20 @@ struct SweepMask {
   const int* st1;  // [nmol] status of the second system, or null
 };
 
+// Tables of the folded contractions (ddc_fold.cu): orbits of the grid under the
+// three reflections and the eight parity classes of the harmonics.
+struct FoldTab {
+  int norb, otiles;  // orbits, tiles of eight orbits
+  int oc;            // orbits per pass of a block
+  int nylm;
+  int psize, xsize;  // entries of pf; of xfw and xfb
+  int cnt[8], poff[8], xoff[8];  // harmonics per class, first entries in pf and xf*
+  const short* img;              // [norb][8] grid point of image k (bits: x, y, z)
+  const uint8_t* first;          // [norb] images that are other points than earlier ones
+  const short* lm;               // [8][32] the classes' harmonics
+  const double *pf, *xfw, *xfb;  // operands in fragment order
+};
+
 #ifdef __CUDACC__
 // The kernels of a solver sweep follow one another with a dependency on all
 // of the previous kernel.  Launched with launch_chained they are scheduled
@@ -332,20 +346,20 @@ cudaError_t launch_lx_gather(Launch L, const DevGeo& g, const double* val, doubl
 cudaError_t launch_lx_gather_f32(Launch L, const DevGeo& g, const float* val, float* pot,
                                  int ldp);
 cudaError_t launch_to_float(Launch L, long long n, const double* x, float* y);
-// dst[c*rows + r] = src[r*cols + c] (FP64)
-cudaError_t launch_transpose(Launch L, int rows, int cols, const double* src, double* dst);
-// C[n*ldc + m] = alpha * sum_k A[k*lda + m] B[n*ldb + k] in FP64 arithmetic;
-// with act set the N columns are spheres and tiles of skipped spheres
-// are left alone
-cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
-                            int lda, const double* B, int ldb, double* C, int ldc,
-                            const SweepMask& act = SweepMask{});
-cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
-                            int lda, const float* B, int ldb, double* C, int ldc,
-                            const SweepMask& act = SweepMask{});
-cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
-                            int lda, const double* B, int ldb, float* C, int ldc,
-                            const SweepMask& act = SweepMask{});
+// projection C(lm,i) = alpha sum_n w_n Y_lm(s_n) B(n,i) and expansion
+// xi(n,i) = [w_n] sum_lm Y_lm(s_n) s(lm,i) over the reflection classes of grid
+// and harmonics (ddc_fold.cu); FP64 arithmetic, FP64 or FP32 grid fields with
+// rows ldb / ldc apart.  With act, blocks of skipped spheres are left alone.
+bool fold_tables(const std::vector<double>& g4, int lmax, FoldTab& t, std::vector<short>& img,
+                 std::vector<uint8_t>& first, std::vector<short>& lm);
+cudaError_t launch_fold_pack(Launch L, const FoldTab& t, const double* basis, const double* bw,
+                             double* pf, double* xw, double* xb);
+template <class TB>
+cudaError_t launch_fold_proj(Launch L, const FoldTab& t, int N, double alpha, const TB* B, int ldb,
+                             double* C, const SweepMask& act);
+template <class TC>
+cudaError_t launch_fold_xi(Launch L, const FoldTab& t, bool weighted, int N, const double* s,
+                           TC* xi, int ldc, const SweepMask& act);
 // FP32 SIMT projection / expansion (mixed path, more than 128 harmonics)
 cudaError_t launch_proj_f32_simt(Launch L, int nylm, int nsph, int ngrid, float alpha,
                                  const float* bw_f, const float* pot, int ldp, double* y);

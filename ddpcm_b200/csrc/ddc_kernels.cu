@@ -767,290 +767,6 @@ cudaError_t gemm2(Launch L, int M, int N, int K, Acc alpha, const TAin* A, int l
   return cudaGetLastError();
 }
 
-// dst[c*rows + r] = src[r*cols + c]
-__global__ void k_transpose(int rows, int cols, const double* __restrict__ src, double* dst) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long long)rows * cols) return;
-  const int r = (int)(e / cols), c = (int)(e - (long long)r * cols);
-  dst[(size_t)c * rows + r] = src[e];
-}
-cudaError_t launch_transpose(Launch L, int rows, int cols, const double* src, double* dst) {
-  const long long n = (long long)rows * cols;
-  if (n == 0) return cudaSuccess;
-  k_transpose<<<(unsigned)((n + 255) / 256), 256, 0, L.st>>>(rows, cols, src, dst);
-  ++*L.launches;
-  return cudaGetLastError();
-}
-// GEMM of the operators' projection and expansion on the FP64 tensor cores
-// (DMMA, mma.sync m8n8k4; tcgen05 has no FP64 kind):
-//   C[n*ldc + m] = alpha * sum_k A[k*lda + m] B[n*ldb + k],
-// B and C in FP64, or (mixed path, smaller molecules) FP32 grid fields.
-// No shared-memory staging: A is the static operand (at most 0.6 MB at lmax
-// 10 and 590 points) and comes from L2 / L1 straight into the fragments, as
-// does B, whose rows are read along k.  A block takes 8 NB spheres and
-// 32 MG rows; its eight warps are MG row groups of 32 rows times KS slices of
-// k, whose partial tiles are summed in slice order through shared memory.  So
-// a few spheres spread over many warps: the kernel this replaces walked k in
-// one 128 x 64 tile per block, 13 us at 12 spheres and 26 us at 600 whatever
-// the arithmetic.  Bound: the FP64 tensor pipe for many spheres, L2 latency
-// for few.
-template <class TB, class TC, int NB, int KS>
-__global__ void __launch_bounds__(256) k_dmma(int M, int N, int K, double alpha,
-                                              const double* __restrict__ A, int lda,
-                                              const TB* __restrict__ B, int ldb,
-                                              TC* __restrict__ C, int ldc, const SweepMask act) {
-  chain_wait();
-  constexpr int MT = 4, MG = 8 / KS;  // 8-row tiles per warp, row groups per block
-  constexpr int TS = MT * NB * 64;    // values of a warp's tile
-  extern __shared__ __align__(16) double dm_smem[];  // [KS - 1][MG][TS]
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * 8 * NB;
-  // columns are spheres: a sweep skips a block whose spheres all belong to
-  // stopped molecules
-  if (act.st0 && __syncthreads_and(tid >= 8 * NB || n0 + tid >= N || sweep_skip(act, n0 + tid)))
-    return;
-  const int ks = w % KS, mg = w / KS;
-  const int m0 = (blockIdx.y * MG + mg) * 8 * MT;
-  const int fr = lane >> 2, fk = lane & 3;  // fragment row (A) or column (B), and k
-  // slice ks takes the k steps ks, ks + KS, ... of four, so that the block's
-  // warps read neighbouring parts of B's rows
-  const int k0 = 4 * ks, nfull = K / 4 > ks ? (K / 4 - ks + KS - 1) / KS : 0;
-  double acc[MT][NB][2];
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  // rows and columns past the end read the last one; they are not stored
-  const double* pa[MT];
-  const TB* pb[NB];
-#pragma unroll
-  for (int i = 0; i < MT; ++i) pa[i] = A + (size_t)(k0 + fk) * lda + min(m0 + 8 * i + fr, M - 1);
-#pragma unroll
-  for (int j = 0; j < NB; ++j) pb[j] = B + (size_t)min(n0 + 8 * j + fr, N - 1) * ldb + k0 + fk;
-  auto mma = [&](const double* a, const double* b) {
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < NB; ++j)
-        asm volatile(
-            "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-            : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
-            : "d"(a[i]), "d"(b[j]));
-  };
-  constexpr int U = NB == 1 ? 4 : 2;  // k steps whose loads are in flight together
-  int t = 0;
-  for (; t + U <= nfull; t += U) {
-    double a[U][MT], b[U][NB];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-#pragma unroll
-      for (int i = 0; i < MT; ++i) a[u][i] = pa[i][(size_t)4 * KS * (t + u) * lda];
-#pragma unroll
-      for (int j = 0; j < NB; ++j) b[u][j] = (double)pb[j][4 * KS * (t + u)];
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) mma(a[u], b[u]);
-  }
-  // the remaining full steps, then the partial one (K not a multiple of four)
-  const int last = (K & 3) && (K / 4) % KS == ks ? nfull + 1 : nfull;
-  for (; t < last; ++t) {
-    const bool ok = k0 + 4 * KS * t + fk < K;
-    double a[MT], b[NB];
-#pragma unroll
-    for (int i = 0; i < MT; ++i) a[i] = ok ? pa[i][(size_t)4 * KS * t * lda] : 0.0;
-#pragma unroll
-    for (int j = 0; j < NB; ++j) b[j] = ok ? (double)pb[j][4 * KS * t] : 0.0;
-    mma(a, b);
-  }
-  // slices 1.. leave their tiles; slice 0 adds them in order and stores
-  if (ks > 0) {
-    double* r = dm_smem + ((size_t)(ks - 1) * MG + mg) * TS;
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) r[((i * NB + j) * 2 + h) * 32 + lane] = acc[i][j][h];
-  }
-  __syncthreads();
-  if (ks > 0) return;
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        double v = acc[i][j][h];
-#pragma unroll
-        for (int q = 0; q < KS - 1; ++q)
-          v += dm_smem[((size_t)q * MG + mg) * TS + ((i * NB + j) * 2 + h) * 32 + lane];
-        const int m = m0 + 8 * i + fr, n = n0 + 8 * j + 2 * fk + h;
-        if (m < M && n < N) C[(size_t)n * ldc + m] = (TC)(alpha * v);
-      }
-}
-template <class TB, class TC, int NB, int KS>
-static cudaError_t dmma_launch(Launch L, int M, int N, int K, double alpha, const double* A,
-                               int lda, const TB* B, int ldb, TC* C, int ldc,
-                               const SweepMask& act) {
-  constexpr int MG = 8 / KS;
-  constexpr size_t sm = sizeof(double) * (KS - 1) * MG * 4 * NB * 64;
-  auto kfn = k_dmma<TB, TC, NB, KS>;
-  if (sm > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e) return e;
-  }
-  const dim3 grid((N + 8 * NB - 1) / (8 * NB), (M + 32 * MG - 1) / (32 * MG));
-  ++*L.launches;
-  return launch_chained(kfn, grid, 256, sm, L.st, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-}
-// The same product for shapes of many tiles (B and C in FP64):
-// 128 x 64 tiles, 8 warps of 32 x 32 (4 x 4 MMA tiles of 8 x 8), 16-deep k
-// slabs copied to shared memory with cp.async (the next slab in flight).
-// Shared rows are padded so that each warp's fragment loads take the
-// minimum two wavefronts: A rows of 136 doubles (a row stride of 16 banks
-// mod 32 separates k and k + 1), B rows of 20 (8 banks mod 32 separates
-// four columns).  Each output is one FMA chain in k order.
-namespace dgp {
-constexpr int BM = 128, BN = 64, BK = 16;
-constexpr int AS = BM + 8, BS = BK + 4;
-constexpr int SMEM = (2 * BK * AS + 2 * BN * BS) * 8;
-}
-__device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
-  const int n = valid ? 8 : 0;  // 0: nothing read, the destination is zero-filled
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gsrc), "r"(n)
-               : "memory");
-}
-__global__ void __launch_bounds__(256, 3) k_dgemm_dmma(int M, int N, int K, double alpha,
-                                                       const double* __restrict__ A, int lda,
-                                                       const double* __restrict__ B, int ldb,
-                                                       double* __restrict__ C, int ldc,
-                                                       const SweepMask act) {
-  chain_wait();
-  using namespace dgp;
-  extern __shared__ __align__(16) double dg_smem[];
-  double* As = dg_smem;                // [2][BK][AS]
-  double* Bs = dg_smem + 2 * BK * AS;  // [2][BN][BS]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = warp & 3, wn = warp >> 2;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  // columns are spheres: a batched sweep skips a tile whose spheres all belong
-  // to stopped molecules
-  if (act.st0 && __syncthreads_and(tid >= BN || n0 + tid >= N || sweep_skip(act, n0 + tid)))
-    return;
-  auto load = [&](int buf, int k0) {
-#pragma unroll
-    for (int u = 0; u < BM * BK / 256; ++u) {
-      const int e = tid + u * 256;
-      const int mm = e % BM, kk = e / BM;
-      const int m = m0 + mm, k = k0 + kk;
-      const bool ok = m < M && k < K;
-      cp_async8(As + (buf * BK + kk) * AS + mm, ok ? A + (size_t)k * lda + m : A, ok);
-    }
-#pragma unroll
-    for (int u = 0; u < BN * BK / 256; ++u) {
-      const int e = tid + u * 256;
-      const int kk = e % BK, nn = e / BK;
-      const int n = n0 + nn, k = k0 + kk;
-      const bool ok = n < N && k < K;
-      cp_async8(Bs + (buf * BN + nn) * BS + kk, ok ? B + (size_t)n * ldb + k : B, ok);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  double acc[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int nk = (K + BK - 1) / BK;
-  const int fr = lane >> 2, fk = lane & 3;  // fragment row / k of this lane
-  load(0, 0);
-  for (int t = 0; t < nk; ++t) {
-    const int buf = t & 1;
-    if (t + 1 < nk) {
-      load(buf ^ 1, (t + 1) * BK);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    const double* as = As + buf * BK * AS;
-    const double* bs = Bs + buf * BN * BS;
-#pragma unroll
-    for (int ks = 0; ks < BK; ks += 4) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = as[(ks + fk) * AS + wm * 32 + i * 8 + fr];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = bs[(wn * 32 + j * 8 + fr) * BS + ks + fk];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          asm volatile(
-              "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-              : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
-              : "d"(a[i]), "d"(b[j]));
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int m = m0 + wm * 32 + i * 8 + fr;
-        const int n = n0 + wn * 32 + j * 8 + 2 * fk + h;
-        if (m < M && n < N) C[(size_t)n * ldc + m] = alpha * acc[i][j][h];
-      }
-}
-// Shapes with fewer 128 x 64 tiles than 1.5 per SM: eight slices of k and
-// eight spheres per block, for the latency (12 spheres, 110 points: 7 to 8 us
-// for either product, 9 to 15 us with two slices); 16 spheres once that fills
-// the device (5,000 spheres, lmax 10, 590 points: projection 48 us, 62 us
-// with eight), for the expansion with two slices, 128 rows per block (2,000
-// spheres, lmax 8, 302 points: 17 us, 20 to 25 us with eight).
-template <class TB, class TC>
-static cudaError_t dgemm_few(Launch L, int M, int N, int K, double alpha, const double* A, int lda,
-                             const TB* B, int ldb, TC* C, int ldc, const SweepMask& act) {
-  if (M == 0 || N == 0) return cudaSuccess;
-  const long long n16 = (N + 15) / 16, rows128 = (M + 127) / 128, rows32 = (M + 31) / 32;
-  if (K < M && n16 * rows128 >= 74)
-    return dmma_launch<TB, TC, 2, 2>(L, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-  if (K >= M && n16 * rows32 >= 296)
-    return dmma_launch<TB, TC, 2, 8>(L, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-  return dmma_launch<TB, TC, 1, 8>(L, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-}
-// From 222 tiles of 128 x 64 on, the staged kernel: it reads A once per 64
-// spheres (20,000 spheres, lmax 10, 590 points: expansion 131 us against 162
-// us, projection 162 against 179 us; 5,000 spheres: expansion 43 against 54
-// us, but projection, 79 tiles, 74 against 48 us).
-cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
-                            int lda, const double* B, int ldb, double* C, int ldc,
-                            const SweepMask& act) {
-  if (M == 0 || N == 0) return cudaSuccess;
-  const dim3 grid((M + dgp::BM - 1) / dgp::BM, (N + dgp::BN - 1) / dgp::BN);
-  if ((long long)grid.x * grid.y < 222)
-    return dgemm_few(L, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-  cudaError_t e = cudaFuncSetAttribute(k_dgemm_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       dgp::SMEM);
-  if (e) return e;
-  ++*L.launches;
-  return launch_chained(k_dgemm_dmma, grid, 256, dgp::SMEM, L.st, M, N, K, alpha, A, lda, B, ldb, C,
-                        ldc, act);
-}
-cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
-                            int lda, const float* B, int ldb, double* C, int ldc,
-                            const SweepMask& act) {
-  return dgemm_few(L, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-}
-cudaError_t launch_dgemm_nn(Launch L, int M, int N, int K, double alpha, const double* A,
-                            int lda, const double* B, int ldb, float* C, int ldc,
-                            const SweepMask& act) {
-  return dgemm_few(L, M, N, K, alpha, A, lda, B, ldb, C, ldc, act);
-}
 // FP32 SIMT contractions of the mixed path where the tensor-core kernels do
 // not apply (more than 128 harmonics): projection into FP64 y, and xi of the
 // FP64 vector s
