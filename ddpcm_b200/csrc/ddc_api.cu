@@ -209,6 +209,7 @@ struct ddc_ctx {
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t st_out = nullptr;  // results to the host beside the force kernels
+  cudaEvent_t ev_out = nullptr;
   cudaEvent_t ev_mark[3] = {};    // ends of the phases of a run
   unsigned int stage_mask = ~0u;  // stages timed when prm.timing is set
 
@@ -703,7 +704,6 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
     CK(cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
-    CK(cudaStreamCreateWithFlags(&ctx->st_out, cudaStreamNonBlocking));
   }
   if (ctx->prm.precision == DDC_PREC_MIXED) {
     // the two contractions run on the tensor cores (split TF32) up to 128
@@ -1309,8 +1309,11 @@ int solute_pot_field(ddc_ctx* ctx, const double* q, double* phi, double* ef, con
                                 ctx->cz.as<double>(), NC, ctx->ccav.as<double>(), phi, ef,
                                 trange));
   } else {
+    const int nchunk = trange ? 1 : efield_chunks(N, NC);
+    CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(NC, 1) * nchunk));
     CK(launch_coulomb_pot(ctx->L(), N, q, ctx->cx.as<double>(), ctx->cy.as<double>(),
-                          ctx->cz.as<double>(), NC, ctx->ccav.as<double>(), phi, trange));
+                          ctx->cz.as<double>(), NC, ctx->ccav.as<double>(), phi,
+                          ctx->ef_scratch.as<double>(), nchunk, trange));
   }
   return DDC_OK;
 }
@@ -1484,6 +1487,7 @@ int ddc_destroy(ddc_ctx* c) {
     if (e) cudaEventDestroy(e);
   if (c->st2) cudaStreamSynchronize(c->st2);
   if (c->st_out) cudaStreamDestroy(c->st_out);
+  if (c->ev_out) cudaEventDestroy(c->ev_out);
   for (cudaEvent_t e : c->ev_mark)
     if (e) cudaEventDestroy(e);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -1665,6 +1669,12 @@ int ddc_get_grid(ddc_ctx* ctx, double* grid, double* w) {
   return DDC_OK;
 }
 
+// the stream of results that go to the host beside kernels
+static int out_stream(ddc_ctx* ctx) {
+  if (!ctx->st_out) CK(cudaStreamCreateWithFlags(&ctx->st_out, cudaStreamNonBlocking));
+  if (!ctx->ev_out) CK(cudaEventCreateWithFlags(&ctx->ev_out, cudaEventDisableTiming));
+  return DDC_OK;
+}
 int ddc_mkrhs(ddc_ctx* ctx, int n, const double* charge, const double* x, const double* y,
               const double* z, int ncav, const double* ccav, double* phi, int nylm, double* psi) {
   if (!ctx) return DDC_ERR_PARAM;
@@ -1684,10 +1694,28 @@ int ddc_mkrhs(ddc_ctx* ctx, int n, const double* charge, const double* x, const 
   double *dphi, *dpsi;
   CKI(out_ptr(ctx, phi, ncav, ctx->phi, &dphi));
   CKI(out_ptr(ctx, psi, (size_t)n * nylm, ctx->out1, &dpsi));
-  CK(launch_coulomb_pot(ctx->L(), n, dq, dx, dy, dz, ncav, dc, dphi, nullptr));
+  const int nchunk = efield_chunks(n, ncav);
+  CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(ncav, 1) * nchunk));
   CK(launch_psi(ctx->L(), n, nylm, dq, dpsi));
+  const bool host = !ctx->prm.device_pointers && psi && n > 0;
+  if (host) {
+    // psi goes to the host while the potential is summed (30,001 charges, 49
+    // harmonics: 12 MB, 0.85 ms with the caller's page faults)
+    CKI(out_stream(ctx));
+    CK(cudaEventRecord(ctx->ev_out, ctx->st));
+    CK(cudaStreamWaitEvent(ctx->st_out, ctx->ev_out, 0));
+  }
+  cudaError_t e = launch_coulomb_pot(ctx->L(), n, dq, dx, dy, dz, ncav, dc, dphi,
+                                     ctx->ef_scratch.as<double>(), nchunk, nullptr);
+  if (host && e == cudaSuccess) {
+    e = cudaMemcpyAsync(psi, dpsi, sizeof(double) * (size_t)n * nylm, cudaMemcpyDeviceToHost,
+                        ctx->st_out);
+    const cudaError_t w = cudaStreamSynchronize(ctx->st_out);
+    if (e == cudaSuccess) e = w;
+  }
+  CK(e);
   CKI(finish_out(ctx, phi, dphi, ncav));
-  CKI(finish_out(ctx, psi, dpsi, (size_t)n * nylm));
+  if (!host) CKI(finish_out(ctx, psi, dpsi, (size_t)n * nylm));
   return sync(ctx);
 }
 
@@ -2071,6 +2099,7 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
       // spheres: 2 x 4.8 MB into memory that is touched for the first time,
       // 3.7 ms beside 4.1 ms of kernels); the solves have ended, so no event
       // is needed
+      CKI(out_stream(ctx));
       cudaError_t e = cudaSuccess;
       for (auto o : {std::make_pair(sigma, dsig), std::make_pair(s, ds)})
         if (e == cudaSuccess && o.first && nv)

@@ -493,9 +493,10 @@ cudaError_t launch_coulomb_pot_field(Launch L, int nsrc, const double* q, const 
                                      const double* sy, const double* sz, int ntrg,
                                      const double* ctrg, double* phi, double* ef,
                                      const int2* trange);
+// phi of charges at any points, partial sums as in launch_efield below
 cudaError_t launch_coulomb_pot(Launch L, int nsrc, const double* q, const double* sx,
                                const double* sy, const double* sz, int ntrg, const double* ctrg,
-                               double* phi, const int2* trange);
+                               double* phi, double* scratch, int nchunk, const int2* trange);
 cudaError_t launch_psi(Launch L, int n, int nylm, const double* q, double* psi);
 // field of sources (q at csrc(3,nsrc)) at targets ctrg(3,ntrg); partial sums
 // over `nchunk` source chunks go to scratch[nchunk][ntrg][3]

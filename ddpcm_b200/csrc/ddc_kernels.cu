@@ -996,12 +996,16 @@ __device__ __forceinline__ SrcRange field_src_range(const int2* trange, int t, i
   return r;
 }
 
+// Potential of point charges; partial sums over chunks of the sources (grid y).
+// Bound by the FP64 pipe, 12 operations per pair.  50,003 targets are 196
+// blocks, one or two per SM: 30,001 sources took 1.86 ms in one piece and take
+// 1.3 ms in seven.
 __global__ void __launch_bounds__(kNbTile) k_coulomb_pot(int nsrc, const double* __restrict__ q,
                                                          const double* __restrict__ sx,
                                                          const double* __restrict__ sy,
                                                          const double* __restrict__ sz,
                                                          int ntrg, const double* __restrict__ ctrg,
-                                                         double* phi,
+                                                         int chunk, double* phi,
                                                          const int2* __restrict__ trange) {
   __shared__ double4 src[kNbTile];
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1011,32 +1015,27 @@ __global__ void __launch_bounds__(kNbTile) k_coulomb_pot(int nsrc, const double*
     py = ctrg[3 * (size_t)t + 1];
     pz = ctrg[3 * (size_t)t + 2];
   }
-  const SrcRange rg = block_src_range(trange, t, ntrg, 0, nsrc);
+  const SrcRange rg = field_src_range(trange, t, ntrg, nsrc, chunk);
   double v = 0.0;
   for (int j0 = rg.ulo; j0 < rg.uhi; j0 += kNbTile) {
-    int j = j0 + threadIdx.x;
+    const int j = j0 + threadIdx.x;
     __syncthreads();
     src[threadIdx.x] = j < rg.uhi ? make_double4(sx[j], sy[j], sz[j], q[j])
-                                  : make_double4(0, 0, 0, 0);
+                              : make_double4(0, 0, 0, 0);
     __syncthreads();
-    int cnt = min(kNbTile, rg.uhi - j0);
-    const int kb = max(rg.lo - j0, 0), ke = min(rg.hi - j0, cnt);
+    const int kb = max(rg.lo - j0, 0), ke = min(rg.hi - j0, min(kNbTile, rg.uhi - j0));
+    auto pair = [&](const double4& s) {
+      const double dx = px - s.x, dy = py - s.y, dz = pz - s.z;
+      v = fma(s.w, rsqrt_pos(dx * dx + dy * dy + dz * dz), v);
+    };
     if (kb == 0 && ke == kNbTile) {
 #pragma unroll 8
-      for (int k = 0; k < kNbTile; ++k) {
-        double4 s = src[k];
-        double dx = px - s.x, dy = py - s.y, dz = pz - s.z;
-        v = fma(s.w, rsqrt_pos(dx * dx + dy * dy + dz * dz), v);
-      }
+      for (int k = 0; k < kNbTile; ++k) pair(src[k]);
     } else {
-      for (int k = kb; k < ke; ++k) {
-        double4 s = src[k];
-        double dx = px - s.x, dy = py - s.y, dz = pz - s.z;
-        v = fma(s.w, rsqrt_pos(dx * dx + dy * dy + dz * dz), v);
-      }
+      for (int k = kb; k < ke; ++k) pair(src[k]);
     }
   }
-  if (t < ntrg) phi[t] = v;
+  if (t < ntrg) phi[(size_t)blockIdx.y * ntrg + t] = v;
 }
 // The potential and, for the forces, the solute's field at the same targets
 // (efld.f90:97-114 with the nuclei as sources) from one pass over the pairs:
@@ -1096,15 +1095,6 @@ cudaError_t launch_coulomb_pot_field(Launch L, int nsrc, const double* q, const 
   ++*L.launches;
   return cudaGetLastError();
 }
-cudaError_t launch_coulomb_pot(Launch L, int nsrc, const double* q, const double* sx,
-                               const double* sy, const double* sz, int ntrg, const double* ctrg,
-                               double* phi, const int2* trange) {
-  if (ntrg == 0) return cudaSuccess;
-  k_coulomb_pot<<<(ntrg + kNbTile - 1) / kNbTile, kNbTile, 0, L.st>>>(nsrc, q, sx, sy, sz, ntrg,
-                                                                       ctrg, phi, trange);
-  ++*L.launches;
-  return cudaGetLastError();
-}
 __global__ void k_psi(int n, int nylm, const double* __restrict__ q, double* psi) {
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (long long)n * nylm) return;
@@ -1122,7 +1112,7 @@ cudaError_t launch_psi(Launch L, int n, int nylm, const double* q, double* psi) 
 // Source chunks of the field kernels for few targets: enough blocks to fill the
 // device, chunks of 1,024 sources or more, as every chunk costs a row of the
 // reduction.  Up to 16 shorter ones are worth that where a chunk is walked
-// alone: 12 targets and 587 sources in FP64 43 -> 13 us with chunks of 64.
+// alone: 12 targets and 587 sources in FP64 50 -> 15 us with chunks of 64.
 static int field_chunks(int nsrc, int blocks, int shortest) {
   const int want = (148 * 8 + blocks - 1) / max(blocks, 1);
   const int maxc = max((nsrc + 4 * kNbTile - 1) / (4 * kNbTile),
@@ -1134,7 +1124,7 @@ int efield_chunks(int nsrc, int ntrg) {
 }
 // Parts of the sources when every target has its own range (batches): a block
 // of 256 targets otherwise walks all sources of its molecules alone.  48
-// molecules of 8 to 1,999 spheres, 18,000 targets in 70 blocks: 3.7 -> 0.5 ms.
+// molecules of 8 to 1,999 spheres, 18,000 targets in 70 blocks: 3.7 -> 0.7 ms.
 int efield_parts(int ntrg) {
   const int tiles = (ntrg + kNbTile - 1) / kNbTile;
   return max(1, min((148 * 8 + tiles - 1) / max(tiles, 1), 64));
@@ -1189,12 +1179,13 @@ __global__ void __launch_bounds__(kNbTile) k_efield(int nsrc, const double* __re
     o[2] = ez;
   }
 }
-__global__ void k_efield_reduce(int ntrg, int nchunk, const double* __restrict__ scratch,
+// the chunks' partial sums of n values, in chunk order
+__global__ void k_efield_reduce(long long n, int nchunk, const double* __restrict__ scratch,
                                 double* ef) {
   long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 3LL * ntrg) return;
+  if (e >= n) return;
   double s = 0.0;
-  for (int c = 0; c < nchunk; ++c) s += scratch[(size_t)c * 3 * ntrg + e];
+  for (int c = 0; c < nchunk; ++c) s += scratch[(size_t)c * n + e];
   ef[e] = s;
 }
 // FP32-pair variant (mixed precision, force terms only): coordinates are
@@ -1348,7 +1339,7 @@ cudaError_t launch_efield_f32(Launch L, int nsrc, const double* q, const double*
   ++*L.launches;
   cudaError_t e = cudaGetLastError();
   if (e || nchunk == 1) return e;
-  k_efield_reduce<<<(unsigned)((3LL * ntrg + 255) / 256), 256, 0, L.st>>>(ntrg, nchunk, scratch, ef);
+  k_efield_reduce<<<(unsigned)((3LL * ntrg + 255) / 256), 256, 0, L.st>>>(3LL * ntrg, nchunk, scratch, ef);
   ++*L.launches;
   return cudaGetLastError();
 }
@@ -1367,7 +1358,24 @@ cudaError_t launch_efield(Launch L, int nsrc, const double* q, const double* csr
   ++*L.launches;
   cudaError_t e = cudaGetLastError();
   if (e || nchunk == 1) return e;
-  k_efield_reduce<<<(unsigned)((3LL * ntrg + 255) / 256), 256, 0, L.st>>>(ntrg, nchunk, scratch, ef);
+  k_efield_reduce<<<(unsigned)((3LL * ntrg + 255) / 256), 256, 0, L.st>>>(3LL * ntrg, nchunk, scratch, ef);
+  ++*L.launches;
+  return cudaGetLastError();
+}
+cudaError_t launch_coulomb_pot(Launch L, int nsrc, const double* q, const double* sx,
+                               const double* sy, const double* sz, int ntrg, const double* ctrg,
+                               double* phi, double* scratch, int nchunk, const int2* trange) {
+  if (ntrg == 0) return cudaSuccess;
+  int chunk = (nsrc + nchunk - 1) / max(nchunk, 1);
+  chunk = max((chunk + kFieldChunk - 1) / kFieldChunk, 1) * kFieldChunk;
+  if (!trange) nchunk = max(1, (nsrc + chunk - 1) / chunk);
+  double* out = nchunk == 1 ? phi : scratch;
+  k_coulomb_pot<<<dim3((ntrg + kNbTile - 1) / kNbTile, nchunk), kNbTile, 0, L.st>>>(
+      nsrc, q, sx, sy, sz, ntrg, ctrg, chunk, out, trange);
+  ++*L.launches;
+  cudaError_t e = cudaGetLastError();
+  if (e || nchunk == 1) return e;
+  k_efield_reduce<<<(ntrg + 255) / 256, 256, 0, L.st>>>(ntrg, nchunk, scratch, phi);
   ++*L.launches;
   return cudaGetLastError();
 }

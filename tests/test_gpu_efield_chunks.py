@@ -29,6 +29,24 @@ def test_field_at_few_targets(oracle, nsrc, ntrg):
     test_field_with_rounded_chunks(oracle, nsrc, ntrg)
 
 
+@pytest.mark.parametrize("nsrc,ntrg", [(587, 12), (64, 1), (65, 300), (1025, 257), (30001, 5003),
+                                       (150000, 2305)])
+def test_potential_in_chunks(oracle, nsrc, ntrg):
+    """mkrhs at points of the caller's (mkrhs.f90:102-120), one chunk and
+    several; psi goes to the host beside the sum and must come out exactly.
+    1e-12 of the largest potential, as above."""
+    from ddpcm_b200.ddcosmo import DDCosmo
+    rng = np.random.default_rng(nsrc)
+    q = rng.uniform(-0.5, 0.5, nsrc)
+    src, trg = rng.uniform(-50.0, 50.0, (nsrc, 3)), rng.uniform(55.0, 80.0, (ntrg, 3))
+    with DDCosmo(lmax=2, ngrid=26) as dd:
+        dd.ddinit(*np.zeros((3, 1)), np.ones(1))
+        phi, psi = dd.mkrhs(q, *src.T, ccav=trg)
+    want, wpsi = oracle.mkrhs(q, *src.T, trg, 9)
+    assert np.abs(phi - want).max() <= 1e-12 * np.abs(want).max()
+    np.testing.assert_array_equal(psi, wpsi)
+
+
 @pytest.mark.parametrize("precision,tol", [(0, 1e-8), (1, 1e-6)])
 def test_field_of_a_batch_in_parts(precision, tol):
     """Blocks of 256 nuclei with one, two and three molecules, their sources
