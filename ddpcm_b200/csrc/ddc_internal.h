@@ -191,6 +191,7 @@ struct DevGeo {
   const int* pn_ptr;
   const uint16_t* pn;
   const int* ls_ptr;
+  const int* ls_order;  // spheres by falling length of their lists, or null: as they are
   const int* ls;  // gather list: a * ngrid + n of each triple
   const int* pt_ptr;   // per point (a, n): its entries of pt_idx
   const int* pt_idx;   // positions of its triples in the gather lists, CSR order
@@ -314,6 +315,8 @@ struct CountStats {
 };
 cudaError_t scan_counts(Launch L, int* cnt, int* out, int n, void* temp, size_t temp_bytes,
                         CountStats* st);
+// order[n]: the lists of ptr[n+1] by falling length (to a 1,024th of the longest)
+cudaError_t launch_ls_order(Launch L, int n, const int* ptr, const CountStats* st, int* order);
 
 // operators over the triples (ddc_lxs.cu): lx values, one per triple in
 // gather-list order, for k_lx_gather, and / or the L* rows.  xi holds the

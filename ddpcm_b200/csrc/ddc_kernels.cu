@@ -548,6 +548,36 @@ __global__ void k_sum_counts(const int* __restrict__ cnt, int n, CountStats* out
     atomicMax(&out->largest, m);
   }
 }
+// Counting sort of the lists by falling length, one block.  Lists of one bucket
+// come in any order: it only sets which block of a pass takes which list.
+constexpr int kOrderB = 1024;
+__global__ void __launch_bounds__(kOrderB) k_ls_order(int n, const int* __restrict__ ptr,
+                                                      const CountStats* __restrict__ st,
+                                                      int* __restrict__ order) {
+  typedef cub::BlockScan<int, kOrderB> BS;
+  __shared__ typename BS::TempStorage tmp;
+  __shared__ int at[kOrderB];
+  const float scale = (float)kOrderB / (float)(st->largest + 1);
+  auto bucket = [&](int i) {
+    return kOrderB - 1 - min(kOrderB - 1, (int)((float)(ptr[i + 1] - ptr[i]) * scale));
+  };
+  at[threadIdx.x] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += kOrderB) atomicAdd(&at[bucket(i)], 1);
+  __syncthreads();
+  int v = at[threadIdx.x];
+  BS(tmp).ExclusiveSum(v, v);
+  at[threadIdx.x] = v;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += kOrderB) order[atomicAdd(&at[bucket(i)], 1)] = i;
+}
+cudaError_t launch_ls_order(Launch L, int n, const int* ptr, const CountStats* st, int* order) {
+  if (n == 0) return cudaSuccess;
+  k_ls_order<<<1, kOrderB, 0, L.st>>>(n, ptr, st, order);
+  ++*L.launches;
+  return cudaGetLastError();
+}
+
 // The scan, the total and the maximum of a short list: one block, eight
 // counts per thread and step.
 constexpr int kScanT = 1024, kScanU = 8;

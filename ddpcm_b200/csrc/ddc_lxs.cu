@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(32 * nroles<Rl>(LMAX), min_blocks<Rl>(LMAX))
   V2<V>* xs = fld + NF * NT;                             // [(l, m)]
   G4* gs = reinterpret_cast<G4*>(xs + lmi(LMAX + 1, 0)); // [NP][NT] (PRE)
   V* lxp = reinterpret_cast<V*>(gs + (PRE ? NP * NT : 0));  // [NR][NT]
-  const int b = blockIdx.x, tid = threadIdx.x;
+  const int b = g.ls_order ? g.ls_order[blockIdx.x] : (int)blockIdx.x, tid = threadIdx.x;
   if (sweep_skip(g.act, b)) return;
   const int role = tid >> 5, lane = tid & 31;
   const int q0 = g.ls_ptr[b], q1 = g.ls_ptr[b + 1];

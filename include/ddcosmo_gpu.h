@@ -192,8 +192,9 @@ int ddc_batch_energy_forces(ddc_ctx* ctx, int nmol, const int* off, const double
  * (lx, :94), y = off-diagonal L* x (lstarx, :161), y = D^-1 x (ldm1x, :246)
  * and the increment norm hnorm (:281).  x, y are (nylm,nsph).  In a
  * DDC_PREC_MIXED context lx, lstarx and lx_lstarx apply the FP32 operators of
- * the inner solves (FP32 sums, tensor-core split-TF32 projection and
- * expansion), read and written as FP64; otherwise everything is FP64. */
+ * the inner solves (FP32 sums; projection and expansion on the tensor cores,
+ * in FP64 up to 2e8 products of harmonics and points and as split TF32
+ * above), read and written as FP64; otherwise everything is FP64. */
 int ddc_lx(ddc_ctx* ctx, const double* x, double* y);
 int ddc_lstarx(ddc_ctx* ctx, const double* x, double* y);
 int ddc_ldm1x(ddc_ctx* ctx, const double* x, double* y);

@@ -28,3 +28,10 @@ def test_chains_at_the_edges_of_the_scan(oracle, sizes):
             v, s = np.random.default_rng(n).normal(size=(2, n, (lmax + 1) ** 2))
             for got, want in zip(dd.lx_lstarx(v, s), (ref.lx(v), ref.lstarx(s))):
                 assert np.linalg.norm(got - want) <= 1e-13 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("sizes", [(148, 149), (65537,)])
+def test_where_the_passes_take_the_longest_lists_first(oracle, sizes):
+    """Spheres in order, sorted (149 to 65,536, the sizes above) and in order
+    again: every sphere's list must be taken once."""
+    test_chains_at_the_edges_of_the_scan(oracle, sizes)
