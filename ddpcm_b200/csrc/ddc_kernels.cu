@@ -2350,7 +2350,7 @@ __device__ __forceinline__ void fa_run_role(int role, const YlmTables& tb, const
 // A(i, lm) for every sphere with cavity points: block per sphere, role warps
 // over chunks of the sources of its molecule.  Per source the thread forms
 // 1/d and 1/sin(theta) with the refined hardware reciprocal square root
-// (rsqrt_pos), the prefix and cos/sin(m phi) (the fields of k_lstarx); the
+// (rsqrt_pos), the prefix and cos/sin(m phi); the
 // roles run the normalised recurrence (fa_column) and store with Kg.
 template <int LMAX>
 __global__ void __launch_bounds__(32 * fa_nroles(LMAX), fa_greedy(LMAX) ? 4 : 1)
