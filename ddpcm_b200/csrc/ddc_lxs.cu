@@ -455,11 +455,11 @@ constexpr size_t lxs_smem(bool pre) {
 // PRE: the geometry comes from tg (built by k_lxs_geo), else it is evaluated
 // per pass (the few FP64 passes of the mixed path).
 template <int LMAX, class Rl, bool PRE, int MODE>
-__global__ void __launch_bounds__(32 * nroles<Rl>(LMAX), min_blocks<Rl>(LMAX))
-    k_lxs(const __grid_constant__ LxsTab tb, const DevGeo g,
-          const typename Slot<Rl>::G4* __restrict__ tg, const double* __restrict__ X,
-          const Rl* __restrict__ xi, Rl* __restrict__ val, double* __restrict__ y) {
-  chain_wait();
+__device__ __forceinline__ void lxs_block(const LxsTab& tb, const DevGeo& g,
+                                          const typename Slot<Rl>::G4* __restrict__ tg,
+                                          const double* __restrict__ X,
+                                          const Rl* __restrict__ xi, Rl* __restrict__ val,
+                                          double* __restrict__ y) {
   typedef Slot<Rl> S;
   typedef typename S::V V;
   typedef typename S::G4 G4;
@@ -597,6 +597,22 @@ __global__ void __launch_bounds__(32 * nroles<Rl>(LMAX), min_blocks<Rl>(LMAX))
   if (MODE != 1) lxs_finish_role<LMAX, NR, 0, Rl>(role, tb, acc, y + (size_t)b * NY, lane);
 }
 
+// MODE 3: lx and L* by blocks of their own (grid y)
+template <int LMAX, class Rl, bool PRE, int MODE>
+__global__ void __launch_bounds__(32 * nroles<Rl>(LMAX), min_blocks<Rl>(LMAX))
+    k_lxs(const __grid_constant__ LxsTab tb, const DevGeo g,
+          const typename Slot<Rl>::G4* __restrict__ tg, const double* __restrict__ X,
+          const Rl* __restrict__ xi, Rl* __restrict__ val, double* __restrict__ y) {
+  chain_wait();
+  if constexpr (MODE < 3) {
+    lxs_block<LMAX, Rl, PRE, MODE>(tb, g, tg, X, xi, val, y);
+  } else if (blockIdx.y == 0) {
+    lxs_block<LMAX, Rl, PRE, 1>(tb, g, tg, X, xi, val, y);
+  } else {
+    lxs_block<LMAX, Rl, PRE, 2>(tb, g, tg, X, xi, val, y);
+  }
+}
+
 LxsTab lxs_tab(const YlmTables& tb) {
   LxsTab t;
   for (int e = 0; e < DDC_NLM_CAP; ++e) t.kp[e] = tb.Kp[e];
@@ -617,7 +633,8 @@ cudaError_t lxs_launch(Launch L, const YlmTables& tb, const DevGeo& g,
   cudaError_t e = cudaSuccess;
 #define CASE(LV)                                                                               \
   case LV: {                                                                                   \
-    e = launch_chained(k_lxs<LV, Rl, PRE, MODE>, g.nsph, 32 * nroles<Rl>(LV),                  \
+    e = launch_chained(k_lxs<LV, Rl, PRE, MODE>, dim3(g.nsph, MODE == 3 ? 2 : 1),              \
+                       32 * nroles<Rl>(LV),                                                    \
                        lxs_smem<LV, Rl>(PRE), L.st, t, g, tg, X, xi, val, y);                  \
     break;                                                                                     \
   }
@@ -653,6 +670,14 @@ cudaError_t lxs_launch64(Launch L, const YlmTables& tb, const DevGeo& g, const d
                   : lxs_launch<double, false, MODE>(L, tb, g, nullptr, X, xi, val, y);
 }
 
+// Few spheres: the two operators by blocks of their own, which takes both
+// halves' latency side by side; beyond two blocks per SM the shared geometry and
+// powers are worth more.  us per pass, together and by halves: 12 spheres, lmax
+// 6, FP64 10.1 / 8.9; 113, lmax 8, FP64 25.2 / 22.9; 200, lmax 8, FP32 15.9 /
+// 15.0; 280, lmax 10, FP32 22.1 / 21.2 (with 4 us of events); energy and forces
+// of 12 spheres 1.06 / 0.99 ms, of 113 mixed 2.22 / 2.07 ms.
+bool split_pass(const DevGeo& g) { return g.nsph <= 2 * 148; }
+
 }  // namespace
 
 cudaError_t prepare_lxs(int lmax) {
@@ -662,6 +687,7 @@ cudaError_t prepare_lxs(int lmax) {
     e = lxs_attributes_mode<LV, 0>();                  \
     if (!e) e = lxs_attributes_mode<LV, 1>();          \
     if (!e) e = lxs_attributes_mode<LV, 2>();          \
+    if (!e) e = lxs_attributes_mode<LV, 3>();          \
     break;
   switch (lmax) { DDC_LMAX_CASES(CASE) }
 #undef CASE
@@ -669,7 +695,8 @@ cudaError_t prepare_lxs(int lmax) {
 }
 cudaError_t launch_lxs(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
                        const double* xi, double* val, double* y) {
-  return lxs_launch64<0>(L, tb, g, X, xi, val, y);
+  return split_pass(g) ? lxs_launch64<3>(L, tb, g, X, xi, val, y)
+                       : lxs_launch64<0>(L, tb, g, X, xi, val, y);
 }
 cudaError_t launch_lx_vals(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
                            double* val) {
@@ -681,7 +708,8 @@ cudaError_t launch_lstarx_acc(Launch L, const YlmTables& tb, const DevGeo& g, co
 }
 cudaError_t launch_lxs_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
                            const float* xi, float* val, double* y) {
-  return lxs_launch<float, true, 0>(L, tb, g, g.tgeo4, X, xi, val, y);
+  return split_pass(g) ? lxs_launch<float, true, 3>(L, tb, g, g.tgeo4, X, xi, val, y)
+                       : lxs_launch<float, true, 0>(L, tb, g, g.tgeo4, X, xi, val, y);
 }
 cudaError_t launch_lx_vals_f32(Launch L, const YlmTables& tb, const DevGeo& g, const double* X,
                                float* val) {

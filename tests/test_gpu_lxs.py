@@ -43,6 +43,25 @@ def test_operators_at_chunk_edges(oracle, kind, ngrid, lmax):
             assert np.all(pair[0][-1] == 0.0) and np.all(pair[1][-1] == 0.0)
 
 
+@pytest.mark.parametrize("n", [296, 297])
+@pytest.mark.parametrize("lmax", [0, 1, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12])
+def test_both_operators_by_halves_and_together(oracle, n, lmax):
+    """lx and lstarx in one launch: by blocks of their own up to 296 spheres,
+    from one pass over the triples beyond."""
+    from ddpcm_b200 import molecules as M
+    from ddpcm_b200.ddcosmo import DDCosmo, PREC_FP64, PREC_MIXED
+    m = M.to_bohr(M.make_molecule(n, 700 + lmax))
+    rng = np.random.default_rng(lmax)
+    x, s = rng.normal(size=(2, n, (lmax + 1) ** 2))
+    ref = oracle.RefDD(lmax, 110, 10, 1, 78.3553, 0.1).init(m["x"], m["y"], m["z"], m["r"])
+    want = ref.lx(x), ref.lstarx(s)
+    for prec, tol in ((PREC_FP64, 1e-13), (PREC_MIXED, 64 * 2.0 ** -24)):
+        with DDCosmo(lmax=lmax, ngrid=110, iconv=10, eta=0.1, precision=prec) as dd:
+            dd.ddinit(m["x"], m["y"], m["z"], m["r"])
+            for got, w in zip(dd.lx_lstarx(x, s), want):
+                assert np.linalg.norm(got - w) <= tol * np.linalg.norm(w)
+
+
 @pytest.mark.parametrize("n,lmax,ngrid", [
     (9, 8, 110),      # eight slices of k, the last block of spheres nearly empty
     (1603, 8, 110),   # projection: 16 spheres per block; expansion: two slices
