@@ -674,12 +674,13 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
                      ctx->cnt.as<int>()));
   CK(scan_counts(L, ctx->cnt.as<int>(), ctx->ls_ptr.as<int>(), N, ctx->scan_tmp.p,
                  ctx->scan_tmp.bytes, stats));
-  // the triple passes take the longest lists first: the blocks of a last wave,
-  // and of an SM that has one more than the others, are then the shortest (lx
-  // and lstarx of 4,999 spheres, lmax 9, FP64: 0.38 -> 0.33 ms; energy and
-  // forces of 2,000, lmax 6, FP64: 10.2 -> 9.4 ms).  Not for one block per SM,
-  // nor where one block would sort for long.
-  ctx->order_on = N > 148 && N <= 65536;
+  // the triple passes take the longest lists first: the blocks of a last wave
+  // are then the shortest (lx and lstarx of 4,999 spheres, lmax 9, FP64: 0.38
+  // -> 0.33 ms; energy and forces of 2,000, lmax 6, FP64: 10.2 -> 9.4 ms).  Not
+  // up to two waves of four blocks per SM, where the pass alone gains 8 % but
+  // the next kernel, scheduled while it ends, loses more (643 spheres routine by
+  // routine 7.1 -> 7.7 ms), nor where one block would sort for long.
+  ctx->order_on = N > 2 * 4 * 148 && N <= 65536;
   if (ctx->order_on) {
     CK(ctx->ls_order.ensure(sizeof(int) * N));
     CK(launch_ls_order(L, N, ctx->ls_ptr.as<int>(), stats, ctx->ls_order.as<int>()));

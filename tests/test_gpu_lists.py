@@ -30,8 +30,8 @@ def test_chains_at_the_edges_of_the_scan(oracle, sizes):
                 assert np.linalg.norm(got - want) <= 1e-13 * np.linalg.norm(want)
 
 
-@pytest.mark.parametrize("sizes", [(148, 149), (65537,)])
+@pytest.mark.parametrize("sizes", [(1184, 1185), (65537,)])
 def test_where_the_passes_take_the_longest_lists_first(oracle, sizes):
-    """Spheres in order, sorted (149 to 65,536, the sizes above) and in order
+    """Spheres in order, sorted (1,185 to 65,536, the sizes above) and in order
     again: every sphere's list must be taken once."""
     test_chains_at_the_edges_of_the_scan(oracle, sizes)
