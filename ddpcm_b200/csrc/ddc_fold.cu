@@ -258,7 +258,11 @@ __global__ void k_fold_pack(FoldTab ft, const double* __restrict__ basis,
 size_t fold_smem_size(const FoldTab& t) {
   return sizeof(double) * std::max(8 * t.oc * 9, 8 * t.nylm);
 }
-
+// the most that any context needs.  The kernels' limit belongs to the function,
+// whatever context set it, so it is the same for all of them (it is a cap: a
+// launch takes what it asks for)
+constexpr int kSmemMost = (int)sizeof(double) * 8 * kChunk * 9;
+static_assert((DDC_MAX_LMAX + 1) * (DDC_MAX_LMAX + 1) <= kChunk * 9, "the result's rows fit");
 
 }  // namespace
 
@@ -318,10 +322,10 @@ bool fold_tables(const std::vector<double>& g4, int lmax, FoldTab& t, std::vecto
 cudaError_t launch_fold_pack(Launch L, const FoldTab& t, const double* basis, const double* bw,
                              double* pf, double* xw, double* xb) {
   cudaError_t e;
-  const int sm = (int)fold_smem_size(t);
   for (auto f : {(const void*)k_fold_proj<double>, (const void*)k_fold_proj<float>,
                  (const void*)k_fold_xi<double>, (const void*)k_fold_xi<float>})
-    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost)))
+      return e;
   const int n = std::max(4 * t.otiles * 2, t.otiles * 7) * 32;
   k_fold_pack<<<dim3((n + kT - 1) / kT, 8), kT, 0, L.st>>>(t, basis, bw, pf, xw, xb);
   ++*L.launches;

@@ -1,0 +1,42 @@
+"""Contexts of different parameters that live side by side in one process:
+what one of them sets for the device's kernels must leave the others as they
+were.  A context's results after another one has been initialised and used
+are the results it gave alone, bit by bit (sums have a fixed order)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _molecule(n, seed):
+    from ddpcm_b200 import molecules as M
+    return M.to_bohr(M.make_molecule(n, seed))
+
+
+def _results(dd, m):
+    out = dd.energy_forces(*(m[k] for k in "qxyzr"))
+    phi, psi = dd.mkrhs(m["q"], m["x"], m["y"], m["z"])
+    pair = dd.lx_lstarx(out["sigma"], out["s"])
+    return [np.float64(out["esolv"]), out["sigma"], out["s"], out["fx"], dd.rhs(phi), psi, *pair,
+            dd.ddmkzeta(out["s"])]
+
+
+def _same(a, b):
+    assert all(np.array_equal(u, v) for u, v in zip(a, b))
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("wide,narrow", [((10, 590), (6, 110)), ((12, 1202), (2, 50)),
+                                         ((9, 434), (10, 302))])
+def test_two_live_contexts(wide, narrow, prec):
+    """More grid points (more shared memory in the folded contractions) in the
+    first context, fewer in the second."""
+    from ddpcm_b200.ddcosmo import DDCosmo
+    m = _molecule(40, 1)
+    with DDCosmo(lmax=wide[0], ngrid=wide[1], eta=0.1, precision=prec) as a:
+        first = _results(a, m)
+        with DDCosmo(lmax=narrow[0], ngrid=narrow[1], eta=0.1, precision=prec) as b:
+            other = _results(b, m)
+            _same(_results(a, m), first)
+            _same(_results(b, m), other)
+        _same(_results(a, m), first)
