@@ -645,6 +645,12 @@ bool tc_supported(int nylm) { return nylm <= 128; }
 
 namespace {
 
+// The limit belongs to the function, whatever plan set it: every plan allows the
+// most that any tile width may ask for, so that one context's narrower tiles do
+// not refuse another's launches.
+cudaError_t allow_smem(const void* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap);
+}
 // tile width bn of the projection: pipeline depth, shared memory and the TMA
 // box of the grid field (bn rows of 32 values)
 cudaError_t cfg_proj(TcPlan& p, int bn) {
@@ -663,8 +669,7 @@ cudaError_t cfg_proj(TcPlan& p, int bn) {
                            box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(k_proj_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              p.smem_proj);
+  return allow_smem((const void*)k_proj_tc);
 }
 // tile width of the expansion: the split coefficients of bn spheres stay
 // resident, the bw chunks stream through a ring of at least two stages
@@ -676,7 +681,7 @@ cudaError_t cfg_xi(TcPlan& p, int bn) {
   p.bn_xi = bn;
   p.ns_xi = ns;
   p.smem_xi = std::max(bsz + ns * 2 * kChunk + kSmemSlack, 120 * 1024);
-  return cudaFuncSetAttribute(k_xi_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem_xi);
+  return allow_smem((const void*)k_xi_tc);
 }
 std::vector<int> bn_candidates(int nsph) {
   std::vector<int> c;

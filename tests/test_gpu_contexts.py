@@ -40,3 +40,25 @@ def test_two_live_contexts(wide, narrow, prec):
             _same(_results(a, m), first)
             _same(_results(b, m), other)
         _same(_results(a, m), first)
+
+
+def test_two_live_contexts_on_tcgen05():
+    """Mixed operators above 2e8 products, where the contractions run on
+    tcgen05: wide tiles (14,000 spheres), then narrow ones (2,900)."""
+    from ddpcm_b200.ddcosmo import DDCosmo, PREC_MIXED
+
+    def pair(dd, n, lmax):
+        rng = np.random.default_rng(n)
+        return dd.lx_lstarx(*rng.normal(size=(2, n, (lmax + 1) ** 2)))
+
+    def context(n, lmax, ngrid):
+        m = _molecule(n, n)
+        return DDCosmo(lmax=lmax, ngrid=ngrid, eta=0.1, precision=PREC_MIXED).ddinit(
+            m["x"], m["y"], m["z"], m["r"])
+
+    with context(14000, 6, 302) as a:
+        first = pair(a, 14000, 6)
+        with context(2900, 10, 590) as b:
+            other = pair(b, 2900, 10)
+            _same(pair(a, 14000, 6), first)
+            _same(pair(b, 2900, 10), other)
