@@ -2037,6 +2037,7 @@ __device__ __forceinline__ void lxs_finish_role(int role, const YlmTables& tb, R
 // one after the other (a pair's points are distinct).
 // ---------------------------------------------------------------------------
 constexpr int kPtWarps = 4;
+constexpr int kMaxGrid = 5810;  // points of the largest Lebedev grid
 __global__ void __launch_bounds__(32 * kPtWarps)
     k_pt_fill(int nsph, int ngrid, const int* __restrict__ inl, const int* __restrict__ pn_ptr,
               const uint16_t* __restrict__ pn, const int* __restrict__ lsstart,
@@ -2080,8 +2081,10 @@ cudaError_t launch_pt_fill(Launch L, int nsph, int ngrid, const int* inl, const 
   if (nsph == 0) return cudaSuccess;
   const size_t sm = sizeof(int) * kPtWarps * ngrid;
   if (sm > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_pt_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    // the limit belongs to the function: the same value whatever the grid, so
+    // that another thread's context cannot lower it before the launch
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_pt_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(int) * kPtWarps * kMaxGrid);
     if (e) return e;
   }
   k_pt_fill<<<(nsph + kPtWarps - 1) / kPtWarps, 32 * kPtWarps, sm, L.st>>>(

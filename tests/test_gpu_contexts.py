@@ -2,6 +2,8 @@
 what one of them sets for the device's kernels must leave the others as they
 were.  A context's results after another one has been initialised and used
 are the results it gave alone, bit by bit (sums have a fixed order)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -62,3 +64,26 @@ def test_two_live_contexts_on_tcgen05():
             other = pair(b, 2900, 10)
             _same(pair(a, 14000, 6), first)
             _same(pair(b, 2900, 10), other)
+
+
+def test_contexts_of_several_threads():
+    """Four threads, each with a context of its own on a grid whose point lists
+    take more than the default 48 KB of shared memory."""
+    from ddpcm_b200.ddcosmo import DDCosmo
+    m = _molecule(4, 3)
+    failed = []
+
+    def work(ngrid):
+        try:
+            with DDCosmo(lmax=2, ngrid=ngrid, eta=0.1) as dd:
+                for _ in range(2000):
+                    dd.ddinit(m["x"], m["y"], m["z"], m["r"])
+        except Exception as e:  # reported by the main thread
+            failed.append(f"{ngrid}: {e}")
+
+    threads = [threading.Thread(target=work, args=(g,)) for g in (3074, 5810, 3470, 5294)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
