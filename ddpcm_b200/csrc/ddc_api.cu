@@ -1887,6 +1887,15 @@ int ddc_lx_lstarx(ddc_ctx* ctx, const double* x, double* y, const double* s, dou
     dz = ctx->in3.as<double>();
   }
   if (!dz) return fail(ctx, DDC_ERR_PARAM, "null output array");
+  // z may lie over x: the pass writes rows of z while other blocks still read
+  // theirs of x, so it then reads a copy (y and s need none: s is read before
+  // the pass, y written after it)
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(dx), za = reinterpret_cast<uintptr_t>(dz);
+  if (xa < za + sizeof(double) * nv && za < xa + sizeof(double) * nv) {
+    CK(ctx->in1.ensure(sizeof(double) * nv));
+    CK(cudaMemcpyAsync(ctx->in1.p, dx, sizeof(double) * nv, cudaMemcpyDeviceToDevice, ctx->st));
+    dx = ctx->in1.as<double>();
+  }
   if (ctx->prm.precision == DDC_PREC_MIXED)
     CKI(op_pair_f32(ctx, dx, dy, ds, dz));
   else
