@@ -1710,9 +1710,9 @@ int ddc_mkrhs(ddc_ctx* ctx, int n, const double* charge, const double* x, const 
   CKI(out_ptr(ctx, psi, (size_t)n * nylm, ctx->out1, &dpsi));
   const int nchunk = efield_chunks(n, ncav);
   CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(ncav, 1) * nchunk));
-  CK(launch_psi(ctx->L(), n, nylm, dq, dpsi));
   const bool host = !ctx->prm.device_pointers && psi && n > 0;
   if (host) {
+    CK(launch_psi(ctx->L(), n, nylm, dq, dpsi));
     // psi goes to the host while the potential is summed (30,001 charges, 49
     // harmonics: 12 MB, 0.85 ms with the caller's page faults)
     CKI(out_stream(ctx));
@@ -1728,6 +1728,8 @@ int ddc_mkrhs(ddc_ctx* ctx, int n, const double* charge, const double* x, const 
     if (e == cudaSuccess) e = w;
   }
   CK(e);
+  // on device arrays psi comes last: it may lie over the charges
+  if (!host) CK(launch_psi(ctx->L(), n, nylm, dq, dpsi));
   CKI(finish_out(ctx, phi, dphi, ncav));
   if (!host) CKI(finish_out(ctx, psi, dpsi, (size_t)n * nylm));
   return sync(ctx);

@@ -1,6 +1,6 @@
-"""Operators on device vectors whose outputs lie over their inputs: lx and
-lstarx together, lx, lstarx, each wholly in place and with a partial overlap,
-against the same call on vectors of their own.  Bit by bit: only where the
+"""Calls on device vectors whose outputs lie over their inputs: lx and
+lstarx together, lx, lstarx, each wholly in place and with a partial overlap, and mkrhs with psi
+over the charges, against the same call on vectors of their own.  Bit by bit: only where the
 results go differs."""
 import ctypes
 
@@ -56,3 +56,21 @@ def test_outputs_over_inputs(n, shift, prec):
             v1, o1 = place(v)
             dd._check(fn(dd.h, _ptr(v1), _ptr(o1)))
             assert torch.equal(o1, want)
+
+
+def test_psi_over_the_charges():
+    """lmax 0: psi has one entry per charge, and may take the charges' place."""
+    import torch
+    from ddpcm_b200.ddcosmo import DDCosmo
+    rng = np.random.default_rng(5)
+    n, nt = 700, 900
+    q, x, y, z = (torch.from_numpy(v).cuda() for v in rng.normal(size=(4, n)))
+    at = torch.from_numpy(50.0 + rng.normal(size=(nt, 3))).cuda()
+    phi, phi1 = torch.zeros(2, nt, dtype=torch.float64, device="cuda")
+    psi = torch.zeros_like(q)
+    torch.cuda.synchronize()
+    with DDCosmo(lmax=0, ngrid=26, device_pointers=1) as dd:
+        for f, p in ((phi, psi), (phi1, q)):
+            dd._check(dd.L.ddc_mkrhs(dd.h, n, *map(_ptr, (q, x, y, z)), nt, _ptr(at), _ptr(f), 1,
+                                     _ptr(p)))
+    assert torch.equal(phi1, phi) and torch.equal(q, psi)
