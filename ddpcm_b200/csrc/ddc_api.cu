@@ -1324,7 +1324,7 @@ int solute_pot_field(ddc_ctx* ctx, const double* q, double* phi, double* ef, con
                                 trange));
   } else {
     const int nchunk = trange ? 1 : efield_chunks(N, NC);
-    CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(NC, 1) * nchunk));
+    if (nchunk > 1) CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(NC, 1) * nchunk));
     CK(launch_coulomb_pot(ctx->L(), N, q, ctx->cx.as<double>(), ctx->cy.as<double>(),
                           ctx->cz.as<double>(), NC, ctx->ccav.as<double>(), phi,
                           ctx->ef_scratch.as<double>(), nchunk, trange));
@@ -1709,7 +1709,8 @@ int ddc_mkrhs(ddc_ctx* ctx, int n, const double* charge, const double* x, const 
   CKI(out_ptr(ctx, phi, ncav, ctx->phi, &dphi));
   CKI(out_ptr(ctx, psi, (size_t)n * nylm, ctx->out1, &dpsi));
   const int nchunk = efield_chunks(n, ncav);
-  CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(ncav, 1) * nchunk));
+  // (one piece goes straight to phi)
+  if (nchunk > 1) CK(ctx->ef_scratch.ensure(sizeof(double) * (size_t)std::max(ncav, 1) * nchunk));
   const bool host = !ctx->prm.device_pointers && psi && n > 0;
   if (host) {
     CK(launch_psi(ctx->L(), n, nylm, dq, dpsi));
