@@ -983,8 +983,12 @@ enum { SI_NMAT, SI_STATUS, SI_ITERS, SI_RESTARTS, SI_EXT, SI_MAXK, SI_RUN, SI_IT
        SI_UPD, SI_CNT, SI_N };
 enum { SD_NORM, SD_LAST, SD_TOLK, SD_N };
 
+// Molecules that a solve treats one by one.  A call on single systems (cosmo)
+// solves whatever the context holds as one, also after a batch.
+int solver_molecules(const ddc_ctx* ctx) { return ctx->batch ? ctx->nmol : 1; }
+
 int solver_setup(ddc_ctx* ctx, SolverArgs& a, const System* sys, int ns, bool mixed) {
-  const int nmol = ctx->nmol, nylm = ctx->nylm;
+  const int nmol = solver_molecules(ctx), nylm = ctx->nylm;
   memset(&a, 0, sizeof(a));
   a.nmol = nmol;
   a.nsph = ctx->nsph;
@@ -1172,9 +1176,9 @@ int print_log(ddc_ctx* ctx, const SolverArgs& a, int ns, const int* from, const 
 int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
   const double t0 = now_s();
   const bool mixed = ctx->prm.precision == DDC_PREC_MIXED;
-  const bool one = ctx->nmol == 1 && !ctx->batch;
+  const bool one = !ctx->batch;
   const bool log = ctx->prm.iprint > 0 && one;
-  const int nmol = ctx->nmol;
+  const int nmol = solver_molecules(ctx);
   if (ctx->batch && ctx->prm.ndiis == 0)
     return fail(ctx, DDC_ERR_UNSUPPORTED, "batched solves need DIIS");
   for (int q = 0; q < ns; q++) memset(sys[q].inf, 0, sizeof(*sys[q].inf));
