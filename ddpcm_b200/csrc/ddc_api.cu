@@ -978,6 +978,8 @@ struct System {
   ddc_solve_info* inf = nullptr;
 };
 
+// norms of a report
+constexpr int kNorms = sizeof(ddc_solve_info::norms) / sizeof(double);
 // integer and double state arrays of a system, nmol entries each
 enum { SI_NMAT, SI_STATUS, SI_ITERS, SI_RESTARTS, SI_EXT, SI_MAXK, SI_RUN, SI_ITS, SI_OUTER, SI_RST,
        SI_UPD, SI_CNT, SI_N };
@@ -1040,7 +1042,10 @@ int solver_setup(ddc_ctx* ctx, SolverArgs& a, const System* sys, int ns, bool mi
   CK(ctx->s_coef.ensure(sizeof(double) * 2 * (size_t)nmol * kMaxHist));
   const size_t parts = (size_t)std::max(solver_parts(a.nchunk, a.chunk), 1) * (kMaxHist + 1);
   CK(ctx->s_part.ensure(sizeof(double) * 2 * parts));
-  if (nmol == 1) CK(ctx->s_log.ensure(sizeof(double) * 2 * (size_t)ctx->prm.max_iter));
+  // the norms of a single solve: what its report holds, and with iprint what is
+  // printed (the first million), not one per iteration that max_iter allows
+  a.nlog = ctx->batch ? 0 : std::min(ctx->prm.max_iter, ctx->prm.iprint > 0 ? 1 << 20 : kNorms);
+  CK(ctx->s_log.ensure(sizeof(double) * 2 * (size_t)a.nlog));
   if (!ctx->hstop) {
     CK(cudaHostAlloc(&ctx->hstop, sizeof(int) * 4, cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer(&ctx->dstop, ctx->hstop, 0));
@@ -1073,7 +1078,7 @@ int solver_setup(ddc_ctx* ctx, SolverArgs& a, const System* sys, int ns, bool mi
     s.gram = ctx->s_gram.as<double>() + (size_t)q * nmol * nd * nd;
     s.coef = ctx->s_coef.as<double>() + (size_t)q * nmol * kMaxHist;
     s.part = ctx->s_part.as<double>() + (size_t)q * parts;
-    s.log = nmol == 1 ? ctx->s_log.as<double>() + (size_t)q * ctx->prm.max_iter : nullptr;
+    s.log = ctx->s_log.as<double>() + (size_t)q * a.nlog;
     s.hx = (q ? ctx->hist_x2 : ctx->hist_x).p;
     s.he = (q ? ctx->hist_e2 : ctx->hist_e).p;
     s.y = (q ? ctx->y2 : ctx->y).as<double>();
@@ -1156,7 +1161,7 @@ int print_log(ddc_ctx* ctx, const SolverArgs& a, int ns, const int* from, const 
   std::vector<double> log[2];
   int most = 0;
   for (int q = 0; q < ns; q++) {
-    log[q].resize(std::max(to[q] - from[q], 0));
+    log[q].resize(std::max(std::min(to[q], a.nlog) - from[q], 0));
     most = std::max(most, (int)log[q].size());
     if (!log[q].empty())
       CK(cudaMemcpyAsync(log[q].data(), a.sys[q].log + from[q], sizeof(double) * log[q].size(),
@@ -1188,7 +1193,7 @@ int solve_systems(ddc_ctx* ctx, const System* sys, int ns) {
   // the state comes back in one go, through pinned memory: the integers, the
   // doubles, and one molecule's norms
   const size_t nsi = 2 * (SI_N * (size_t)nmol + 1), nsd = 2 * SD_N * (size_t)nmol;
-  const int nlog = one ? std::max(std::min(256, ctx->prm.max_iter), 0) : 0;
+  const int nlog = std::min(kNorms, a.nlog);
   CK(ctx->hstate.ensure(sizeof(double) * (nsd + 2 * (size_t)nlog) + sizeof(int) * nsi));
   double* sd = static_cast<double*>(ctx->hstate.p);
   double* slog = sd + nsd;

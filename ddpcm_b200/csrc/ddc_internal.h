@@ -243,13 +243,14 @@ struct SolverSys {
   double* coef;   // [nmol][kMaxHist] extrapolation coefficients
   double* gram;   // [nmol][ndiis][ndiis] inner products by physical slot
   double* part;   // [nchunk][kMaxHist+1] per-chunk partial sums
-  double* log;    // increment norm of every iteration (one molecule), or null
+  double* log;    // [nlog] increment norms of the first iterations (one molecule)
 };
 struct SolverArgs {
   int nmol, nonempty, nsph, nylm, ndiis, max_iter;
   int nchunk, chunk;  // chunks of `chunk` elements
   int first;          // system of grid row 0
   int sweep;          // number of the sweep, from 1
+  int nlog;           // length of the systems' logs
   double tol;
   long long n_total;
   const int* off;     // [nmol+1] sphere offsets of the molecules; with cmol

@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kT) k_extrap(const __grid_constant__ SolverArg
     s.norm[k] = nrm;
     const int it = s.iters[k] + 1;
     s.iters[k] = it;
-    if (s.log) s.log[s.its[k] + it - 1] = nrm;
+    if (s.its[k] + it <= a.nlog) s.log[s.its[k] + it - 1] = nrm;
     const int now = nrm < s.tolk[k] ? 1 : (it >= s.maxk[k] ? 2 : (isfinite(nrm) ? 0 : 3));
     if (now != 0) {
       s.status[k] = now;
