@@ -100,8 +100,7 @@ __device__ __forceinline__ void proj_class(double (&acc)[4][2], const double* F,
 
 template <class TB>
 __global__ void __launch_bounds__(kT, 4) k_fold_proj(const __grid_constant__ FoldTab ft, int N,
-                                                     double alpha, const TB* __restrict__ B,
-                                                     int ldb, double* __restrict__ C,
+                                                     double alpha, const TB* B, int ldb, double* C,
                                                      const SweepMask act) {
   extern __shared__ __align__(16) double fold_smem[];  // [8][oc][9]; then [8][nylm]
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, n0 = blockIdx.x * 8;
@@ -160,8 +159,7 @@ __global__ void __launch_bounds__(kT, 4) k_fold_proj(const __grid_constant__ Fol
 template <class TC>
 __global__ void __launch_bounds__(kT, 4) k_fold_xi(const __grid_constant__ FoldTab ft,
                                                    const double* __restrict__ xf, int N,
-                                                   const double* __restrict__ s,
-                                                   TC* __restrict__ xi, int ldc,
+                                                   const double* s, TC* xi, int ldc,
                                                    const SweepMask act) {
   extern __shared__ __align__(16) double fold_smem[];  // [8][oc][9]
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, n0 = blockIdx.x * 8;

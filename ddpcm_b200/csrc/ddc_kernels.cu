@@ -2108,7 +2108,7 @@ cudaError_t launch_pt_fill(Launch L, int nsph, int ngrid, const int* inl, const 
 constexpr int kPtPoints = 2;
 template <class Rl>
 __global__ void __launch_bounds__(256)
-    k_lx_gather(const DevGeo g, const Rl* __restrict__ val, Rl* pot, int ldp, bool chi) {
+    k_lx_gather(const DevGeo g, const Rl* val, Rl* pot, int ldp, bool chi) {
   chain_wait();
   constexpr int P = kPtPoints;
   constexpr int U = 4;  // triples of a point in flight

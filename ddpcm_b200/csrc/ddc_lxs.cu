@@ -58,19 +58,23 @@ __host__ __device__ constexpr int lmi(int l, int m) { return l * (l + 1) / 2 + m
 // ---------------------------------------------------------------------------
 // Loads that stay where they are written: issued ahead of the role work that
 // hides their latency (the compiler would sink them to their first use).
-__device__ __forceinline__ int ld_here(const int* p) {
+// ld_list goes through the read-only path and is for the lists and other tables
+// of the molecule; what the preceding kernel of a sweep writes (X, xi) is not
+// read-only while this one is resident (chain_wait), so it takes ordinary loads
+// and its pointers carry no __restrict__.
+__device__ __forceinline__ int ld_list(const int* p) {
   int v;
   asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ float ld_here(const float* p) {
   float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ double ld_here(const double* p) {
   double v;
-  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -457,9 +461,7 @@ constexpr size_t lxs_smem(bool pre) {
 template <int LMAX, class Rl, bool PRE, int MODE>
 __device__ __forceinline__ void lxs_block(const LxsTab& tb, const DevGeo& g,
                                           const typename Slot<Rl>::G4* __restrict__ tg,
-                                          const double* __restrict__ X,
-                                          const Rl* __restrict__ xi, Rl* __restrict__ val,
-                                          double* __restrict__ y) {
+                                          const double* X, const Rl* xi, Rl* val, double* y) {
   typedef Slot<Rl> S;
   typedef typename S::V V;
   typedef typename S::G4 G4;
@@ -501,7 +503,7 @@ __device__ __forceinline__ void lxs_block(const LxsTab& tb, const DevGeo& g,
   auto points = [&](int k, int* pa) {
     if (k < nch) {
 #pragma unroll
-      for (int p = 0; p < NP; ++p) pa[p] = ld_here(g.ls + triple(k, p));
+      for (int p = 0; p < NP; ++p) pa[p] = ld_list(g.ls + triple(k, p));
     }
   };
   struct In {
@@ -601,8 +603,8 @@ __device__ __forceinline__ void lxs_block(const LxsTab& tb, const DevGeo& g,
 template <int LMAX, class Rl, bool PRE, int MODE>
 __global__ void __launch_bounds__(32 * nroles<Rl>(LMAX), min_blocks<Rl>(LMAX))
     k_lxs(const __grid_constant__ LxsTab tb, const DevGeo g,
-          const typename Slot<Rl>::G4* __restrict__ tg, const double* __restrict__ X,
-          const Rl* __restrict__ xi, Rl* __restrict__ val, double* __restrict__ y) {
+          const typename Slot<Rl>::G4* __restrict__ tg, const double* X, const Rl* xi, Rl* val,
+          double* y) {
   chain_wait();
   if constexpr (MODE < 3) {
     lxs_block<LMAX, Rl, PRE, MODE>(tb, g, tg, X, xi, val, y);
