@@ -130,6 +130,19 @@ struct FoldTab {
   const double *pf, *xfw, *xfb;  // operands in fragment order
 };
 
+// Indices into lists and fields of up to 2^31 - 2 entries, formed so that no
+// sum passes 2^31 where threads of a last block lie beyond the end.
+// Entry k of the list [q0, q1), its last where the list is shorter:
+__host__ __device__ inline int list_entry(int q0, int q1, int k) {
+  const int last = q1 - q0 - 1;
+  return q0 + (k < last ? k : last);
+}
+// Point of thread tid in step i of a block of n threads that takes `steps` steps:
+__host__ __device__ inline unsigned step_point(unsigned block, unsigned steps, unsigned i,
+                                               unsigned n, unsigned tid) {
+  return (block * steps + i) * n + tid;
+}
+
 #ifdef __CUDACC__
 // The kernels of a solver sweep follow one another with a dependency on all
 // of the previous kernel.  Launched with launch_chained they are scheduled

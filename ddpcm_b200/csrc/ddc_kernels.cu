@@ -521,7 +521,7 @@ __global__ void k_ls_fill(int nsph, const int* __restrict__ inl, const int* __re
     int kk = rev[k], j = nl[k];
     int a = pn_ptr[kk], b = pn_ptr[kk + 1];
     if (threadIdx.x == 0) lsstart[kk] = off;  // where pair (j, i) sits in i's gather list
-    for (int q = a + threadIdx.x; q < b; q += blockDim.x) ls[off + (q - a)] = j * ngrid + pn[q];
+    for (int t = threadIdx.x; t < b - a; t += blockDim.x) ls[off + t] = j * ngrid + pn[a + t];
     off += b - a;
   }
 }
@@ -1700,7 +1700,9 @@ __global__ void __launch_bounds__(128) k_forces_a(const YlmTables tb, const DevG
   double f0 = 0.0, f1 = 0.0, f2 = 0.0;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const double* si = sigma + (size_t)i * NY;
-  for (int q = g.ls_ptr[i] + threadIdx.x; q < g.ls_ptr[i + 1]; q += blockDim.x) {
+  const int q0 = g.ls_ptr[i], nq = g.ls_ptr[i + 1] - q0;
+  for (int t = threadIdx.x; t < nq; t += blockDim.x) {
+    const int q = q0 + t;
     const int pj = g.ls[q], j = pj / G, n = pj - j * G;
     const double4 cj = g.sph[j];
     const double4 gn = g.grid[n];
@@ -2066,11 +2068,11 @@ __global__ void __launch_bounds__(32 * kPtWarps)
   if (a == nsph - 1 && lane == 0) pt_ptr[p0 + ngrid] = run;
   __syncwarp();
   for (int k = inl[a]; k < inl[a + 1]; ++k) {
-    const int q0 = pn_ptr[k], q1 = pn_ptr[k + 1], base = lsstart[k] - q0;
-    for (int q = q0 + lane; q < q1; q += 32) {
-      const int n = pn[q], at = cur[n];
+    const int q0 = pn_ptr[k], cnt = pn_ptr[k + 1] - q0, base = lsstart[k];
+    for (int t = lane; t < cnt; t += 32) {
+      const int n = pn[q0 + t], at = cur[n];
       cur[n] = at + 1;
-      pt_idx[at] = base + q;
+      pt_idx[at] = base + t;
     }
     __syncwarp();
   }
@@ -2112,15 +2114,15 @@ __global__ void __launch_bounds__(256)
   chain_wait();
   constexpr int P = kPtPoints;
   constexpr int U = 4;  // triples of a point in flight
-  const int np = g.nsph * g.ngrid;
+  const unsigned np = (unsigned)g.nsph * g.ngrid, G = g.ngrid;
   int q[P], q1[P];
   Rl v[P];
 #pragma unroll
   for (int i = 0; i < P; ++i) {
-    const int p = (blockIdx.x * P + i) * 256 + threadIdx.x;
+    const unsigned p = step_point(blockIdx.x, P, i, 256, threadIdx.x);
     q[i] = q1[i] = 0;
     v[i] = 0;
-    if (p < np && !sweep_skip(g.act, p / g.ngrid)) {
+    if (p < np && !sweep_skip(g.act, p / G)) {
       q[i] = g.pt_ptr[p];
       q1[i] = g.pt_ptr[p + 1];
     }
@@ -2131,7 +2133,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int u = 0; u < U; ++u) at[i][u] = q[i] + u < q1[i] ? g.pt_idx[q[i] + u] : -1;
+      for (int u = 0; u < U; ++u) at[i][u] = u < q1[i] - q[i] ? g.pt_idx[q[i] + u] : -1;
 #pragma unroll
     for (int i = 0; i < P; ++i)
 #pragma unroll
@@ -2141,18 +2143,18 @@ __global__ void __launch_bounds__(256)
     for (int i = 0; i < P; ++i) {
 #pragma unroll
       for (int u = 0; u < U; ++u) v[i] += x[i][u];
-      q[i] += U;
+      q[i] = min(q[i], q1[i] - U) + U;  // at most q1
       more |= q[i] < q1[i];
     }
   }
 #pragma unroll
   for (int i = 0; i < P; ++i) {
-    const int p = (blockIdx.x * P + i) * 256 + threadIdx.x;
+    const unsigned p = step_point(blockIdx.x, P, i, 256, threadIdx.x);
     if (p >= np) continue;
-    const int a = p / g.ngrid;
+    const unsigned a = p / G;
     if (sweep_skip(g.act, a)) continue;
     if (chi) v[i] *= (Rl)fmax(g.fi[p], 1.0);
-    pot[(size_t)a * ldp + (p - a * g.ngrid)] = v[i];
+    pot[(size_t)a * ldp + (p - a * G)] = v[i];
   }
 }
 

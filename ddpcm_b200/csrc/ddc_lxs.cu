@@ -433,7 +433,9 @@ __global__ void __launch_bounds__(128) k_lxs_geo(const LxsTab tb, const DevGeo g
   const int b = blockIdx.x;
   const double4 cb = g.sph[b];
   const double irb = 1.0 / cb.w;
-  for (int q = g.ls_ptr[b] + threadIdx.x; q < g.ls_ptr[b + 1]; q += blockDim.x) {
+  const int q0 = g.ls_ptr[b], n1 = g.ls_ptr[b + 1] - q0;
+  for (int k = threadIdx.x; k < n1; k += blockDim.x) {
+    const int q = q0 + k;
     const int pa = g.ls[q], a = pa / g.ngrid, n = pa - a * g.ngrid;
     set4(tg[q], lxs_geom(tb, g.sph[a], g.grid[n], g.fi[pa], cb, irb));
   }
@@ -485,8 +487,9 @@ __device__ __forceinline__ void lxs_block(const LxsTab& tb, const DevGeo& g,
   const int left = q1 - q0 - (nch - 1) * CH;
   const int hlast = NP == 1 ? left : min(NT, ((left + 1) / 2 + 31) & ~31);
   auto slots = [&](int k) { return k == nch - 1 ? hlast : NT; };
-  auto triple = [&](int k, int p) { return min(q0 + k * CH + tid + p * slots(k), q1 - 1); };
-  auto mine = [&](int k, int p) { return tid < slots(k) && q0 + k * CH + tid + p * slots(k) < q1; };
+  auto entry = [&](int k, int p) { return k * CH + tid + p * slots(k); };
+  auto triple = [&](int k, int p) { return list_entry(q0, q1, entry(k, p)); };
+  auto mine = [&](int k, int p) { return tid < slots(k) && entry(k, p) < q1 - q0; };
   auto geo_copy = [&](int k) {  // chunk k's geometry into this thread's slots of gs
     if (PRE && k < nch) {
 #pragma unroll
@@ -564,7 +567,7 @@ __device__ __forceinline__ void lxs_block(const LxsTab& tb, const DevGeo& g,
     S::unpack(sv, o);
 #pragma unroll
     for (int p = 0; p < NP; ++p)
-      if (k < nch - 1 || mine(k, p)) val[q0 + k * CH + tid + p * slots(k)] = o[p];
+      if (k < nch - 1 || mine(k, p)) val[q0 + entry(k, p)] = o[p];
   };
   geo_copy(0);
   int pa[NP] = {};
