@@ -720,18 +720,25 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
     CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
   }
   if (ctx->prm.precision == DDC_PREC_MIXED) {
-    // the two contractions run on the tensor cores (split TF32) up to 128
-    // harmonics (lmax 10), else as FP32 SIMT GEMMs on an FP32 copy of bw
-    // DDC_TC_OFF=1 in the environment selects the SIMT contractions (a
-    // diagnostic switch: the tests compare the two paths' accuracy)
+    // The two contractions of the FP32 operators: folded (FP64 arithmetic,
+    // ddc_fold.cu) up to kFoldProducts products; above that on tcgen05 (split
+    // TF32, ddc_tc.cu) up to 128 harmonics (lmax 10) and as FP32 SIMT GEMMs on an
+    // FP32 copy of bw beyond.  The folded kernels' blocks are short, the tcgen05
+    // ones' wide; projection + expansion us, folded against tcgen05, with 4 us of
+    // events: lmax 6, 302 points, 8,000 spheres (1.2e8 products) 15 + 20 against
+    // 21 + 20, 13,000 (1.9e8) 19 + 27 against 23 + 23, 18,000 (2.7e8) 24 + 35
+    // against 24 + 25; lmax 8, 302 points, 18,000 (4.4e8) 27 + 36 against 25 + 31.
+    // (lmax 10, 590 points is for the folded ones longer, 5,000 spheres, 3.6e8,
+    // 24 + 25 against 29 + 35; 20,000, 1.4e9, 49 + 63 against 37 + 49.)  With few
+    // harmonics only molecules of a size that no program solves pass the line
+    // (lmax 0, 110 points: 1.8 million spheres).
+    // Diagnostic switches of the environment, with which the tests compare the
+    // paths: DDC_TC_OFF=1 takes the SIMT contractions at any size, DDC_FOLD=0
+    // never folds, DDC_FOLD=1 always.
     const char* tc_off = std::getenv("DDC_TC_OFF");
+    const char* fold = std::getenv("DDC_FOLD");
     const bool tc_env = !(tc_off && tc_off[0] == '1');
-    // up to 2e8 products (harmonics x points) the folded FP64 kernels instead,
-    // whose blocks are short (projection / expansion us, folded against
-    // tcgen05): 5,000 spheres, lmax 6, 302 points (7.4e7) 13 / 19 against 21 /
-    // 20, 8,000 (1.2e8) 15 / 20 against 21 / 20; 48 molecules, 18,000 spheres,
-    // lmax 8 (4.5e8) 22 / 32 against 24 / 24
-    ctx->fold_f32 = tc_env && (long long)NY * NP <= kFoldProducts;
+    ctx->fold_f32 = tc_env && (fold && fold[0] ? fold[0] == '1' : (long long)NY * NP <= kFoldProducts);
     const bool tc = tc_supported(NY) && tc_env && !ctx->fold_f32;
     ctx->ldp_f = tc ? (G + 3) / 4 * 4 : G;
     CK(ctx->pot_f.ensure(sizeof(float) * std::max<long long>((long long)N * ctx->ldp_f, 1LL)));
