@@ -431,27 +431,20 @@ void build_tables(ddc_ctx* c) {
   build_tables_for(c->tbP, kFarDegree, c->prm.eta, c->ngrid);
 }
 
-// deterministic reduction of `nvals` partial columns into red[0..nvals-1], copied to host.
-// stride: the partial row length of the producing kernel (kMaxHist + 1 for the
-// Jacobi step's Gram row, whatever its current length; 1 for single sums).
-// nblk: the producing kernel's block count (partial rows).
-int reduce_to_pinned(ddc_ctx* ctx, int nvals, int stride = 1, int nblk = 0) {
-  if (nvals > kMaxHist + 1 || !ctx->hred)
-    return fail(ctx, DDC_ERR_STATE, "reduction read beyond the pinned buffer");
+// the sum of the blocks' partial sums, in a fixed order, to hred[0]
+int reduce_to_pinned(ddc_ctx* ctx) {
   {
     StageScope sc(ctx, ST_REDUCE);
-    CK(launch_reduce_partials(ctx->L(), ctx->partials.as<double>(),
-                              nblk > 0 ? nblk : reduce_blocks(), nvals, stride,
+    CK(launch_reduce_partials(ctx->L(), ctx->partials.as<double>(), reduce_blocks(),
                               ctx->red.as<double>()));
   }
-  CK(cudaMemcpyAsync(ctx->hred, ctx->red.p, sizeof(double) * nvals, cudaMemcpyDeviceToHost,
-                     ctx->st));
+  CK(cudaMemcpyAsync(ctx->hred, ctx->red.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
   return DDC_OK;
 }
-int reduce_to_host(ddc_ctx* ctx, int nvals, double* host, int stride = 1, int nblk = 0) {
-  CKI(reduce_to_pinned(ctx, nvals, stride, nblk));
+int reduce_to_host(ddc_ctx* ctx, double* host) {
+  CKI(reduce_to_pinned(ctx));
   CKI(sync(ctx));
-  memcpy(host, ctx->hred, sizeof(double) * nvals);
+  *host = ctx->hred[0];
   return DDC_OK;
 }
 
@@ -712,7 +705,7 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
     CK(b->ensure(sizeof(double) * std::max(nv, (size_t)1)));
   CK(ctx->hist_x.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
   CK(ctx->hist_e.ensure(sizeof(double) * std::max(nv, (size_t)1) * nd));
-  CK(ctx->partials.ensure(sizeof(double) * reduce_blocks() * (kMaxHist + 1)));
+  CK(ctx->partials.ensure(sizeof(double) * reduce_blocks()));
   CK(ctx->red.ensure(sizeof(double) * 2 * (kMaxHist + 1)));
   if (ctx->prm.igrad && !ctx->st2) {
     CK(cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking));
@@ -1318,7 +1311,7 @@ int need_ready(ddc_ctx* ctx) {
 // dot product on device, deterministic
 int dot_dev(ddc_ctx* ctx, long long n, const double* a, const double* b, double* out) {
   CK(launch_dot_partial(ctx->L(), n, a, b, ctx->partials.as<double>(), reduce_blocks()));
-  return reduce_to_host(ctx, 1, out);
+  return reduce_to_host(ctx, out);
 }
 
 // Solute potential (and, with ef, field) at the context's cavity points from
@@ -1945,7 +1938,7 @@ int ddc_hnorm(ddc_ctx* ctx, const double* x, double* norm) {
   CK(launch_hnorm_partial(ctx->L(), ctx->tb, (long long)nv, dx, ctx->partials.as<double>(),
                           reduce_blocks()));
   double ss = 0.0;
-  CKI(reduce_to_host(ctx, 1, &ss));
+  CKI(reduce_to_host(ctx, &ss));
   *norm = std::sqrt(ss / (double)std::max(ctx->nsph, 1));
   return DDC_OK;
 }
@@ -2045,7 +2038,7 @@ int ddc_energy_forces(ddc_ctx* ctx, int n, const double* charge, const double* x
     CKI(run.mark());
     CK(launch_dot_partial(ctx->L(), (long long)nv, dsig, dpsi, ctx->partials.as<double>(),
                           reduce_blocks()));
-    CKI(reduce_to_pinned(ctx, 1));
+    CKI(reduce_to_pinned(ctx));
     run.esolv = esolv;
     run.fac = 0.5 * ((ctx->prm.eps - 1.0) / ctx->prm.eps);
   } else {

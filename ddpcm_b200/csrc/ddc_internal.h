@@ -89,7 +89,7 @@ struct YlmTables {
   double K[DDC_NLM_CAP];          // facs / facl
   double A[DDC_NLM_CAP];          // (2l-1)/(l-m): Legendre recurrence
   double B[DDC_NLM_CAP];          // (l+m-1)/(l-m)
-  // normalised recurrence of the fused L / L* kernel: Pt_l^m = gam_lm Q_l^m with
+  // normalised recurrence of the far-field and force kernels: Pt_l^m = gam_lm Q_l^m with
   // Q_m = Pt_m^m, Q_{m+1} = c t Q_m, Q_l = c t Q_{l-1} - beta_lm t^2 Q_{l-2};
   // Kg = K * gam folds the scale into the contractions
   double Bn[DDC_NLM_CAP], Kg[DDC_NLM_CAP];
@@ -439,10 +439,8 @@ cudaError_t launch_hnorm_partial(Launch L, const YlmTables& tb, long long n, con
                                  double* partials, int nblk);
 cudaError_t launch_dot_partial(Launch L, long long n, const double* a, const double* b,
                                double* partials, int nblk);
-// out[k] = sum_b partials[b*stride + k], k < nvals, fixed order; stride is
-// the row length the producing kernel stores (block_sum_store's NV)
-cudaError_t launch_reduce_partials(Launch L, const double* partials, int nblk, int nvals,
-                                   int stride, double* out);
+// out[0] = sum_b partials[b], fixed order
+cudaError_t launch_reduce_partials(Launch L, const double* partials, int nblk, double* out);
 int reduce_blocks();
 
 // electrostatics

@@ -672,19 +672,19 @@ __host__ __device__ constexpr int ls_nvals_m(int L, int m) { return m == 0 ? L +
 // shared-memory fields per triple: ct, t2, then pmm[m], cos[m], sin[m]
 __host__ __device__ constexpr int ls_nfields(int L) { return 2 + 3 * (L + 1); }
 
-// GAM: accumulators of the normalised recurrence (scale Kg instead of K)
-template <int LMAX, int M, int OFF, class Rl, bool GAM = false>
-__device__ __forceinline__ void ls_store(const YlmTables& tb, const Rl* acc, double* yi,
+// column M of the normalised recurrence's accumulators, with its scale
+template <int LMAX, int M, int OFF>
+__device__ __forceinline__ void ls_store(const YlmTables& tb, const double* acc, double* yi,
                                          int lane) {
 #pragma unroll
   for (int l = M; l <= LMAX; ++l) {
     const int ind = l * l + l;
-    const double k = GAM ? tb.Kg[lmi(l, M)] : tb.K[lmi(l, M)];
+    const double k = tb.Kg[lmi(l, M)];
     if (M == 0) {
-      if (lane == 0) yi[ind] = -k * (double)acc[OFF + (l - M)];
+      if (lane == 0) yi[ind] = -k * acc[OFF + (l - M)];
     } else if (lane == 0) {
-      yi[ind + M] = -k * (double)acc[OFF + (l - M)];
-      yi[ind - M] = -k * (double)acc[OFF + (LMAX + 1 - M) + (l - M)];
+      yi[ind + M] = -k * acc[OFF + (l - M)];
+      yi[ind - M] = -k * acc[OFF + (LMAX + 1 - M) + (l - M)];
     }
   }
 }
@@ -885,26 +885,18 @@ cudaError_t launch_guess(Launch L, const YlmTables& tb, long long n, const doubl
 
 int reduce_blocks() { return 148 * 4; }
 
-// block sums of v[0..nv) into partials[blockIdx.x * STRIDE + k] (blocks of
-// at most 256 threads)
-template <int NV, int STRIDE = NV>
-__device__ __forceinline__ void block_sum_store(double (&v)[NV], int nv, double* partials) {
-  __shared__ double sh[NV][8];
+// block sum of x into partials[blockIdx.x] (blocks of at most 256 threads)
+__device__ __forceinline__ void block_sum_store(double x, double* partials) {
+  __shared__ double sh[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    if (k < nv) {
-      double x = v[k];
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) sh[k][w] = x;
-    }
-  }
+  for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  if (lane == 0) sh[w] = x;
   __syncthreads();
-  if (threadIdx.x < nv) {
+  if (threadIdx.x == 0) {
     double s = 0.0;
-    for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) s += sh[threadIdx.x][ww];
-    partials[(size_t)blockIdx.x * STRIDE + threadIdx.x] = s;
+    for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) s += sh[ww];
+    partials[blockIdx.x] = s;
   }
 }
 
@@ -917,8 +909,7 @@ __global__ void __launch_bounds__(256) k_hnorm_partial(const YlmTables tb, long 
     int l = l_of((int)(q % tb.nylm));
     acc = fma(x[q] * x[q], 1.0 / (1.0 + l), acc);
   }
-  double v[1] = {acc};
-  block_sum_store<1>(v, 1, partials);
+  block_sum_store(acc, partials);
 }
 cudaError_t launch_hnorm_partial(Launch L, const YlmTables& tb, long long n, const double* x,
                                  double* partials, int nblk) {
@@ -934,8 +925,7 @@ __global__ void __launch_bounds__(256) k_dot_partial(long long n, const double* 
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n;
        q += (long long)gridDim.x * blockDim.x)
     acc = fma(a[q], b[q], acc);
-  double v[1] = {acc};
-  block_sum_store<1>(v, 1, partials);
+  block_sum_store(acc, partials);
 }
 cudaError_t launch_dot_partial(Launch L, long long n, const double* a, const double* b,
                                double* partials, int nblk) {
@@ -944,25 +934,21 @@ cudaError_t launch_dot_partial(Launch L, long long n, const double* a, const dou
   return cudaGetLastError();
 }
 
-// out[k] = sum over blocks of partials[b][k] in a fixed tree order
-__global__ void k_reduce_partials(const double* __restrict__ partials, int nblk, int stride,
-                                  double* out) {
+// out[0] = sum over blocks of partials[b] in a fixed tree order
+__global__ void k_reduce_partials(const double* __restrict__ partials, int nblk, double* out) {
   __shared__ double sh[256];
-  const int k = blockIdx.x;
   double s = 0.0;
-  for (int b = threadIdx.x; b < nblk; b += 256) s += partials[(size_t)b * stride + k];
+  for (int b = threadIdx.x; b < nblk; b += 256) s += partials[b];
   sh[threadIdx.x] = s;
   __syncthreads();
   for (int h = 128; h >= 1; h >>= 1) {
     if (threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[k] = sh[0];
+  if (threadIdx.x == 0) out[0] = sh[0];
 }
-cudaError_t launch_reduce_partials(Launch L, const double* partials, int nblk, int nvals,
-                                   int stride, double* out) {
-  if (nvals > stride) return cudaErrorInvalidValue;
-  k_reduce_partials<<<nvals, 256, 0, L.st>>>(partials, nblk, stride, out);
+cudaError_t launch_reduce_partials(Launch L, const double* partials, int nblk, double* out) {
+  k_reduce_partials<<<1, 256, 0, L.st>>>(partials, nblk, out);
   ++*L.launches;
   return cudaGetLastError();
 }
@@ -1537,7 +1523,7 @@ __device__ void dbasis_contract(const YlmTables& tb, double sx, double sy, doubl
   }
 }
 
-// The same alp and beta from the recurrence of the fused L / L* pass.  With
+// The same alp and beta from the normalised recurrence (YlmTables::Bn).  With
 // u = v / r_i (|u| = t, u / |u| = s) and the real solid harmonics
 // R_lm(u) = t^l Y_lm(s), the contraction above is
 //   beta  = sum_lm w_lm R_lm(u),   alp_k = sum_lm w_lm d_k R_lm(u),
@@ -1964,6 +1950,8 @@ cudaError_t launch_csph_pack(Launch L, int n, const double4* sph, double* csph, 
   return cudaGetLastError();
 }
 
+// Roles of the local expansions (k_far_acc): the columns m shared out over the
+// warps of a block, greedily by cost or in pairs m / L - m
 __host__ __device__ constexpr int lxs_cost(int L, int m) {
   return m == 0 ? 5 * (L + 1) + 4 : 7 * (L + 1 - m) + 4;
 }
@@ -2004,18 +1992,17 @@ __host__ __device__ constexpr int lxs_max_nvals(int L, int NR, bool g) {
     mx = lxs_role_nvals(L, NR, r, g) > mx ? lxs_role_nvals(L, NR, r, g) : mx;
   return mx;
 }
-// the L* rows of role R: lane sums by a fixed shuffle tree, then its columns
-// G: the greedy column map (else the pairing); the fused pass's choice by
-// default
-template <int LMAX, int NR, int R, int M, class Rl, bool GAM, bool G = sizeof(Rl) == 4>
-__device__ __forceinline__ void lxs_store_cols(const YlmTables& tb, const Rl* acc, double* yi,
+// the rows of role R: lane sums by a fixed shuffle tree, then its columns
+// G: the greedy column map (else the pairing)
+template <int LMAX, int NR, int R, int M, bool G>
+__device__ __forceinline__ void lxs_store_cols(const YlmTables& tb, const double* acc, double* yi,
                                                int lane) {
   if constexpr (lxs_role_of(LMAX, NR, M, G) == R)
-    ls_store<LMAX, M, lxs_off_of(LMAX, NR, M, G), Rl, GAM>(tb, acc, yi, lane);
-  if constexpr (M < LMAX) lxs_store_cols<LMAX, NR, R, M + 1, Rl, GAM, G>(tb, acc, yi, lane);
+    ls_store<LMAX, M, lxs_off_of(LMAX, NR, M, G)>(tb, acc, yi, lane);
+  if constexpr (M < LMAX) lxs_store_cols<LMAX, NR, R, M + 1, G>(tb, acc, yi, lane);
 }
-template <int LMAX, int NR, int R, class Rl, bool GAM, bool G = sizeof(Rl) == 4>
-__device__ __forceinline__ void lxs_finish_role(int role, const YlmTables& tb, Rl* acc,
+template <int LMAX, int NR, int R, bool G>
+__device__ __forceinline__ void lxs_finish_role(int role, const YlmTables& tb, double* acc,
                                                 double* yi, int lane) {
   if (role == R) {
     constexpr int NV = lxs_role_nvals(LMAX, NR, R, G);
@@ -2024,11 +2011,11 @@ __device__ __forceinline__ void lxs_finish_role(int role, const YlmTables& tb, R
 #pragma unroll
       for (int o = 16; o >= 1; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
     }
-    lxs_store_cols<LMAX, NR, R, 0, Rl, GAM, G>(tb, acc, yi, lane);
+    lxs_store_cols<LMAX, NR, R, 0, G>(tb, acc, yi, lane);
     return;
   }
   if constexpr (R + 1 < NR)
-    lxs_finish_role<LMAX, NR, R + 1, Rl, GAM, G>(role, tb, acc, yi, lane);
+    lxs_finish_role<LMAX, NR, R + 1, G>(role, tb, acc, yi, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -2287,10 +2274,9 @@ namespace ddc {
 // are summed directly.  Truncation: at most t^(P+1) / (1 - t) of each far
 // term, 1e-10 for P = 10, rho = 8.
 // ---------------------------------------------------------------------------
-// The L* half of the normalised recurrence of the fused pass, FP64:
-// Q_l = ct Q_{l-1} - Bn t^2 Q_{l-2} (three operations per value; the scale
-// gam_lm sits in Kg, applied when the rows are stored), accumulated into the
-// column's register rows (layout of ls_column)
+// The adjrhs sum by the normalised recurrence, FP64: Q_l = ct Q_{l-1}
+// - Bn t^2 Q_{l-2} (three operations per value; the scale gam_lm sits in Kg,
+// applied when the rows are stored), accumulated into the column's register rows
 template <int LMAX, int M, int OFF>
 __device__ __forceinline__ void fa_column(const YlmTables& tb, double ct, double t2, double q0,
                                           double cm, double sm, double* acc) {
@@ -2318,8 +2304,8 @@ __device__ __forceinline__ void fa_column(const YlmTables& tb, double ct, double
   }
 }
 // Roles of k_far_acc: at lmax 10 four roles of about three columns each
-// (the greedy map of the FP32 fused pass: each role's per-source fixed cost
-// paid four times instead of six), else the pairing m / lmax-m
+// (the greedy map: each role's per-source fixed cost paid four times instead
+// of six), else the pairing m / lmax-m
 __host__ __device__ constexpr bool fa_greedy(int L) { return L == 10; }
 __host__ __device__ constexpr int fa_nroles(int L) { return fa_greedy(L) ? 4 : L / 2 + 1; }
 template <int LMAX, int R, int M>
@@ -2428,8 +2414,7 @@ __global__ void __launch_bounds__(32 * fa_nroles(LMAX), fa_greedy(LMAX) ? 4 : 1)
     fa_run_role<LMAX, 0>(role, tb, sh, CH, chunk, lane, acc);
     __syncthreads();
   }
-  lxs_finish_role<LMAX, NR, 0, double, true, fa_greedy(LMAX)>(role, tb, acc,
-                                                              A + (size_t)i * tb.nylm, lane);
+  lxs_finish_role<LMAX, NR, 0, fa_greedy(LMAX)>(role, tb, acc, A + (size_t)i * tb.nylm, lane);
 }
 
 // Tables on the grid, once per context: BT[lm][n] = Y_lm(s_n) and
