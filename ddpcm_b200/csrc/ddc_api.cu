@@ -667,12 +667,23 @@ int do_init(ddc_ctx* ctx, int n, const std::vector<double4>& hsph) {
                      ctx->cnt.as<int>()));
   CK(scan_counts(L, ctx->cnt.as<int>(), ctx->ls_ptr.as<int>(), N, ctx->scan_tmp.p,
                  ctx->scan_tmp.bytes, stats));
-  // the triple passes take the longest lists first: the blocks of a last wave
-  // are then the shortest (lx and lstarx of 4,999 spheres, lmax 9, FP64: 0.38
-  // -> 0.33 ms; energy and forces of 2,000, lmax 6, FP64: 10.2 -> 9.4 ms).  Not
-  // up to two waves of four blocks per SM, where the pass alone gains 8 % but
-  // the next kernel, scheduled while it ends, loses more (643 spheres routine by
-  // routine 7.1 -> 7.7 ms), nor where one block would sort for long.
+  // The triple passes take the longest lists first: the blocks of a last wave
+  // are then the shortest.  The pass gains at every size (lx alone 4 to 15 %, lmax
+  // 8 and 10), whole solves only with enough spheres; why few lose was not
+  // traced.  ms to 1e-9 by rising index / longest first:
+  //   energy and forces (both systems), 302 points:
+  //     lmax 6, FP64     2,000 spheres 8.87 / 8.03, 5,000 16.8 / 15.8
+  //     lmax 6, mixed    900 4.42 / 4.65, 1,184 5.06 / 5.33, 1,300 4.41 / 4.33, 2,000 7.16 / 6.66
+  //     lmax 8, FP64     320 3.89 / 4.22, 643 4.93 / 5.05, 900 5.55 / 5.25, 2,000 11.0 / 10.2
+  //     lmax 10, mixed   320 4.04 / 4.20, 643 5.03 / 4.92, 2,000 10.4 / 9.9
+  //   one system (cosmo):
+  //     lmax 6, FP64, 110 points  643 2.17 / 2.69, 1,300 2.60 / 2.83, 1,600 3.53 / 3.77, 2,000 4.06 / 3.94
+  //     lmax 8, FP64     643 3.43 / 3.64, 900 3.56 / 3.70, 1,184 4.74 / 4.55, 2,000 7.55 / 6.78
+  //     lmax 10, mixed   643 3.26 / 3.41, 900 3.58 / 3.45
+  // So the line lies between 600 and 1,800 spheres, by degree, precision and
+  // number of systems, and not at a number of waves (lmax 6 in FP32 has eight
+  // blocks per SM, lmax 8 four); one line stands for all.  Nor where one block
+  // would sort for long.
   ctx->order_on = N > 2 * 4 * 148 && N <= 65536;
   if (ctx->order_on) {
     CK(ctx->ls_order.ensure(sizeof(int) * N));

@@ -22,9 +22,8 @@
 // shared memory between the two, its rows 9 doubles apart so that neither
 // side's accesses collide.
 //
-// Both kernels replace plain FP64 GEMMs (128 x 64 tiles staged in shared memory,
-// or slices of k straight from L2) that stood at 40 % of the FP64 peak at best;
-// projection / expansion us, then and now, with 4 us of events:
+// Projection / expansion us (with 4 us of events), unfolded on the same tensor
+// cores (40 % of the FP64 peak at best) and folded:
 //   12 spheres, lmax 6, 110 points      6.9 /  7.9    8.0 /  8.6
 //   600, lmax 8, 302 (FP32 fields)     10.7 / 11.0    8.6 / 10.7
 //   2,000, lmax 8, 302                   17 / 17.6   10.7 / 11.6

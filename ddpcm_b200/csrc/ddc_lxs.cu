@@ -676,11 +676,17 @@ cudaError_t lxs_launch64(Launch L, const YlmTables& tb, const DevGeo& g, const d
 }
 
 // Few spheres: the two operators by blocks of their own, which takes both
-// halves' latency side by side; beyond two blocks per SM the shared geometry and
-// powers are worth more.  us per pass, together and by halves: 12 spheres, lmax
-// 6, FP64 10.1 / 8.9; 113, lmax 8, FP64 25.2 / 22.9; 200, lmax 8, FP32 15.9 /
-// 15.0; 280, lmax 10, FP32 22.1 / 21.2 (with 4 us of events); energy and forces
-// of 12 spheres 1.06 / 0.99 ms, of 113 mixed 2.22 / 2.07 ms.
+// halves' latency side by side; with more the shared geometry and powers are worth
+// more.  us of a call of lx and lstarx on device vectors (some 25 of them the call and
+// the other kernels), by one pass / by halves:
+//   lmax 10, 302 points, FP64   12 spheres 41.8 / 38.0, 60 54.5 / 47.3, 200 63.8 / 62.8,
+//                               296 68.2 / 69.2, 450 77.3 / 77.3, 900 100 / 108
+//   lmax 10, mixed              60 44.8 / 42.1, 200 49.6 / 50.3, 450 59.1 / 58.2, 900 71.7 / 77.5
+//   lmax 8, 302 points, FP64    60 49.4 / 45.2, 200 53.7 / 51.5, 296 55.5 / 61.4, 900 79.7 / 86.4
+//   lmax 6, 302 points, mixed   60 43.0 / 40.3, 296 46.5 / 46.6, 900 54.2 / 59.9
+//   lmax 6, 110 points, FP64    113 39.5 / 35.7, 296 38.7 / 38.4, 450 38.7 / 43.5
+// and ms of energy and forces, lmax 10, FP64: 60 spheres 2.09 / 1.93, 296 3.73 / 3.62,
+// 600 4.86 / 4.97, 900 7.12 / 7.46.
 bool split_pass(const DevGeo& g) { return g.nsph <= 2 * 148; }
 
 }  // namespace

@@ -5,12 +5,10 @@
 // Every molecule of every system runs the reference's algorithm on its own
 // segment of the vectors: own history, Gram matrix, restarts and convergence
 // test, all in device memory, so that the host only launches sweeps and looks
-// now and then whether anything still runs.  With the bordered system solved
-// on the host an iteration waited for two round trips; energy and forces of
-// 12 / 113 / 600 spheres took 3.9 / 7.0 / 11.4 ms so and take 2.4 / 4.2 /
-// 7.0 ms now, a batch of 64 small molecules 17.9 and 10.7 ms.  The vectors are cut into chunks of CK consecutive
-// elements; a chunk is a block.  Two kernels per iteration, each over the
-// chunks of all running systems (grid y):
+// now and then whether anything still runs (with the bordered system solved on
+// the host an iteration would wait for two round trips).  The vectors are cut
+// into chunks of CK consecutive elements; a chunk is a block.  Two kernels per
+// iteration, each over the chunks of all running systems (grid y):
 //   k_gram    Jacobi iterate, increment, the chunk's part of the Gram row; the
 //             molecule's last chunk to arrive sums the parts in chunk order
 //             and solves the bordered system (the whole block, one barrier
@@ -134,10 +132,12 @@ __device__ __forceinline__ void sum_parts(const SolverArgs& a, const SolverSys& 
 // n x n system, n <= 32, by the whole block: thread (w, lane) holds column
 // `lane` of the rows w, w + 8, w + 16, w + 24 in a[], the rows' right-hand
 // sides in b[] (every lane).  The pivot is the largest |a| over free rows and
-// columns, compared by its high word (to 20 bits of the mantissa), the first
-// in the reference's scan order (rows outer, columns inner) among equals;
-// rows stay in place (myrow: the row that column `lane` was pivoted in)
-// instead of being swapped, which changes no value.  A chain of n dependent
+// columns, compared by its high word alone (20 bits of the mantissa), the first
+// in the reference's scan order (rows outer, columns inner) among equals: a
+// pivot within 2^-20 of the largest, so not always the reference's, nor its
+// rounding bit for bit; singular, as there, only without a pivot (here: one of
+// 2^-1042 or more).  Rows stay in place (myrow: the row that column `lane` was
+// pivoted in) instead of being swapped, which changes no value.  A chain of n dependent
 // pivots, each some hundred cycles of latency: one barrier per pivot, the
 // rows mirrored in shared memory as they are updated, so that every warp
 // reads the pivot row of whichever warp offers it; 650 cycles per pivot
@@ -312,10 +312,13 @@ __global__ void __launch_bounds__(kT, 4) k_gram(const __grid_constant__ SolverAr
   // history span many decades and their products twice as many, and unscaled
   // the elimination loses the small ones to the rounding of the large; the
   // coefficients of the last iterations are then noise that slows the solve
-  // and now and then stops it early (12-sphere molecules to 1e-12: 24.1
-  // iterations on average, 3 of 40 solutions off by 1e-10 to 2e-9; scaled 20.6
-  // and none above 7e-12, the same as with the system solved exactly).  The
-  // border row's scale is the smallest, so that the border stays below 1.
+  // and now and then stops it early.  200 chains of 12 spheres, lmax 6, to 1e-12,
+  // both solutions against direct ones: unscaled (the reference's elimination) 24.5 and
+  // 24.8 iterations on average, errors of 5e-13 and 1e-13 in the median, 89 of
+  // 400 above 1e-10 and up to 1.2e-8; scaled 21.2 and 21.0 iterations, 9e-12 and
+  // 2e-12, none above 4e-11.  (The median is larger because a solve stops where the
+  // test says; with noise for coefficients it ran on and ended far below it.)
+  // The border row's scale is the smallest, so that the border stays below 1.
   const int n1 = nm + 1, pn = pm[nm - 1];
   __shared__ int ex[kMaxHist + 1];  // row r is scaled by 2^-ex[r]
   if (w == 0) {

@@ -63,10 +63,12 @@ def test_both_operators_by_halves_and_together(oracle, n, lmax):
 
 
 @pytest.mark.parametrize("n,lmax,ngrid", [
-    (9, 8, 110),      # eight slices of k, the last block of spheres nearly empty
-    (1603, 8, 110),   # projection: 16 spheres per block; expansion: two slices
+    # all folded (ddc_fold.cu: eight spheres per block); the other paths of the
+    # mixed operators are held in test_gpu_tcgen05.py
+    (9, 8, 110),      # one sphere in the last block
+    (1603, 8, 110),   # three, of many blocks
     (1190, 10, 110),  # fewer points than harmonics
-    (14305, 2, 26)])  # staged 128 x 64 tiles
+    (14305, 2, 26)])  # few harmonics, a class of them without any
 def test_contractions_by_shape(oracle, n, lmax, ngrid):
     """The projection and expansion GEMMs of every dispatch branch (remainders
     in all three dimensions), through lx and lstarx."""

@@ -18,6 +18,9 @@ The cases cover every harmonic count the tensor-core kernels take (lmax 0, 6,
 grid tiles), tile widths from 16 to 64 spheres and the FP32 SIMT fallback
 above 128 harmonics (lmax 11, 12).
 """
+# These sizes lie below the line from which the mixed operators leave the folded
+# contractions (2e8 products): without a switch the folded ones run here.  The
+# tcgen05 kernels at these sizes are held in test_gpu_tcgen05.py.
 import os
 
 import numpy as np
